@@ -709,6 +709,57 @@ int nsvf_prune_exact_dev(int64_t n_voxels, int bits, int rule, double threshold,
                          const int64_t *n_list, int64_t list_cap, uint8_t *keep, int32_t *err,
                          void *stream);
 
+/* Training on compacted samples (fairnr/modules/encoder.py:558-592 and
+ * fairnr/modules/renderer.py:94-126 under autograd, with per-chunk
+ * recomputation). A batch's rows [rays, max_steps] are compacted once, the
+ * valid samples (sampled_idx != -1) of row r in slot order at
+ * [offset[r], offset[r + 1]), offset the prefix sum of the counts:
+ *  - train_rows_count, train_rows_pack: voxel int32, xyz_dist float4 (x, y, z,
+ *    distance) and depth per sample;
+ *  - field_train_pack: the 4 x 128 field's FP32 weights (row-major [out, in],
+ *    32-128-128-128-128-4) and biases into field_train_packed_floats() floats,
+ *    16-byte aligned;
+ *  - field_train_forward: out[s] = (sigma, r, g, b), interpolation and field in
+ *    FP32 with the operations of nsvf_trilinear_embed and of an FP32 GEMM that
+ *    adds over k in order (fused multiply-add from zero, then the bias). Ids
+ *    out of range as nsvf_trilinear_embed (embedding 0, err bit 2);
+ *  - composite_rows (+ _backward): compositing with the free energy relu(sigma)
+ *    * dist * sigma_scale; the backward gives d loss / d out [samples, 4] (any
+ *    of the three gradients may be NULL);
+ *  - field_train_backward: the field's gradients (overwritten, a fixed sum
+ *    order) and grad_values (added to, float4 atomics), the activations
+ *    recomputed for chunk_samples (a multiple of 128) samples at a time in a
+ *    workspace of field_train_backward_floats() floats. */
+int nsvf_train_rows_count(int64_t rays, int max_steps, const int32_t *sampled_idx, int32_t *count,
+                          void *stream);
+int nsvf_train_rows_pack(int64_t rays, int max_steps, const int32_t *sampled_idx, const float *xyz,
+                         const float *dists, const float *depths, const int64_t *offset,
+                         int32_t *voxel, float *xyz_dist, float *depth, void *stream);
+int64_t nsvf_field_train_packed_floats(void);
+int nsvf_field_train_pack(const float *const weights[5], const float *const biases[5],
+                          float *packed, void *stream);
+int nsvf_field_train_forward(int64_t n_samples, const int32_t *voxel, const float *xyz_dist,
+                             int64_t n_voxels, int64_t n_keys, float voxel_size,
+                             const float *centers, const int32_t *feats, const float *values,
+                             const float *packed, float *out, int32_t *err, void *stream);
+int nsvf_composite_rows(int64_t rays, const int64_t *offset, const float *field,
+                        const float *xyz_dist, const float *depth, float sigma_scale,
+                        float *out_color, float *out_depth, float *out_missed, int kahan,
+                        void *stream);
+int nsvf_composite_rows_backward(int64_t rays, const int64_t *offset, const float *field,
+                                 const float *xyz_dist, const float *depth, float sigma_scale,
+                                 const float *grad_color, const float *grad_depth,
+                                 const float *grad_missed, float *grad_field, int kahan,
+                                 void *stream);
+int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_samples);
+int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
+                              const float *xyz_dist, int64_t n_voxels, int64_t n_keys,
+                              float voxel_size, const float *centers, const int32_t *feats,
+                              const float *values, const float *packed, const float *grad_out,
+                              float *workspace, int64_t workspace_floats, float *grad_values,
+                              float *const grad_weights[5], float *const grad_biases[5],
+                              void *stream);
+
 #ifdef __cplusplus
 }
 #endif

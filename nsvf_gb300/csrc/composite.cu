@@ -34,6 +34,9 @@ __device__ __forceinline__ float warp_incl_scan(float x, int lane) {
   return x;
 }
 
+// torch.relu: NaN stays NaN
+__device__ __forceinline__ float relu_nan(float x) { return x <= 0.0f ? 0.0f : x; }
+
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -217,6 +220,92 @@ __global__ void __launch_bounds__(kWarps * 32) composite_segments_kernel(
   }
 }
 
+// Training: compositing of compacted samples and its backward. Ray r owns
+// samples [offset[r], offset[r + 1]); field, xyzd and depth as in
+// composite_segments_kernel, the free energy in the same operations. Against
+// the padded kernels above on [rays, steps] arrays this reads and writes
+// valid samples only and carries the free energy's own forward and backward:
+// d sigma = d fe * dist * sigma_scale where sigma > 0.
+__global__ void __launch_bounds__(kWarps * 32) composite_rows_kernel(
+    int64_t rays, const int64_t *__restrict__ offset, const float4 *__restrict__ field,
+    const float4 *__restrict__ xyzd, const float *__restrict__ depth, float sigma_scale,
+    float *__restrict__ out_color, float *__restrict__ out_depth, float *__restrict__ out_missed,
+    int kahan) {
+  int lane = threadIdx.x & 31;
+  int64_t r = blockIdx.x * (int64_t)kWarps + (threadIdx.x >> 5);
+  if (r >= rays) return;
+  const int64_t a = offset[r], n = offset[r + 1] - a;
+  Prefix carry{0.f, 0.f};
+  float sp = 0.f, sd = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
+  for (int64_t base = 0; base < n; base += 32) {
+    const int64_t i = base + lane;
+    const bool in = i < n;
+    const float4 f = in ? field[a + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float dist = in ? xyzd[a + i].w : 0.f;
+    const float fe = (relu_nan(f.x) * dist) * sigma_scale;
+    const float pre = chunk_prefix(fe, lane, carry, kahan != 0);
+    if (in) {
+      const float p = (1.0f - expf(-fe)) * expf(-pre);
+      sp += p;
+      sd += p * depth[a + i];
+      c0 += p * f.y; c1 += p * f.z; c2 += p * f.w;
+    }
+  }
+  sp = warp_sum(sp);
+  sd = warp_sum(sd);
+  c0 = warp_sum(c0); c1 = warp_sum(c1); c2 = warp_sum(c2);
+  if (lane == 0) {
+    out_color[r * 3 + 0] = c0; out_color[r * 3 + 1] = c1; out_color[r * 3 + 2] = c2;
+    out_depth[r] = sd;
+    out_missed[r] = 1.0f - sp;
+  }
+}
+
+__global__ void __launch_bounds__(kWarps * 32) composite_rows_bwd_kernel(
+    int64_t rays, const int64_t *__restrict__ offset, const float4 *__restrict__ field,
+    const float4 *__restrict__ xyzd, const float *__restrict__ depth, float sigma_scale,
+    const float *__restrict__ g_color, const float *__restrict__ g_depth,
+    const float *__restrict__ g_missed, float4 *__restrict__ g_field, int kahan) {
+  int lane = threadIdx.x & 31;
+  int64_t r = blockIdx.x * (int64_t)kWarps + (threadIdx.x >> 5);
+  if (r >= rays) return;
+  const int64_t a = offset[r], n = offset[r + 1] - a;
+  const float gd = g_depth ? g_depth[r] : 0.f;
+  const float gm = g_missed ? g_missed[r] : 0.f;
+  float gc0 = 0.f, gc1 = 0.f, gc2 = 0.f;
+  if (g_color) { gc0 = g_color[r * 3]; gc1 = g_color[r * 3 + 1]; gc2 = g_color[r * 3 + 2]; }
+  // pass 1: total = sum_i g_i p_i; pass 2: suffix_j = total - inclusive prefix
+  float total = 0.f, gp_carry = 0.f;
+  for (int pass = 0; pass < 2; ++pass) {
+    Prefix carry{0.f, 0.f};
+    for (int64_t base = 0; base < n; base += 32) {
+      const int64_t i = base + lane;
+      const bool in = i < n;
+      const float4 f = in ? field[a + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float dist = in ? xyzd[a + i].w : 0.f;
+      const float fe = (relu_nan(f.x) * dist) * sigma_scale;
+      const float pre = chunk_prefix(fe, lane, carry, kahan != 0);
+      const float T = expf(-pre), e = expf(-fe);
+      const float p = in ? (1.0f - e) * T : 0.f;
+      float g = 0.f;
+      if (in) g = (gd * depth[a + i] - gm) + (gc0 * f.y + gc1 * f.z + gc2 * f.w);
+      const float gp = g * p;
+      if (pass == 0) {
+        total += gp;
+        continue;
+      }
+      const float incl = warp_incl_scan(gp, lane) + gp_carry;
+      gp_carry = __shfl_sync(0xffffffffu, incl, 31);
+      if (in) {
+        const float g_fe = g * e * T - (total - incl);
+        g_field[a + i] = make_float4((g_fe * dist) * sigma_scale * (f.x > 0.0f ? 1.0f : 0.0f),
+                                     gc0 * p, gc1 * p, gc2 * p);
+      }
+    }
+    if (pass == 0) total = warp_sum(total);
+  }
+}
+
 }  // namespace
 
 extern "C" {
@@ -280,6 +369,37 @@ int nsvf_composite_backward(int64_t rays, int max_steps, const float *free_energ
   composite_bwd_kernel<<<nsvf_grid(rays, kWarps), kWarps * 32, 0, (cudaStream_t)stream>>>(
       rays, max_steps, free_energy, texture, sampled_depth, grad_probs, grad_depth, grad_missed,
       grad_colors, grad_free_energy, grad_texture, kahan);
+  return nsvf_launch_status();
+}
+
+int nsvf_composite_rows(int64_t rays, const int64_t *offset, const float *field,
+                        const float *xyz_dist, const float *depth, float sigma_scale,
+                        float *out_color, float *out_depth, float *out_missed, int kahan,
+                        void *stream) {
+  if (rays < 0) return NSVF_ERR_INVALID;
+  if (rays == 0) return NSVF_OK;
+  if (!offset || !field || !xyz_dist || !depth || !out_color || !out_depth || !out_missed ||
+      ((((uintptr_t)field) | ((uintptr_t)xyz_dist)) & 15))
+    return NSVF_ERR_INVALID;
+  composite_rows_kernel<<<nsvf_grid(rays, kWarps), kWarps * 32, 0, (cudaStream_t)stream>>>(
+      rays, offset, (const float4 *)field, (const float4 *)xyz_dist, depth, sigma_scale, out_color,
+      out_depth, out_missed, kahan);
+  return nsvf_launch_status();
+}
+
+int nsvf_composite_rows_backward(int64_t rays, const int64_t *offset, const float *field,
+                                 const float *xyz_dist, const float *depth, float sigma_scale,
+                                 const float *grad_color, const float *grad_depth,
+                                 const float *grad_missed, float *grad_field, int kahan,
+                                 void *stream) {
+  if (rays < 0) return NSVF_ERR_INVALID;
+  if (rays == 0) return NSVF_OK;
+  if (!offset || !field || !xyz_dist || !depth || !grad_field ||
+      ((((uintptr_t)field) | ((uintptr_t)xyz_dist) | ((uintptr_t)grad_field)) & 15))
+    return NSVF_ERR_INVALID;
+  composite_rows_bwd_kernel<<<nsvf_grid(rays, kWarps), kWarps * 32, 0, (cudaStream_t)stream>>>(
+      rays, offset, (const float4 *)field, (const float4 *)xyz_dist, depth, sigma_scale, grad_color,
+      grad_depth, grad_missed, (float4 *)grad_field, kahan);
   return nsvf_launch_status();
 }
 

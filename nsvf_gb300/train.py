@@ -4,22 +4,24 @@ FP32 forward and a hand-written backward with per-chunk recomputation.
 The reference trains through autograd and keeps every ray chunk's graph
 alive until the loss's backward (fairnr/modules/renderer.py:135-232): the
 [samples, 8, 32] corner gathers and every MLP activation of the whole batch.
-Here `RayChunk` is one torch.autograd.Function per chunk of rays that keeps
-only the chunk's inputs (sample voxel ids, positions, depths, lengths). Its
-backward evaluates the chunk again and runs
+Here `RayBatch` is one torch.autograd.Function per batch of rays that keeps
+its compacted samples (voxel ids, positions, depths, lengths: 28 bytes each)
+and their field values. Its backward runs
 
-  compositing backward     nsvf_composite_backward (transmittance prefix
-                           recomputed in the kernel)
-  free energy backward     d sigma = d fe * dist * 7 where sigma > 0
-  MLP backward             per layer, from the saved pre-activations:
-                           dW = dZ^T A, db = sum dZ, dA = dZ W, dZ = dA (Z > 0)
-                           (FP32 GEMMs, cuBLAS through torch.mm)
-  interpolation backward   nsvf_trilinear_embed_backward (float4 atomics
-                           into the corner embeddings)
+  compositing backward     nsvf_composite_rows_backward (transmittance prefix
+                           recomputed in the kernel), with the free energy's:
+                           d sigma = d fe * dist * 7 where sigma > 0
+  field backward           nsvf_field_train_backward: per chunk of samples,
+                           interpolation and activations again, dZ = dA (Z >
+                           0), dA = dZ W through all layers of a tile in
+                           shared memory, then dW = dZ^T A, db = sum dZ
+  interpolation backward   float4 atomics into the corner embeddings, from the
+                           same tiles
 
 so a batch needs one chunk's activations at a time. The field is the
 workloads' 4 x 128 ReLU MLP (field.StandInField); the embeddings are the
-encoder's `values` table.
+encoder's `values` table. Fields of other widths (and tensors that are not
+FP32) go through `RayChunk`, one Function per chunk of rays on cuBLAS GEMMs.
 
 `train_step` renders a batch of rays (intersection, sampling distribution,
 inverse-CDF samples: no gradient), takes the squared colour error against
@@ -28,6 +30,8 @@ The sigma noise the reference adds in training mode
 (fairnr/modules/renderer.py:119) is left out, as in evaluation mode, so that
 gradients are reproducible.
 """
+import ctypes
+
 import torch
 from torch.autograd import Function
 
@@ -144,6 +148,113 @@ class RayChunk(Function):
         return (g_values, *grads) + (None,) * 8
 
 
+# Samples of one wave of nsvf_field_train_backward: 304 blocks (two per SM) of
+# one 128-sample tile. A chunk is whole waves, so that no SM idles between the
+# chunks of a batch.
+WAVE = 304 * 128
+
+
+def _ptrs(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+
+class RayBatch(Function):
+    """(values, W0, b0, ..., W4, b4, sampled_idx [R, M], xyz [R, M, 3],
+    dists [R, M], depths [R, M], centers, feats, voxel_size, kahan,
+    chunk_rays) -> (colors [R, 3], depth [R], missed [R]) of a batch of rays.
+    chunk_rays rays' samples (on average, rounded to whole waves) are
+    recomputed at a time in the backward."""
+
+    @staticmethod
+    def forward(ctx, values, *args):
+        params = args[:10]
+        sidx, xyz, dists, depths, centers, feats, voxel_size, kahan, chunk_rays = args[10:]
+        dev = values.device
+        stream = ext.ctypes_stream(dev)
+        R, M = sidx.shape
+        count = torch.empty(R, dtype=torch.int32, device=dev)
+        check(LIB.nsvf_train_rows_count(R, M, _p(sidx), _p(count), stream), "train_rows_count")
+        offset = torch.zeros(R + 1, dtype=torch.int64, device=dev)
+        torch.cumsum(count, 0, out=offset[1:])
+        ns = int(offset[R])
+        f = lambda *shape: torch.empty(*shape, dtype=torch.float32, device=dev)
+        vox = torch.empty(max(ns, 1), dtype=torch.int32, device=dev)
+        xyzd, depth, field = f(max(ns, 1), 4), f(max(ns, 1)), f(max(ns, 1), 4)
+        if ns:
+            check(LIB.nsvf_train_rows_pack(R, M, _p(sidx), _p(xyz), _p(dists), _p(depths),
+                                           _p(offset), _p(vox), _p(xyzd), _p(depth), stream),
+                  "train_rows_pack")
+            packed = RayBatch._packed(params, stream)
+            check(LIB.nsvf_field_train_forward(
+                ns, _p(vox), _p(xyzd), centers.size(0), values.size(0), float(voxel_size),
+                _p(centers), _p(feats), _p(values), _p(packed), _p(field),
+                _p(ext.error_word(dev)), stream), "field_train_forward")
+        colors, out_depth, missed = f(R, 3), f(R), f(R)
+        check(LIB.nsvf_composite_rows(R, _p(offset), _p(field), _p(xyzd), _p(depth), SIGMA_SCALE,
+                                      _p(colors), _p(out_depth), _p(missed), int(bool(kahan)),
+                                      stream), "composite_rows")
+        ctx.save_for_backward(values, *params, vox, xyzd, depth, offset, field, centers, feats)
+        ctx.voxel_size, ctx.kahan, ctx.ns = float(voxel_size), bool(kahan), ns
+        waves = max(1, round(ns * int(chunk_rays) / max(R, 1) / WAVE))
+        ctx.chunk = waves * WAVE
+        return colors, out_depth, missed
+
+    @staticmethod
+    def _packed(params, stream):
+        packed = torch.empty(int(LIB.nsvf_field_train_packed_floats()), dtype=torch.float32,
+                             device=params[0].device)
+        check(LIB.nsvf_field_train_pack(_ptrs(params[0::2]), _ptrs(params[1::2]), _p(packed),
+                                        stream), "field_train_pack")
+        return packed
+
+    @staticmethod
+    def backward(ctx, g_colors, g_depth, g_missed):
+        saved = ctx.saved_tensors
+        values, params = saved[0], saved[1:11]
+        vox, xyzd, depth, offset, field, centers, feats = saved[11:]
+        dev = values.device
+        stream = ext.ctypes_stream(dev)
+        R, ns = offset.numel() - 1, ctx.ns
+        c = lambda g: g.float().contiguous() if g is not None else None
+        g_colors, g_depth, g_missed = c(g_colors), c(g_depth), c(g_missed)
+        with torch.no_grad():
+            g_field = torch.empty_like(field)
+            check(LIB.nsvf_composite_rows_backward(
+                R, _p(offset), _p(field), _p(xyzd), _p(depth), SIGMA_SCALE, _p(g_colors),
+                _p(g_depth), _p(g_missed), _p(g_field), int(ctx.kahan), stream),
+                "composite_rows_backward")
+            g_values = torch.zeros_like(values)
+            grads = [torch.empty_like(t) for t in params]
+            n = int(LIB.nsvf_field_train_backward_floats(ns, ctx.chunk))
+            work = torch.empty(n, dtype=torch.float32, device=dev)
+            packed = RayBatch._packed(params, stream)
+            check(LIB.nsvf_field_train_backward(
+                ns, ctx.chunk, _p(vox), _p(xyzd), centers.size(0), values.size(0), ctx.voxel_size,
+                _p(centers), _p(feats), _p(values), _p(packed), _p(g_field), _p(work), n,
+                _p(g_values), _ptrs(grads[0::2]), _ptrs(grads[1::2]), stream),
+                "field_train_backward")
+        return (g_values, *grads) + (None,) * 9
+
+
+FIELD_SHAPES = [(128, 32), (128,)] + [(128, 128), (128,)] * 3 + [(4, 128), (4,)]
+
+
+def _batch_ok(values, params, sidx, xyz, dists, depths, centers, feats):
+    """RayBatch takes FP32 tensors on one GPU, the 4 x 128 field and 32
+    channels in 16-byte aligned rows; anything else goes through RayChunk."""
+    if [tuple(t.shape) for t in params] != FIELD_SHAPES or values.dim() != 2 or \
+            values.size(1) != 32 or sidx.dim() != 2 or xyz.shape != (*sidx.shape, 3) or \
+            dists.shape != sidx.shape or depths.shape != sidx.shape or \
+            centers.dim() != 2 or centers.size(1) != 3 or feats.shape != (centers.size(0), 8):
+        return False
+    if not all(t.is_cuda and t.dtype == torch.float32 and t.device == values.device
+               for t in (values, *params, xyz, dists, depths, centers)):
+        return False
+    return sidx.device == feats.device == values.device and not sidx.is_floating_point() and \
+        values.data_ptr() % 16 == 0 and all(t.is_contiguous() for t in (values, *params)) and \
+        not torch.is_autocast_enabled()
+
+
 def field_params(field):
     out = []
     for lin in field.layers:
@@ -198,7 +309,13 @@ def render_batch(encoder, field, ray_start, ray_dir, chunk_rays=1024, states=Non
     bg = field.bg_color.bg_color.float()
     colors_hit, missed_hit = [], []
     n = sidx.shape[0]
-    for i in range(0, n, chunk_rays):
+    starts = range(0, n, chunk_rays)
+    if starts and _batch_ok(values, params, sidx, xyz, dists, depths, centers, feats):
+        c, _, m = RayBatch.apply(values, *params, sidx.int().contiguous(), xyz.contiguous(),
+                                 dists.contiguous(), depths.contiguous(), centers, feats,
+                                 float(encoder.voxel_size), kahan, chunk_rays)
+        colors_hit, missed_hit, starts = [c], [m], ()
+    for i in starts:
         c, _, m = RayChunk.apply(values, *params, sidx[i:i + chunk_rays].contiguous(),
                                  xyz[i:i + chunk_rays].contiguous(),
                                  dists[i:i + chunk_rays].contiguous(),

@@ -1,0 +1,140 @@
+"""The training batch's kernels (nsvf_gb300/csrc/train.cu) at sizes around
+their tiles: the FP32 field forward against a chain of cuBLAS FP32 layers
+(bit for bit) and the whole batch's colours and gradients against float64
+torch autograd."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(cuda, n_vox, seed):
+    g = torch.Generator().manual_seed(seed)
+    vs = 0.25
+    centers = torch.rand(n_vox, 3, generator=g) * 2 - 1
+    feats = torch.randint(0, 3 * n_vox, (n_vox, 8), generator=g, dtype=torch.int32)
+    values = torch.randn(3 * n_vox, 32, generator=g) * 0.3
+    dims = [32, 128, 128, 128, 128, 4]
+    params = []
+    for a, b in zip(dims[:-1], dims[1:]):
+        params += [torch.randn(b, a, generator=g) * a ** -0.5, torch.randn(b, generator=g) * 0.1]
+    return vs, centers.to(cuda), feats.to(cuda), values.to(cuda), [p.to(cuda) for p in params]
+
+
+def _rows(cuda, rays, steps, n_vox, vs, centers, seed):
+    """sampled_idx with -1 both inside and at the end of the rows (and empty
+    rows), positions inside the sampled voxels, increasing depths."""
+    g = torch.Generator().manual_seed(seed + 1)
+    idx = torch.randint(0, n_vox, (rays, steps), generator=g, dtype=torch.int32)
+    runs = torch.randint(0, n_vox, (rays, max(1, steps // 5 + 1)), generator=g, dtype=torch.int32)
+    idx = torch.where(torch.rand(rays, 1, generator=g) < 0.7,
+                      runs.repeat_interleave(5, 1)[:, :steps], idx)
+    idx[torch.rand(rays, steps, generator=g) < 0.1] = -1
+    idx[torch.arange(steps)[None] >= torch.randint(0, steps + 1, (rays, 1), generator=g)] = -1
+    off = (torch.rand(rays, steps, 3, generator=g) - 0.5) * vs
+    idx, off = idx.to(cuda), off.to(cuda)
+    xyz = centers[idx.clamp(min=0).long()] + off
+    dists = torch.rand(rays, steps, generator=g).to(cuda) * 0.1
+    depths = torch.rand(rays, steps, generator=g).cumsum(1).to(cuda)
+    return idx, xyz.contiguous(), dists, depths
+
+
+def _field64(idx, xyz, centers, feats, values, params, vs):
+    m = idx.ne(-1)
+    v = idx[m].long()
+    p = (xyz[m] - centers[v]) / vs + 0.5
+    x = 0
+    for k in range(8):
+        w = 1
+        for d, bit in enumerate((4, 2, 1)):
+            w = w * (p[:, d] if k & bit else 1 - p[:, d])
+        x = x + w[:, None] * values[feats[v, k].long()]
+    for l in range(5):
+        x = x @ params[2 * l].t() + params[2 * l + 1]
+        x = torch.relu(x) if l < 4 else x
+    return m, x
+
+
+# samples: below one tile, across a tile's edge, more tiles than blocks (304
+# tiles of 128), and a backward in several chunks
+@pytest.mark.parametrize("rays,steps,chunk_rays", [(1, 1, 1), (3, 47, 2), (130, 3, 1024),
+                                                   (257, 64, 64), (900, 100, 300)])
+def test_batch_matches_float64_autograd(cuda, rays, steps, chunk_rays):
+    from nsvf_gb300 import ext, train
+    n_vox = 97
+    vs, centers, feats, values, params = _scene(cuda, n_vox, rays)
+    idx, xyz, dists, depths = _rows(cuda, rays, steps, n_vox, vs, centers, rays)
+    values.requires_grad_(True)
+    for p in params:
+        p.requires_grad_(True)
+    g = torch.Generator().manual_seed(5)
+    gc, gd, gm = (torch.randn(*s, generator=g).to(cuda) for s in ((rays, 3), (rays,), (rays,)))
+    out = train.RayBatch.apply(values, *params, idx, xyz, dists, depths, centers, feats, vs, False,
+                               chunk_rays)
+    grads = torch.autograd.grad(out, [values, *params], (gc, gd, gm))
+    ext.check_errors(cuda)
+    v64 = values.detach().double().requires_grad_(True)
+    p64 = [p.detach().double().requires_grad_(True) for p in params]
+    vs32 = float(np.float32(vs))
+    m, x = _field64(idx, xyz.double(), centers.double(), feats, v64, p64, vs32)
+    z = torch.zeros(rays, steps, dtype=torch.float64, device=cuda)
+    fe = z.masked_scatter(m, torch.relu(x[:, 0]) * dists.double()[m] * 7.0)
+    tex = torch.stack([z.masked_scatter(m, x[:, 1 + c]) for c in range(3)], -1)
+    T = torch.exp(-torch.cat([z[:, :1], fe[:, :-1]], 1).cumsum(1))
+    pr = (1 - torch.exp(-fe)) * T
+    ref = ((pr[..., None] * tex).sum(1), (pr * depths.double()).sum(1), 1 - pr.sum(1))
+    ref_g = torch.autograd.grad(ref, [v64, *p64], (gc.double(), gd.double(), gm.double()))
+    # FP32 sums of at most 100 terms of order 1 along a ray (colours), then of
+    # all samples (gradients); a sign of a pre-activation within FP32 rounding
+    # of zero (about one in 1e7 of the 512 per sample) changes a gradient by
+    # one sample's share
+    for a, b in zip(out, ref):
+        assert float((a.detach().double() - b.detach()).abs().max()) <= 2e-5 * (1 + float(b.abs().max()))
+    for a, b in zip(grads, ref_g):
+        scale = float(b.norm()) + 1e-12
+        assert float((a.detach().double() - b.detach()).norm()) <= 2e-3 * scale
+
+
+@pytest.mark.parametrize("ns", [100, 128, 129, 40000])
+def test_forward_bits_of_a_gemm_chain(cuda, ns):
+    """out = the bits of nsvf_trilinear_embed followed by torch.addmm / relu
+    (FP32 cuBLAS: one fused multiply-add chain over k, then the bias), so a
+    training run keeps every ReLU's sign."""
+    from nsvf_gb300 import ext, train
+    from nsvf_gb300._lib import LIB, check
+    from nsvf_gb300.functional import trilinear_embed
+    n_vox = 61
+    vs, centers, feats, values, params = _scene(cuda, n_vox, ns)
+    g = torch.Generator().manual_seed(ns)
+    vid = torch.randint(0, n_vox, (ns,), generator=g, dtype=torch.int32).to(cuda)
+    xyz = centers[vid.long()] + (torch.rand(ns, 3, generator=g).to(cuda) - 0.5) * vs
+    xyzd = torch.cat([xyz, torch.ones(ns, 1, device=cuda)], 1).contiguous()
+    stream = ext.ctypes_stream(cuda)
+    packed = train.RayBatch._packed(params, stream)
+    out = torch.empty(ns, 4, device=cuda)
+    check(LIB.nsvf_field_train_forward(
+        ns, vid.data_ptr(), xyzd.data_ptr(), n_vox, values.size(0), vs, centers.data_ptr(),
+        feats.data_ptr(), values.data_ptr(), packed.data_ptr(), out.data_ptr(),
+        ext.error_word(cuda).data_ptr(), stream), "field_train_forward")
+    x = trilinear_embed(vid, xyz.contiguous(), centers, feats, values, vs)
+    for l in range(5):
+        x = torch.addmm(params[2 * l + 1], x, params[2 * l].t())
+        x = torch.relu(x) if l < 4 else x
+    ext.check_errors(cuda)
+    assert torch.equal(out, x)
+
+
+def test_other_widths_keep_the_general_path(cuda):
+    """A field that is not 4 x 128 trains through RayChunk."""
+    from nsvf_gb300 import train
+    vs, centers, feats, values, _ = _scene(cuda, 20, 1)
+    g = torch.Generator().manual_seed(2)
+    dims = [32, 64, 64, 64, 64, 4]
+    params = []
+    for a, b in zip(dims[:-1], dims[1:]):
+        params += [torch.randn(b, a, generator=g).to(cuda), torch.zeros(b, device=cuda)]
+    idx, xyz, dists, depths = _rows(cuda, 5, 8, 20, vs, centers, 3)
+    assert not train._batch_ok(values, params, idx, xyz, dists, depths, centers, feats)
+    out = train.RayChunk.apply(values, *params, idx, xyz, dists, depths, centers, feats, vs, False)
+    assert out[0].shape == (5, 3)
