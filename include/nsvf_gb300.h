@@ -702,6 +702,18 @@ int nsvf_prune_screen_bf16(int64_t n_voxels, int bits, int rule, float step, flo
                            const void *const weights[5], const float *const biases[5],
                            uint32_t *score, uint8_t *keep, int64_t *list, int64_t *n_list,
                            int64_t list_cap, int32_t *err, void *stream);
+/* prune_fp32_dev: between the two, the listed points of voxels not yet kept in
+ * FP32 (packed weights as nsvf_field_train_pack). A point with sigma - margin >
+ * threshold sets keep, margin = band * M + 1e-6 threshold; the points within
+ * the margin go to `undecided`, prune_exact_dev's list (the screen's own list
+ * buffer may be passed; n_live and n_undecided zeroed by the caller; live and
+ * undecided hold list_cap entries). FP32 rounds 2^15 times finer than BF16;
+ * a band of 1/64 of the screen's leaves 2^9 for the longer accumulation. */
+int nsvf_prune_fp32_dev(int64_t n_voxels, int bits, float threshold, float band, int64_t n_keys,
+                        float voxel_size, const float *centers, const int32_t *feats,
+                        const float *values, const float *packed, const int64_t *list,
+                        const int64_t *n_list, int64_t list_cap, uint8_t *keep, int64_t *live,
+                        int64_t *n_live, int64_t *undecided, int64_t *n_undecided, void *stream);
 int nsvf_prune_exact_dev(int64_t n_voxels, int bits, int rule, double threshold, int64_t n_keys,
                          float voxel_size, const float *centers, const int32_t *feats,
                          const float *values, const float *const weights_t[5],

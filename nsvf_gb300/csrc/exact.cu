@@ -25,9 +25,9 @@
 //
 // The same evaluation decides the pruning mask exactly (nsvf_prune_exact_dev):
 // the tensor-core pruning kernel screens every point in BF16 with an error
-// scale M (mlp_tc.cu), and only the points it cannot decide -- about 0.3 %
-// of a c2 pass -- are evaluated here, their sigma compared with the
-// threshold in double-float.
+// scale M (mlp_tc.cu), nsvf_prune_fp32_dev (train.cu) evaluates the points of
+// undecided voxels in FP32, and only what that cannot decide is evaluated
+// here, its sigma compared with the threshold in double-float.
 //
 // A sample is flagged when any trilinear coordinate leaves [-0.5, 1.5]: half
 // a voxel beyond the voxel's faces, well past the x-shift of the reference's

@@ -16,7 +16,7 @@
 // elementwise operation; here a tile of 128 samples goes through all layers
 // in shared memory.
 //
-// field_train_kernel<BWD>, 256 threads, two blocks per SM (while one gathers,
+// field_train_kernel<MODE>, 256 threads, two blocks per SM (while one gathers,
 // scatters or waits for weights, the other computes):
 //   * activations [unit][sample] in shared memory (64 KB), each thread an 8 x
 //     8 block of (unit, sample) accumulators, two samples per fma.rn.f32x2;
@@ -55,12 +55,19 @@ constexpr int kBlocks = 2 * 152;           // two per SM
 // cost about a third
 constexpr int kSplit = 90, kSplit0 = kBlocks - 3 * kSplit;
 constexpr int kRows = 16, kGradStages = 4;
-// per half block of field_train_kernel<true>: dW4 [4][128], db0..db3 [4][128]
+// per half block of field_train_kernel<kBackward>: dW4 [4][128], db0..db3 [4][128]
 constexpr int kSmall = 8 * kHid;
 
 __host__ __device__ constexpr int act_swz(int row) {
-  return ((row >> 2) ^ ((row & 3) << 1)) & 7;
+  return (((row >> 2) & 3) << 1) ^ (row & 1) ^ ((row & 2) << 1);
 }
+
+// A warp's 8 x 4 block of threads. Lanes that differ in bit 0 share lane_x and
+// lanes that differ in bit 1 share lane_y: with either, a 128-bit shared load
+// takes 2 cycles of the 128-byte data path instead of the 4 of a broadcast
+// between 8-lane groups (measured: x = lane & 7 and y = lane >> 3 take 4 and 2).
+__device__ __forceinline__ int lane_x(int lane) { return (lane >> 1) & 7; }
+__device__ __forceinline__ int lane_y(int lane) { return (lane & 1) | ((lane >> 4) << 1); }
 
 __device__ __forceinline__ void cp16(float *dst, const float *src, int bytes = 16) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
@@ -87,17 +94,27 @@ __device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// acc[j][p] += w_j * (samples 2p, 2p + 1) for one k: w = 8 units, a = 8 samples
+// acc[j][p] += w_j * (samples 2p, 2p + 1) for one k: w = 8 units, a = 8
+// samples. Every other row of pairs runs backwards, so that neighbouring FMAs
+// share an operand (a copy of this loop alone: 67 TFLOP/s, 65 in plain order,
+// 57 with one FMA per instruction).
 __device__ __forceinline__ void outer(uint64_t (&acc)[8][4], const float4 &w0, const float4 &w1,
                                       const ulonglong2 &a0, const ulonglong2 &a1) {
   const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const uint64_t ww = pk(w[j], w[j]);
-    fma2(acc[j][0], ww, a0.x);
-    fma2(acc[j][1], ww, a0.y);
-    fma2(acc[j][2], ww, a1.x);
-    fma2(acc[j][3], ww, a1.y);
+    if (j & 1) {
+      fma2(acc[j][3], ww, a1.y);
+      fma2(acc[j][2], ww, a1.x);
+      fma2(acc[j][1], ww, a0.y);
+      fma2(acc[j][0], ww, a0.x);
+    } else {
+      fma2(acc[j][0], ww, a0.x);
+      fma2(acc[j][1], ww, a0.y);
+      fma2(acc[j][2], ww, a1.x);
+      fma2(acc[j][3], ww, a1.y);
+    }
   }
 }
 
@@ -129,7 +146,23 @@ struct TrainParams {
   int add;                    // backward: add to the slots (0: overwrite)
   float4 *g_values;           // backward: [n_keys, 32]
   int32_t *err;
+  // pruning (kPrune): sample s is point list[s] % bits^3 of voxel list[s] /
+  // bits^3, *n_list of them (at most ns)
+  const int64_t *list;
+  const unsigned long long *n_list;
+  int bits;
+  float T, band;
+  uint8_t *keep;              // [n_vox]
+  int64_t *undecided;         // points within the band of T
+  unsigned long long *n_undecided;
 };
+
+enum Mode { kForward, kBackward, kPrune };
+
+// offset_points' FP32 position of point i of the voxel around c (exact.cu)
+__device__ __forceinline__ float point_pos(float c, int o, int bits, float hv) {
+  return __fadd_rn(c, __fmul_rn(__fdiv_rn((float)(2 * o + 1 - bits), (float)(bits - 1)), hv));
+}
 
 // The weight stages, streamed in order and around.
 struct Stream {
@@ -185,10 +218,9 @@ __device__ __forceinline__ void gemm128(uint64_t (&acc)[8][4], int stages, Strea
   for (int c = 0; c < stages; ++c) {
     const float *w = st.take() + tx * 4;
     const float *a = act + c * 16 * kTile;
-    const int par = (c & 1) << 2;          // act_swz(16 c + kk) = act_swz(kk) ^ par
 #pragma unroll
     for (int kk = 0; kk < 16; ++kk) {
-      const float *row = a + kk * kTile + ((ty ^ act_swz(kk) ^ par) << 2);
+      const float *row = a + kk * kTile + ((ty ^ act_swz(kk)) << 2);
       const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(row);
       const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(row + 64);
       const float4 w0 = *reinterpret_cast<const float4 *>(w + kk * kHid);
@@ -233,12 +265,13 @@ __device__ __forceinline__ float row_sum(const float *act, int n, int half) {
   return s;
 }
 
-template <bool BWD>
+template <int MODE>
 __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p) {
+  constexpr bool BWD = MODE == kBackward;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   Smem &S = *reinterpret_cast<Smem *>(smem_raw);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int tx = (warp >> 2) * 8 + (lane & 7), ty = (warp & 3) * 4 + (lane >> 3);
+  const int tx = (warp >> 2) * 8 + lane_x(lane), ty = (warp & 3) * 4 + lane_y(lane);
   const int unit = t & 127, half = t >> 7;
   for (int i = t; i < 4 * kHid; i += kT) {
     S.w4[i] = p.packed[kW4Off + i];
@@ -252,7 +285,9 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
   st.start();
   float dw4[4] = {0.f, 0.f, 0.f, 0.f}, db[4] = {0.f, 0.f, 0.f, 0.f};
   float4 db4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int64_t tiles = (p.ns + kTile - 1) / kTile;
+  int64_t ns = p.ns;
+  if (MODE == kPrune && (int64_t)*p.n_list < ns) ns = (int64_t)*p.n_list;
+  const int64_t tiles = (ns + kTile - 1) / kTile;
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t s0 = tile * kTile;
     // interpolation: 8 threads per sample, 4 channels each (interp.cu's
@@ -263,12 +298,26 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
       const int sl = it * 32 + (t >> 3), ch = t & 7;
       const int64_t s = s0 + sl;
       float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (s < p.ns) {
-        const int64_t v = p.vox[s];
-        if (v < 0 || v >= p.n_vox) {
-          if (!BWD && p.err && ch == 0) atomicOr(p.err, 4);
+      if (s < ns) {
+        int64_t v;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (MODE == kPrune) {
+          const int P = p.bits * p.bits * p.bits;
+          v = p.list[s] / P;
+          const int i = (int)(p.list[s] % P);
+          if (v >= 0 && v < p.n_vox) {
+            const float hv = p.voxel_size / 2.0f;
+            x.x = point_pos(p.centers[v * 3 + 0], i / (p.bits * p.bits), p.bits, hv);
+            x.y = point_pos(p.centers[v * 3 + 1], i / p.bits % p.bits, p.bits, hv);
+            x.z = point_pos(p.centers[v * 3 + 2], i % p.bits, p.bits, hv);
+          }
         } else {
-          const float4 x = p.xyzd[s];
+          v = p.vox[s];
+        }
+        if (v < 0 || v >= p.n_vox) {
+          if (MODE == kForward && p.err && ch == 0) atomicOr(p.err, 4);
+        } else {
+          if (MODE != kPrune) x = p.xyzd[s];
           const float q[3] = {(x.x - p.centers[v * 3 + 0]) / p.voxel_size + 0.5f,
                               (x.y - p.centers[v * 3 + 1]) / p.voxel_size + 0.5f,
                               (x.z - p.centers[v * 3 + 2]) / p.voxel_size + 0.5f};
@@ -276,7 +325,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
           for (int k = 0; k < 8; ++k) {
             const int64_t key = p.feats[v * 8 + k];
             if (key < 0 || key >= p.n_keys) {
-              if (!BWD && p.err) atomicOr(p.err, 4);
+              if (MODE == kForward && p.err) atomicOr(p.err, 4);
               continue;
             }
             const float w = corner_weight(q, k);
@@ -296,7 +345,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
     }
     if (BWD && t < kTile) {
       const int64_t s = s0 + t;
-      const float4 d = s < p.ns ? p.d_out[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 d = s < ns ? p.d_out[s] : make_float4(0.f, 0.f, 0.f, 0.f);
       S.dout[t] = d;
       db4.x += d.x; db4.y += d.y; db4.z += d.z; db4.w += d.w;
     }
@@ -333,6 +382,29 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
       store_act(S.act, y, tx, ty);
     }
     __syncthreads();
+    if (MODE == kPrune) {
+      // sigma (threads of half 0) and M = sum |W4[0]| h (half 1) of point
+      // `unit`: the point is decided where sigma lies further from T than the
+      // band; the others (and NaN) are listed
+      float o = 0.0f;
+#pragma unroll 8
+      for (int k = 0; k < kHid; ++k) {
+        const float a = S.act[k * kTile + (((unit >> 2) ^ act_swz(k)) << 2) + (unit & 3)];
+        o = fmaf(a, half ? fabsf(S.w4[k]) : S.w4[k], o);
+      }
+      if (half) S.dout[unit].x = o;
+      __syncthreads();
+      if (!half && s0 + unit < ns) {
+        const float sigma = __fadd_rn(o, S.b4[0]);
+        const float margin = p.band * S.dout[unit].x + 1e-6f * p.T;
+        const int64_t row = p.list[s0 + unit];
+        if (sigma - margin > p.T)
+          p.keep[row / (p.bits * p.bits * p.bits)] = 1;
+        else if (!(sigma + margin < p.T))
+          p.undecided[atomicAdd(p.n_undecided, 1ull)] = row;
+      }
+      continue;
+    }
     if (!BWD) {
       // head: outputs 2 half, 2 half + 1 of sample `unit`
       const float *w = S.w4 + half * 2 * kHid;
@@ -343,7 +415,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
         o0 = fmaf(a, w[k], o0);
         o1 = fmaf(a, w[kHid + k], o1);
       }
-      if (s0 + unit < p.ns)
+      if (s0 + unit < ns)
         reinterpret_cast<float2 *>(p.out + s0 + unit)[half] =
             make_float2(__fadd_rn(o0, S.b4[half * 2]), __fadd_rn(o1, S.b4[half * 2 + 1]));
       continue;
@@ -409,7 +481,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
     }
     // dA0 = dZ0 W0 [128 samples x 32 channels]: 4 samples x 4 channels a thread
     {
-      const int cg = t & 7, sg = t >> 3;
+      const int cg = lane_x(lane), sg = warp * 4 + lane_y(lane);
       float4 g[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -445,7 +517,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
 #pragma unroll 1
       for (int i = 0; i < 4; ++i) {
         const int64_t s = s0 + sg * 4 + i;
-        int64_t v = s < p.ns ? (int64_t)p.vox[s] : -1;
+        int64_t v = s < ns ? (int64_t)p.vox[s] : -1;
         if (v >= p.n_vox) v = -1;
         if (v < 0) continue;
         if (v != prev) {
@@ -530,9 +602,9 @@ __global__ void __launch_bounds__(kT, 2) weight_grad_kernel(int64_t ns, int64_t 
     cp_commit();
   };
   for (int q = 0; q < kGradStages - 1; ++q) issue(q);
+  const int lane = t & 31, warp = t >> 5;
   if (l) {
-    const int lane = t & 31, warp = t >> 5;
-    const int tx = (warp >> 2) * 8 + (lane & 7), ty = (warp & 3) * 4 + (lane >> 3);
+    const int tx = (warp >> 2) * 8 + lane_x(lane), ty = (warp & 3) * 4 + lane_y(lane);
     uint64_t acc[8][4];
 #pragma unroll
     for (int a = 0; a < 8; ++a)
@@ -572,7 +644,7 @@ __global__ void __launch_bounds__(kT, 2) weight_grad_kernel(int64_t ns, int64_t 
       }
     }
   } else {
-    const int kg = t & 7, ng = t >> 3;         // 4 channels, 4 units
+    const int kg = lane_x(lane), ng = warp * 4 + lane_y(lane);   // 4 channels, 4 units
     float4 g[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -719,12 +791,37 @@ bool bad_scene(int64_t ns, const int32_t *vox, const float *xyzd, int64_t n_vox,
          ((((uintptr_t)xyzd) | ((uintptr_t)values) | ((uintptr_t)packed)) & 15);
 }
 
-template <bool BWD>
+// The points of `in` whose voxel is not kept yet, to `out` (any order).
+__global__ void __launch_bounds__(kT) undecided_kernel(
+    const int64_t *__restrict__ in, const unsigned long long *__restrict__ n_in, int64_t cap, int P,
+    int64_t n_vox, const uint8_t *__restrict__ keep, int64_t *__restrict__ out,
+    unsigned long long *__restrict__ n_out) {
+  const int64_t n = (int64_t)*n_in < cap ? (int64_t)*n_in : cap;
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * kT;
+  for (int64_t base = blockIdx.x * (int64_t)kT; base < n; base += stride) {
+    const int64_t i = base + threadIdx.x;
+    int64_t row = 0;
+    bool live = i < n;
+    if (live) {
+      row = in[i];
+      const int64_t v = row / P;
+      live = row >= 0 && v < n_vox && !keep[v];
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, live);
+    unsigned long long at = 0;
+    if (m && lane == 0) at = atomicAdd(n_out, (unsigned long long)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (live) out[at + __popc(m & ((1u << lane) - 1u))] = row;
+  }
+}
+
+template <int MODE>
 int launch_train(const TrainParams &p, int64_t blocks, cudaStream_t s) {
-  if (cudaFuncSetAttribute(field_train_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(field_train_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)sizeof(Smem)) != cudaSuccess)
     return NSVF_ERR_CUDA;
-  field_train_kernel<BWD><<<(int)blocks, kT, sizeof(Smem), s>>>(p);
+  field_train_kernel<MODE><<<(int)blocks, kT, sizeof(Smem), s>>>(p);
   return nsvf_launch_status();
 }
 
@@ -802,7 +899,7 @@ int nsvf_field_train_forward(int64_t n_samples, const int32_t *voxel, const floa
   p.out = (float4 *)out;
   p.err = err;
   const int64_t tiles = (n_samples + kTile - 1) / kTile;
-  return launch_train<false>(p, tiles < kBlocks ? tiles : kBlocks, (cudaStream_t)stream);
+  return launch_train<kForward>(p, tiles < kBlocks ? tiles : kBlocks, (cudaStream_t)stream);
 }
 
 int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_samples) {
@@ -863,7 +960,7 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
     p.xyzd = (const float4 *)xyz_dist + a;
     p.d_out = (const float4 *)grad_out + a;
     p.add = a > 0;
-    int st = launch_train<true>(p, kBlocks, s);
+    int st = launch_train<kBackward>(p, kBlocks, s);
     if (st != NSVF_OK) return st;
     weight_grad_kernel<<<kBlocks, kT, smem, s>>>(p.ns, rows, acts, grads, part, p.add);
     st = nsvf_launch_status();
@@ -872,6 +969,46 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
   constexpr int n_grads = 3 * kHid * kHid + kHid * kE + kSmall + 4;
   grad_reduce_kernel<<<nsvf_grid(n_grads, kT), kT, 0, s>>>(part, small, db4, g);
   return nsvf_launch_status();
+}
+
+int nsvf_prune_fp32_dev(int64_t n_voxels, int bits, float threshold, float band, int64_t n_keys,
+                        float voxel_size, const float *centers, const int32_t *feats,
+                        const float *values, const float *packed, const int64_t *list,
+                        const int64_t *n_list, int64_t list_cap, uint8_t *keep, int64_t *live,
+                        int64_t *n_live, int64_t *undecided, int64_t *n_undecided, void *stream) {
+  if (n_voxels < 0 || bits < 2 || bits > 64 || n_keys < 1 || list_cap < 0 || !(threshold > 0.0f) ||
+      !(band > 0.0f))
+    return NSVF_ERR_INVALID;
+  if (n_voxels == 0 || list_cap == 0) return NSVF_OK;
+  if (!centers || !feats || !values || !packed || !list || !n_list || !keep || !live || !n_live ||
+      !undecided || !n_undecided || live == list || undecided == live ||
+      ((((uintptr_t)values) | ((uintptr_t)packed)) & 15))
+    return NSVF_ERR_INVALID;
+  cudaStream_t s = (cudaStream_t)stream;
+  const int64_t need = (list_cap + kT - 1) / kT;
+  undecided_kernel<<<(int)(need < 152 * 8 ? need : 152 * 8), kT, 0, s>>>(
+      list, (const unsigned long long *)n_list, list_cap, bits * bits * bits, n_voxels, keep, live,
+      (unsigned long long *)n_live);
+  int st = nsvf_launch_status();
+  if (st != NSVF_OK) return st;
+  TrainParams p = {};
+  p.ns = list_cap;
+  p.n_vox = n_voxels;
+  p.n_keys = n_keys;
+  p.voxel_size = voxel_size;
+  p.centers = centers;
+  p.feats = feats;
+  p.values = (const float4 *)values;
+  p.packed = packed;
+  p.list = live;
+  p.n_list = (const unsigned long long *)n_live;
+  p.bits = bits;
+  p.T = threshold;
+  p.band = band;
+  p.keep = keep;
+  p.undecided = undecided;
+  p.n_undecided = (unsigned long long *)n_undecided;
+  return launch_train<kPrune>(p, kBlocks, s);
 }
 
 }  // extern "C"

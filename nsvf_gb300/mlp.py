@@ -148,6 +148,9 @@ class TensorCoreMLP:
     # 0.005 M (c2 pruning field, 768k points), so 0.02 leaves a factor 4.
     PRUNE_BAND = 0.02
 
+    # The FP32 pass's band is PRUNE_BAND / 64 (nsvf_prune_fp32_dev).
+    FP32_BAND = 64.0
+
     def prune_mask(self, centers, feats, values, voxel_size, th=0.5, bits=8, rule=1, step=0.0,
                    band=PRUNE_BAND):
         """Exact pruning mask [V] (bool) for 0 < th < 1: rule 0 (the
@@ -155,10 +158,11 @@ class TensorCoreMLP:
         1 - min exp(-relu sigma) > th, rule 1 those with max 1 - exp(-relu(sigma)
         step) >= th, sigma at bits^3 offset_points positions per voxel. The
         tensor-core pass screens every point in BF16 and decides all but the
-        points within `band` M of the threshold, which are evaluated in
-        double-float (nsvf_prune_screen_bf16, nsvf_prune_exact_dev). Also
-        returns the BF16 scores (as prune_scores) and the number of points the
-        double-float pass had to examine."""
+        points within `band` M of the threshold. Those of voxels not kept yet
+        are evaluated in FP32 with a band of `band` / FP32_BAND, and what that
+        leaves in double-float (nsvf_prune_screen_bf16, nsvf_prune_fp32_dev,
+        nsvf_prune_exact_dev). Also returns the BF16 scores (as prune_scores)
+        and the number of points that the BF16 pass left undecided."""
         if not 0.0 < th < 1.0:
             raise ValueError("pruning threshold must lie in (0, 1), got %r" % (th,))
         if rule == 1 and not step > 0.0:
@@ -171,7 +175,9 @@ class TensorCoreMLP:
         keep = torch.empty(V, dtype=torch.uint8, device=dev)
         n_list = torch.empty(1, dtype=torch.int64, device=dev)
         err = ext.error_word(dev)
-        cap = max(65536, V * bits ** 3 // 128)
+        # room for 3 % of the points (1.65 % of the c2 pass are undecided): a
+        # second screen pass (7.5 ms there) costs more than the list
+        cap = max(65536, V * bits ** 3 // 32)
         for _ in range(3):
             lst = torch.empty(cap, dtype=torch.int64, device=dev)
             score.fill_(init)
@@ -187,6 +193,28 @@ class TensorCoreMLP:
             if n <= cap:
                 break
             cap = n + n // 4
+        # double-float costs about 60 times FP32 a point (131 against 2.2 us per
+        # thousand), so FP32 decides what it can first: the c2 pass's 23.0 ms
+        # of double-float become 0.39 ms of FP32 and 0.07 ms
+        if n and band > 0.0 and 1e-30 < T < 1e30:
+            stream = ext.ctypes_stream(dev)
+            # the weights of the double-float pass, as they are laid out there
+            w = [t.t().contiguous() for t in self.wt32]
+            packed = torch.empty(int(LIB.nsvf_field_train_packed_floats()), dtype=torch.float32,
+                                 device=dev)
+            check(LIB.nsvf_field_train_pack((ctypes.c_void_p * 5)(*[t.data_ptr() for t in w]),
+                                            self._bp, packed.data_ptr(), stream),
+                  "field_train_pack")
+            live = torch.empty(cap, dtype=torch.int64, device=dev)
+            n_live = torch.zeros(1, dtype=torch.int64, device=dev)
+            n_listed, n_list = n_list, torch.zeros(1, dtype=torch.int64, device=dev)
+            with ext._timed("prune_fp32", dev):
+                check(LIB.nsvf_prune_fp32_dev(
+                    V, int(bits), float(T), float(band) / self.FP32_BAND, values.size(0),
+                    float(voxel_size), centers.data_ptr(), feats.data_ptr(), values.data_ptr(),
+                    packed.data_ptr(), lst.data_ptr(), n_listed.data_ptr(), cap,
+                    keep.data_ptr(), live.data_ptr(), n_live.data_ptr(), lst.data_ptr(),
+                    n_list.data_ptr(), stream), "prune_fp32_dev")
         with ext._timed("prune_exact", dev):
             check(LIB.nsvf_prune_exact_dev(
                 V, int(bits), int(rule), float(T), values.size(0), float(voxel_size),

@@ -90,7 +90,8 @@ def test_batch_matches_float64_autograd(cuda, rays, steps, chunk_rays):
     # of zero (about one in 1e7 of the 512 per sample) changes a gradient by
     # one sample's share
     for a, b in zip(out, ref):
-        assert float((a.detach().double() - b.detach()).abs().max()) <= 2e-5 * (1 + float(b.abs().max()))
+        a, b = a.detach().double(), b.detach()
+        assert float((a - b).abs().max()) <= 2e-5 * (1 + float(b.abs().max()))
     for a, b in zip(grads, ref_g):
         scale = float(b.norm()) + 1e-12
         assert float((a.detach().double() - b.detach()).norm()) <= 2e-3 * scale
@@ -138,3 +139,31 @@ def test_other_widths_keep_the_general_path(cuda):
     assert not train._batch_ok(values, params, idx, xyz, dists, depths, centers, feats)
     out = train.RayChunk.apply(values, *params, idx, xyz, dists, depths, centers, feats, vs, False)
     assert out[0].shape == (5, 3)
+
+
+@pytest.mark.parametrize("n_vox,bits,rule", [(3, 4, 1), (40, 8, 1), (301, 8, 0), (9, 16, 0)])
+def test_prune_fp32_stage_keeps_the_mask(cuda, n_vox, bits, rule):
+    """prune_mask with its FP32 stage against float64 torch at every point,
+    thresholds through the middle of the voxels' scores, so that many points
+    are close. A wide band sends most points through the FP32 stage."""
+    from nsvf_gb300 import ext, geometry
+    from nsvf_gb300.field import StandInField
+    from nsvf_gb300.mlp import TensorCoreMLP
+    vs, centers, feats, values, params = _scene(cuda, n_vox, n_vox)
+    field = StandInField(weights=[(params[2 * l].cpu(), params[2 * l + 1].cpu())
+                                  for l in range(5)]).to(cuda)
+    mlp = TensorCoreMLP(field)
+    pts = geometry.offset_points(centers, torch.tensor(vs / 2.0, device=cuda), bits=bits)
+    idx = torch.arange(n_vox, device=cuda)[:, None].expand(*pts.shape[:2])
+    _, x = _field64(idx, pts.double(), centers.double(), feats, values.double(),
+                    [p.double() for p in params], float(np.float32(vs)))
+    top = x[:, 0].reshape(n_vox, -1).max(1)[0]
+    T = float(top[top > 0].median()) * (1 + 1e-9)
+    step = 0.01 if rule else 0.0
+    th = -np.expm1(-T * (step if rule else 1.0))
+    want = top >= T
+    for band in (0.02, 0.5):
+        keep, _, n = mlp.prune_mask(centers, feats, values, vs, th=th, bits=bits, rule=rule,
+                                    step=step, band=band)
+        ext.check_errors(cuda)
+        assert torch.equal(keep, want) and n > 0
