@@ -269,15 +269,15 @@ __global__ void __launch_bounds__(kBlock) icdf_compact_kernel(
 // cdf_t = (t + 0.5) * step, this sequence: for each bin b, the steps that
 // land in it, then (when a later step passes the bin's upper CDF bound) the
 // bin's closing segment; after the last valid bin is closed the walk is
-// done; then the tail loop. With sf[b + 1] = #{t : cdf_t <= cdf_hi[b]} (a
-// binary search, cdf_t is increasing) every position is closed-form:
+// done; then the tail loop. With sf[b + 1] = #{t : cdf_t <= cdf_hi[b]} (cdf_t
+// is increasing) every position is closed-form:
 //   step t in bin b          at t + b,
 //   closing segment of bin b at sf[b + 1] + b,   emitted iff sf[b + 1] < T,
 // and a step's z_low is the previous step's z when that step is in the same
 // bin, else the bin's min depth. So 32 lanes place 32 consecutive samples
 // at once, with the walk's exact FP32 operations, and write them coalesced.
-// The CDF bounds are the walk's sequential FP32 prefix (one lane); the tail
-// loop runs on one lane. Rows with max_hits > kMaxH use the per-thread walk.
+// The CDF bounds are the walk's sequential FP32 prefix; the tail loop runs on
+// one lane. Rows with max_hits > kMaxH use the per-thread walk.
 constexpr int kMaxH = 128;
 constexpr int kWarpRays = 8;                 // warps (rays in flight) per block
 
@@ -288,20 +288,32 @@ struct RayTab {
   int end[kMaxH];
 };
 
-__device__ __forceinline__ float tab_cdf(int t, float step) {
-  return __fmul_rn(__fadd_rn((float)t, 0.5f), step);
+// The jitter of step t: 0.5, or the row's noise.
+struct HalfJitter {
+  __device__ __forceinline__ float operator()(int) const { return 0.5f; }
+};
+struct RowJitter {
+  const float *U;   // NULL: 0.5
+  __device__ __forceinline__ float operator()(int t) const { return U ? U[t] : 0.5f; }
+};
+
+template <typename J>
+__device__ __forceinline__ float tab_cdf(int t, float step, const J &u) {
+  return __fmul_rn(__fadd_rn((float)t, u(t)), step);
 }
 
 // z of step t in bin b (the walk's in-bin placement)
-__device__ __forceinline__ float tab_z(const RayTab &T, int t, int b, float step) {
+template <typename J>
+__device__ __forceinline__ float tab_z(const RayTab &T, int t, int b, float step, const J &jit) {
   float cl = b > 0 ? T.cdf_hi[b - 1] : 0.0f;
-  float u = __fdiv_rn(__fsub_rn(tab_cdf(t, step), cl), __fsub_rn(T.cdf_hi[b], cl));
+  float u = __fdiv_rn(__fsub_rn(tab_cdf(t, step, jit), cl), __fsub_rn(T.cdf_hi[b], cl));
   return __fmaf_rn(u, __fsub_rn(T.hi[b], T.lo[b]), T.lo[b]);
 }
 
 // z_low of bin b's closing segment: its last step's z, or its min depth
-__device__ __forceinline__ float tab_zlow_close(const RayTab &T, int b, float step) {
-  return T.sf[b + 1] > T.sf[b] ? tab_z(T, T.sf[b + 1] - 1, b, step) : T.lo[b];
+template <typename J>
+__device__ __forceinline__ float tab_zlow_close(const RayTab &T, int b, float step, const J &jit) {
+  return T.sf[b + 1] > T.sf[b] ? tab_z(T, T.sf[b + 1] - 1, b, step, jit) : T.lo[b];
 }
 
 struct WarpRay {
@@ -310,50 +322,69 @@ struct WarpRay {
   bool done;
 };
 
-// Builds the ray's table (all 32 lanes; returns the same WarpRay on every
-// lane). B == 0 (an empty first slot) is left to the caller.
-__device__ __forceinline__ WarpRay build_tab(RayTab &T, int H, const int32_t *__restrict__ I,
-                                             const float *__restrict__ lo,
-                                             const float *__restrict__ hi,
-                                             const float *__restrict__ pr, float steps, int lane) {
+// Loads the row's slots into the table; returns the number of valid bins
+// (ids before the first -1) on every lane.
+__device__ __forceinline__ int load_tab(RayTab &T, int H, const int32_t *__restrict__ I,
+                                        const float *__restrict__ lo,
+                                        const float *__restrict__ hi, int lane) {
   for (int b = lane; b < H; b += 32) { T.id[b] = I[b]; T.lo[b] = lo[b]; T.hi[b] = hi[b]; }
   __syncwarp();
-  WarpRay w;
-  w.step = __double2float_rn(__ddiv_rn(1.0, (double)steps));
-  w.total = (int)ceilf(steps);
-  int B = H;
   for (int b0 = 0; b0 < H; b0 += 32) {
     uint32_t m = __ballot_sync(0xffffffffu, b0 + lane < H && T.id[b0 + lane] == -1);
-    if (m) { B = b0 + __ffs(m) - 1; break; }
+    if (m) return b0 + __ffs(m) - 1;
   }
+  return H;
+}
+
+// Fills the rest of the table of a row of B valid bins (loaded by load_tab)
+// walked in `total` steps of `step` (all 32 lanes; the same WarpRay on every
+// lane). B == 0 (an empty first slot) is left to the caller.
+template <typename J>
+__device__ __forceinline__ WarpRay build_tab(RayTab &T, int B, const float *__restrict__ pr,
+                                             float step, int total, int lane, const J &jit) {
+  WarpRay w;
+  w.step = step;
+  w.total = total;
   w.B = B;
-  if (lane == 0) {
-    float c = pr[0];
-    if (B > 0) T.cdf_hi[0] = c;
-    for (int b = 1; b < B; ++b) { c = __fadd_rn(c, pr[b]); T.cdf_hi[b] = c; }
-    T.sf[0] = 0;
+  // the CDF bounds: one lane after the other adds its slot (the walk's order)
+  float c = 0.0f;
+  for (int b0 = 0; b0 < B; b0 += 32) {
+    const float v = b0 + lane < B ? pr[b0 + lane] : 0.0f;
+    const int n = B - b0 < 32 ? B - b0 : 32;
+    float mine = 0.0f;
+    for (int j = 0; j < n; ++j) {
+      const float x = __shfl_sync(0xffffffffu, v, j);
+      c = b0 + j == 0 ? x : __fadd_rn(c, x);
+      if (lane == j) mine = c;
+    }
+    if (b0 + lane < B) T.cdf_hi[b0 + lane] = mine;
   }
+  if (lane == 0) T.sf[0] = 0;
   __syncwarp();
   for (int b = lane; b < B; b += 32) {
+    // the first step past the bin's bound: cdf_t increases with t and t is
+    // about bound / step, from where a step or two settle it
     const float bound = T.cdf_hi[b];
-    int a = 0, e = w.total;
-    while (a < e) {
-      int mid = (a + e) >> 1;
-      if (tab_cdf(mid, w.step) <= bound) a = mid + 1;
-      else e = mid;
-    }
+    int a = (int)fminf(fmaxf(__fdiv_rn(bound, step), 0.0f), 1.0e9f);
+    a = a < total ? a : (total > 0 ? total : 0);
+    while (a > 0 && !(tab_cdf(a - 1, step, jit) <= bound)) --a;
+    while (a < total && tab_cdf(a, step, jit) <= bound) ++a;
     T.sf[b + 1] = a;
   }
   __syncwarp();
   int nb = 0;
   for (int b0 = 0; b0 < B; b0 += 32)
-    nb += __popc(__ballot_sync(0xffffffffu, b0 + lane < B && T.sf[b0 + lane + 1] < w.total));
+    nb += __popc(__ballot_sync(0xffffffffu, b0 + lane < B && T.sf[b0 + lane + 1] < total));
   for (int b = lane; b < nb; b += 32) T.end[b] = T.sf[b + 1] + b + 1;
   __syncwarp();
   w.nb = nb;
-  w.done = B > 0 && T.sf[B] < w.total;
+  w.done = B > 0 && T.sf[B] < total;
   w.M = B > 0 ? T.sf[B] + nb : 0;
   return w;
+}
+
+__device__ __forceinline__ float walk_step(float steps) {
+  return __double2float_rn(__ddiv_rn(1.0, (double)steps));
 }
 
 // Main-sequence sample j (0 <= j < M): voxel id, depth, distance, in two
@@ -369,19 +400,29 @@ struct TabStep {
   float z = 0.0f;
 };
 
-__device__ __forceinline__ TabStep tab_step(const RayTab &T, const WarpRay &w, int j) {
-  TabStep sp;
-  int a = 0, e = w.nb;
-  while (a < e) {
-    int mid = (a + e) >> 1;
-    if (T.end[mid] <= j) a = mid + 1;
-    else e = mid;
+// Bit k: sample j0 + k is a closing segment, with `cur` the bins closed before
+// j0. A bin's samples end with its closing segment, so the bin of lane k's
+// sample is cur plus the closings before it: one reduction for 32 samples in
+// place of a binary search each.
+__device__ __forceinline__ uint32_t closing_mask(const RayTab &T, const WarpRay &w, int j0, int cur,
+                                                 int lane) {
+  uint32_t m = 0;
+  if (cur + lane < w.nb) {
+    const int at = T.end[cur + lane] - 1 - j0;
+    if (at < 32) m = 1u << at;
   }
-  sp.b = a;
-  sp.closing = a < w.nb && j == T.end[a] - 1;
+  return __reduce_or_sync(0xffffffffu, m);
+}
+
+template <typename J>
+__device__ __forceinline__ TabStep tab_step(const RayTab &T, const WarpRay &w, int j, uint32_t closing,
+                                            int cur, int lane, const J &jit) {
+  TabStep sp;
+  sp.b = cur + __popc(closing & ((1u << lane) - 1u));
+  sp.closing = (closing >> lane) & 1u;
   if (!sp.closing) {
-    sp.st = j - a;
-    sp.z = tab_z(T, sp.st, a, w.step);
+    sp.st = j - sp.b;
+    sp.z = tab_z(T, sp.st, sp.b, w.step, jit);
   }
   return sp;
 }
@@ -404,17 +445,17 @@ __device__ __forceinline__ void tab_finish(const RayTab &T, const WarpRay &w, co
 }
 
 // The tail loop of the walk from its end state, calling emit(id, t, dist).
-template <typename Emit>
+template <typename Emit, typename J>
 __device__ __forceinline__ void tab_tail(const RayTab &T, const WarpRay &w, int H,
                                          const int32_t *__restrict__ I0,
                                          const int32_t *__restrict__ pts_all, int64_t nxt,
-                                         Emit &emit) {
+                                         Emit &emit, const J &jit) {
   int bin;
   float cmax, z_low;
   if (w.done) {
-    bin = w.B; cmax = T.hi[w.B - 1]; z_low = tab_zlow_close(T, w.B - 1, w.step);
+    bin = w.B; cmax = T.hi[w.B - 1]; z_low = tab_zlow_close(T, w.B - 1, w.step, jit);
   } else if (w.total > 0) {
-    bin = w.nb; cmax = T.hi[w.nb]; z_low = tab_z(T, w.total - 1, w.nb, w.step);
+    bin = w.nb; cmax = T.hi[w.nb]; z_low = tab_z(T, w.total - 1, w.nb, w.step, jit);
   } else {
     bin = 0; cmax = T.hi[0]; z_low = T.lo[0];
   }
@@ -488,10 +529,13 @@ __device__ __forceinline__ void warp_write_samples(
   // one bin: lane - 1 computed it (lane 31 of the previous round for lane
   // 0), so each step's division runs once.
   float z_last = 0.0f;
+  int cur = 0;
   for (int j0 = 0; j0 < w.M; j0 += 32) {
     const int j = j0 + lane;
+    const uint32_t closing = closing_mask(T, w, j0, cur, lane);
     TabStep sp;
-    if (j < w.M) sp = tab_step(T, w, j);
+    if (j < w.M) sp = tab_step(T, w, j, closing, cur, lane, HalfJitter());
+    cur += __popc(closing);
     float z_prev = __shfl_up_sync(0xffffffffu, sp.z, 1);
     if (lane == 0) z_prev = z_last;
     z_last = __shfl_sync(0xffffffffu, sp.z, 31);
@@ -511,7 +555,7 @@ __device__ __forceinline__ void warp_write_samples(
   if (lane == 0) {
     TailWrite tw{vox, xyzd, depth, ox, oy, oz, dx, dy, dz, base + w.M, lim, false};
     if (base + w.M > lim) tw.over = true;
-    tab_tail(T, w, H, pts_idx + tail * H, pts_idx, nxt, tw);
+    tab_tail(T, w, H, pts_idx + tail * H, pts_idx, nxt, tw, HalfJitter());
     if ((tw.over || tw.pos != end || end > sample_cap) && err) atomicOr(err, 2);
   }
 }
@@ -533,7 +577,7 @@ __device__ __forceinline__ int warp_count_samples(const RayTab &T, const WarpRay
       n = em.n;
     } else {
       TailCount tc{0};
-      tab_tail(T, w, H, pts_idx + tail * H, pts_idx, nxt, tc);
+      tab_tail(T, w, H, pts_idx + tail * H, pts_idx, nxt, tc, HalfJitter());
       n = w.M + tc.n;
     }
   }
@@ -567,9 +611,9 @@ __global__ void __launch_bounds__(32 * kWarpRays) icdf_warp_kernel(
     }
     int64_t tail, nxt;
     row_layout(r, K, C, N, G, piece_rows, max_pieces, tail, nxt);
-    const int32_t *I = pts_idx + r * H;
-    WarpRay w = build_tab(T, H, I, min_depth + r * H, max_depth + r * H, probs + r * H,
-                          steps[r], lane);
+    const int B = load_tab(T, H, pts_idx + r * H, min_depth + r * H, max_depth + r * H, lane);
+    const WarpRay w = build_tab(T, B, probs + r * H, walk_step(steps[r]), (int)ceilf(steps[r]),
+                                lane, HalfJitter());
     if (!WRITE) {
       const int n = warp_count_samples(T, w, H, r, tail, nxt, lane, pts_idx, min_depth,
                                        max_depth, probs, steps);
@@ -581,6 +625,100 @@ __global__ void __launch_bounds__(32 * kWarpRays) icdf_warp_kernel(
     }
     __syncwarp();                          // the table is rebuilt for the next ray
   }
+}
+
+// The padded [rows, M] outputs of the reference op, a warp per row: the
+// closed form above, 32 consecutive samples at a time, written coalesced.
+// Bound by instruction issue (the closed form's division), then by the
+// padded rows' stores. A thread per row wrote 12 bytes here and there in its
+// own row, and 8,192 rows are 64 such blocks for 152 SMs: 120,000 rows of 64
+// slots and 320 columns 0.95 -> 0.22 ms, 8,192 rows with jitter 190 -> 25 us.
+// The closed form needs a CDF that does not decrease and jitter in [0, 1]; a
+// row that has neither (or whose steps exceed its columns, where the walk
+// stops in the middle) is walked by one lane.
+struct PadTail {
+  int32_t *SI;
+  float *SD, *SS;
+  int M, s, valid;
+  bool over;
+  __device__ void operator()(int32_t id, float t, float dist) {
+    if (s >= M) { over = true; return; }
+    SI[s] = id; SD[s] = t; SS[s] = dist;
+    valid += (id != -1);
+    ++s;
+  }
+};
+
+__global__ void __launch_bounds__(32 * kWarpRays) inverse_cdf_warp_kernel(
+    int64_t rows, int H, int M, int noise_stride, float fixed_step_size,
+    const int32_t *__restrict__ pts_idx, const float *__restrict__ min_depth,
+    const float *__restrict__ max_depth, const float *__restrict__ noise,
+    const float *__restrict__ probs, const float *__restrict__ steps, int64_t K, int64_t C,
+    int64_t N, int64_t G, int32_t *__restrict__ s_idx, float *__restrict__ s_depth,
+    float *__restrict__ s_dist, int32_t *__restrict__ max_len, int32_t *__restrict__ err) {
+  __shared__ RayTab tabs[kWarpRays];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  RayTab &T = tabs[wib];
+  const int64_t stride = (int64_t)gridDim.x * kWarpRays;
+  int longest = 0;
+  for (int64_t r = (int64_t)blockIdx.x * kWarpRays + wib; r < rows; r += stride) {
+    int64_t tail, nxt;
+    icdf_rows(r, K, C, N, G, tail, nxt);
+    const int32_t *I0 = pts_idx + tail * H;
+    const float *pr = probs + r * H;
+    const RowJitter jit{noise ? noise + r * noise_stride : nullptr};
+    PadTail em{s_idx + r * M, s_depth + r * M, s_dist + r * M, M, 0, 0, false};
+    const int B = load_tab(T, H, pts_idx + r * H, min_depth + r * H, max_depth + r * H, lane);
+    const int total = max((int)ceilf(steps[r]), 0);
+    const float step = fixed_step_size > 0.0f ? fixed_step_size : walk_step(steps[r]);
+    bool fine = B > 0 && total <= M && (!noise || total <= noise_stride);
+    if (fine) {
+      bool ok = total == 0 || isfinite(step);
+      for (int b = lane; b < B; b += 32) ok = ok && pr[b] >= 0.0f;
+      if (noise)
+        for (int t = lane; t < total; t += 32) ok = ok && jit.U[t] >= 0.0f && jit.U[t] <= 1.0f;
+      fine = __all_sync(0xffffffffu, ok);
+    }
+    if (fine) {
+      const WarpRay w = build_tab(T, B, pr, step, total, lane, jit);
+      const int n = min(w.M, M);
+      float z_last = 0.0f;
+      int cur = 0;
+      for (int j0 = 0; j0 < n; j0 += 32) {
+        const int j = j0 + lane;
+        const uint32_t closing = closing_mask(T, w, j0, cur, lane);
+        TabStep sp;
+        if (j < n) sp = tab_step(T, w, j, closing, cur, lane, jit);
+        cur += __popc(closing);
+        float z_prev = __shfl_up_sync(0xffffffffu, sp.z, 1);
+        if (lane == 0) z_prev = z_last;
+        z_last = __shfl_sync(0xffffffffu, sp.z, 31);
+        if (j < n) {
+          int32_t id;
+          float t, dist;
+          tab_finish(T, w, sp, z_prev, id, t, dist);
+          em.SI[j] = id; em.SD[j] = t; em.SS[j] = dist;
+        }
+      }
+      em.s = em.valid = n;
+      em.over = w.M > M;
+      if (lane == 0 && !em.over) tab_tail(T, w, H, I0, pts_idx, nxt, em, jit);
+    } else if (lane == 0) {
+      RowEmit re{em.SI, em.SD, em.SS, M, 0, 0};
+      em.over = icdf_walk(H, pts_idx + r * H, I0, pts_idx, nxt, min_depth + r * H,
+                          max_depth + r * H, pr, steps[r], jit.U, noise_stride, fixed_step_size,
+                          re);
+      em.s = re.s;
+      em.valid = re.valid;
+    }
+    if (lane == 0 && em.over && err) atomicOr(err, 2);
+    longest = max(longest, em.valid);                 // lane 0's counts
+    for (int q = __shfl_sync(0xffffffffu, em.s, 0) + lane; q < M; q += 32) {
+      em.SI[q] = -1; em.SD[q] = 0.0f; em.SS[q] = 0.0f;
+    }
+    __syncwarp();                                     // the table is rebuilt for the next row
+  }
+  if (lane == 0 && max_len) atomicMax(max_len, longest);
 }
 
 int scan_sms() {
@@ -663,8 +801,9 @@ __global__ void __launch_bounds__(32 * kScanWarps) icdf_scan_kernel(
     int n = 0;
     if (r < rows) {
       row_layout(r, K, C, N, G, piece_rows, max_pieces, tail, nxt);
-      w = build_tab(T, H, pts_idx + r * H, min_depth + r * H, max_depth + r * H, probs + r * H,
-                    steps[r], lane);
+      const int B = load_tab(T, H, pts_idx + r * H, min_depth + r * H, max_depth + r * H, lane);
+      w = build_tab(T, B, probs + r * H, walk_step(steps[r]), (int)ceilf(steps[r]), lane,
+                    HalfJitter());
       n = warp_count_samples(T, w, H, r, tail, nxt, lane, pts_idx, min_depth, max_depth, probs,
                              steps);
     }
@@ -723,14 +862,16 @@ __global__ void __launch_bounds__(32 * kScanWarps) icdf_scan_kernel(
 // Uniform sampler (fairnr/clib/src/sample_gpu.cu:15-106): merge interval
 // starts, interval ends and jittered steps into one sorted depth list in the
 // output row, then turn it into midpoints/lengths and keep those inside a
-// voxel, compacting in place.
-__global__ void __launch_bounds__(kBlock) uniform_kernel(
-    int64_t rows, int H, int M, float step_size, const int32_t *__restrict__ pts_idx,
-    const float *__restrict__ min_depth, const float *__restrict__ max_depth,
-    const float *__restrict__ noise, int32_t *__restrict__ s_idx, float *__restrict__ s_depth,
-    float *__restrict__ s_dist, int32_t *__restrict__ err) {
-  int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-  if (r >= rows) return;
+// voxel, compacting in place. Returns true when the row has no room for the
+// whole list.
+__device__ __forceinline__ bool uniform_walk(int64_t r, int H, int M, float step_size,
+                                             const int32_t *__restrict__ pts_idx,
+                                             const float *__restrict__ min_depth,
+                                             const float *__restrict__ max_depth,
+                                             const float *__restrict__ noise,
+                                             int32_t *__restrict__ s_idx,
+                                             float *__restrict__ s_depth,
+                                             float *__restrict__ s_dist) {
   const int32_t *I = pts_idx + r * H;
   const float *lo = min_depth + r * H, *hi = max_depth + r * H;
   const float *U = noise + r * M;
@@ -777,7 +918,231 @@ __global__ void __launch_bounds__(kBlock) uniform_kernel(
     }
   }
   for (int q = step; q < M; ++q) SI[q] = -1;
-  if (overflow && err) atomicOr(err, 2);
+  return overflow;
+}
+
+__global__ void __launch_bounds__(kBlock) uniform_kernel(
+    int64_t rows, int H, int M, float step_size, const int32_t *__restrict__ pts_idx,
+    const float *__restrict__ min_depth, const float *__restrict__ max_depth,
+    const float *__restrict__ noise, int32_t *__restrict__ s_idx, float *__restrict__ s_depth,
+    float *__restrict__ s_dist, int32_t *__restrict__ err) {
+  int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+  if (r >= rows) return;
+  if (uniform_walk(r, H, M, step_size, pts_idx, min_depth, max_depth, noise, s_idx, s_depth,
+                   s_dist) &&
+      err)
+    atomicOr(err, 2);
+}
+
+__device__ __forceinline__ int warp_min_scan(int x, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x = min(x, y);
+  }
+  return x;
+}
+
+// The same rows, a warp per row: a thread per row leaves a small batch on a
+// few SMs, in one serial chain of loads and 12-byte stores a row (1,070 rows
+// of 20 slots and 151 columns: 119 -> 6 us). Latency-bound at that size.
+//
+// The merge. With B valid slots whose starts lo and ends hi do not decrease
+// and steps u_t that do not either, the walk's list is all ends, steps and
+// starts by value, ties in that order, up to the last end: an end's place is
+// its own index plus the steps and the starts below it, a start's its index
+// plus the ends and the steps not above it, and the steps fill the places in
+// between. The places of ends and starts are found once (uniform_steps_below:
+// a guess and a step or two); 32 places at a time, two bit masks tell each
+// lane what its event is.
+//
+// The second pass. Segment e lies between events e and e + 1. The walk keeps
+// umin and umax, which grow by at most one a segment towards n_e, the number
+// of starts (ends) not above the segment's midpoint: umin_e = min(umin_(e-1)
+// + 1, n_e), which is e plus the running minimum of n_e - e (a warp scan). It
+// stops before the first segment whose next event has no id and after the
+// first one with umax_e = B, and leaves midpoints and lengths behind the kept
+// ones, as the reference does.
+//
+// Rows that are not in this form (unsorted or NaN depths, jitter outside [0,
+// 1], misses that sort before the last end, no room for the steps) are
+// walked by one lane.
+__device__ __forceinline__ int uniform_steps_below(const float *__restrict__ U, float lo0,
+                                                   float step, int limit, float v, bool equal) {
+  int a = (int)fminf(fmaxf(__fdiv_rn(__fsub_rn(v, lo0), step), 0.0f), 1.0e9f);
+  a = a < limit ? a : limit;
+  auto below = [&](int t) {
+    const float c = __fmaf_rn(__fadd_rn((float)t, U[t]), step, lo0);
+    return equal ? c <= v : c < v;
+  };
+  while (a > 0 && !below(a - 1)) --a;
+  while (a < limit && below(a)) ++a;
+  return a;
+}
+
+struct UniRow {
+  float lo[kMaxH], hi[kMaxH];
+  int32_t id[kMaxH];
+  int at_lo[kMaxH], at_hi[kMaxH];   // places in the merged list
+};
+
+__global__ void __launch_bounds__(32 * kWarpRays) uniform_warp_kernel(
+    int64_t rows, int H, int M, float step_size, const int32_t *__restrict__ pts_idx,
+    const float *__restrict__ min_depth, const float *__restrict__ max_depth,
+    const float *__restrict__ noise, int32_t *__restrict__ s_idx, float *__restrict__ s_depth,
+    float *__restrict__ s_dist, int32_t *__restrict__ err) {
+  __shared__ UniRow tabs[kWarpRays];
+  const uint32_t full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const uint32_t below = (1u << lane) - 1u;
+  UniRow &T = tabs[wib];
+  const int64_t stride = (int64_t)gridDim.x * kWarpRays;
+  for (int64_t r = (int64_t)blockIdx.x * kWarpRays + wib; r < rows; r += stride) {
+    const float *U = noise + r * M;
+    int32_t *SI = s_idx + r * M;
+    float *SD = s_depth + r * M, *SS = s_dist + r * M;
+    __syncwarp();                            // the table of the previous row is done with
+    for (int b = lane; b < H; b += 32) {
+      T.id[b] = pts_idx[r * H + b];
+      T.lo[b] = min_depth[r * H + b];
+      T.hi[b] = max_depth[r * H + b];
+    }
+    __syncwarp();
+    int B = H;
+    for (int b0 = 0; b0 < H; b0 += 32) {
+      const uint32_t m = __ballot_sync(full, b0 + lane < H && T.id[b0 + lane] == -1);
+      if (m) { B = b0 + __ffs(m) - 1; break; }
+    }
+    int E = 0, limit = 0;                    // events; steps looked at
+    bool fine = true, over = false;
+    const float lo0 = T.lo[0];
+    if (B > 0) {
+      const float last = T.hi[B - 1];
+      bool ok = step_size > 0.0f && isfinite(step_size) && fabsf(lo0) < 1.0e30f &&
+                last <= 10000.0f && (B == H || T.lo[B] >= last);
+      for (int b = lane; b < B; b += 32)
+        ok = ok && T.id[b] >= 0 && T.lo[b] >= (b ? T.lo[b - 1] : lo0) &&
+             T.hi[b] >= (b ? T.hi[b - 1] : T.hi[0]);
+      const float span = __fdiv_rn(__fsub_rn(last, lo0), step_size);
+      limit = span < (float)(M - 4) ? (int)fmaxf(span, 0.0f) + 3 : M;
+      limit = limit < M ? limit : M;
+      for (int t = lane; t < limit; t += 32) ok = ok && U[t] >= 0.0f && U[t] <= 1.0f;
+      // some step lies past the last end
+      ok = ok && __fmaf_rn(__fadd_rn((float)(limit - 1), U[limit - 1]), step_size, lo0) > last;
+      fine = __all_sync(full, ok);
+      if (fine) {
+        for (int b = lane; b < B; b += 32) {
+          const float v = T.hi[b], u = T.lo[b];
+          int n = 0, m = 0;                  // starts below this end, ends not above this start
+          for (int k = 0; k < B; ++k) {
+            n += T.lo[k] < v;
+            m += T.hi[k] <= u;
+          }
+          T.at_hi[b] = b + n + uniform_steps_below(U, lo0, step_size, limit, v, false);
+          T.at_lo[b] = b + m + uniform_steps_below(U, lo0, step_size, limit, u, true);
+        }
+        __syncwarp();
+        E = T.at_hi[B - 1] + 1;
+        over = E > M;
+        E = min(E, M);
+      }
+    }
+    if (!fine) {
+      if (lane == 0)
+        over = uniform_walk(r, H, M, step_size, pts_idx, min_depth, max_depth, noise, s_idx,
+                            s_depth, s_dist);
+      if (lane == 0 && over && err) atomicOr(err, 2);
+      continue;
+    }
+    // event e of the merged list: value and id (-1 past the list), with i
+    // ends and j starts before the 32 events from e0
+    int ci = 0, cj = 0;
+    auto events = [&](int e0, float &val, int32_t &id, int &n_hi, int &n_lo) {
+      uint32_t mi = 0, mj = 0;
+      if (ci + lane < B) {
+        const int at = T.at_hi[ci + lane] - e0;
+        if (at < 32) mi = 1u << at;
+      }
+      if (cj + lane < B) {
+        const int at = T.at_lo[cj + lane] - e0;
+        if (at < 32) mj = 1u << at;
+      }
+      mi = __reduce_or_sync(full, mi);
+      mj = __reduce_or_sync(full, mj);
+      const int i = ci + __popc(mi & below), j = cj + __popc(mj & below), e = e0 + lane;
+      const bool is_hi = (mi >> lane) & 1u, is_lo = (mj >> lane) & 1u;
+      val = 0.0f;
+      id = -1;
+      if (e < E) {
+        if (is_hi) {
+          val = T.hi[i];
+          id = T.id[i];
+        } else if (is_lo) {
+          val = T.lo[j];
+          id = T.id[j];
+        } else {
+          const int t = e - i - j;
+          val = __fmaf_rn(__fadd_rn((float)t, U[t]), step_size, lo0);
+          // before the first start (a jitter of exactly 0) the reference reads
+          // the element before the row
+          id = j > 0 ? T.id[j - 1] : (r > 0 ? pts_idx[r * H - 1] : -1);
+        }
+      }
+      n_hi = i + is_hi;                      // ends and starts among events 0..e
+      n_lo = j + is_lo;
+      ci += __popc(mi);
+      cj += __popc(mj);
+    };
+    float val, nval;
+    int32_t id, nid;
+    int n_hi, n_lo, nn_hi, nn_lo;
+    int lo_min = 1, hi_min = 1;              // running minima of n_e - e
+    int kept = 0;
+    bool stopped = false;
+    events(0, val, id, n_hi, n_lo);
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      events(e0 + 32, nval, nid, nn_hi, nn_lo);
+      const int e = e0 + lane;
+      float rv = __shfl_down_sync(full, val, 1);
+      int32_t rid = __shfl_down_sync(full, id, 1);
+      const float v0 = __shfl_sync(full, nval, 0);
+      const int32_t id0 = __shfl_sync(full, nid, 0);
+      if (lane == 31) { rv = v0; rid = id0; }
+      const float mid = __fmul_rn(__fadd_rn(val, rv), 0.5f), len = __fsub_rn(rv, val);
+      if (e < E) {
+        while (n_lo < B && mid >= T.lo[n_lo]) ++n_lo;
+        while (n_hi < B && mid >= T.hi[n_hi]) ++n_hi;
+      }
+      const int a = min(warp_min_scan(n_lo - e, lane), lo_min);
+      const int c = min(warp_min_scan(n_hi - e, lane), hi_min);
+      lo_min = __shfl_sync(full, a, 31);
+      hi_min = __shfl_sync(full, c, 31);
+      const int umin = a + e, umax = c + e;
+      const bool before = stopped || rid == -1 || e >= M - 1;   // not processed
+      const bool after = umax == B;                             // processed, not kept
+      const uint32_t stops = __ballot_sync(full, before || after);
+      const int first = stops ? __ffs(stops) - 1 : 32;
+      const bool done = lane < first || (lane == first && !before);
+      const bool keep = lane < first && umin - 1 == umax && len > 0.0f;
+      if (e < M) {
+        SI[e] = -1;
+        SD[e] = done ? mid : val;
+        SS[e] = done ? len : 0.0f;
+      }
+      __syncwarp();
+      const uint32_t km = __ballot_sync(full, keep);
+      if (keep) {
+        const int q = kept + __popc(km & below);
+        SI[q] = id; SD[q] = mid; SS[q] = len;
+      }
+      kept += __popc(km);
+      stopped = stopped || stops != 0;
+      __syncwarp();
+      val = nval; id = nid; n_hi = nn_hi; n_lo = nn_lo;
+    }
+    for (int q = (E + 31) / 32 * 32 + lane; q < M; q += 32) { SI[q] = -1; SD[q] = 0.0f; SS[q] = 0.0f; }
+    if (lane == 0 && over && err) atomicOr(err, 2);
+  }
 }
 
 // Parallel uniform sampler: the pure-torch backup sampler of the reference's
@@ -971,9 +1336,15 @@ int nsvf_inverse_cdf_sampling(int64_t rows, int max_hits, int max_steps, int noi
   int64_t K = layout[0], C = layout[1], N = layout[2], G = layout[3];
   if (K < 1 || C < 1 || N < rows || G < 1 || G * K < N) return NSVF_ERR_INVALID;
   if (rows == 0) return NSVF_OK;
-  inverse_cdf_kernel<<<nsvf_grid(rows, kBlock), kBlock, 0, (cudaStream_t)stream>>>(
-      rows, max_hits, max_steps, noise_stride, fixed_step_size, pts_idx, min_depth, max_depth,
-      noise, probs, steps, K, C, N, G, sampled_idx, sampled_depth, sampled_dists, max_len, err);
+  // (rows of more than kMaxH slots don't fit the warp's table)
+  if (max_hits <= kMaxH)
+    inverse_cdf_warp_kernel<<<warp_grid(rows), 32 * kWarpRays, 0, (cudaStream_t)stream>>>(
+        rows, max_hits, max_steps, noise_stride, fixed_step_size, pts_idx, min_depth, max_depth,
+        noise, probs, steps, K, C, N, G, sampled_idx, sampled_depth, sampled_dists, max_len, err);
+  else
+    inverse_cdf_kernel<<<nsvf_grid(rows, kBlock), kBlock, 0, (cudaStream_t)stream>>>(
+        rows, max_hits, max_steps, noise_stride, fixed_step_size, pts_idx, min_depth, max_depth,
+        noise, probs, steps, K, C, N, G, sampled_idx, sampled_depth, sampled_dists, max_len, err);
   return nsvf_launch_status();
 }
 
@@ -1162,9 +1533,15 @@ int nsvf_uniform_ray_sampling(int b, int m, int max_hits, int max_steps, float s
     return NSVF_ERR_INVALID;
   int64_t rows = (int64_t)b * m;
   if (rows == 0) return NSVF_OK;
-  uniform_kernel<<<nsvf_grid(rows, kBlock), kBlock, 0, (cudaStream_t)stream>>>(
-      rows, max_hits, max_steps, step_size, pts_idx, min_depth, max_depth, noise, sampled_idx,
-      sampled_depth, sampled_dists, err);
+  // (rows of more than kMaxH slots don't fit the warp's table)
+  if (max_hits <= kMaxH)
+    uniform_warp_kernel<<<warp_grid(rows), 32 * kWarpRays, 0, (cudaStream_t)stream>>>(
+        rows, max_hits, max_steps, step_size, pts_idx, min_depth, max_depth, noise, sampled_idx,
+        sampled_depth, sampled_dists, err);
+  else
+    uniform_kernel<<<nsvf_grid(rows, kBlock), kBlock, 0, (cudaStream_t)stream>>>(
+        rows, max_hits, max_steps, step_size, pts_idx, min_depth, max_depth, noise, sampled_idx,
+        sampled_depth, sampled_dists, err);
   return nsvf_launch_status();
 }
 

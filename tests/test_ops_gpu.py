@@ -415,3 +415,108 @@ def test_sample_compact_matches_inverse_cdf_op(cuda, case):
     row = torch.arange(n, device=cuda)[:, None].expand_as(si)[valid]
     xyz = ro[row] + rd[row] * sd[valid][:, None]
     assert torch.equal(xyzd[:, :3], xyz)
+
+
+@pytest.mark.parametrize("H", [1, 31, 33, 64, 127])
+@pytest.mark.parametrize("form", ["half", "jitter", "wild_noise", "wild_probs", "narrow",
+                                  "fixed_step"])
+def test_inverse_cdf_warp_rows_equal_thread_rows(cuda, H, form):
+    """Rows of up to 128 slots are sampled by a warp each, wider ones by a
+    thread: the same rows padded with misses to 130 slots give the same
+    samples, over every form the op takes (jitter outside [0, 1], NaN and
+    negative probabilities, too few columns, empty rows, a fixed step).
+    (Rows that fill all H slots read on into the next row, so they keep one
+    miss here.)"""
+    from nsvf_gb300 import ext
+    rows = 333
+    idx, lo, hi, probs, steps = _random_intervals(rows, H, seed=H + 7)
+    idx[:, -1] = -1
+    idx[::50] = -1
+    rng = np.random.RandomState(H)
+    fixed = 0.013 if form == "fixed_step" else -1.0
+    if form == "wild_probs":
+        probs[::3] *= rng.choice([-1.0, 1.0, np.nan], probs[::3].shape).astype(np.float32)
+        steps[::7] = np.nan
+        steps[1::7] = 1e-42
+        steps[2::7] = -3.0
+    M = 40 if form == "narrow" else int(np.nanmax(np.ceil(steps))) + H + 4
+    noise = None if form == "half" else rng.uniform(0.0, 1.0, (rows, M)).astype(np.float32)
+    if form == "wild_noise":
+        noise[::2] = rng.uniform(-3.0, 4.0, noise[::2].shape).astype(np.float32)
+        noise[::5, ::9] = np.nan
+
+    def run(pad):
+        p = lambda a, v: np.pad(a, ((0, 0), (0, pad)), constant_values=v)
+        ml = torch.zeros(1, dtype=torch.int32, device=cuda)
+        ext.error_word(cuda).zero_()
+        out = ext.inverse_cdf_sampling_rows(
+            _t(p(idx, -1), cuda), _t(p(lo, 10000.0), cuda), _t(p(hi, 10000.0), cuda),
+            _t(noise, cuda) if noise is not None else None, _t(p(probs, 0.0), cuda),
+            _t(steps, cuda), fixed, (2, 800, rows, 200), M, ml)
+        err = int(ext.error_word(cuda).item())
+        ext.error_word(cuda).zero_()
+        return [_np(o) for o in out] + [int(ml), err]
+
+    a, b = run(0), run(130 - H)
+    for x, y in zip(a[:3], b[:3]):
+        assert np.array_equal(x.view(np.int32), y.view(np.int32))
+    assert a[3:] == b[3:]
+    if form == "narrow" and H > 1:
+        assert a[4] & 2
+
+
+@pytest.mark.parametrize("H", [1, 31, 33, 64, 127])
+@pytest.mark.parametrize("form", ["contiguous", "gaps", "equal_depths", "edge_noise", "wild_noise",
+                                  "raw_misses", "unsorted", "narrow"])
+def test_uniform_warp_rows_equal_thread_rows(cuda, H, form):
+    """Rows of up to 128 slots are sampled by a warp each, wider ones by a
+    thread: the same rows padded with misses to 130 slots give the same whole
+    output rows (left-over depths included), over every form the op takes."""
+    from nsvf_gb300 import ext
+    rows, step = 217, 0.02
+    rng = np.random.RandomState(H)
+    idx, lo, hi, _, _ = _random_intervals(rows, H, seed=H + 3)
+    idx[:, -1] = -1
+    idx[::40] = -1
+    for r in range(rows):
+        n = int((idx[r] != -1).argmin()) if (idx[r] == -1).any() else H
+        if form != "unsorted" and n:
+            # intervals one after the other: touching, or with gaps
+            cut = np.sort(rng.uniform(1.0, 4.0, 2 * n).astype(np.float32))
+            if form == "equal_depths":
+                cut = np.sort(rng.choice(cut, cut.size))
+            lo[r, :n], hi[r, :n] = cut[0::2], cut[1::2]
+            if form == "contiguous":
+                lo[r, 1:n] = hi[r, :n - 1]
+        lo[r, n:] = hi[r, n:] = 0.0 if form == "raw_misses" else 10000.0
+    M = 60 if form == "narrow" else int(4.0 / step) + 2 * H + 3
+    noise = rng.rand(rows, M).astype(np.float32)
+    if form == "edge_noise":
+        noise = rng.choice(np.float32([0.0, 0.25, 0.5, 1.0]), (rows, M)).astype(np.float32)
+        lo, hi = (np.where(a < 9000, np.round(a / (step / 4)) * np.float32(step / 4), a)
+                  .astype(np.float32) for a in (lo, hi))
+    if form == "wild_noise":
+        noise[::2] = rng.uniform(-3.0, 4.0, noise[::2].shape)
+        noise[::5, ::9] = np.nan
+
+    def run(pad):
+        p = lambda a, v: np.pad(a, ((0, 0), (0, pad)), constant_values=v)[None]
+        ext.error_word(cuda).zero_()
+        out = ext.uniform_ray_sampling(_t(p(idx, -1), cuda),
+                                       _t(p(lo, 0.0 if form == "raw_misses" else 10000.0), cuda),
+                                       _t(p(hi, 0.0 if form == "raw_misses" else 10000.0), cuda),
+                                       _t(noise[None], cuda), step, M)
+        err = int(ext.error_word(cuda).item())
+        ext.error_word(cuda).zero_()
+        return [_np(o) for o in out] + [err]
+
+    a = run(0)
+    if form == "raw_misses":
+        # (misses at depth 0 sort before the hits: each one is an event, so
+        # padding changes the row's own result)
+        b = [*cpu.uniform_ray_sampling(idx[None], lo[None], hi[None], noise[None], step, M), 0]
+    else:
+        b = run(130 - H)
+    for x, y in zip(a[:3], b[:3]):
+        assert np.array_equal(x.view(np.int32), y.view(np.int32))
+    assert a[3] == b[3]
