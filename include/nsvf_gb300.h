@@ -55,6 +55,16 @@ int nsvf_aabb_intersect(int b, int b_pts, int n, int m, float voxelsize, int n_m
                         const float *ray_start, const float *ray_dir, const float *points,
                         int32_t *idx, float *min_depth, float *max_depth, void *stream);
 
+/* The same op with a workspace of nsvf_aabb_workspace_bytes (16-byte aligned)
+ * for one box per 32 consecutive voxels, which lets a ray skip the groups whose
+ * box it misses: the same hits, bit for bit. */
+int64_t nsvf_aabb_workspace_bytes(int b_pts, int n);
+int nsvf_aabb_intersect_boxes(int b, int b_pts, int n, int m, float voxelsize, int n_max,
+                              const float *ray_start, const float *ray_dir, const float *points,
+                              int32_t *idx, float *min_depth, float *max_depth, void *workspace,
+                              void *stream);
+
+
 /* svo_intersect: replaces `svo_intersect(ray_start, ray_dir, points,
  * children, voxelsize, n_max)` (fairnr/clib/src/intersect.cpp:84-112,
  * fairnr/clib/src/intersect_gpu.cu:170-237).

@@ -141,9 +141,13 @@ def aabb_intersect(ray_start, ray_dir, points, voxelsize, n_max):
     idx = torch.empty(B, M, n_max, dtype=torch.int32, device=dev)
     lo = torch.empty(B, M, n_max, dtype=torch.float32, device=dev)
     hi = torch.empty(B, M, n_max, dtype=torch.float32, device=dev)
-    check(LIB.nsvf_aabb_intersect(B, bp, N, M, float(voxelsize), int(n_max), _ptr(ray_start),
-                                  _ptr(ray_dir), _ptr(points), _ptr(idx), _ptr(lo), _ptr(hi),
-                                  _stream(ray_start)), "aabb_intersect")
+    # boxes of 32 voxels (nsvf_aabb_intersect_boxes)
+    ws = torch.empty(max(int(LIB.nsvf_aabb_workspace_bytes(bp, N)), 16), dtype=torch.uint8,
+                     device=dev)
+    check(LIB.nsvf_aabb_intersect_boxes(B, bp, N, M, float(voxelsize), int(n_max),
+                                        _ptr(ray_start), _ptr(ray_dir), _ptr(points), _ptr(idx),
+                                        _ptr(lo), _ptr(hi), _ptr(ws), _stream(ray_start)),
+          "aabb_intersect")
     return idx, lo, hi
 
 

@@ -520,3 +520,31 @@ def test_uniform_warp_rows_equal_thread_rows(cuda, H, form):
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x.view(np.int32), y.view(np.int32))
     assert a[3] == b[3]
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 256, 257, 1025, 3000])
+@pytest.mark.parametrize("order", ["grid", "random", "odd"])
+def test_aabb_boxes_equal_oracle(cuda, n, order):
+    """The brute-force op skips groups of 32 voxels whose box a ray misses:
+    the oracle's hits, for voxel lists in grid and in random order, NaN and
+    infinite centres, rays along the axes and grid planes and from inside."""
+    from nsvf_gb300 import ext
+    rng = np.random.RandomState(n)
+    vs, m = 0.05, 120
+    g = np.stack(np.meshgrid(*[np.arange(-20, 21)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pts = (g[np.linalg.norm(g, axis=1) < 12][:n] if order == "grid"
+           else g[rng.permutation(len(g))[:n]]).astype(np.float32) * np.float32(vs)
+    if order == "odd":
+        pts[::37, 0] = np.nan
+        pts[5::41, 1] = np.inf
+    o = rng.uniform(-1.5, 1.5, (1, m, 3)).astype(np.float32)
+    d = rng.normal(size=(1, m, 3)).astype(np.float32)
+    d /= np.linalg.norm(d, axis=-1, keepdims=True)
+    d[0, ::7, rng.randint(3)] = 0.0
+    d[0, 1::11] = np.float32([0, 0, -1])
+    o[0, 2::9] = np.round(o[0, 2::9] / (vs / 2)) * np.float32(vs / 2)
+    for n_max in (1, 20):
+        ref = cpu.aabb_intersect(o, d, pts[None], vs, n_max)
+        out = ext.aabb_intersect(_t(o, cuda), _t(d, cuda), _t(pts[None], cuda), vs, n_max)
+        for a, b in zip(out, ref):
+            assert np.array_equal(_np(a), b)
