@@ -79,6 +79,7 @@ int nsvf_aabb_intersect_boxes(int b, int b_pts, int n, int m, float voxelsize, i
  * outside [0, n), a cycle, or deeper than 36 levels); such rays stop early
  * instead of reading out of bounds (the reference asserts or faults). */
 int64_t nsvf_svo_workspace_bytes(int b_pts, int n);
+int64_t nsvf_svo_packed_bytes(int n);   /* of nsvf_svo_pack */
 int nsvf_svo_intersect(int b, int b_pts, int n, int m, float voxelsize, int n_max,
                        const float *ray_start, const float *ray_dir, const float *points,
                        const int32_t *children, int32_t *idx, float *min_depth,
@@ -86,7 +87,7 @@ int nsvf_svo_intersect(int b, int b_pts, int n, int m, float voxelsize, int n_ma
 
 /* svo_pack: writes the packed copy of ONE octree (points [n, 3], children
  * [n, 9]) that the sorted traversal reads into `workspace`
- * (nsvf_svo_workspace_bytes(1, n) bytes, 16-byte aligned), so that
+ * (nsvf_svo_packed_bytes(n) bytes, 16-byte aligned), so that
  * nsvf_svo_intersect_grid can reuse it across calls. The packing step of
  * fairnr/clib/__init__.py:101-111 (the reference copies the octree once per
  * ray block on every call). */

@@ -32,6 +32,7 @@ def _load():
         "nsvf_aabb_workspace_bytes": ([i32, i32], i64),
         "nsvf_aabb_intersect_boxes": ([i32, i32, i32, i32, f32, i32, P, P, P, P, P, P, P, P], i32),
         "nsvf_svo_workspace_bytes": ([i32, i32], i64),
+        "nsvf_svo_packed_bytes": ([i32], i64),
         "nsvf_svo_intersect": ([i32, i32, i32, i32, f32, i32, P, P, P, P, P, P, P, P, P, P], i32),
         "nsvf_svo_intersect_sorted": ([i32, i32, i32, i32, f32, i32, P, P, P, P, P, P, P, P, P,
                                        P, P], i32),
@@ -131,7 +132,7 @@ def exported_symbols():
     """Names declared in include/nsvf_gb300.h that the library must export."""
     return [
         "nsvf_status_string", "nsvf_launch_count", "nsvf_aabb_intersect", "nsvf_svo_workspace_bytes",
-        "nsvf_aabb_workspace_bytes", "nsvf_aabb_intersect_boxes",
+        "nsvf_aabb_workspace_bytes", "nsvf_aabb_intersect_boxes", "nsvf_svo_packed_bytes",
         "nsvf_svo_intersect", "nsvf_svo_intersect_sorted", "nsvf_svo_pack",
         "nsvf_svo_grid_build", "nsvf_svo_grid_info", "nsvf_svo_grid_list_bytes",
         "nsvf_svo_intersect_grid", "nsvf_svo_intersect_grid_rows", "nsvf_ball_intersect",

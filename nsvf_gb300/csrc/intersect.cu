@@ -195,6 +195,193 @@ __global__ void pack_octree_kernel(int64_t total, int n, float hv, const float *
   if (k == n - 1 && j == 0) B[(int64_t)n * 8] = node_box(P, C, n - 1, hv);
 }
 
+// The tight form of the packed octree, for the calls that traverse a tree once
+// (svo_launch with a workspace). A node's cube in the input reaches far beyond
+// its leaves (a frame's ray that hits the 125,476-voxel shell enters 311 nodes
+// to find 23 leaves), so a child's box here is the bounding box of its
+// leaves' faces: 69 nodes for such a ray, 1 instead of 14 for one that misses.
+//
+// Same hits, bit for bit. The search reports a leaf iff its own slab test and
+// every ancestor's hit. A leaf's box here is its own (its FP32 faces c - h, c +
+// h). For an internal node, the slab arithmetic is monotone in the face
+// coordinate (see common.cuh): a ray that hits a leaf hits any box whose faces
+// contain the leaf's, so skipping a node whose tight box is missed loses
+// nothing, and where the node's cube contains its tight box, hitting the
+// latter implies hitting the former. Where it does not (rounded centres of
+// non-dyadic voxels), the node keeps its cube. So do all nodes of an input
+// that is not a tree of at most 14 levels with ids in range (a node reached
+// twice, a cycle, an id >= n), so that what the search reports about it stays.
+//
+// Layout, per node: 12 float4 of boxes, children c and c + 4 paired: (lo_c,
+// lo_c+4, hi_c, hi_c+4) of x, y and z at tbox[12 k + 3 c ..]; 8 ids as in the
+// packed octree, a leaf's with kLeafBit, an id out of range as kBadId. Per set
+// two float4 with the root's box (the first's w < 0: the root is a leaf). Then
+// the links (parent * 8 + slot) and a flag, both -1 at first.
+constexpr int32_t kLeafBit = 1 << 30, kBadId = kLeafBit - 1;
+constexpr int kTightMaxNodes = 1 << 27;       // links are 32-bit
+constexpr int kTightMaxDepth = 14;
+
+struct TightOctree {
+  float4 *boxes, *root;
+  int32_t *kids, *link, *flag;
+};
+
+__host__ __device__ __forceinline__ TightOctree tight_view(void *ws, int64_t b_pts, int64_t n) {
+  TightOctree t;
+  t.boxes = (float4 *)ws;
+  t.root = t.boxes + b_pts * n * 12;
+  t.kids = (int32_t *)(t.root + b_pts * 2);
+  t.link = t.kids + b_pts * n * 8;
+  t.flag = t.link + b_pts * n;
+  return t;
+}
+
+// Float k (0..5: lo x y z, hi x y z) of child slot c of node k0 (in the set).
+__device__ __forceinline__ float *tight_face(float4 *boxes, int64_t node, int c, int f) {
+  return (float *)(boxes + node * 12 + 3 * (c & 3)) + (f % 3) * 4 + (f / 3) * 2 + (c >> 2);
+}
+
+// A box's FP32 faces: lo x y z, hi x y z
+__device__ __forceinline__ void box_faces(const float4 &b, float (&f)[6]) {
+  const float h = fabsf(b.w), c[3] = {b.x, b.y, b.z};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    f[d] = __fsub_rn(c[d], h);
+    f[3 + d] = __fadd_rn(c[d], h);
+  }
+}
+
+// Child ids, leaf boxes and links; empty boxes for internal children.
+__global__ void tight_link_kernel(int64_t total, int n, float hv, const float *__restrict__ points,
+                                  const int32_t *__restrict__ children, TightOctree t) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;   // (set, node, child)
+  if (q >= total * 8) return;
+  const int j = (int)(q & 7);
+  const int64_t gk = q >> 3, g = gk / n;
+  const int k = (int)(gk - g * n);
+  const int32_t *C = children + g * (int64_t)n * 9;
+  const float *P = points + g * (int64_t)n * 3;
+  const float inf = __int_as_float(0x7f800000);
+  const int cid = C[(int64_t)k * 9 + j];
+  float f[6] = {inf, inf, inf, -inf, -inf, -inf};
+  int id = -1;
+  if (cid >= n) {
+    id = kBadId;
+    atomicExch(t.flag + g, 0);
+  } else if (cid > -1) {
+    const float4 b = node_box(P, C, cid, hv);
+    id = cid;
+    if (b.w < 0.0f) {
+      id |= kLeafBit;
+      box_faces(b, f);
+    }
+    if (atomicCAS(t.link + g * n + cid, -1, k * 8 + j) != -1) atomicExch(t.flag + g, 0);
+  }
+#pragma unroll
+  for (int d = 0; d < 6; ++d) *tight_face(t.boxes, gk, j, d) = f[d];
+  t.kids[gk * 8 + 2 * (j & 3) + (j >> 2)] = id;
+  if (k == n - 1 && j == 0) {
+    const float4 b = node_box(P, C, n - 1, hv);
+    if (b.w < 0.0f) box_faces(b, f);
+    else { f[0] = f[1] = f[2] = inf; f[3] = f[4] = f[5] = -inf; }
+    t.root[g * 2] = make_float4(f[0], f[1], f[2], b.w < 0.0f ? -1.0f : 1.0f);
+    t.root[g * 2 + 1] = make_float4(f[3], f[4], f[5], 0.0f);
+  }
+}
+
+// Float minimum / maximum by the order of the bits (no NaN, no -0).
+__device__ __forceinline__ void atomic_fmin(float *a, float v) {
+  if (v >= 0.0f) atomicMin((int *)a, __float_as_int(v));
+  else atomicMax((unsigned *)a, __float_as_uint(v));
+}
+__device__ __forceinline__ void atomic_fmax(float *a, float v) {
+  if (v >= 0.0f) atomicMax((int *)a, __float_as_int(v));
+  else atomicMin((unsigned *)a, __float_as_uint(v));
+}
+
+// A thread per node walks to the root: every leaf widens its ancestors' boxes
+// until one already contains it (whoever widened that one carries it on), and
+// every node checks its depth.
+__global__ void tight_widen_kernel(int64_t total, int n, float hv, const float *__restrict__ points,
+                                   const int32_t *__restrict__ children, TightOctree t) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;   // (set, node)
+  if (q >= total) return;
+  const int64_t g = q / n;
+  const int i = (int)(q - g * n);
+  const int32_t *link = t.link + g * n;
+  const float4 b = node_box(points + g * (int64_t)n * 3, children + g * (int64_t)n * 9, i, hv);
+  bool widen = b.w < 0.0f;
+  float f[6];
+  box_faces(b, f);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (f[d] != f[d] || f[3 + d] != f[3 + d]) {          // a NaN axis counts as hit
+      f[d] = -__int_as_float(0x7f800000);
+      f[3 + d] = __int_as_float(0x7f800000);
+    }
+    f[d] = __fadd_rn(f[d], 0.0f);
+    f[3 + d] = __fadd_rn(f[3 + d], 0.0f);
+  }
+  int node = i, depth = 0;
+  while (link[node] >= 0 && depth <= kTightMaxDepth) {
+    node = link[node] >> 3;
+    ++depth;
+    const int up = link[node];
+    // below a leaf, or not below the root: never visited
+    if (up >= 0 ? (t.kids[(g * n + (up >> 3)) * 8 + 2 * (up & 3) + ((up >> 2) & 1)] & kLeafBit) != 0
+                : node != n - 1 || t.root[g * 2].w < 0.0f)
+      break;
+    if (!widen) continue;
+    widen = false;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+      float *a = up >= 0 ? tight_face(t.boxes, g * n + (up >> 3), up & 7, d)
+                         : (float *)(t.root + g * 2 + d / 3) + d % 3;
+      const float v = *(volatile float *)a;
+      if (d < 3 ? f[d] < v : f[d] > v) {
+        if (d < 3) atomic_fmin(a, f[d]);
+        else atomic_fmax(a, f[d]);
+        widen = true;
+      }
+    }
+  }
+  if (depth > kTightMaxDepth || (i == n - 1 && link[i] >= 0)) atomicExch(t.flag + g, 0);
+}
+
+// Internal nodes whose cube does not contain their tight box, and all of a
+// flagged set, keep the cube.
+__global__ void tight_check_kernel(int64_t total, int n, float hv, const float *__restrict__ points,
+                                   const int32_t *__restrict__ children, TightOctree t) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;   // (set, node)
+  if (q >= total) return;
+  const int64_t g = q / n;
+  const int i = (int)(q - g * n);
+  const int32_t *C = children + g * (int64_t)n * 9;
+  const float *P = points + g * (int64_t)n * 3;
+  const bool flagged = t.flag[g] >= 0;
+  auto fix = [&](const float4 &b, auto face) {
+    float f[6];
+    box_faces(b, f);
+    bool inside = !flagged;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) inside = inside && *face(d) >= f[d] && *face(3 + d) <= f[3 + d];
+    if (!inside) {
+#pragma unroll
+      for (int d = 0; d < 6; ++d) *face(d) = f[d];
+    }
+  };
+  for (int j = 0; j < 8; ++j) {
+    const int cid = C[(int64_t)i * 9 + j];
+    if (cid < 0 || cid >= n) continue;
+    const float4 b = node_box(P, C, cid, hv);
+    if (!(b.w < 0.0f)) fix(b, [&](int d) { return tight_face(t.boxes, q, j, d); });
+  }
+  if (i == n - 1) {
+    const float4 b = node_box(P, C, i, hv);
+    if (!(b.w < 0.0f)) fix(b, [&](int d) { return (float *)(t.root + g * 2 + d / 3) + d % 3; });
+  }
+}
+
 constexpr int kSvoLevels = 16;
 constexpr int kLanesPerRay = 4;                       // lane j owns children j and j + 4
 static_assert(kLanesPerRay == 4, "the packed octree pairs children c and c + 4 for one lane");
@@ -348,11 +535,59 @@ __device__ __forceinline__ void slab_fast_pair(float ox, float oy, float oz, flo
   }
 }
 
-template <bool SORTED>
+// The slab tests on a box's faces: the same values as from its centre and
+// half size, whose faces these are.
+__device__ __forceinline__ bool slab_faces(float ox, float oy, float oz, float ix, float iy,
+                                           float iz, const float (&f)[6], float &t_lo,
+                                           float &t_hi) {
+  float lo = 0.0f, hi = 100000.0f;
+  auto axis = [&](float a, float b, float o, float inv) {
+    float l = __fmul_rn(__fsub_rn(a, o), inv), u = __fmul_rn(__fsub_rn(b, o), inv);
+    if (u < l) { const float t = l; l = u; u = t; }
+    lo = (l > lo) ? l : lo;
+    hi = (u < hi) ? u : hi;
+  };
+  axis(f[0], f[3], ox, ix);
+  axis(f[1], f[4], oy, iy);
+  axis(f[2], f[5], oz, iz);
+  t_lo = lo;
+  t_hi = hi;
+  return !(lo > hi);
+}
+
+// slab_fast_pair on the pairs of near and far faces.
+__device__ __forceinline__ void slab_near_pair(float ox, float oy, float oz, float ix, float iy,
+                                               float iz, const uint64_t (&nf)[6], bool (&hit)[2],
+                                               float (&t_lo)[2], float (&t_hi)[2]) {
+  float lo[2] = {0.0f, 0.0f}, hi[2] = {100000.0f, 100000.0f};
+  auto axis = [&](uint64_t near, uint64_t far, float o, float inv) {
+    const uint64_t oo = f2(o, o), ii = f2(inv, inv);
+    const uint64_t l = f2_add(f2_mul(f2_sub(near, oo), ii), 0), u = f2_mul(f2_sub(far, oo), ii);
+    float l0, l1, u0, u1;
+    f2_split(l, l0, l1);
+    f2_split(u, u0, u1);
+    lo[0] = fmaxf(lo[0], l0);
+    lo[1] = fmaxf(lo[1], l1);
+    hi[0] = (u0 < hi[0]) ? u0 : hi[0];
+    hi[1] = (u1 < hi[1]) ? u1 : hi[1];
+  };
+  axis(nf[0], nf[1], ox, ix);
+  axis(nf[2], nf[3], oy, iy);
+  axis(nf[4], nf[5], oz, iz);
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    t_lo[e] = lo[e];
+    t_hi[e] = hi[e];
+    hit[e] = !(lo[e] > hi[e]);
+  }
+}
+
+template <bool SORTED, bool TIGHT>
 __global__ void __launch_bounds__(kRayBlock) svo_kernel(
     int64_t rays, int m, int b_pts, int n, int n_max, const float *__restrict__ ray_start,
     const float *__restrict__ ray_dir, const float4 *__restrict__ cbox_all,
-    const int32_t *__restrict__ kids_all, int32_t *__restrict__ idx, float *__restrict__ min_depth,
+    const int32_t *__restrict__ kids_all, const float4 *__restrict__ roots,
+    int32_t *__restrict__ idx, float *__restrict__ min_depth,
     float *__restrict__ max_depth, uint8_t *__restrict__ hits, int32_t *__restrict__ err,
     const int32_t *__restrict__ ray_list, const int32_t *__restrict__ n_list) {
   // per ray and stack level: the expanded node's 8 child ids (lane j writes
@@ -381,7 +616,8 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
 
   const int64_t rr = live ? r : 0;
   const int64_t g = (b_pts == 1) ? 0 : rr / m;
-  const float4 *CB = cbox_all + g * ((int64_t)n * 8 + 1);
+  // (cubes: 8n boxes and the root's; TIGHT: 12n float4, the root's apart)
+  const float4 *CB = cbox_all + g * (TIGHT ? (int64_t)n * 12 : (int64_t)n * 8 + 1);
   const int32_t *KD = kids_all + g * (int64_t)n * 8;
   const float ox = ray_start[rr * 3 + 0], oy = ray_start[rr * 3 + 1], oz = ray_start[rr * 3 + 2];
   const float ix = nsvf_rcp(ray_dir[rr * 3 + 0]), iy = nsvf_rcp(ray_dir[rr * 3 + 1]),
@@ -401,9 +637,16 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
   // root
   int level = -1;
   {
-    float4 rb = CB[(int64_t)n * 8];
+    const float4 rb = TIGHT ? roots[g * 2] : CB[(int64_t)n * 8];
     float lo, hi;
-    bool rh = live && slab(rb.x, rb.y, rb.z, fabsf(rb.w), lo, hi);
+    bool rh = live;
+    if (TIGHT) {
+      const float4 rh4 = roots[g * 2 + 1];
+      const float f[6] = {rb.x, rb.y, rb.z, rh4.x, rh4.y, rh4.z};
+      rh = slab_faces(ox, oy, oz, ix, iy, iz, f, lo, hi) && rh;
+    } else {
+      rh = slab(rb.x, rb.y, rb.z, fabsf(rb.w), lo, hi) && rh;
+    }
     if (rh && rb.w < 0.0f) {            // a single-leaf octree
       if (j == 0) { I[0] = n - 1; LO[0] = lo; HI[0] = hi; }
       cnt = 1;
@@ -437,19 +680,43 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
     if (expand) {
       // children j and j + 4: ids, and both boxes as component pairs
       const int2 ids = *reinterpret_cast<const int2 *>(KD + (int64_t)node * 8 + 2 * j);
-      const float4 qa = CB[(int64_t)node * 8 + 2 * j], qb = CB[(int64_t)node * 8 + 2 * j + 1];
       bool sh[NC];
-      if (fast) {
-        slab_fast_pair(ox, oy, oz, ix, iy, iz, sx, sy, sz, f2(qa.x, qa.y), f2(qa.z, qa.w),
-                       f2(qb.x, qb.y), f2(fabsf(qb.z), fabsf(qb.w)), sh, clo, chi);
+      if (TIGHT) {
+        // (lo pair, hi pair) of x, y, z; the near faces first
+        const uint64_t *q = reinterpret_cast<const uint64_t *>(CB + (int64_t)node * 12 + 3 * j);
+        if (fast) {
+          const int nx = sx < 0.0f, ny = sy < 0.0f, nz = sz < 0.0f;
+          const uint64_t nf[6] = {q[nx], q[nx ^ 1], q[2 + ny], q[2 + (ny ^ 1)], q[4 + nz],
+                                  q[4 + (nz ^ 1)]};
+          slab_near_pair(ox, oy, oz, ix, iy, iz, nf, sh, clo, chi);
+        } else {
+          float f[2][6];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            f2_split(q[2 * d], f[0][d], f[1][d]);
+            f2_split(q[2 * d + 1], f[0][3 + d], f[1][3 + d]);
+          }
+          sh[0] = slab_faces(ox, oy, oz, ix, iy, iz, f[0], clo[0], chi[0]);
+          sh[1] = slab_faces(ox, oy, oz, ix, iy, iz, f[1], clo[1], chi[1]);
+        }
+        cbw[0] = ids.x >= kLeafBit ? -1.0f : 1.0f;
+        cbw[1] = ids.y >= kLeafBit ? -1.0f : 1.0f;
+        cid[0] = ids.x >= kLeafBit ? ids.x - kLeafBit : ids.x;
+        cid[1] = ids.y >= kLeafBit ? ids.y - kLeafBit : ids.y;
       } else {
-        sh[0] = nsvf_slab(ox, oy, oz, ix, iy, iz, qa.x, qa.z, qb.x, fabsf(qb.z), clo[0], chi[0]);
-        sh[1] = nsvf_slab(ox, oy, oz, ix, iy, iz, qa.y, qa.w, qb.y, fabsf(qb.w), clo[1], chi[1]);
+        const float4 qa = CB[(int64_t)node * 8 + 2 * j], qb = CB[(int64_t)node * 8 + 2 * j + 1];
+        if (fast) {
+          slab_fast_pair(ox, oy, oz, ix, iy, iz, sx, sy, sz, f2(qa.x, qa.y), f2(qa.z, qa.w),
+                         f2(qb.x, qb.y), f2(fabsf(qb.z), fabsf(qb.w)), sh, clo, chi);
+        } else {
+          sh[0] = nsvf_slab(ox, oy, oz, ix, iy, iz, qa.x, qa.z, qb.x, fabsf(qb.z), clo[0], chi[0]);
+          sh[1] = nsvf_slab(ox, oy, oz, ix, iy, iz, qa.y, qa.w, qb.y, fabsf(qb.w), clo[1], chi[1]);
+        }
+        cbw[0] = qb.z;
+        cbw[1] = qb.w;
+        cid[0] = ids.x;
+        cid[1] = ids.y;
       }
-      cbw[0] = qb.z;
-      cbw[1] = qb.w;
-      cid[0] = ids.x;
-      cid[1] = ids.y;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         if (cid[c] > -1) {
@@ -536,11 +803,18 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
           top = t;
           if (isleaf) {
             if (j == 0) {
-              const float *cb =
-                  reinterpret_cast<const float *>(CB + (int64_t)s_node[base] * 8 + 2 * (u & 3)) +
-                  (u >> 2);
               float a, b2;
-              slab(cb[0], cb[2], cb[4], -cb[6], a, b2);
+              if (TIGHT) {
+                const float *cb = reinterpret_cast<const float *>(
+                                      CB + (int64_t)s_node[base] * 12 + 3 * (u & 3)) + (u >> 2);
+                const float f[6] = {cb[0], cb[4], cb[8], cb[2], cb[6], cb[10]};
+                slab_faces(ox, oy, oz, ix, iy, iz, f, a, b2);
+              } else {
+                const float *cb =
+                    reinterpret_cast<const float *>(CB + (int64_t)s_node[base] * 8 + 2 * (u & 3)) +
+                    (u >> 2);
+                slab(cb[0], cb[2], cb[4], -cb[6], a, b2);
+              }
               I[cnt] = ch; LO[cnt] = a; HI[cnt] = b2;
             }
             ++cnt;
@@ -814,15 +1088,25 @@ int nsvf_aabb_intersect_boxes(int b, int b_pts, int n, int m, float voxelsize, i
 
 // Packed octree per point set: (8n + 1) boxes of 16 bytes, then (for all
 // sets) 8n child ids of 4 bytes.
-int64_t nsvf_svo_workspace_bytes(int b_pts, int n) {
-  return (int64_t)b_pts * (((int64_t)n * 8 + 1) * (int64_t)sizeof(float4) +
-                           (int64_t)n * 8 * (int64_t)sizeof(int32_t));
+int64_t nsvf_svo_packed_bytes(int n) {
+  return ((int64_t)n * 8 + 1) * (int64_t)sizeof(float4) + (int64_t)n * 8 * (int64_t)sizeof(int32_t);
 }
 
-static int svo_launch(bool sorted, int b, int b_pts, int n, int m, float voxelsize, int n_max,
-                      const float *ray_start, const float *ray_dir, const float *points,
-                      const int32_t *children, int32_t *idx, float *min_depth, float *max_depth,
-                      uint8_t *hits, int32_t *err, void *workspace, void *stream) {
+// The workspace of a traversal: the tight form (a packed octree of the same
+// sets takes less).
+int64_t nsvf_svo_workspace_bytes(int b_pts, int n) {
+  const int64_t total = (int64_t)b_pts * n;
+  return (total * (12 * (int64_t)sizeof(float4) + 9 * (int64_t)sizeof(int32_t)) +
+          (int64_t)b_pts * (2 * (int64_t)sizeof(float4) + (int64_t)sizeof(int32_t)) + 15) / 16 * 16;
+}
+
+// tight: traverse the tight form, built in the workspace; otherwise the cubes
+// (packed in less of it).
+static int svo_launch(bool sorted, bool tight, int b, int b_pts, int n, int m, float voxelsize,
+                      int n_max, const float *ray_start, const float *ray_dir,
+                      const float *points, const int32_t *children, int32_t *idx,
+                      float *min_depth, float *max_depth, uint8_t *hits, int32_t *err,
+                      void *workspace, void *stream) {
   if (bad_common(b, b_pts, n, m, n_max, ray_start, ray_dir, points) || !children || !workspace ||
       (sorted && n_max > 128))
     return NSVF_ERR_INVALID;
@@ -830,23 +1114,34 @@ static int svo_launch(bool sorted, int b, int b_pts, int n, int m, float voxelsi
     return NSVF_ERR_INVALID;
   if (((uintptr_t)workspace) & 15) return NSVF_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
-  int64_t total = (int64_t)b_pts * n;
+  const int64_t total = (int64_t)b_pts * n, rays = (int64_t)b * m;
+  const float hv = voxelsize * 0.5f;
+  const int grid = nsvf_grid(rays, kRaysPerBlock);
+  if (tight && n <= kTightMaxNodes) {
+    if (rays == 0) return NSVF_OK;
+    const TightOctree t = tight_view(workspace, b_pts, n);
+    if (cudaMemsetAsync(t.link, 0xff, (size_t)(total + b_pts) * sizeof(int32_t), s) != cudaSuccess)
+      return NSVF_ERR_CUDA;
+    tight_link_kernel<<<nsvf_grid(total * 8, 256), 256, 0, s>>>(total, n, hv, points, children, t);
+    tight_widen_kernel<<<nsvf_grid(total, 256), 256, 0, s>>>(total, n, hv, points, children, t);
+    tight_check_kernel<<<nsvf_grid(total, 256), 256, 0, s>>>(total, n, hv, points, children, t);
+    for (int k = 0; k < 3; ++k) nsvf_count_launch();
+    auto kernel = sorted ? svo_kernel<true, true> : svo_kernel<false, true>;
+    kernel<<<grid, kRayBlock, 0, s>>>(rays, m, b_pts, n, n_max, ray_start, ray_dir, t.boxes, t.kids,
+                                      t.root, idx, min_depth, max_depth, hits, err, nullptr,
+                                      nullptr);
+    return nsvf_launch_status();
+  }
   float4 *cbox = (float4 *)workspace;
   int32_t *kids = (int32_t *)(cbox + (int64_t)b_pts * ((int64_t)n * 8 + 1));
-  float hv = voxelsize * 0.5f;
   pack_octree_kernel<<<nsvf_grid(total * 8, 256), 256, 0, s>>>(total, n, hv, points, children,
                                                                cbox, kids);
   nsvf_count_launch();
-  int64_t rays = (int64_t)b * m;
   if (rays == 0) return nsvf_launch_status();
-  if (sorted)
-    svo_kernel<true><<<nsvf_grid(rays, kRaysPerBlock), kRayBlock, 0, s>>>(
-        rays, m, b_pts, n, n_max, ray_start, ray_dir, cbox, kids, idx, min_depth, max_depth, hits,
-        err, nullptr, nullptr);
-  else
-    svo_kernel<false><<<nsvf_grid(rays, kRaysPerBlock), kRayBlock, 0, s>>>(
-        rays, m, b_pts, n, n_max, ray_start, ray_dir, cbox, kids, idx, min_depth, max_depth, hits,
-        err, nullptr, nullptr);
+  auto kernel = sorted ? svo_kernel<true, false> : svo_kernel<false, false>;
+  kernel<<<grid, kRayBlock, 0, s>>>(rays, m, b_pts, n, n_max, ray_start, ray_dir, cbox, kids,
+                                    nullptr, idx, min_depth, max_depth, hits, err, nullptr,
+                                    nullptr);
   return nsvf_launch_status();
 }
 
@@ -854,7 +1149,7 @@ int nsvf_svo_intersect(int b, int b_pts, int n, int m, float voxelsize, int n_ma
                        const float *ray_start, const float *ray_dir, const float *points,
                        const int32_t *children, int32_t *idx, float *min_depth,
                        float *max_depth, int32_t *err, void *workspace, void *stream) {
-  return svo_launch(false, b, b_pts, n, m, voxelsize, n_max, ray_start, ray_dir, points, children,
+  return svo_launch(false, true, b, b_pts, n, m, voxelsize, n_max, ray_start, ray_dir, points, children,
                     idx, min_depth, max_depth, nullptr, err, workspace, stream);
 }
 
@@ -863,7 +1158,7 @@ int nsvf_svo_intersect_sorted(int b, int b_pts, int n, int m, float voxelsize, i
                               const int32_t *children, int32_t *idx, float *min_depth,
                               float *max_depth, uint8_t *hits, int32_t *err, void *workspace,
                               void *stream) {
-  return svo_launch(true, b, b_pts, n, m, voxelsize, n_max, ray_start, ray_dir, points, children,
+  return svo_launch(true, true, b, b_pts, n, m, voxelsize, n_max, ray_start, ray_dir, points, children,
                     idx, min_depth, max_depth, hits, err, workspace, stream);
 }
 
@@ -892,9 +1187,9 @@ int nsvf_svo_sorted_list_launch(int64_t rays, int64_t cap, int n, int n_max,
   if (cap <= 0) return NSVF_OK;
   const float4 *cbox = (const float4 *)packed;
   const int32_t *kids = (const int32_t *)(cbox + ((int64_t)n * 8 + 1));
-  svo_kernel<true><<<nsvf_grid(cap, kRaysPerBlock), kRayBlock, 0, stream>>>(
+  svo_kernel<true, false><<<nsvf_grid(cap, kRaysPerBlock), kRayBlock, 0, stream>>>(
       rays, (int)(rays > 0x7fffffff ? 0x7fffffff : rays), 1, n, n_max, ray_start, ray_dir, cbox,
-      kids, idx, min_depth, max_depth, hits, err, ray_list, n_list);
+      kids, nullptr, idx, min_depth, max_depth, hits, err, ray_list, n_list);
   return nsvf_launch_status();
 }
 
@@ -950,7 +1245,7 @@ int nsvf_svo_intersect_noalloc(int b, int b_pts, int n, int m, float voxelsize, 
   if (!scratch) return status;
   // the pack kernel rewrites all b_pts * n scratch entries before the
   // traversal reads them, so nothing left by an earlier call is read
-  return svo_launch(false, b, b_pts, n, m, voxelsize, n_max, ray_start, ray_dir, points, children,
+  return svo_launch(false, false, b, b_pts, n, m, voxelsize, n_max, ray_start, ray_dir, points, children,
                     idx, min_depth, max_depth, nullptr, err, scratch, stream);
 }
 

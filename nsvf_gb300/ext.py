@@ -240,7 +240,8 @@ class SvoGrid:
         self.lines = tuple(int(v) for v in info[:3])
         self.n_leaves, self.n_flagged = int(info[3]), int(info[4])
         self.grid = torch.from_numpy(blob).to(dev)
-        self.packed = _svo_workspace(1, self.n, dev)
+        self.packed = torch.empty(int(LIB.nsvf_svo_packed_bytes(self.n)), dtype=torch.uint8,
+                                  device=dev)
         check(LIB.nsvf_svo_pack(self.n, self.voxel_size, _ptr(self.centers), _ptr(self.children),
                                 _ptr(self.packed), _stream(self.centers)), "svo_pack")
         self._lists = {}

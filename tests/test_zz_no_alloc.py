@@ -120,3 +120,96 @@ def test_noalloc_at_its_capacity(cuda):
     assert int(err.item()) == 0
     assert torch.equal(idx, ref[0]) and torch.equal(lo, ref[1]) and torch.equal(hi, ref[2])
     assert int((ref[0] != -1).sum()) > 100
+
+
+def _mixed(seed, sizes):
+    from test_ops_gpu import _mixed_tree
+    cen, chi = _mixed_tree(seed)
+    rng = np.random.RandomState(seed)
+    internal = np.flatnonzero(chi[:, 8] > 1)
+    leaves = np.flatnonzero(chi[:, 8] == 1)
+    n = len(cen)
+    if sizes == "two_parents":          # a subtree reached twice
+        k = internal[internal < n - 1]
+        for a in k[:3]:
+            free = [p for p in internal if p > a and (chi[p, :8] == -1).any()]
+            p = free[rng.randint(len(free))]
+            chi[p, np.flatnonzero(chi[p, :8] == -1)[0]] = a
+    elif sizes == "bad_id":
+        chi[internal[len(internal) // 2], 3] = n + 5
+        chi[internal[0], 1] = -7
+    elif sizes == "leaf_children":      # a leaf that lists children
+        chi[leaves[1::5], 0] = leaves[0]
+        chi[leaves[2::5], 2] = internal[0]
+    elif sizes == "nan":
+        cen[leaves[::9], 1] = np.nan
+        cen[leaves[1::9], 0] = np.inf
+    elif sizes == "odd_sizes":          # sizes that are not the tree's
+        chi[internal[::3], 8] = 3
+        chi[internal[1::7], 8] = -2
+        chi[leaves[::11], 8] = 0
+    elif sizes == "shifted":            # cubes that do not contain their leaves
+        cen[internal[:-1:2]] += rng.uniform(-0.05, 0.05, (len(internal[:-1:2]), 3)).astype(np.float32)
+    elif sizes == "cycle":
+        p = internal[len(internal) // 2]
+        chi[p, 0] = n - 1
+    return cen, chi
+
+
+@pytest.mark.parametrize("form", ["shell", "odd_voxel", "mixed", "two_parents", "bad_id",
+                                  "leaf_children", "nan", "odd_sizes", "shifted", "cycle",
+                                  "single_leaf", "chain", "chain_center"])
+def test_tight_boxes_equal_the_cubes(cuda, form):
+    """nsvf_svo_intersect traverses the bounding boxes of the leaves, the
+    allocation-free entry point the input's cubes: the same hits and the same
+    error bits, for every kind of input table and ray."""
+    from nsvf_gb300 import ext, geometry, scenes
+    R, H = 3000, 33
+    o, d = _rays(R, seed=11)
+    rng = np.random.RandomState(1)
+    if form in ("shell", "odd_voxel"):
+        vs = 1.0 / 32 if form == "shell" else 0.037
+        p = scenes.shell_voxels(vs, scenes.sphere_torus_sdf)
+        cen, chi = (t.numpy() for t in geometry.build_easy_octree(torch.from_numpy(p), vs / 2))
+    elif form == "single_leaf":
+        vs, cen, chi = 0.5, np.zeros((1, 3), np.float32), np.array([[-1] * 8 + [1]], np.int32)
+    elif form.startswith("chain"):      # 21 levels: deeper than the traversal's stack
+        vs, L = 1e-5, 21
+        cen = np.zeros((L, 3), np.float32)
+        chi = np.full((L, 9), -1, np.int32)
+        chi[:, 8] = 2 ** np.arange(L)
+        chi[1:, 7] = np.arange(L - 1)
+    else:
+        vs = 0.04
+        cen, chi = _mixed(3, form)
+    o[::5] = rng.uniform(-0.3, 0.3, o[::5].shape)            # from inside
+    d[::7, 0] = 0.0
+    d[1::13] = np.float32([0, 0, -1])
+    o[2::9] = np.round(o[2::9] / (vs / 2)) * np.float32(vs / 2)   # on grid planes
+    if form == "chain_center":
+        d[3::4] = -o[3::4] / np.linalg.norm(o[3::4], axis=1, keepdims=True)
+    cen, chi = np.ascontiguousarray(cen, np.float32), np.ascontiguousarray(chi, np.int32)
+    t = lambda a: torch.from_numpy(a)[None].contiguous().to(cuda)
+    rs, rd, tc, tch = t(o), t(d), t(cen), t(chi)
+    ext.error_word(cuda).zero_()
+    out = ext.svo_intersect(rs, rd, tc, tch, vs, H)
+    srt = ext.svo_intersect_sorted(rs, rd, tc, tch, vs, H)
+    got_err = int(ext.error_word(cuda).item())
+    ext.error_word(cuda).zero_()
+    ref = [torch.empty_like(a) for a in out]
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+    status = _noalloc_fn()(1, 1, len(cen), R, vs, H, rs.data_ptr(), rd.data_ptr(), tc.data_ptr(),
+                           tch.data_ptr(), *[a.data_ptr() for a in ref], err.data_ptr(),
+                           torch.cuda.current_stream(cuda).cuda_stream)
+    assert status == 0
+    for a, b in zip(out, ref):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert got_err == int(err.item())
+    assert (form in ("bad_id", "cycle", "chain_center")) == (got_err != 0)
+    if form != "single_leaf" and not form.startswith("chain"):
+        assert int(out[0].ne(-1).sum()) > 0
+    # the sorted variant: the same rows in depth order, slot order at ties
+    m = ref[0].eq(-1)
+    lo, order = ref[1].masked_fill(m, 10000.0).sort(dim=-1, stable=True)
+    assert torch.equal(srt[1], lo) and torch.equal(srt[0], ref[0].gather(-1, order))
+    assert torch.equal(srt[2], ref[2].masked_fill(m, 10000.0).gather(-1, order))
