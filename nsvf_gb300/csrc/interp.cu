@@ -6,9 +6,14 @@
 // voxel v with centre c, p = (x - c) / voxel_size + 0.5, corner k = 4*ix +
 // 2*iy + iz (offset_points order) has weight prod_d (q_kd ? p_d : 1 - p_d)
 // and emb = sum_k w_k * values[feats[v, k]]. The reference materialises the
-// 8 gathered rows per sample ([Ns, 8, E]) with two F.embedding calls; here
-// one thread produces 4 channels of one sample from 8 float4 loads, and the
-// 8 threads of a sample read each 128-byte corner row together.
+// 8 gathered rows per sample ([Ns, 8, E]) with two F.embedding calls.
+//
+// Two pairs of kernels. The general ones: E / 4 threads per sample, 4 channels
+// each, one sample per thread. For E = 32, the embeddings' width, 8 lanes walk
+// consecutive samples (trilinear_*_run_kernel): along a ray about eight in a
+// row lie in the same voxel, so its corner rows stay in registers until the
+// voxel changes, and so do the backward's eight corner sums, whose float4
+// atomics were the bound. Measured at 1.26 M samples: see there.
 #include "common.cuh"
 
 namespace {
@@ -118,6 +123,211 @@ __global__ void __launch_bounds__(kBlock) trilinear_bwd_kernel(
   }
 }
 
+// ------------------------------------------------------ runs, E = 32 ----
+//
+// A group of 8 lanes takes 4 consecutive samples, a lane 4 channels of each.
+// Lane c of the first four reads sample c (voxel, position, centre) and
+// divides; lane c of all eight reads corner c of the samples' voxels; the rest
+// comes by shuffles. Corner rows are fetched, and the backward's corner sums
+// flushed, where the voxel changes. Latency-bound (four dependent trips to L2),
+// so the work per thread is kept short and the blocks small: 1.26 M samples
+// along rays take 80 us forward and 141 us backward (86 us for the embeddings'
+// gradient alone, 90 for the positions'), where one sample per thread took 152
+// and 228 (203, 170), and groups that walk 32 samples with the next batch's
+// loads in flight 85 and 222. Floor 30 and 55 us: the embeddings written; read,
+// and the table updated. Blocks of 256: 84 and 148 us, of 512: 88 and 164.
+constexpr int kLanes = 8, kRun = 4, kRunBlock = 128;
+
+template <typename FeatT>
+struct Group {
+  int64_t v[kRun];          // voxel of each sample, -1 where there is none
+  int key[kRun];            // this lane's corner of it, -1 where it is out of range
+  float mine[3];            // trilinear coordinates of sample (lane & 3)
+
+  template <typename IdxT>
+  __device__ __forceinline__ void load(int64_t s0, int64_t ns, float voxel_size, int64_t n_vox,
+                                       int64_t n_keys, const IdxT *__restrict__ sidx,
+                                       const float *__restrict__ xyz,
+                                       const float *__restrict__ centers,
+                                       const FeatT *__restrict__ feats, int lane, int32_t *err) {
+    const int64_t s = s0 + (lane & (kRun - 1));
+    int64_t my = -1;
+    mine[0] = mine[1] = mine[2] = 0.0f;
+    if (s < ns) {
+      my = (int64_t)sidx[s];
+      if (my < 0 || my >= n_vox) {
+        if (err) atomicOr(err, 4);
+        my = -1;
+      } else {
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          mine[d] = (xyz[s * 3 + d] - centers[my * 3 + d]) / voxel_size + 0.5f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+      v[i] = __shfl_sync(0xffffffffu, my, i, kLanes);
+      if (i > 0 && v[i] == v[i - 1]) {
+        key[i] = key[i - 1];
+        continue;
+      }
+      key[i] = -1;
+      if (v[i] < 0) continue;
+      const int64_t k = (int64_t)feats[v[i] * 8 + lane];
+      if (k >= 0 && k < n_keys) key[i] = (int)k;
+      else if (err) atomicOr(err, 4);
+    }
+  }
+  __device__ __forceinline__ bool change(int i) const { return i == 0 || v[i] != v[i - 1]; }
+  __device__ __forceinline__ void coords(int i, float (&p)[3]) const {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) p[d] = __shfl_sync(0xffffffffu, mine[d], i, kLanes);
+  }
+};
+
+template <typename IdxT, typename FeatT>
+__global__ void __launch_bounds__(kRunBlock) trilinear_fwd_run_kernel(
+    int64_t ns, float voxel_size, int64_t n_vox, int64_t n_keys, const IdxT *__restrict__ sidx,
+    const float *__restrict__ xyz, const float *__restrict__ centers,
+    const FeatT *__restrict__ feats, const float4 *__restrict__ values, float4 *__restrict__ emb,
+    int32_t *__restrict__ err) {
+  const int64_t t = blockIdx.x * (int64_t)kRunBlock + threadIdx.x;
+  const int64_t s0 = t / kLanes * kRun;
+  const int ch = threadIdx.x % kLanes;
+  Group<FeatT> g;
+  g.load(s0, ns, voxel_size, n_vox, n_keys, sidx, xyz, centers, feats, ch, err);
+  float4 x[8];
+  unsigned mask = 0;
+#pragma unroll
+  for (int i = 0; i < kRun; ++i) {
+    float p[3];
+    g.coords(i, p);
+    int key[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) key[k] = __shfl_sync(0xffffffffu, g.key[i], k, kLanes);
+    if (g.change(i)) {
+      mask = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (key[k] >= 0) {
+          x[k] = __ldg(values + (int64_t)key[k] * kLanes + ch);
+          mask |= 1u << k;
+        }
+      }
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (mask != 0xffu && !((mask >> k) & 1u)) continue;
+      const float w = corner_w(p, k);
+      acc.x = fmaf(w, x[k].x, acc.x); acc.y = fmaf(w, x[k].y, acc.y);
+      acc.z = fmaf(w, x[k].z, acc.z); acc.w = fmaf(w, x[k].w, acc.w);
+    }
+    if (s0 + i < ns) emb[(s0 + i) * kLanes + ch] = acc;
+  }
+}
+
+// The corners in two halves (ix = 0, then 1), so that four rows and four sums
+// are live at a time. With D_k = <values_k, g>, a half adds to grad_xyz
+//   x: (-1 or 1) sum_yz b_y c_z D_yz, y: a sum_z c_z (D_1z - D_0z),
+//   z: a sum_y b_y (D_y1 - D_y0).
+template <typename IdxT, typename FeatT, bool GV, bool GX>
+__global__ void __launch_bounds__(kRunBlock, GV && GX ? 6 : 8) trilinear_bwd_run_kernel(
+    int64_t ns, float voxel_size, int64_t n_vox, int64_t n_keys, const IdxT *__restrict__ sidx,
+    const float *__restrict__ xyz, const float *__restrict__ centers,
+    const FeatT *__restrict__ feats, const float4 *__restrict__ values,
+    const float4 *__restrict__ grad_emb, float4 *__restrict__ grad_values,
+    float *__restrict__ grad_xyz) {
+  const unsigned full = 0xffffffffu;
+  const int64_t t = blockIdx.x * (int64_t)kRunBlock + threadIdx.x;
+  const int64_t s0 = t / kLanes * kRun;
+  const int ch = threadIdx.x % kLanes;
+  float4 ge[kRun];
+#pragma unroll
+  for (int i = 0; i < kRun; ++i)
+    ge[i] = s0 + i < ns ? grad_emb[(s0 + i) * kLanes + ch] : make_float4(0.f, 0.f, 0.f, 0.f);
+  Group<FeatT> g;
+  g.load(s0, ns, voxel_size, n_vox, n_keys, sidx, xyz, centers, feats, ch, nullptr);
+  float d[kRun][3];
+#pragma unroll
+  for (int i = 0; i < kRun; ++i) d[i][0] = d[i][1] = d[i][2] = 0.0f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float4 x[4], sum[4];
+    int last[4] = {-1, -1, -1, -1};          // rows of the sums
+    auto flush = [&]() {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (GV && last[k] >= 0) atomicAdd(grad_values + (int64_t)last[k] * kLanes + ch, sum[k]);
+    };
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+      float p[3];
+      g.coords(i, p);
+      int key[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) key[k] = __shfl_sync(full, g.key[i], h * 4 + k, kLanes);
+      if (g.change(i)) {
+        if (i > 0) flush();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          last[k] = key[k];
+          sum[k] = x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (GX && key[k] >= 0) x[k] = __ldg(values + (int64_t)key[k] * kLanes + ch);
+        }
+      }
+      const float a = h ? p[0] : 1.0f - p[0];
+      const float b[2] = {1.0f - p[1], p[1]}, c[2] = {1.0f - p[2], p[2]};
+      const float4 gi = ge[i];
+      if (GV) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float w = a * b[k >> 1] * c[k & 1];
+          sum[k].x = fmaf(w, gi.x, sum[k].x); sum[k].y = fmaf(w, gi.y, sum[k].y);
+          sum[k].z = fmaf(w, gi.z, sum[k].z); sum[k].w = fmaf(w, gi.w, sum[k].w);
+        }
+      }
+      if (GX) {
+        float D[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          D[k] = last[k] < 0 ? 0.0f
+                             : x[k].x * gi.x + x[k].y * gi.y + x[k].z * gi.z + x[k].w * gi.w;
+        const float ex = b[0] * (c[0] * D[0] + c[1] * D[1]) + b[1] * (c[0] * D[2] + c[1] * D[3]);
+        d[i][0] += h ? ex : -ex;
+        d[i][1] += a * (c[0] * (D[2] - D[0]) + c[1] * (D[3] - D[1]));
+        d[i][2] += a * (b[0] * (D[1] - D[0]) + b[1] * (D[3] - D[2]));
+      }
+    }
+    flush();
+  }
+  if (GX) {
+    // over the sample's 8 lanes, the four samples folded onto the lanes: after
+    // the exchange over 4 lanes a lane holds two samples, then one
+    const bool up = ch & 4, mid = ch & 2;
+    float e[2][3], f[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float keep = up ? d[2 + i][c] : d[i][c], give = up ? d[i][c] : d[2 + i][c];
+        e[i][c] = keep + __shfl_xor_sync(full, give, 4);
+      }
+      const float keep = mid ? e[1][c] : e[0][c], give = mid ? e[0][c] : e[1][c];
+      f[c] = keep + __shfl_xor_sync(full, give, 2);
+      f[c] += __shfl_xor_sync(full, f[c], 1);
+    }
+    const int64_t s = s0 + (ch >> 1);
+    if (!(ch & 1) && s < ns) {
+      const float inv = 1.0f / voxel_size;
+      grad_xyz[s * 3 + 0] = f[0] * inv;
+      grad_xyz[s * 3 + 1] = f[1] * inv;
+      grad_xyz[s * 3 + 2] = f[2] * inv;
+    }
+  }
+}
+
 struct InterpArgs {
   int64_t ns;
   int e;
@@ -129,23 +339,43 @@ struct InterpArgs {
   const float *values;
 };
 
+// The run kernels take E = 32 and tables whose rows 31 bits can number.
+bool use_runs(const InterpArgs &a) { return a.e == 32 && a.n_keys <= 0x7fffffff; }
+
+int run_grid(int64_t ns) { return nsvf_grid((ns + kRun - 1) / kRun * kLanes, kRunBlock); }
+
 template <typename IdxT, typename FeatT>
 int launch_fwd(const InterpArgs &a, float *emb, int32_t *err, cudaStream_t s) {
-  int e4 = a.e / 4;
-  trilinear_fwd_kernel<IdxT, FeatT><<<nsvf_grid(a.ns * e4, kBlock), kBlock, 0, s>>>(
-      a.ns, e4, a.vs, a.n_vox, a.n_keys, (const IdxT *)a.sidx, a.xyz, a.centers,
-      (const FeatT *)a.feats, (const float4 *)a.values, (float4 *)emb, err);
+  const int e4 = a.e / 4;
+  if (use_runs(a))
+    trilinear_fwd_run_kernel<IdxT, FeatT><<<run_grid(a.ns), kRunBlock, 0, s>>>(
+        a.ns, a.vs, a.n_vox, a.n_keys, (const IdxT *)a.sidx, a.xyz, a.centers,
+        (const FeatT *)a.feats, (const float4 *)a.values, (float4 *)emb, err);
+  else
+    trilinear_fwd_kernel<IdxT, FeatT><<<nsvf_grid(a.ns * e4, kBlock), kBlock, 0, s>>>(
+        a.ns, e4, a.vs, a.n_vox, a.n_keys, (const IdxT *)a.sidx, a.xyz, a.centers,
+        (const FeatT *)a.feats, (const float4 *)a.values, (float4 *)emb, err);
   return nsvf_launch_status();
 }
 
 template <typename IdxT, typename FeatT>
 int launch_bwd(const InterpArgs &a, const float *grad_emb, float *grad_values, float *grad_xyz,
                cudaStream_t s) {
-  int e4 = a.e / 4;
-  trilinear_bwd_kernel<IdxT, FeatT><<<nsvf_grid(a.ns * e4, kBlock), kBlock, 0, s>>>(
-      a.ns, e4, a.vs, a.n_vox, a.n_keys, (const IdxT *)a.sidx, a.xyz, a.centers,
-      (const FeatT *)a.feats, (const float4 *)a.values, (const float4 *)grad_emb,
-      (float4 *)grad_values, grad_xyz);
+  const int e4 = a.e / 4;
+  if (use_runs(a)) {
+    auto kernel = grad_values && grad_xyz ? trilinear_bwd_run_kernel<IdxT, FeatT, true, true>
+                  : grad_values           ? trilinear_bwd_run_kernel<IdxT, FeatT, true, false>
+                                          : trilinear_bwd_run_kernel<IdxT, FeatT, false, true>;
+    kernel<<<run_grid(a.ns), kRunBlock, 0, s>>>(
+        a.ns, a.vs, a.n_vox, a.n_keys, (const IdxT *)a.sidx, a.xyz, a.centers,
+        (const FeatT *)a.feats, (const float4 *)a.values, (const float4 *)grad_emb,
+        (float4 *)grad_values, grad_xyz);
+  } else {
+    trilinear_bwd_kernel<IdxT, FeatT><<<nsvf_grid(a.ns * e4, kBlock), kBlock, 0, s>>>(
+        a.ns, e4, a.vs, a.n_vox, a.n_keys, (const IdxT *)a.sidx, a.xyz, a.centers,
+        (const FeatT *)a.feats, (const float4 *)a.values, (const float4 *)grad_emb,
+        (float4 *)grad_values, grad_xyz);
+  }
   return nsvf_launch_status();
 }
 

@@ -167,3 +167,54 @@ def test_prune_fp32_stage_keeps_the_mask(cuda, n_vox, bits, rule):
                                     step=step, band=band)
         ext.check_errors(cuda)
         assert torch.equal(keep, want) and n > 0
+
+
+@pytest.mark.parametrize("ns", [1, 7, 257, 90001])
+@pytest.mark.parametrize("E,dtypes", [(4, (torch.int64, torch.int64)),
+                                      (32, (torch.int64, torch.int64)),
+                                      (32, (torch.int32, torch.int32)),
+                                      (128, (torch.int32, torch.int64))])
+def test_interpolation_runs(cuda, ns, E, dtypes):
+    """trilinear_embed forward and backward, the kernels for 32 channels (4
+    samples per group of lanes) and the general ones: runs of samples in one
+    voxel longer and shorter than a group, voxel and corner ids out of range:
+    against float64 torch."""
+    from nsvf_gb300 import ext
+    from nsvf_gb300.functional import trilinear_embed
+    n_vox = 50
+    vs, centers, feats, _, _ = _scene(cuda, n_vox, E)
+    g = torch.Generator().manual_seed(ns + E)
+    values = torch.randn(3 * n_vox, E, generator=g).to(cuda).requires_grad_(True)
+    lens = torch.randint(1, 40, (ns,), generator=g)
+    vid = torch.randint(0, n_vox, (ns,), generator=g).repeat_interleave(lens)[:ns]
+    bad = torch.rand(ns, generator=g) < 0.02
+    vid = torch.where(bad, torch.where(torch.rand(ns, generator=g) < 0.5, -1, n_vox), vid)
+    feats = feats.clone()
+    feats[7, 3], feats[9, 0] = -1, 3 * n_vox
+    vid, feats, bad = vid.to(cuda), feats.to(dtypes[1]), bad.to(cuda)
+    xyz = centers[vid.clamp(0, n_vox - 1)] + (torch.rand(ns, 3, generator=g).to(cuda) - 0.5) * vs
+    xyz = xyz.requires_grad_(True)
+    gr = torch.randn(ns, E, generator=g).to(cuda)
+    ext.error_word(cuda).zero_()
+    emb = trilinear_embed(vid.to(dtypes[0]), xyz, centers, feats, values, vs)
+    gx, gv = torch.autograd.grad(emb, (xyz, values), gr)
+    flagged = int(ext.error_word(cuda).item())
+    ext.error_word(cuda).zero_()
+    v = vid.clamp(0, n_vox - 1)
+    assert flagged == (4 if bad.any() or ((v == 7) | (v == 9)).any() else 0)
+    x64, v64 = xyz.detach().double().requires_grad_(True), values.detach().double().requires_grad_(True)
+    p = (x64 - centers[v].double()) / vs + 0.5
+    ref = 0
+    for k in range(8):
+        w = 1
+        for d, bit in enumerate((4, 2, 1)):
+            w = w * (p[:, d] if k & bit else 1 - p[:, d])
+        key = feats[v, k].long()
+        ok = ((key >= 0) & (key < values.size(0)) & ~bad).double()
+        ref = ref + (w * ok)[:, None] * v64[key.clamp(0, values.size(0) - 1)]
+    rx, rv = torch.autograd.grad(ref, (x64, v64), gr.double())
+    # 8 products of order 1; gradients: a sum over the channels times 1 / vs,
+    # and over up to ns / 150 * 8 samples per corner row
+    assert float((emb.detach().double() - ref.detach()).abs().max()) <= 1e-5
+    assert float((gx.double() - rx).norm()) <= 2e-6 * float(rx.norm()) + 1e-12
+    assert float((gv.double() - rv).norm()) <= 2e-6 * float(rv.norm()) + 1e-12
