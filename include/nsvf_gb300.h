@@ -713,6 +713,18 @@ int nsvf_prune_screen_bf16(int64_t n_voxels, int bits, int rule, float step, flo
                            const void *const weights[5], const float *const biases[5],
                            uint32_t *score, uint8_t *keep, int64_t *list, int64_t *n_list,
                            int64_t list_cap, int32_t *err, void *stream);
+/* prune_screen_live_bf16: the screen without scores, on sub^3 of each voxel's
+ * points (sub per axis, both faces among them; 2 <= sub <= bits, all points for
+ * sub == bits) and, with `live` (int32 [n_voxels], n_live one int64), only for
+ * the voxels that keep does not hold yet. Two calls, a few points of every
+ * voxel and then all points of the rest, set the same keep flags and list the
+ * undecided points of every voxel not kept. */
+int nsvf_prune_screen_live_bf16(int64_t n_voxels, int bits, int sub, int rule, float threshold,
+                                float band, int64_t n_keys, float voxel_size,
+                                const float *centers, const int32_t *feats, const float *values,
+                                const void *const weights[5], const float *const biases[5],
+                                uint8_t *keep, int32_t *live, int64_t *n_live, int64_t *list,
+                                int64_t *n_list, int64_t list_cap, int32_t *err, void *stream);
 /* prune_fp32_dev: between the two, the listed points of voxels not yet kept in
  * FP32 (packed weights as nsvf_field_train_pack). A point with sigma - margin >
  * threshold sets keep, margin = band * M + 1e-6 threshold; the points within

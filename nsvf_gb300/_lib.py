@@ -98,6 +98,8 @@ def _load():
         "nsvf_field_refine_fp32_dev": ([P, P, i64, i64, P, P, i64, P, P, i64, i64, f32, P, P, P, P,
                                         P, P, P], i32),
         "nsvf_wait_timeout_selftest": ([ctypes.c_uint64, P, P], i32),
+        "nsvf_prune_screen_live_bf16": ([i64, i32, i32, i32, f32, f32, i64, f32, P, P, P, P, P, P,
+                                         P, P, P, P, i64, P, P], i32),
         "nsvf_prune_fp32_dev": ([i64, i32, f32, f32, i64, f32, P, P, P, P, P, P, i64, P, P, P, P, P,
                                  P], i32),
         "nsvf_train_rows_count": ([i64, i32, P, P, P], i32),
@@ -150,7 +152,7 @@ def exported_symbols():
         "nsvf_parallel_sampling_smem_bytes", "nsvf_pinhole_rays_multi", "nsvf_piece_rows",
         "nsvf_sample_count_pieces", "nsvf_sample_compact_pieces",
         "nsvf_sample_scan_bytes", "nsvf_sample_scan_compact_dev", "nsvf_sample_scan_compact_pieces",
-        "nsvf_prune_fp32_dev", "nsvf_train_rows_count", "nsvf_train_rows_pack", "nsvf_field_train_packed_floats",
+        "nsvf_prune_fp32_dev", "nsvf_prune_screen_live_bf16", "nsvf_train_rows_count", "nsvf_train_rows_pack", "nsvf_field_train_packed_floats",
         "nsvf_field_train_pack", "nsvf_field_train_forward", "nsvf_composite_rows",
         "nsvf_composite_rows_backward", "nsvf_field_train_backward_floats",
         "nsvf_field_train_backward",

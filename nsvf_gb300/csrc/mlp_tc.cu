@@ -133,7 +133,11 @@ enum Mode : int {
                    // the input stage; out[n] = (sigma, r, g, b)
   kPrune = 2,      // rows = bits^3 points per voxel; per-voxel score reduced
                    // with atomics into score[v]
+  kScreen = 3,     // kPrune's screen without scores, on sub^3 of a voxel's
+                   // points and on the listed voxels only
 };
+
+__host__ __device__ constexpr bool is_prune(int mode) { return mode == kPrune || mode == kScreen; }
 
 struct MlpParams {
   const float *emb;                  // kEmbIn: [ns, 32] fp32
@@ -158,6 +162,10 @@ struct MlpParams {
   int64_t *plist;
   unsigned long long *n_plist;
   int64_t plist_cap;
+  // kScreen: points per axis of the sub-grid (every one for sub == bits), the
+  // voxels (NULL: all of them); ns_dev then counts voxels
+  int sub;
+  const int32_t *vlist;
   const __nv_bfloat16 *w[5];         // row-major [N, K]: 128x32, 3x 128x128, 4x128
   const float *b[5];                 // [128] x4, [4]
   // FP8 variant: the hidden layers 1-3 as E4M3 bytes (row-major [128, 128],
@@ -282,6 +290,20 @@ constexpr int kSkipKey = -1;
 // invalid voxels / corner ids get kSkipKey (they contribute nothing; invalid
 // ids set `bad`). The weights are the interpolation kernel's, same
 // operations in the same order.
+// kScreen: the voxel of row r, and the row's point in the voxel's full grid of
+// bits^3 (offset_points order): sub-grid index j of an axis is full index
+// j (bits - 1) / (sub - 1), rounded, so both faces are in it.
+__device__ __forceinline__ int64_t screen_voxel(const MlpParams &p, int64_t r) {
+  const int64_t li = r / ((int64_t)p.sub * p.sub * p.sub);
+  return p.vlist ? (int64_t)p.vlist[li] : li;
+}
+__device__ __forceinline__ int64_t screen_point(const MlpParams &p, int64_t r) {
+  const int g = p.sub, b = p.bits - 1;
+  const int i = (int)(r % ((int64_t)g * g * g));
+  auto full = [&](int j) { return (j * b + (g - 1) / 2) / (g - 1); };
+  return ((int64_t)full(i / (g * g)) * p.bits + full(i / g % g)) * p.bits + full(i % g);
+}
+
 // A sample row's voxel id and position, loaded one tile ahead of its use.
 struct SampleRow {
   int32_t vox;
@@ -297,6 +319,7 @@ __device__ __forceinline__ SampleRow load_sample(const MlpParams &p, int64_t r, 
     s.vox = p.vox[r];
     s.xyz = p.xyzd[r];
   }
+  if (MODE == kScreen && r < ns) s.vox = (int32_t)screen_voxel(p, r);
   return s;
 }
 
@@ -305,7 +328,7 @@ template <int MODE>
 __device__ __forceinline__ int64_t row_voxel(const MlpParams &p, int64_t r, int64_t ns,
                                              const SampleRow &smp) {
   if (r >= ns) return -1;
-  if (MODE == kSamplesIn) return smp.vox;
+  if (MODE == kSamplesIn || MODE == kScreen) return smp.vox;
   return r / ((int64_t)p.bits * p.bits * p.bits);
 }
 
@@ -350,8 +373,8 @@ __device__ __forceinline__ void row_meta(const MlpParams &p, int64_t r, int64_t 
       // point i of voxel v: offset_points order (x slowest), offset
       // ((2 i_d + 1) - bits) / (bits - 1) times half a voxel
       int64_t P = (int64_t)p.bits * p.bits * p.bits;
-      v = r / P;
-      int64_t i = r % P;
+      v = MODE == kScreen ? (int64_t)smp.vox : r / P;
+      int64_t i = MODE == kScreen ? screen_point(p, r) : r % P;
       int ix = (int)(i / (p.bits * p.bits)), iy = (int)((i / p.bits) % p.bits), iz = (int)(i % p.bits);
       // offset_points' FP32 operations: fl(fl(o / (bits - 1)) * hv), then
       // added to the centre (separate roundings, no contraction)
@@ -506,7 +529,7 @@ __device__ __forceinline__ void head_store(const MlpParams &p, const float *bias
   tmem_wait_ld();
   fence_before_sync();
   float sigma = v[0] + bias4[0];
-  if (MODE != kPrune) {
+  if (!is_prune(MODE)) {
     if (r < ns)
       reinterpret_cast<float4 *>(p.out)[r] =
           make_float4(sigma, v[1] + bias4[1], v[2] + bias4[2], v[3] + bias4[3]);
@@ -516,8 +539,9 @@ __device__ __forceinline__ void head_store(const MlpParams &p, const float *bias
     // Both are >= 0, so their float bits order like unsigned ints. A warp
     // whose rows all belong to one voxel reduces before its one atomic.
     bool live = r < ns;
-    int64_t vv = live ? r / ((int64_t)p.bits * p.bits * p.bits) : -1;
-    uint32_t val;
+    const int64_t P = (int64_t)p.bits * p.bits * p.bits;
+    int64_t vv = live && MODE == kPrune ? r / P : -1;
+    uint32_t val = 0;
     if (p.rule == 0) val = __float_as_uint(expf(-fmaxf(sigma, 0.0f)));
     else val = __float_as_uint(fmaxf(1.0f - expf(-(fmaxf(sigma, 0.0f) * p.step)), 0.0f));
     if (p.keep) {
@@ -527,6 +551,10 @@ __device__ __forceinline__ void head_store(const MlpParams &p, const float *bias
       const float lo = sigma - p.prune_c * M, hi = sigma + p.prune_c * M;
       const bool certain = live && (p.rule == 1 ? lo >= p.prune_T : lo > p.prune_T);
       const bool maybe = live && !certain && hi >= p.prune_T;
+      if (MODE == kScreen && (certain || maybe)) {
+        vv = screen_voxel(p, r);
+        r = vv * P + screen_point(p, r);
+      }
       if (certain) p.keep[vv] = 1;
       const unsigned m = __ballot_sync(0xffffffffu, maybe);
       if (m) {
@@ -541,6 +569,7 @@ __device__ __forceinline__ void head_store(const MlpParams &p, const float *bias
         }
       }
     }
+    if (MODE == kScreen) return;
     int64_t v0 = __shfl_sync(0xffffffffu, vv, 0);
     if (__all_sync(0xffffffffu, vv == v0 && live)) {
 #pragma unroll
@@ -585,7 +614,7 @@ __global__ void __launch_bounds__(Cfg<F8>::kThreads, 1) mlp_tc_kernel(const MlpP
     else stage_weights(reinterpret_cast<__nv_bfloat16 *>(S.wh[l]), p.w[l + 1], HID, HID, HID);
   }
   stage_weights(S.w4, p.w[4], NOUT, 4, HID);
-  if (MODE == kPrune && p.keep) {
+  if (is_prune(MODE) && p.keep) {
     // head row 4 = |W4[0]|: column 4 of the head output is M = sum_j
     // |W4[0][j]| h_j, the scale of sigma's BF16 rounding error
     // (each chunk written by the thread stage_weights gave it, after its
@@ -629,6 +658,7 @@ __global__ void __launch_bounds__(Cfg<F8>::kThreads, 1) mlp_tc_kernel(const MlpP
   int64_t ns = p.ns;
   if (p.ns_dev) {
     int64_t d = *p.ns_dev;
+    if (MODE == kScreen) d *= (int64_t)p.sub * p.sub * p.sub;
     if (d > ns && tid == 0 && p.err) atomicOr(p.err, 2);
     ns = d < 0 ? 0 : (d < ns ? d : ns);
   }
@@ -897,6 +927,21 @@ int launch_mlp(const MlpParams &p, cudaStream_t stream) {
   return launch_mlp_grid<MODE, F8>(p, stream, 0);
 }
 
+// The voxels not kept yet (in blocks of 32 in index order).
+__global__ void __launch_bounds__(256) live_voxels_kernel(int64_t n,
+                                                          const uint8_t *__restrict__ keep,
+                                                          int32_t *__restrict__ live,
+                                                          unsigned long long *__restrict__ n_live) {
+  const int64_t v = blockIdx.x * (int64_t)256 + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool in = v < n && !keep[v];
+  const unsigned m = __ballot_sync(0xffffffffu, in);
+  unsigned long long at = 0;
+  if (m && lane == 0) at = atomicAdd(n_live, (unsigned long long)__popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (in) live[at + __popc(m & ((1u << lane) - 1u))] = (int32_t)v;
+}
+
 // grid_override < 0: one CTA per SM (the row count is only known on the
 // device); 0: sized from p.ns.
 template <int MODE, bool F8>
@@ -1103,6 +1148,52 @@ int nsvf_prune_screen_bf16(int64_t n_voxels, int bits, int rule, float step, flo
   p.ns = n_voxels * (int64_t)bits * bits * bits;
   p.err = err;
   return launch_mlp<kPrune>(p, (cudaStream_t)stream);
+}
+
+int nsvf_prune_screen_live_bf16(int64_t n_voxels, int bits, int sub, int rule, float threshold,
+                                float band, int64_t n_keys, float voxel_size,
+                                const float *centers, const int32_t *feats, const float *values,
+                                const void *const weights[5], const float *const biases[5],
+                                uint8_t *keep, int32_t *live, int64_t *n_live, int64_t *list,
+                                int64_t *n_list, int64_t list_cap, int32_t *err, void *stream) {
+  if (n_voxels < 0 || n_voxels > 0x7fffffff || bits < 2 || bits > 64 || sub < 2 || sub > bits ||
+      (rule != 0 && rule != 1) || n_keys < 1 || list_cap < 0 || !(threshold > 0.0f) ||
+      !(band >= 0.0f) || !(threshold < 3.0e38f) || (live && !n_live))
+    return NSVF_ERR_INVALID;
+  if (n_voxels == 0) return NSVF_OK;
+  MlpParams p = {};
+  if (!centers || !feats || !values || !keep || !n_list || (list_cap > 0 && !list) ||
+      !set_weights(p, weights, biases))
+    return NSVF_ERR_INVALID;
+  if ((((uintptr_t)values) | ((uintptr_t)feats)) & 15) return NSVF_ERR_INVALID;
+  cudaStream_t s = (cudaStream_t)stream;
+  p.ns = n_voxels * (int64_t)sub * sub * sub;
+  if (live) {
+    if (cudaMemsetAsync(n_live, 0, sizeof(int64_t), s) != cudaSuccess) return NSVF_ERR_CUDA;
+    live_voxels_kernel<<<nsvf_grid(n_voxels, 256), 256, 0, s>>>(n_voxels, keep, live,
+                                                                (unsigned long long *)n_live);
+    const int st = nsvf_launch_status();
+    if (st != NSVF_OK) return st;
+    p.vlist = live;
+    p.ns_dev = n_live;
+  }
+  p.centers = centers;
+  p.feats = feats;
+  p.values = (const float4 *)values;
+  p.n_vox = n_voxels;
+  p.n_keys = n_keys;
+  p.voxel_size = voxel_size;
+  p.bits = bits;
+  p.sub = sub;
+  p.rule = rule;
+  p.keep = keep;
+  p.prune_T = threshold;
+  p.prune_c = band;
+  p.plist = list;
+  p.n_plist = (unsigned long long *)n_list;
+  p.plist_cap = list_cap;
+  p.err = err;
+  return launch_mlp_grid<kScreen, false>(p, s, live ? -1 : 0);
 }
 
 int nsvf_field_samples_fp8_dev(int64_t capacity, const int64_t *n_samples_dev,

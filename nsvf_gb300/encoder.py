@@ -359,7 +359,7 @@ class SparseVoxelEncoder(nn.Module):
         values = states['voxel_vertex_emb'].detach().float().contiguous()
         keep, _, n = mlp.prune_mask(centers, feats, values, float(self.voxel_size), th=th,
                                     bits=bits, rule=1 if use_step else 0,
-                                    step=float(self.step_size))
+                                    step=float(self.step_size), scores=False)
         self.last_prune_undecided_points = n
         if apply:
             self.keep.masked_scatter_(self.keep.bool(), keep.long())

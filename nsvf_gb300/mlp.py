@@ -152,7 +152,7 @@ class TensorCoreMLP:
     FP32_BAND = 64.0
 
     def prune_mask(self, centers, feats, values, voxel_size, th=0.5, bits=8, rule=1, step=0.0,
-                   band=PRUNE_BAND):
+                   band=PRUNE_BAND, scores=True):
         """Exact pruning mask [V] (bool) for 0 < th < 1: rule 0 (the
         reference's, fairnr/modules/encoder.py:609-610) keeps voxels with
         1 - min exp(-relu sigma) > th, rule 1 those with max 1 - exp(-relu(sigma)
@@ -162,7 +162,10 @@ class TensorCoreMLP:
         are evaluated in FP32 with a band of `band` / FP32_BAND, and what that
         leaves in double-float (nsvf_prune_screen_bf16, nsvf_prune_fp32_dev,
         nsvf_prune_exact_dev). Also returns the BF16 scores (as prune_scores)
-        and the number of points that the BF16 pass left undecided."""
+        and the number of points that the BF16 pass left undecided. With
+        scores=False (the second result is then None) the BF16 pass first
+        takes a few points of every voxel and then all points of the voxels
+        that those do not keep."""
         if not 0.0 < th < 1.0:
             raise ValueError("pruning threshold must lie in (0, 1), got %r" % (th,))
         if rule == 1 and not step > 0.0:
@@ -171,24 +174,42 @@ class TensorCoreMLP:
         V = centers.size(0)
         dev = centers.device
         init = 0x7F800000 if rule == 0 else 0
-        score = torch.empty(V, dtype=torch.int32, device=dev)
+        score = torch.empty(V, dtype=torch.int32, device=dev) if scores else None
         keep = torch.empty(V, dtype=torch.uint8, device=dev)
         n_list = torch.empty(1, dtype=torch.int64, device=dev)
         err = ext.error_word(dev)
+        stream = ext.ctypes_stream(dev)
         # room for 3 % of the points (1.65 % of the c2 pass are undecided): a
         # second screen pass (7.5 ms there) costs more than the list
         cap = max(65536, V * bits ** 3 // 32)
+        # The points of the first pass, per axis: at most 1.6 % of them (on
+        # the c2 pass the corners keep 66 % of the voxels that are kept, and
+        # 4 points per axis 87 %)
+        sub = 4 if bits >= 12 else 2
+        live = torch.empty(V, dtype=torch.int32, device=dev) if not scores else None
+        n_live = torch.empty(1, dtype=torch.int64, device=dev) if not scores else None
+        common = (values.size(0), float(voxel_size), centers.data_ptr(), feats.data_ptr(),
+                  values.data_ptr(), self._wp, self._bp)
         for _ in range(3):
             lst = torch.empty(cap, dtype=torch.int64, device=dev)
-            score.fill_(init)
             keep.zero_()
             n_list.zero_()
             with ext._timed("prune_screen_bf16", dev):
-                check(LIB.nsvf_prune_screen_bf16(
-                    V, int(bits), int(rule), float(step), float(T), float(band), values.size(0),
-                    float(voxel_size), centers.data_ptr(), feats.data_ptr(), values.data_ptr(),
-                    self._wp, self._bp, score.data_ptr(), keep.data_ptr(), lst.data_ptr(),
-                    n_list.data_ptr(), cap, None, ext.ctypes_stream(dev)), "prune_screen_bf16")
+                if scores:
+                    score.fill_(init)
+                    check(LIB.nsvf_prune_screen_bf16(
+                        V, int(bits), int(rule), float(step), float(T), float(band), *common,
+                        score.data_ptr(), keep.data_ptr(), lst.data_ptr(), n_list.data_ptr(), cap,
+                        None, stream), "prune_screen_bf16")
+                else:
+                    for g, lv, nl in ((sub, None, None), (bits, live, n_live)):
+                        if lv is None and bits < 4:
+                            continue
+                        check(LIB.nsvf_prune_screen_live_bf16(
+                            V, int(bits), int(g), int(rule), float(T), float(band), *common,
+                            keep.data_ptr(), lv.data_ptr() if lv is not None else None,
+                            nl.data_ptr() if nl is not None else None, lst.data_ptr(),
+                            n_list.data_ptr(), cap, None, stream), "prune_screen_live_bf16")
             n = int(n_list.item())
             if n <= cap:
                 break
@@ -197,7 +218,6 @@ class TensorCoreMLP:
         # thousand), so FP32 decides what it can first: the c2 pass's 23.0 ms
         # of double-float become 0.39 ms of FP32 and 0.07 ms
         if n and band > 0.0 and 1e-30 < T < 1e30:
-            stream = ext.ctypes_stream(dev)
             # the weights of the double-float pass, as they are laid out there
             w = [t.t().contiguous() for t in self.wt32]
             packed = torch.empty(int(LIB.nsvf_field_train_packed_floats()), dtype=torch.float32,
@@ -221,7 +241,7 @@ class TensorCoreMLP:
                 centers.data_ptr(), feats.data_ptr(), values.data_ptr(), self._wtp, self._bp,
                 lst.data_ptr(), n_list.data_ptr(), cap, keep.data_ptr(), err.data_ptr(),
                 ext.ctypes_stream(dev)), "prune_exact_dev")
-        return keep.bool(), score.view(torch.float32), n
+        return keep.bool(), score.view(torch.float32) if scores else None, n
 
     def reference_bf16(self, emb):
         """torch emulation of the kernel's rounding: bf16 operands, FP32 sums

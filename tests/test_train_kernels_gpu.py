@@ -141,7 +141,8 @@ def test_other_widths_keep_the_general_path(cuda):
     assert out[0].shape == (5, 3)
 
 
-@pytest.mark.parametrize("n_vox,bits,rule", [(3, 4, 1), (40, 8, 1), (301, 8, 0), (9, 16, 0)])
+@pytest.mark.parametrize("n_vox,bits,rule", [(3, 4, 1), (40, 8, 1), (301, 8, 0), (9, 16, 0),
+                                             (500, 2, 1), (77, 5, 0)])
 def test_prune_fp32_stage_keeps_the_mask(cuda, n_vox, bits, rule):
     """prune_mask with its FP32 stage against float64 torch at every point,
     thresholds through the middle of the voxels' scores, so that many points
@@ -167,6 +168,11 @@ def test_prune_fp32_stage_keeps_the_mask(cuda, n_vox, bits, rule):
                                     step=step, band=band)
         ext.check_errors(cuda)
         assert torch.equal(keep, want) and n > 0
+        # a few points of every voxel first, then the rest's
+        keep2, none, _ = mlp.prune_mask(centers, feats, values, vs, th=th, bits=bits, rule=rule,
+                                        step=step, band=band, scores=False)
+        ext.check_errors(cuda)
+        assert torch.equal(keep2, want) and none is None
 
 
 @pytest.mark.parametrize("ns", [1, 7, 257, 90001])
