@@ -744,6 +744,19 @@ int nsvf_prune_exact_dev(int64_t n_voxels, int bits, int rule, double threshold,
                          const int64_t *n_list, int64_t list_cap, uint8_t *keep, int32_t *err,
                          void *stream);
 
+/* frame_begin: the background colour, depth and missed = 1 into a frame of n
+ * rays, the shared `origin` [3] (device; may be NULL) into ray_start [n, 3], and
+ * zeros into zero_words 8-byte words.
+ * compact_scan: nsvf_compact_hits without a prefix sum to prepare: pix and
+ * *n_hit from the flags in one pass; ws: nsvf_compact_scan_words(n) 8-byte
+ * words, zeroed by the caller (bit 8 of *err: a bounded wait gave up). */
+int nsvf_frame_begin(int64_t n, const float bg[3], float bg_depth, float *color, float *depth,
+                     float *missed, const float *origin, float *ray_start, void *zero,
+                     int64_t zero_words, void *stream);
+int64_t nsvf_compact_scan_words(int64_t n);
+int nsvf_compact_scan(int64_t n, const uint8_t *hits, int64_t *pix, int64_t *n_hit, void *ws,
+                      int32_t *err, void *stream);
+
 /* Training on compacted samples (fairnr/modules/encoder.py:558-592 and
  * fairnr/modules/renderer.py:94-126 under autograd, with per-chunk
  * recomputation). A batch's rows [rays, max_steps] are compacted once, the

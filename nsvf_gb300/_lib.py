@@ -98,6 +98,9 @@ def _load():
         "nsvf_field_refine_fp32_dev": ([P, P, i64, i64, P, P, i64, P, P, i64, i64, f32, P, P, P, P,
                                         P, P, P], i32),
         "nsvf_wait_timeout_selftest": ([ctypes.c_uint64, P, P], i32),
+        "nsvf_frame_begin": ([i64, P, f32, P, P, P, P, P, P, i64, P], i32),
+        "nsvf_compact_scan_words": ([i64], i64),
+        "nsvf_compact_scan": ([i64, P, P, P, P, P, P], i32),
         "nsvf_prune_screen_live_bf16": ([i64, i32, i32, i32, f32, f32, i64, f32, P, P, P, P, P, P,
                                          P, P, P, P, i64, P, P], i32),
         "nsvf_prune_fp32_dev": ([i64, i32, f32, f32, i64, f32, P, P, P, P, P, P, i64, P, P, P, P, P,
@@ -152,6 +155,7 @@ def exported_symbols():
         "nsvf_parallel_sampling_smem_bytes", "nsvf_pinhole_rays_multi", "nsvf_piece_rows",
         "nsvf_sample_count_pieces", "nsvf_sample_compact_pieces",
         "nsvf_sample_scan_bytes", "nsvf_sample_scan_compact_dev", "nsvf_sample_scan_compact_pieces",
+        "nsvf_frame_begin", "nsvf_compact_scan_words", "nsvf_compact_scan",
         "nsvf_prune_fp32_dev", "nsvf_prune_screen_live_bf16", "nsvf_train_rows_count", "nsvf_train_rows_pack", "nsvf_field_train_packed_floats",
         "nsvf_field_train_pack", "nsvf_field_train_forward", "nsvf_composite_rows",
         "nsvf_composite_rows_backward", "nsvf_field_train_backward_floats",

@@ -5,8 +5,8 @@ For one frame of rays of a resident scene:
 1. nsvf_svo_intersect_grid    -- the octree's hit lists in depth order from a
    sweep over the leaf grid (FP32, exact; nsvf_svo_intersect_sorted, the
    depth-first traversal + sort, for trees not in leaf-grid form)
-2. nsvf_compact_hits          -- order-preserving compaction of the hit rays
-   (on a torch prefix sum of the hit flags)
+2. nsvf_compact_scan          -- order-preserving compaction of the hit rays,
+   in one pass over the hit flags
 3. nsvf_gather_probs          -- the hit rays' lists and their sampling
    distribution (fairnr/models/nsvf.py:65-74), warp per ray
 4. nsvf_sample_scan_compact_dev -- the inverse-CDF walk (deterministic
@@ -18,7 +18,8 @@ For one frame of rays of a resident scene:
                                  tcgen05 BF16 field MLP (FP32 accumulation);
                                  embeddings and activations stay on chip
 6. nsvf_composite_segments    -- compensated transmittance compositing into
-                                 the frame (the background is filled first)
+                                 the frame (nsvf_frame_begin fills the
+                                 background first and zeroes the counters)
 
 With the tensor-core field the whole chain runs on device-side counts (hit
 rays, samples), so the host enqueues the frame while the traversal runs and
@@ -141,19 +142,23 @@ def _frame_buffers(scene, R, stream):
     def e(*shape, dtype=torch.float32):
         return torch.empty(*shape, dtype=dtype, device=dev)
 
+    # the samples' offsets, then the frame's counters (sample count = the last
+    # offset, hit rays, far-outside samples, refined rays, error bits), read
+    # back with one copy, then the compaction's words: one range to zero
+    words = R + 1 + 4 + int(LIB.nsvf_compact_scan_words(R))
+    off = torch.zeros(words, dtype=i64, device=dev)
     b = {"R": R, "ro": e(R, 3), "idx": e(R, H, dtype=i32), "lo": e(R, H), "hi": e(R, H),
-         "hits": e(R, dtype=torch.uint8), "scan": e(R, dtype=i32), "pix": e(R, dtype=i64),
-         "n_hit": e(1, dtype=i64), "I": e(R, H, dtype=i32), "L": e(R, H), "U": e(R, H),
+         "hits": e(R, dtype=torch.uint8), "pix": e(R, dtype=i64),
+         "n_hit": off[R + 1:R + 2], "I": e(R, H, dtype=i32), "L": e(R, H), "U": e(R, H),
          "probs": e(R, H), "steps": e(R), "count": e(R, dtype=i32),
-         "offset": torch.zeros(R + 1, dtype=i64, device=dev),
+         "offset": off[:R + 1], "counts": off[R:R + 5], "zero": off[R:], "scan_words": off[R + 5:],
          "scan_ws": torch.empty(int(LIB.nsvf_sample_scan_bytes(R)), dtype=torch.uint8, device=dev),
          "ws": ext._svo_workspace(1, scene.octree_centers.shape[0], dev),
          "bg": torch.tensor(list(scene.bg), dtype=torch.float32, device=dev),
-         "err": torch.zeros(1, dtype=i32, device=dev),
-         "counts_host": torch.zeros(4, dtype=i64).pin_memory(),
-         "err_host": torch.zeros(1, dtype=i32).pin_memory(), "cap": 0,
-         "n_outl": torch.zeros(1, dtype=i64, device=dev), "outl": None, "outl_cap": 0,
-         "n_refine": torch.zeros(1, dtype=i64, device=dev)}
+         "err": off[R + 4:R + 5].view(i32)[:1],
+         "counts_host": torch.zeros(5, dtype=i64).pin_memory(), "cap": 0,
+         "n_outl": off[R + 2:R + 3], "outl": None, "outl_cap": 0,
+         "n_refine": off[R + 3:R + 4]}
     frames[stream] = b
     return b
 
@@ -199,11 +204,10 @@ def _exact_pass(scene, b, R, ro, rd, vox, xyzd, depth, field, err, stream, cap, 
     field in double-float, written over `field`; then the rays whose listed
     sample's colour exceeds REFINE_ABOVE get their other samples in FP32
     (nsvf_field_refine_fp32_dev). The second half of the outlier buffer holds
-    those rays."""
+    those rays (counted in b["n_refine"], zero before)."""
     m = scene.mlp
     ocap = b["outl_cap"]
     rows = b["outl"][ocap:]
-    b["n_refine"].zero_()
     with ext._timed("field_exact", scene.device):
         check(LIB.nsvf_field_exact_dev(R, _p(b["n_hit"]), _p(b["offset"]), _p(b["pix"]), _p(ro), 3,
                                        _p(rd), _p(depth), _p(vox), scene.centers.size(0),
@@ -255,7 +259,7 @@ def _count(scene, b, R, stream):
         check(LIB.nsvf_sample_count_dev(R, _p(b["n_hit"]), scene.max_hits, _p(b["I"]), _p(b["L"]),
                                         _p(b["U"]), _p(b["probs"]), _p(b["steps"]), _p(b["count"]),
                                         stream), "sample_count_dev")
-    torch.cumsum(b["count"], 0, out=b["offset"][1:])
+    torch.cumsum(b["count"], 0, out=b["offset"][1:])   # (up to offset[R])
 
 
 def _samples_on_device(scene, b, R, ro, rd, out, mlp, kahan, exact, stream):
@@ -267,17 +271,16 @@ def _samples_on_device(scene, b, R, ro, rd, out, mlp, kahan, exact, stream):
     composited again with room for all of them."""
     dev = scene.device
     err = b["err"]
-    counts, err_h = b["counts_host"], b["err_host"]
+    counts = b["counts_host"]
     cap = max(b["cap"], INITIAL_SAMPLES_PER_RAY * R)
     ocap = max(b["outl_cap"], INITIAL_OUTLIERS)
-    for _ in range(3):
+    for attempt in range(3):
         vox, xyzd, depth, field = _sample_buffers(b, cap)
         cap = b["cap"]
         outl, ocap = _outlier_list(b, ocap) if exact else (None, 0)
         n_outl = b["n_outl"] if exact else None
-        err.zero_()
-        if exact:
-            n_outl.zero_()
+        if attempt:                          # (nsvf_frame_begin zeroed them)
+            b["counts"][2:].zero_()
         if scene.max_hits <= SCAN_MAX_HITS:
             _scan_compact(scene, b, R, ro, rd, cap, vox, xyzd, depth, _p(err), stream)
         else:
@@ -306,16 +309,9 @@ def _samples_on_device(scene, b, R, ro, rd, out, mlp, kahan, exact, stream):
                 R, _p(b["n_hit"]), _p(b["offset"]), cap, _p(field), _p(xyzd), _p(depth), _p(b["pix"]),
                 7.0, scene.bg, scene.bg_depth, _p(out["colors"]), _p(out["depths"]),
                 _p(out["missed"]), int(bool(kahan)), stream), "composite_segments_dev")
-        counts[0:1].copy_(b["n_hit"], non_blocking=True)
-        counts[1:2].copy_(b["offset"][R:], non_blocking=True)
-        if exact:
-            counts[2:3].copy_(n_outl, non_blocking=True)
-            counts[3:4].copy_(b["n_refine"], non_blocking=True)
-        err_h.copy_(err, non_blocking=True)
+        counts.copy_(b["counts"], non_blocking=True)
         torch.cuda.current_stream(dev).synchronize()
-        n, ns, e = int(counts[0]), int(counts[1]), int(err_h[0])
-        n_far = int(counts[2]) if exact else 0
-        n_ref = int(counts[3]) if exact else 0
+        ns, n, n_far, n_ref, e = counts.tolist()
         if not (e & (2 | 16)):
             break
         if e & 2:
@@ -369,11 +365,22 @@ def render_frame(scene, ray_start, ray_dir, kahan=True, out=None, mlp="tc", exac
     stream = ext.ctypes_stream(dev)
     b = _frame_buffers(scene, R, stream)
     rd = ray_dir.float().contiguous()
+    # one launch for the background, the shared origin and the counters, for
+    # outputs and origins in the form that the kernel writes and reads
+    plain = lambda t, *shape: t.dtype == torch.float32 and t.device == dev and \
+        t.is_contiguous() and t.shape == shape
+    fill = all(plain(out[k], R, *s) for k, s in (("colors", (3,)), ("depths", ()), ("missed", ())))
+    spread = fill and ray_start.dim() == 1 and plain(ray_start, 3)
     if ray_start.dim() == 1:
         ro = b["ro"]
-        ro.copy_(ray_start.float().reshape(1, 3).expand(R, 3))
+        if not spread:
+            ro.copy_(ray_start.float().reshape(1, 3).expand(R, 3))
     else:
         ro = ray_start.float().contiguous()
+    o3 = (out["colors"], out["depths"], out["missed"]) if fill else (None,) * 3
+    check(LIB.nsvf_frame_begin(R if fill else 0, scene.bg, scene.bg_depth, *map(_p, o3),
+                               _p(ray_start) if spread else None, _p(ro), _p(b["zero"]),
+                               b["zero"].numel(), stream), "frame_begin")
     err = _p(ext.error_word(dev))
     n_nodes = scene.octree_centers.shape[0]
     if traversal == "grid" and scene.svo_grid.ok:
@@ -389,25 +396,24 @@ def render_frame(scene, ray_start, ray_dir, kahan=True, out=None, mlp="tc", exac
                                                 _p(b["lo"]), _p(b["hi"]), _p(b["hits"]), err,
                                                 _p(b["ws"]), stream), "svo_intersect_sorted")
     with ext._timed("hit_rows", dev):
-        torch.cumsum(b["hits"], 0, dtype=torch.int32, out=b["scan"])
-        check(LIB.nsvf_compact_hits(R, _p(b["hits"]), _p(b["scan"]), _p(b["pix"]), _p(b["n_hit"]),
-                                    stream), "compact_hits")
+        check(LIB.nsvf_compact_scan(R, _p(b["hits"]), _p(b["pix"]), _p(b["n_hit"]),
+                                    _p(b["scan_words"]), err, stream), "compact_scan")
         check(LIB.nsvf_gather_probs(R, _p(b["n_hit"]), H, scene.step_size, _p(b["pix"]),
                                     _p(b["idx"]), _p(b["lo"]), _p(b["hi"]), _p(b["I"]), _p(b["L"]),
                                     _p(b["U"]), _p(b["probs"]), _p(b["steps"]), stream),
               "gather_probs")
-    out["colors"].copy_(b["bg"].expand(R, 3))
-    out["depths"].fill_(scene.bg_depth)
-    out["missed"].fill_(1.0)
+    if not fill:
+        out["colors"].copy_(b["bg"].expand(R, 3))
+        out["depths"].fill_(scene.bg_depth)
+        out["missed"].fill_(1.0)
     if mlp in ("tc", "tc_fp8"):
         return _samples_on_device(scene, b, R, ro, rd, out, mlp, kahan, exact, stream)
     _count(scene, b, R, stream)
     offset = b["offset"]
     counts = b["counts_host"]
-    counts[0:1].copy_(b["n_hit"], non_blocking=True)
-    counts[1:2].copy_(offset[R:], non_blocking=True)
+    counts.copy_(b["counts"], non_blocking=True)
     torch.cuda.current_stream(dev).synchronize()
-    n, ns = int(counts[0]), int(counts[1])
+    ns, n = counts.tolist()[:2]
     out["n_hit_rays"], out["n_samples"] = n, ns
     if n == 0:
         return out

@@ -400,3 +400,52 @@ def test_scan_compact_equals_two_pass(cuda, rows):
         assert torch.equal(v1[:k], v2[:k]) and torch.equal(d1[:k], d2[:k])
         assert torch.equal(x1[:k], x2[:k])
         assert bool((v1[k:] == -7).all())
+
+
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 33000, 640000])
+@pytest.mark.parametrize("fill", [0.0, 0.01, 0.6, 1.0])
+def test_compact_scan_equals_nonzero(cuda, n, fill):
+    """The one-pass compaction of the hit flags (chunks of 1,024) against
+    torch.nonzero, with frame_begin's fills and zeros before it."""
+    import ctypes
+    from nsvf_gb300 import ext
+    from nsvf_gb300._lib import LIB, check
+    g = torch.Generator(device="cuda").manual_seed(n)
+    hits = (torch.rand(n, generator=g, device=cuda) < fill).to(torch.uint8)
+    words = int(LIB.nsvf_compact_scan_words(n))
+    ws = torch.full((words + 3,), -1, dtype=torch.int64, device=cuda)
+    col, dep, mis = torch.empty(n, 3, device=cuda), torch.empty(n, device=cuda), torch.empty(n, device=cuda)
+    ro, o = torch.empty(n, 3, device=cuda), torch.tensor([1.0, -2.0, 3.0], device=cuda)
+    stream = ext.ctypes_stream(cuda)
+    check(LIB.nsvf_frame_begin(n, (ctypes.c_float * 3)(0.25, 0.5, 0.75), 5.0, col.data_ptr(),
+                               dep.data_ptr(), mis.data_ptr(), o.data_ptr(), ro.data_ptr(),
+                               ws.data_ptr(), words, stream), "frame_begin")
+    assert int(ws[:words].abs().sum()) == 0 and int((ws[words:] + 1).abs().sum()) == 0
+    assert torch.equal(col, torch.tensor([0.25, 0.5, 0.75], device=cuda).expand(n, 3))
+    assert bool((dep == 5.0).all()) and bool((mis == 1.0).all()) and torch.equal(ro, o.expand(n, 3))
+    pix = torch.full((n,), -1, dtype=torch.int64, device=cuda)
+    n_hit = torch.full((1,), -1, dtype=torch.int64, device=cuda)
+    check(LIB.nsvf_compact_scan(n, hits.data_ptr(), pix.data_ptr(), n_hit.data_ptr(), ws.data_ptr(),
+                                ext.error_word(cuda).data_ptr(), stream), "compact_scan")
+    ref = hits.nonzero()[:, 0]
+    ext.check_errors(cuda)
+    assert int(n_hit) == ref.numel() and torch.equal(pix[:ref.numel()], ref)
+    assert bool((pix[ref.numel():] == -1).all())
+
+
+def test_frame_outputs_in_other_forms(cuda):
+    """Origins and output tensors that the one-launch start of a frame does
+    not take (strided, another dtype) still give the same frame."""
+    from nsvf_gb300 import scenes
+    from nsvf_gb300.served import SceneState, render_frame
+    enc, field, _, _ = _scene(cuda, 0.25, 1.0, 60.0, 0.5, 20)
+    sc = SceneState(enc, field)
+    rs, rd = (torch.from_numpy(a).to(cuda) for a in scenes.small_view(0))
+    ref = render_frame(sc, rs, rd)
+    a = render_frame(sc, rs.double(), rd)
+    wide = torch.zeros(6, device=cuda)
+    wide[::2] = rs
+    b = render_frame(sc, wide[::2], rd)
+    for o in (a, b):
+        for k in ("colors", "depths", "missed"):
+            assert torch.equal(o[k], ref[k])
