@@ -565,8 +565,8 @@ __global__ void __launch_bounds__(kGridBlock) svo_grid_kernel(
     float *__restrict__ min_depth, float *__restrict__ max_depth, uint8_t *__restrict__ hits,
     int32_t *__restrict__ list, int32_t *__restrict__ n_list, int32_t *__restrict__ over,
     int32_t *__restrict__ over_cnt, int32_t *__restrict__ n_over, OverHit *__restrict__ scratch,
-    int over_cap, unsigned long long *__restrict__ next_ray, bool pad_rows) {
-  // Persistent warps: each warp takes the next 32 rays from a global
+    int over_cap, unsigned long long *__restrict__ next_ray, int take, bool pad_rows) {
+  // Persistent warps: each warp takes the next `take` rays from a global
   // counter until there are none left, so the SMs stay full to the end of
   // the frame (rays differ a lot in length: fixed blocks left the SMs active
   // 57 % of the time, with 7 of 20 possible warps resident on average). A
@@ -576,11 +576,11 @@ __global__ void __launch_bounds__(kGridBlock) svo_grid_kernel(
   const unsigned full = 0xffffffffu;
   for (;;) {
     unsigned long long base0 = 0;
-    if (lane == 0) base0 = atomicAdd(next_ray, 32ull);
+    if (lane == 0) base0 = atomicAdd(next_ray, (unsigned long long)take);
     const int64_t base = (int64_t)__shfl_sync(full, base0, 0);
     if (base >= rays) break;
     const int64_t r = base + lane;
-    const bool live = r < rays;
+    const bool live = lane < take && r < rays;
     const int64_t rr = live ? r : 0;
     RowEmit em{idx + rr * n_max, min_depth + rr * n_max, max_depth + rr * n_max, G.rank_of,
                n_max, 0, -1.0f, n_over, scratch, over_cap, -1, 0};
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(kGridBlock) svo_grid_kernel(
     }
     // pad the rows (misses: id -1, depths 10000), a warp per row
     const bool pad = live && st == kSweepDone && em.q < 0;
-    for (int q = 0; q < 32; ++q) {
+    for (int q = 0; q < take; ++q) {
       const int cq = __shfl_sync(full, em.cnt, q);
       if (!__shfl_sync(full, (int)pad, q)) continue;
       const int64_t rq = base + q;
@@ -822,12 +822,22 @@ int nsvf_svo_intersect_grid_rows(int64_t rays, int n, float voxelsize, int n_max
   G.points = points;
   G.children = children;
   G.hv = voxelsize * 0.5f;
-  const int64_t need = (rays + kGridBlock - 1) / kGridBlock;
+  // A warp takes the fewest rays (1 to 32) that leave no more warps than the
+  // device holds at once: a few rays are bound by each one's own chain of
+  // cells, which the other lanes of its warp, at other places of the code,
+  // only make longer. c2 rays: 2,048 that all hit 528 -> 188 us (32 -> 1 rays a
+  // warp), 8,192 532 -> 313 (2), 20,000 at voxel 1/32 333 -> 271 (8); a view's
+  // 65,536 473 -> 412 (16), 262,144 535 (32; 599 with 16).
+  const int64_t warps = (int64_t)g_grid_blocks[dev] * (kGridBlock / 32);
+  int take = 1;
+  while (take < 32 && rays > warps * take) take <<= 1;
+  const int64_t per_block = (int64_t)take * (kGridBlock / 32);
+  const int64_t need = (rays + per_block - 1) / per_block;
   const int blocks = (int)(need < g_grid_blocks[dev] ? need : g_grid_blocks[dev]);
   svo_grid_kernel<<<blocks, kGridBlock, 0, s>>>(rays, n_max, ray_start, ray_dir, G, idx,
                                                 min_depth, max_depth, hits, list, n_list, over,
                                                 over_cnt, n_over, scratch, (int)over_cap,
-                                                next_ray, pad_rows != 0);
+                                                next_ray, take, pad_rows != 0);
   st = nsvf_launch_status();
   if (st != NSVF_OK) return st;
   // the overflow rays: their count is on the device; 8 blocks of 4 warps per

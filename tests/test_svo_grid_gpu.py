@@ -210,3 +210,23 @@ def test_served_frame_same_with_either_traversal(cuda):
     for k in ["colors", "depths", "missed"]:
         assert torch.equal(a[k], b[k]), k
     assert a["n_samples"] == b["n_samples"] > 0
+
+
+@pytest.mark.parametrize("rays", [1, 33, 2047, 4099, 9000, 40000, 150000])
+def test_rays_per_warp(cuda, rays):
+    """Few rays are spread over more warps (1 to 32 rays each): the same lists
+    as the depth-first kernel at counts on both sides of each step."""
+    from nsvf_gb300 import ext, geometry, scenes
+    p, vs = scenes.scene_shell(1.0 / 32)
+    cen, chi = (t.to(cuda) for t in geometry.build_easy_octree(torch.from_numpy(p), vs / 2))
+    grid = ext.SvoGrid(cen, chi, vs)
+    rng = np.random.RandomState(rays)
+    o = rng.normal(size=(rays, 3))
+    o = 3 * o / np.linalg.norm(o, axis=1, keepdims=True)
+    d = -o + rng.normal(scale=0.3, size=(rays, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    ro, rd = (torch.from_numpy(a.astype(np.float32)).to(cuda) for a in (o, d))
+    ref = ext.svo_intersect_sorted(ro[None], rd[None], cen[None], chi[None], vs, 24)
+    for a, b in zip(ext.svo_intersect_grid(grid, ro, rd, 24), ref):
+        assert torch.equal(a, b)
+    ext.check_errors(cuda)
