@@ -226,6 +226,14 @@ int nsvf_uniform_ray_sampling(int b, int m, int max_hits, int max_steps, float s
                               const float *max_depth, const float *noise, int32_t *sampled_idx,
                               float *sampled_depth, float *sampled_dists, int32_t *err,
                               void *stream);
+/* ... and the largest number of samples (id != -1) of a row into *max_len (device,
+ * zeroed by the caller; may be NULL). */
+int nsvf_uniform_ray_sampling_len(int b, int m, int max_hits, int max_steps, float step_size,
+                                  const int32_t *pts_idx, const float *min_depth,
+                                  const float *max_depth, const float *noise,
+                                  int32_t *sampled_idx, float *sampled_depth,
+                                  float *sampled_dists, int32_t *max_len, int32_t *err,
+                                  void *stream);
 
 /* parallel_ray_sampling: the reference's back-up uniform sampler
  * (`_parallel_ray_sampling`, fairnr/clib/__init__.py:303-349, pure torch

@@ -47,6 +47,8 @@ def _load():
         "nsvf_ball_intersect": ([i32, i32, i32, i32, f32, i32, P, P, P, P, P, P, P], i32),
         "nsvf_triangle_intersect": ([i32, i32, i32, i32, f32, f32, i32, P, P, P, P, P, P, P], i32),
         "nsvf_uniform_ray_sampling": ([i32, i32, i32, i32, f32, P, P, P, P, P, P, P, P, P], i32),
+        "nsvf_uniform_ray_sampling_len": ([i32, i32, i32, i32, f32, P, P, P, P, P, P, P, P, P, P],
+                                          i32),
         "nsvf_inverse_cdf_sampling": ([i64, i32, i32, i32, f32, P, P, P, P, P, P, P, P, P, P,
                                        P, P, P], i32),
         "nsvf_build_octree": ([P, P, i64, i32, P, P, i64], i64),
@@ -155,8 +157,9 @@ def exported_symbols():
         "nsvf_parallel_sampling_smem_bytes", "nsvf_pinhole_rays_multi", "nsvf_piece_rows",
         "nsvf_sample_count_pieces", "nsvf_sample_compact_pieces",
         "nsvf_sample_scan_bytes", "nsvf_sample_scan_compact_dev", "nsvf_sample_scan_compact_pieces",
-        "nsvf_frame_begin", "nsvf_compact_scan_words", "nsvf_compact_scan",
-        "nsvf_prune_fp32_dev", "nsvf_prune_screen_live_bf16", "nsvf_train_rows_count", "nsvf_train_rows_pack", "nsvf_field_train_packed_floats",
+        "nsvf_uniform_ray_sampling_len", "nsvf_frame_begin", "nsvf_compact_scan_words",
+        "nsvf_compact_scan", "nsvf_prune_fp32_dev", "nsvf_prune_screen_live_bf16",
+        "nsvf_train_rows_count", "nsvf_train_rows_pack", "nsvf_field_train_packed_floats",
         "nsvf_field_train_pack", "nsvf_field_train_forward", "nsvf_composite_rows",
         "nsvf_composite_rows_backward", "nsvf_field_train_backward_floats",
         "nsvf_field_train_backward",

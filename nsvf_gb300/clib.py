@@ -15,6 +15,8 @@ work reaches the GPU:
   layout parameters, and the noise tensor is drawn with the same shape and
   torch RNG calls, so results are identical for the same seed.
 """
+import math
+
 import numpy as np
 import torch
 from torch.autograd import Function
@@ -121,22 +123,19 @@ class UniformRaySampling(Function):
         H = int(np.ceil(N / G)) * G
         max_steps = int(max_ray_length / step_size) + P * 2
         # noise drawn exactly as the reference: [G, H/G, max_steps], U(0, 1)
-        noise = min_depth.new_zeros(H, max_steps)
-        if deterministic:
-            noise += 0.5
-        else:
-            noise = noise.uniform_()
+        noise = min_depth.new_empty(H, max_steps)
+        noise = noise.fill_(0.5) if deterministic else noise.uniform_()
+        max_len = torch.zeros(1, dtype=torch.int32, device=pts_idx.device)
         # the reference pads rows by repeating the FIRST H-N rows; rows are
         # independent except that a jitter of exactly 0 reads the previous
         # row's last id, which is the same element here
         si, sd, ss = ext.uniform_ray_sampling(
             pts_idx.int().contiguous().view(1, N, P), min_depth.float().contiguous().view(1, N, P),
             max_depth.float().contiguous().view(1, N, P),
-            noise.float()[:N].contiguous().view(1, N, max_steps), float(step_size), max_steps)
+            noise.float()[:N].contiguous().view(1, N, max_steps), float(step_size), max_steps,
+            max_len)
         si, sd, ss = si.view(N, -1), sd.view(N, -1).type_as(min_depth), ss.view(N, -1).type_as(min_depth)
-        ext.check_errors(pts_idx.device)
-        max_len = si.ne(-1).sum(-1).max()
-        si, sd, ss = _truncate(si, sd, ss, max_len)
+        si, sd, ss = _truncate(si, sd, ss, ext.check_errors_with(max_len))
         ctx.mark_non_differentiable(si, sd, ss)
         return si, sd, ss
 
@@ -161,13 +160,17 @@ class InverseCDFRaySampling(Function):
                 deterministic=False):
         G, N, P = 200, pts_idx.size(0), pts_idx.size(1)
         H = int(np.ceil(N / G)) * G
-        # max_steps over the padded rows (padding copies row 0): same as over N
-        max_steps = int(steps.ceil().long().max()) + P
+        # max_steps over the padded rows (padding copies row 0): same as over
+        # N; ceil keeps the order, so it comes after the maximum (a NaN, which
+        # the maximum would pass on, before it)
+        most = steps.max().item()
+        most = int(math.ceil(most)) if math.isfinite(most) else int(steps.ceil().long().max())
+        max_steps = most + P
         if deterministic:
             noise = None   # the kernel's built-in 0.5 jitter
         else:
             # drawn exactly as the reference: [G, H/G, max_steps], clamped
-            noise = min_depth.new_zeros(H, max_steps).uniform_().clamp(min=0.001, max=0.999)
+            noise = min_depth.new_empty(H, max_steps).uniform_().clamp_(min=0.001, max=0.999)
             noise = noise.float()
         dev = pts_idx.device
         max_len = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -177,9 +180,7 @@ class InverseCDFRaySampling(Function):
             steps.float().contiguous(), float(fixed_step_size), inverse_cdf_layout(N),
             max_steps, max_len)
         sd, ss = sd.type_as(min_depth), ss.type_as(min_depth)
-        ext.check_errors(dev)
-        L = int(max_len.item())
-        si, sd, ss = _truncate(si, sd, ss, L)
+        si, sd, ss = _truncate(si, sd, ss, ext.check_errors_with(max_len))
         ctx.mark_non_differentiable(si, sd, ss)
         return si, sd, ss
 

@@ -863,7 +863,7 @@ __global__ void __launch_bounds__(32 * kScanWarps) icdf_scan_kernel(
 // starts, interval ends and jittered steps into one sorted depth list in the
 // output row, then turn it into midpoints/lengths and keep those inside a
 // voxel, compacting in place. Returns true when the row has no room for the
-// whole list.
+// whole list; `valid` gets the number of samples (id != -1).
 __device__ __forceinline__ bool uniform_walk(int64_t r, int H, int M, float step_size,
                                              const int32_t *__restrict__ pts_idx,
                                              const float *__restrict__ min_depth,
@@ -871,7 +871,8 @@ __device__ __forceinline__ bool uniform_walk(int64_t r, int H, int M, float step
                                              const float *__restrict__ noise,
                                              int32_t *__restrict__ s_idx,
                                              float *__restrict__ s_depth,
-                                             float *__restrict__ s_dist) {
+                                             float *__restrict__ s_dist, int &valid) {
+  valid = 0;
   const int32_t *I = pts_idx + r * H;
   const float *lo = min_depth + r * H, *hi = max_depth + r * H;
   const float *U = noise + r * M;
@@ -914,7 +915,9 @@ __device__ __forceinline__ bool uniform_walk(int64_t r, int H, int M, float step
     if (umax < H && SD[ucur] >= hi[umax] && I[umax] > -1) umax++;
     if (umax == H || I[umax] == -1) break;
     if (umin - 1 == umax && SS[ucur] > 0) {
-      SD[step] = SD[ucur]; SS[step] = SS[ucur]; SI[step] = SI[ucur]; step++;
+      SD[step] = SD[ucur]; SS[step] = SS[ucur]; SI[step] = SI[ucur];
+      valid += SI[step] != -1;
+      step++;
     }
   }
   for (int q = step; q < M; ++q) SI[q] = -1;
@@ -925,13 +928,15 @@ __global__ void __launch_bounds__(kBlock) uniform_kernel(
     int64_t rows, int H, int M, float step_size, const int32_t *__restrict__ pts_idx,
     const float *__restrict__ min_depth, const float *__restrict__ max_depth,
     const float *__restrict__ noise, int32_t *__restrict__ s_idx, float *__restrict__ s_depth,
-    float *__restrict__ s_dist, int32_t *__restrict__ err) {
+    float *__restrict__ s_dist, int32_t *__restrict__ max_len, int32_t *__restrict__ err) {
   int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-  if (r >= rows) return;
-  if (uniform_walk(r, H, M, step_size, pts_idx, min_depth, max_depth, noise, s_idx, s_depth,
-                   s_dist) &&
+  int valid = 0;
+  if (r < rows && uniform_walk(r, H, M, step_size, pts_idx, min_depth, max_depth, noise, s_idx,
+                               s_depth, s_dist, valid) &&
       err)
     atomicOr(err, 2);
+  valid = __reduce_max_sync(0xffffffffu, valid);
+  if ((threadIdx.x & 31) == 0 && max_len) atomicMax(max_len, valid);
 }
 
 __device__ __forceinline__ int warp_min_scan(int x, int lane) {
@@ -990,13 +995,14 @@ __global__ void __launch_bounds__(32 * kWarpRays) uniform_warp_kernel(
     int64_t rows, int H, int M, float step_size, const int32_t *__restrict__ pts_idx,
     const float *__restrict__ min_depth, const float *__restrict__ max_depth,
     const float *__restrict__ noise, int32_t *__restrict__ s_idx, float *__restrict__ s_depth,
-    float *__restrict__ s_dist, int32_t *__restrict__ err) {
+    float *__restrict__ s_dist, int32_t *__restrict__ max_len, int32_t *__restrict__ err) {
   __shared__ UniRow tabs[kWarpRays];
   const uint32_t full = 0xffffffffu;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t below = (1u << lane) - 1u;
   UniRow &T = tabs[wib];
   const int64_t stride = (int64_t)gridDim.x * kWarpRays;
+  int longest = 0;
   for (int64_t r = (int64_t)blockIdx.x * kWarpRays + wib; r < rows; r += stride) {
     const float *U = noise + r * M;
     int32_t *SI = s_idx + r * M;
@@ -1048,9 +1054,11 @@ __global__ void __launch_bounds__(32 * kWarpRays) uniform_warp_kernel(
       }
     }
     if (!fine) {
+      int valid = 0;
       if (lane == 0)
         over = uniform_walk(r, H, M, step_size, pts_idx, min_depth, max_depth, noise, s_idx,
-                            s_depth, s_dist);
+                            s_depth, s_dist, valid);
+      longest = max(longest, valid);         // lane 0's count
       if (lane == 0 && over && err) atomicOr(err, 2);
       continue;
     }
@@ -1097,7 +1105,7 @@ __global__ void __launch_bounds__(32 * kWarpRays) uniform_warp_kernel(
     int32_t id, nid;
     int n_hi, n_lo, nn_hi, nn_lo;
     int lo_min = 1, hi_min = 1;              // running minima of n_e - e
-    int kept = 0;
+    int kept = 0, valid = 0;
     bool stopped = false;
     events(0, val, id, n_hi, n_lo);
     for (int e0 = 0; e0 < E; e0 += 32) {
@@ -1136,13 +1144,16 @@ __global__ void __launch_bounds__(32 * kWarpRays) uniform_warp_kernel(
         SI[q] = id; SD[q] = mid; SS[q] = len;
       }
       kept += __popc(km);
+      valid += __popc(__ballot_sync(full, keep && id != -1));
       stopped = stopped || stops != 0;
       __syncwarp();
       val = nval; id = nid; n_hi = nn_hi; n_lo = nn_lo;
     }
     for (int q = (E + 31) / 32 * 32 + lane; q < M; q += 32) { SI[q] = -1; SD[q] = 0.0f; SS[q] = 0.0f; }
     if (lane == 0 && over && err) atomicOr(err, 2);
+    longest = max(longest, valid);
   }
+  if (lane == 0 && max_len) atomicMax(max_len, longest);
 }
 
 // Parallel uniform sampler: the pure-torch backup sampler of the reference's
@@ -1528,6 +1539,17 @@ int nsvf_uniform_ray_sampling(int b, int m, int max_hits, int max_steps, float s
                               const float *max_depth, const float *noise, int32_t *sampled_idx,
                               float *sampled_depth, float *sampled_dists, int32_t *err,
                               void *stream) {
+  return nsvf_uniform_ray_sampling_len(b, m, max_hits, max_steps, step_size, pts_idx, min_depth,
+                                       max_depth, noise, sampled_idx, sampled_depth, sampled_dists,
+                                       nullptr, err, stream);
+}
+
+int nsvf_uniform_ray_sampling_len(int b, int m, int max_hits, int max_steps, float step_size,
+                                  const int32_t *pts_idx, const float *min_depth,
+                                  const float *max_depth, const float *noise,
+                                  int32_t *sampled_idx, float *sampled_depth,
+                                  float *sampled_dists, int32_t *max_len, int32_t *err,
+                                  void *stream) {
   if (b < 0 || m < 0 || max_hits < 1 || max_steps < 1 || !pts_idx || !min_depth || !max_depth ||
       !noise || !sampled_idx || !sampled_depth || !sampled_dists)
     return NSVF_ERR_INVALID;
@@ -1537,11 +1559,11 @@ int nsvf_uniform_ray_sampling(int b, int m, int max_hits, int max_steps, float s
   if (max_hits <= kMaxH)
     uniform_warp_kernel<<<warp_grid(rows), 32 * kWarpRays, 0, (cudaStream_t)stream>>>(
         rows, max_hits, max_steps, step_size, pts_idx, min_depth, max_depth, noise, sampled_idx,
-        sampled_depth, sampled_dists, err);
+        sampled_depth, sampled_dists, max_len, err);
   else
     uniform_kernel<<<nsvf_grid(rows, kBlock), kBlock, 0, (cudaStream_t)stream>>>(
         rows, max_hits, max_steps, step_size, pts_idx, min_depth, max_depth, noise, sampled_idx,
-        sampled_depth, sampled_dists, err);
+        sampled_depth, sampled_dists, max_len, err);
   return nsvf_launch_status();
 }
 

@@ -32,11 +32,15 @@ KERNEL_TIMING = False
 kernel_events = []
 
 
-@contextlib.contextmanager
+_untimed = contextlib.nullcontext()
+
+
 def _timed(name, device):
-    if not KERNEL_TIMING:
-        yield
-        return
+    return _events(name, device) if KERNEL_TIMING else _untimed
+
+
+@contextlib.contextmanager
+def _events(name, device):
     s = torch.cuda.Event(enable_timing=True)
     e = torch.cuda.Event(enable_timing=True)
     s.record(torch.cuda.current_stream(device))
@@ -65,7 +69,10 @@ def _stream(t):
 
 
 def ctypes_stream(device):
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream's handle on `device` (the call behind
+    torch.cuda.current_stream, without the Stream object around it)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def error_word(device):
@@ -98,6 +105,15 @@ def check_errors(device=None):
         if v & 16:
             what.append("more samples far outside their voxel than the outlier list holds")
         raise RuntimeError("nsvf_gb300: " + "; ".join(what))
+
+
+def check_errors_with(value):
+    """check_errors on `value`'s device, and the int32 tensor `value` [1] as an
+    int, with one read for both."""
+    v, bits = torch.cat((value, error_word(value.device))).tolist()
+    if bits:
+        check_errors(value.device)
+    return v
 
 
 def _ptr(t):
@@ -335,8 +351,10 @@ def triangle_intersect(ray_start, ray_dir, face_points, cagesize, blur, n_max):
     return idx, depth, uv
 
 
-def uniform_ray_sampling(pts_idx, min_depth, max_depth, uniform_noise, step_size, max_steps):
-    """fairnr/clib/src/sample.cpp:23-55: -> (sampled_idx, sampled_depth, sampled_dists) [B, M, max_steps]."""
+def uniform_ray_sampling(pts_idx, min_depth, max_depth, uniform_noise, step_size, max_steps,
+                         max_len=None):
+    """fairnr/clib/src/sample.cpp:23-55: -> (sampled_idx, sampled_depth, sampled_dists) [B, M, max_steps].
+    max_len, if given (one int32, zeroed): the largest number of samples of a row."""
     _check_int("pts_idx", pts_idx)
     for n, t in (("min_depth", min_depth), ("max_depth", max_depth),
                  ("uniform_noise", uniform_noise)):
@@ -350,10 +368,10 @@ def uniform_ray_sampling(pts_idx, min_depth, max_depth, uniform_noise, step_size
     si = torch.empty(B, M, max_steps, dtype=torch.int32, device=dev)
     sd = torch.empty(B, M, max_steps, dtype=torch.float32, device=dev)
     ss = torch.empty(B, M, max_steps, dtype=torch.float32, device=dev)
-    check(LIB.nsvf_uniform_ray_sampling(B, M, H, int(max_steps), float(step_size), _ptr(pts_idx),
-                                        _ptr(min_depth), _ptr(max_depth), _ptr(uniform_noise),
-                                        _ptr(si), _ptr(sd), _ptr(ss), _ptr(error_word(dev)),
-                                        _stream(pts_idx)), "uniform_ray_sampling")
+    check(LIB.nsvf_uniform_ray_sampling_len(
+        B, M, H, int(max_steps), float(step_size), _ptr(pts_idx), _ptr(min_depth),
+        _ptr(max_depth), _ptr(uniform_noise), _ptr(si), _ptr(sd), _ptr(ss), _ptr(max_len),
+        _ptr(error_word(dev)), _stream(pts_idx)), "uniform_ray_sampling")
     return si, sd, ss
 
 
@@ -367,12 +385,12 @@ def inverse_cdf_sampling_rows(pts_idx, min_depth, max_depth, noise, probs, steps
     si = torch.empty(rows, max_steps, dtype=torch.int32, device=dev)
     sd = torch.empty(rows, max_steps, dtype=torch.float32, device=dev)
     ss = torch.empty(rows, max_steps, dtype=torch.float32, device=dev)
-    lay = (torch.tensor(layout, dtype=torch.int64)).contiguous()
+    lay = (ctypes.c_int64 * 4)(*layout)
     with _timed("inverse_cdf_sampling", dev):
         check(LIB.nsvf_inverse_cdf_sampling(
             rows, H, int(max_steps), noise.size(-1) if noise is not None else 0,
             float(fixed_step_size), _ptr(pts_idx), _ptr(min_depth), _ptr(max_depth), _ptr(noise),
-            _ptr(probs), _ptr(steps), lay.data_ptr(), _ptr(si), _ptr(sd), _ptr(ss), _ptr(max_len),
+            _ptr(probs), _ptr(steps), ctypes.addressof(lay), _ptr(si), _ptr(sd), _ptr(ss), _ptr(max_len),
             _ptr(error_word(dev)), _stream(pts_idx)), "inverse_cdf_sampling")
     return si, sd, ss
 

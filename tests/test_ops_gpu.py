@@ -465,6 +465,27 @@ def test_inverse_cdf_warp_rows_equal_thread_rows(cuda, H, form):
         assert a[4] & 2
 
 
+@pytest.mark.parametrize("H", [1, 33, 128, 129])
+@pytest.mark.parametrize("rows", [1, 31, 257])
+def test_uniform_longest_row(cuda, H, rows):
+    """The samplers' own longest row (a warp per row up to 128 slots, a thread
+    per row beyond; touching intervals and unordered ones) is the one that the
+    ids show, with ids of -1 inside a row not counted."""
+    from nsvf_gb300 import ext
+    step = 0.05
+    idx, lo, hi, _, _ = _random_intervals(rows, H, seed=H + rows)
+    if rows > 1:
+        idx[::2] = -1                        # empty rows
+    M = int(7.0 / step) + 2 * H + 3
+    noise = np.random.RandomState(5).rand(rows, M).astype(np.float32)
+    longest = torch.zeros(1, dtype=torch.int32, device=cuda)
+    ext.error_word(cuda).zero_()
+    out = ext.uniform_ray_sampling(_t(idx[None], cuda), _t(lo[None], cuda), _t(hi[None], cuda),
+                                   _t(noise[None], cuda), step, M, longest)
+    ext.error_word(cuda).zero_()
+    assert int(longest) == int(out[0].ne(-1).sum(-1).max())
+
+
 @pytest.mark.parametrize("H", [1, 31, 33, 64, 127])
 @pytest.mark.parametrize("form", ["contiguous", "gaps", "equal_depths", "edge_noise", "wild_noise",
                                   "raw_misses", "unsorted", "narrow"])
