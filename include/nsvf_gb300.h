@@ -779,13 +779,17 @@ int nsvf_compact_scan(int64_t n, const uint8_t *hits, int64_t *pix, int64_t *n_h
  *    FP32 with the operations of nsvf_trilinear_embed and of an FP32 GEMM that
  *    adds over k in order (fused multiply-add from zero, then the bias). Ids
  *    out of range as nsvf_trilinear_embed (embedding 0, err bit 2);
+ *  - field_train_forward_signs: also signs [4][n_samples][16 bytes], 16-byte
+ *    aligned: unit n of layer l is active (pre-activation > 0) where byte n / 4
+ *    % 16 has bit n % 4 + (n < 64 ? 0 : 4);
  *  - composite_rows (+ _backward): compositing with the free energy relu(sigma)
  *    * dist * sigma_scale; the backward gives d loss / d out [samples, 4] (any
  *    of the three gradients may be NULL);
  *  - field_train_backward: the field's gradients (overwritten, a fixed sum
  *    order) and grad_values (added to, float4 atomics), the activations
- *    recomputed for chunk_samples (a multiple of 128) samples at a time in a
- *    workspace of field_train_backward_floats() floats. */
+ *    recomputed (with the forward's signs) for chunk_samples (a multiple of
+ *    128) samples at a time in a workspace of field_train_backward_floats()
+ *    floats. A tensor-core wait that runs out sets err bit 3. */
 int nsvf_train_rows_count(int64_t rays, int max_steps, const int32_t *sampled_idx, int32_t *count,
                           void *stream);
 int nsvf_train_rows_pack(int64_t rays, int max_steps, const int32_t *sampled_idx, const float *xyz,
@@ -798,6 +802,11 @@ int nsvf_field_train_forward(int64_t n_samples, const int32_t *voxel, const floa
                              int64_t n_voxels, int64_t n_keys, float voxel_size,
                              const float *centers, const int32_t *feats, const float *values,
                              const float *packed, float *out, int32_t *err, void *stream);
+int nsvf_field_train_forward_signs(int64_t n_samples, const int32_t *voxel, const float *xyz_dist,
+                                   int64_t n_voxels, int64_t n_keys, float voxel_size,
+                                   const float *centers, const int32_t *feats,
+                                   const float *values, const float *packed, float *out,
+                                   uint8_t *signs, int32_t *err, void *stream);
 int nsvf_composite_rows(int64_t rays, const int64_t *offset, const float *field,
                         const float *xyz_dist, const float *depth, float sigma_scale,
                         float *out_color, float *out_depth, float *out_missed, int kahan,
@@ -811,10 +820,10 @@ int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_sample
 int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
                               const float *xyz_dist, int64_t n_voxels, int64_t n_keys,
                               float voxel_size, const float *centers, const int32_t *feats,
-                              const float *values, const float *packed, const float *grad_out,
-                              float *workspace, int64_t workspace_floats, float *grad_values,
-                              float *const grad_weights[5], float *const grad_biases[5],
-                              void *stream);
+                              const float *values, const float *packed, const uint8_t *signs,
+                              const float *grad_out, float *workspace, int64_t workspace_floats,
+                              float *grad_values, float *const grad_weights[5],
+                              float *const grad_biases[5], int32_t *err, void *stream);
 
 #ifdef __cplusplus
 }

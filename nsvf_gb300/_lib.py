@@ -112,11 +112,13 @@ def _load():
         "nsvf_field_train_packed_floats": ([], i64),
         "nsvf_field_train_pack": ([P, P, P, P], i32),
         "nsvf_field_train_forward": ([i64, P, P, i64, i64, f32, P, P, P, P, P, P, P], i32),
+        "nsvf_field_train_forward_signs": ([i64, P, P, i64, i64, f32, P, P, P, P, P, P, P, P],
+                                           i32),
         "nsvf_composite_rows": ([i64, P, P, P, P, f32, P, P, P, i32, P], i32),
         "nsvf_composite_rows_backward": ([i64, P, P, P, P, f32, P, P, P, P, i32, P], i32),
         "nsvf_field_train_backward_floats": ([i64, i64], i64),
-        "nsvf_field_train_backward": ([i64, i64, P, P, i64, i64, f32, P, P, P, P, P, P, i64, P, P,
-                                       P, P], i32),
+        "nsvf_field_train_backward": ([i64, i64, P, P, i64, i64, f32, P, P, P, P, P, P, P, i64, P,
+                                       P, P, P, P], i32),
     }
     for name, (args, res) in sig.items():
         fn = getattr(lib, name)
@@ -162,5 +164,5 @@ def exported_symbols():
         "nsvf_train_rows_count", "nsvf_train_rows_pack", "nsvf_field_train_packed_floats",
         "nsvf_field_train_pack", "nsvf_field_train_forward", "nsvf_composite_rows",
         "nsvf_composite_rows_backward", "nsvf_field_train_backward_floats",
-        "nsvf_field_train_backward",
+        "nsvf_field_train_backward", "nsvf_field_train_forward_signs",
     ]

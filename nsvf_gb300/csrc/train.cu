@@ -1,6 +1,5 @@
-// The differentiable part of a training batch on compacted samples: FP32
-// interpolation + 4 x 128 field forward, and the field's and the
-// interpolation's backward with the activations recomputed.
+// The forward of a training batch on compacted samples: FP32 interpolation and
+// the 4 x 128 field (backward: train_bwd.cu), and the FP32 stage of pruning.
 //
 // Reference: SparseVoxelEncoder.forward (fairnr/modules/encoder.py:558-592),
 // the field and VolumeRenderer.forward_chunk (fairnr/modules/renderer.py:
@@ -10,53 +9,36 @@
 // pre-activation changes sign, so the forward has to keep FP32 and its order
 // (one fused multiply-add chain over k = 0..K-1 from zero, then the bias:
 // the bits of an FP32 SIMT GEMM with a bias epilogue), which leaves the
-// tensor cores out. The bound is the FP32 pipe: 53,760 FMAs a sample forward,
-// four times that for a training step. A chain of library GEMMs runs it at
-// about 30 TFLOP/s and moves every activation through memory once per
-// elementwise operation; here a tile of 128 samples goes through all layers
-// in shared memory.
+// tensor cores out. The bound is the FP32 pipe: 53,760 FMAs a sample. A chain
+// of library GEMMs runs it at about 30 TFLOP/s and moves every activation
+// through memory once per elementwise operation; here a tile of 128 samples
+// goes through all layers in shared memory (1.40 M samples: 2.92 ms, 51
+// TFLOP/s).
 //
-// field_train_kernel<MODE>, 256 threads, two blocks per SM (while one gathers,
-// scatters or waits for weights, the other computes):
+// field_train_kernel<MODE>, 256 threads, two blocks per SM (while one gathers
+// or waits for weights, the other computes):
 //   * activations [unit][sample] in shared memory (64 KB), each thread an 8 x
 //     8 block of (unit, sample) accumulators, two samples per fma.rn.f32x2;
 //   * the weights stream through three 8 KB stages by cp.async, in one
-//     packed buffer that holds them in the order in which they are used
-//     (forward: W_l transposed; backward: W_l as it is), so a stage is 2,048
-//     consecutive floats and the next layer's weights arrive during an
-//     epilogue;
+//     packed buffer that holds them in the order in which they are used, so a
+//     stage is 2,048 consecutive floats and the next layer's weights arrive
+//     during an epilogue;
 //   * rows of 16-byte groups are XOR-swizzled by act_swz(row), so that the
 //     epilogue's stores (8 rows, 4 apart), the GEMM's loads (one row) and the
-//     per-unit sums (consecutive rows) are all free of bank conflicts.
-// The backward writes the layer inputs A_l and the pre-activation gradients
-// dZ_l of a chunk of samples to memory; weight_grad_kernel contracts them
-// (dW_l = dZ_l^T A_l) with 128 x 128 accumulators per block over a range of
-// samples. Partial sums live in per-block slots and are added in a fixed
-// order, so the field's gradients are reproducible; the embeddings' are
-// float4 atomics (merged over consecutive samples of one voxel).
-#include "common.cuh"
+//     head's loads are all free of bank conflicts.
+// For a backward (kForwardSigns) it also writes the sign of every
+// pre-activation, 64 bytes a sample: the backward recomputes activations to
+// FP32 accuracy, but not to these bits.
+#include "train_common.cuh"
+
+using namespace nsvf_train;
 
 namespace {
 
-constexpr int kT = 256;
-constexpr int kTile = 128;                 // samples per tile
-constexpr int kHid = 128, kE = 32;
 constexpr int kStages = 3;
 constexpr int kStage = 2048;               // floats per weight stage
-constexpr int kFwdStages = (kE + 3 * kHid) * kHid / kStage;   // 26
-constexpr int kAllStages = 2 * kFwdStages;
-// packed weights: the stages, then W4 [4][128], b0..b3 [4][128], b4 [4]
-constexpr int kW4Off = kAllStages * kStage;
-constexpr int kBiasOff = kW4Off + 4 * kHid;
-constexpr int kB4Off = kBiasOff + 4 * kHid;
-constexpr int kPacked = kB4Off + 4;
-constexpr int kBlocks = 2 * 152;           // two per SM
-// weight_grad_kernel: blocks of layers 1..3 (each) and of layer 0, whose rows
-// cost about a third
-constexpr int kSplit = 90, kSplit0 = kBlocks - 3 * kSplit;
-constexpr int kRows = 16, kGradStages = 4;
-// per half block of field_train_kernel<kBackward>: dW4 [4][128], db0..db3 [4][128]
-constexpr int kSmall = 8 * kHid;
+constexpr int kWStages = kW4Off / kStage;  // 26
+constexpr int kBlocks = 2 * kSMs;          // two per SM
 
 __host__ __device__ constexpr int act_swz(int row) {
   return (((row >> 2) & 3) << 1) ^ (row & 1) ^ ((row & 2) << 1);
@@ -118,14 +100,6 @@ __device__ __forceinline__ void outer(uint64_t (&acc)[8][4], const float4 &w0, c
   }
 }
 
-// w_k for corner k, multiplied in dimension order (interp.cu)
-__device__ __forceinline__ float corner_weight(const float p[3], int k) {
-  const float a = (k & 4) ? p[0] : 1.0f - p[0];
-  const float b = (k & 2) ? p[1] : 1.0f - p[1];
-  const float c = (k & 1) ? p[2] : 1.0f - p[2];
-  return a * b * c;
-}
-
 struct TrainParams {
   int64_t ns;                 // samples of this launch
   const int32_t *vox;         // [ns]
@@ -136,15 +110,8 @@ struct TrainParams {
   const int32_t *feats;       // [n_vox, 8]
   const float4 *values;       // [n_keys, 32]
   const float *packed;        // kPacked floats
-  float4 *out;                // forward: [ns] (sigma, r, g, b)
-  const float4 *d_out;        // backward: [ns]
-  float *acts;                // backward: A0 [rows, 32], then A1, A2, A3 [rows, 128]
-  float *grads;               // backward: dZ0..dZ3 [rows, 128]
-  int64_t rows;               // rows of each of these arrays (>= ns, whole tiles)
-  float *small;               // backward: per half block kSmall floats
-  float *db4;                 // backward: per block 4 floats
-  int add;                    // backward: add to the slots (0: overwrite)
-  float4 *g_values;           // backward: [n_keys, 32]
+  float4 *out;                // [ns] (sigma, r, g, b)
+  uint8_t *signs;             // kForwardSigns: [4][ns][16], see nsvf_field_train_forward_signs
   int32_t *err;
   // pruning (kPrune): sample s is point list[s] % bits^3 of voxel list[s] /
   // bits^3, *n_list of them (at most ns)
@@ -157,7 +124,7 @@ struct TrainParams {
   unsigned long long *n_undecided;
 };
 
-enum Mode { kForward, kBackward, kPrune };
+enum Mode { kForward, kForwardSigns, kPrune };
 
 // offset_points' FP32 position of point i of the voxel around c (exact.cu)
 __device__ __forceinline__ float point_pos(float c, int o, int bits, float hv) {
@@ -168,7 +135,7 @@ __device__ __forceinline__ float point_pos(float c, int o, int bits, float hv) {
 struct Stream {
   const float *base;
   float *ws;
-  int period, next, stage;    // next stage to issue; stage slot to read
+  int next, stage;            // next stage to issue; stage slot to read
 
   __device__ __forceinline__ void issue(int slot) {
     const int t = threadIdx.x;
@@ -176,7 +143,7 @@ struct Stream {
     cp16(ws + slot * kStage + t * 4, src + t * 4);
     cp16(ws + slot * kStage + 1024 + t * 4, src + 1024 + t * 4);
     cp_commit();
-    next = next + 1 == period ? 0 : next + 1;
+    next = next + 1 == kWStages ? 0 : next + 1;
   }
   __device__ __forceinline__ void start() {
     next = 0;
@@ -203,8 +170,7 @@ struct Smem {
   float w4[4 * kHid];
   float bias[4 * kHid];
   float b4[4];
-  float4 dout[kTile];
-  uint32_t mask[4][2][kT];    // sign bits of each thread's pre-activations
+  float margin[kTile];        // kPrune
 };
 
 // acc = sum over k of w[k][unit] * act[k][sample], K = 16 * stages
@@ -242,32 +208,9 @@ __device__ __forceinline__ void store_act(float *act, const float (&y)[8][8], in
   }
 }
 
-// Stores a thread's block to rows [sample][128] of a chunk array.
-__device__ __forceinline__ void store_rows(float *out, const float (&y)[8][8], int tx, int ty) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float *row = out + (int64_t)((i < 4 ? 0 : 64) + ty * 4 + (i & 3)) * kHid + tx * 4;
-    *reinterpret_cast<float4 *>(row) = make_float4(y[0][i], y[1][i], y[2][i], y[3][i]);
-    *reinterpret_cast<float4 *>(row + 64) = make_float4(y[4][i], y[5][i], y[6][i], y[7][i]);
-  }
-}
-
-// Sum over half the tile's samples of unit row n.
-__device__ __forceinline__ float row_sum(const float *act, int n, int half) {
-  const int f = act_swz(n);
-  float s = 0.0f;
-#pragma unroll
-  for (int g = 0; g < 16; ++g) {
-    const float4 v =
-        *reinterpret_cast<const float4 *>(act + n * kTile + (((half * 16 + g) ^ f) << 2));
-    s += (v.x + v.y) + (v.z + v.w);
-  }
-  return s;
-}
-
 template <int MODE>
 __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p) {
-  constexpr bool BWD = MODE == kBackward;
+  constexpr bool SIGNS = MODE == kForwardSigns;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   Smem &S = *reinterpret_cast<Smem *>(smem_raw);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -281,10 +224,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
   Stream st;
   st.base = p.packed;
   st.ws = S.ws;
-  st.period = BWD ? kAllStages : kFwdStages;
   st.start();
-  float dw4[4] = {0.f, 0.f, 0.f, 0.f}, db[4] = {0.f, 0.f, 0.f, 0.f};
-  float4 db4 = make_float4(0.f, 0.f, 0.f, 0.f);
   int64_t ns = p.ns;
   if (MODE == kPrune && (int64_t)*p.n_list < ns) ns = (int64_t)*p.n_list;
   const int64_t tiles = (ns + kTile - 1) / kTile;
@@ -315,7 +255,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
           v = p.vox[s];
         }
         if (v < 0 || v >= p.n_vox) {
-          if (MODE == kForward && p.err && ch == 0) atomicOr(p.err, 4);
+          if (MODE != kPrune && p.err && ch == 0) atomicOr(p.err, 4);
         } else {
           if (MODE != kPrune) x = p.xyzd[s];
           const float q[3] = {(x.x - p.centers[v * 3 + 0]) / p.voxel_size + 0.5f,
@@ -325,7 +265,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
           for (int k = 0; k < 8; ++k) {
             const int64_t key = p.feats[v * 8 + k];
             if (key < 0 || key >= p.n_keys) {
-              if (MODE == kForward && p.err) atomicOr(p.err, 4);
+              if (MODE != kPrune && p.err) atomicOr(p.err, 4);
               continue;
             }
             const float w = corner_weight(q, k);
@@ -341,13 +281,6 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
         const int row = ch * 4 + j;
         S.act[row * kTile + (((sl >> 2) ^ act_swz(row)) << 2) + (sl & 3)] = ev[j];
       }
-      if (BWD) reinterpret_cast<float4 *>(p.acts)[s * (kE / 4) + ch] = e;
-    }
-    if (BWD && t < kTile) {
-      const int64_t s = s0 + t;
-      const float4 d = s < ns ? p.d_out[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-      S.dout[t] = d;
-      db4.x += d.x; db4.y += d.y; db4.z += d.z; db4.w += d.w;
     }
     uint64_t acc[8][4];
     float y[8][8];
@@ -365,7 +298,7 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
           unpk(acc[j][q], z0, z1);
           z0 = __fadd_rn(z0, b);
           z1 = __fadd_rn(z1, b);
-          if (BWD) {
+          if (SIGNS) {
             m[j >> 2] |= (z0 > 0.0f ? 1u : 0u) << ((j & 3) * 8 + 2 * q);
             m[j >> 2] |= (z1 > 0.0f ? 1u : 0u) << ((j & 3) * 8 + 2 * q + 1);
           }
@@ -373,11 +306,16 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
           y[j][2 * q + 1] = z1 <= 0.0f ? 0.0f : z1;
         }
       }
-      if (BWD) {
-        S.mask[l][0][t] = m[0];
-        S.mask[l][1][t] = m[1];
-        if (l < 3)
-          store_rows(p.acts + p.rows * kE + (int64_t)l * p.rows * kHid + s0 * kHid, y, tx, ty);
+      if (SIGNS) {
+        // units tx * 4 + 0..3 in the low half of the byte, 64 above them in
+        // the high half
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int64_t q = s0 + (i < 4 ? 0 : 64) + ty * 4 + (i & 3);
+          const uint32_t lo = ((m[0] >> i & 0x01010101u) * 0x01020408u) >> 24;
+          const uint32_t hi = ((m[1] >> i & 0x01010101u) * 0x01020408u) >> 24;
+          if (q < ns) p.signs[((int64_t)l * ns + q) * 16 + tx] = (uint8_t)(lo | hi << 4);
+        }
       }
       store_act(S.act, y, tx, ty);
     }
@@ -392,11 +330,11 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
         const float a = S.act[k * kTile + (((unit >> 2) ^ act_swz(k)) << 2) + (unit & 3)];
         o = fmaf(a, half ? fabsf(S.w4[k]) : S.w4[k], o);
       }
-      if (half) S.dout[unit].x = o;
+      if (half) S.margin[unit] = o;
       __syncthreads();
       if (!half && s0 + unit < ns) {
         const float sigma = __fadd_rn(o, S.b4[0]);
-        const float margin = p.band * S.dout[unit].x + 1e-6f * p.T;
+        const float margin = p.band * S.margin[unit] + 1e-6f * p.T;
         const int64_t row = p.list[s0 + unit];
         if (sigma - margin > p.T)
           p.keep[row / (p.bits * p.bits * p.bits)] = 1;
@@ -405,319 +343,20 @@ __global__ void __launch_bounds__(kT, 2) field_train_kernel(const TrainParams p)
       }
       continue;
     }
-    if (!BWD) {
-      // head: outputs 2 half, 2 half + 1 of sample `unit`
-      const float *w = S.w4 + half * 2 * kHid;
-      float o0 = 0.0f, o1 = 0.0f;
+    // head: outputs 2 half, 2 half + 1 of sample `unit`
+    const float *w = S.w4 + half * 2 * kHid;
+    float o0 = 0.0f, o1 = 0.0f;
 #pragma unroll 8
-      for (int k = 0; k < kHid; ++k) {
-        const float a = S.act[k * kTile + (((unit >> 2) ^ act_swz(k)) << 2) + (unit & 3)];
-        o0 = fmaf(a, w[k], o0);
-        o1 = fmaf(a, w[kHid + k], o1);
-      }
-      if (s0 + unit < ns)
-        reinterpret_cast<float2 *>(p.out + s0 + unit)[half] =
-            make_float2(__fadd_rn(o0, S.b4[half * 2]), __fadd_rn(o1, S.b4[half * 2 + 1]));
-      continue;
+    for (int k = 0; k < kHid; ++k) {
+      const float a = S.act[k * kTile + (((unit >> 2) ^ act_swz(k)) << 2) + (unit & 3)];
+      o0 = fmaf(a, w[k], o0);
+      o1 = fmaf(a, w[kHid + k], o1);
     }
-    // dW4 += d_out^T A4: unit `unit`, half of the samples
-    {
-      const int f = act_swz(unit);
-#pragma unroll 4
-      for (int g = 0; g < 16; ++g) {
-        const int gg = half * 16 + g;
-        const float4 a =
-            *reinterpret_cast<const float4 *>(S.act + unit * kTile + ((gg ^ f) << 2));
-        const float av[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 d = S.dout[gg * 4 + i];
-          dw4[0] = fmaf(av[i], d.x, dw4[0]);
-          dw4[1] = fmaf(av[i], d.y, dw4[1]);
-          dw4[2] = fmaf(av[i], d.z, dw4[2]);
-          dw4[3] = fmaf(av[i], d.w, dw4[3]);
-        }
-      }
-    }
-    // dA4 = d_out W4
-    {
-      const float4 *w4 = reinterpret_cast<const float4 *>(S.w4);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 d = S.dout[(i < 4 ? 0 : 64) + ty * 4 + (i & 3)];
-        const float dv[4] = {d.x, d.y, d.z, d.w};
-#pragma unroll
-        for (int j = 0; j < 8; ++j) y[j][i] = 0.0f;
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-          const float4 a = w4[o * 32 + tx], b = w4[o * 32 + 16 + tx];
-          y[0][i] = fmaf(dv[o], a.x, y[0][i]); y[1][i] = fmaf(dv[o], a.y, y[1][i]);
-          y[2][i] = fmaf(dv[o], a.z, y[2][i]); y[3][i] = fmaf(dv[o], a.w, y[3][i]);
-          y[4][i] = fmaf(dv[o], b.x, y[4][i]); y[5][i] = fmaf(dv[o], b.y, y[5][i]);
-          y[6][i] = fmaf(dv[o], b.z, y[6][i]); y[7][i] = fmaf(dv[o], b.w, y[7][i]);
-        }
-      }
-    }
-    // dZ_l = dA_{l+1} (z_l > 0), then dA_l = dZ_l W_l
-#pragma unroll
-    for (int l = 3; l >= 0; --l) {
-      if (l < 3) {
-        gemm128(acc, kHid / 16, st, S.act, tx, ty);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) unpk(acc[j][q], y[j][2 * q], y[j][2 * q + 1]);
-      }
-      const uint32_t m0 = S.mask[l][0][t], m1 = S.mask[l][1][t];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          y[j][i] *= (((j < 4 ? m0 : m1) >> ((j & 3) * 8 + i)) & 1u) ? 1.0f : 0.0f;
-      store_rows(p.grads + (int64_t)l * p.rows * kHid + s0 * kHid, y, tx, ty);
-      store_act(S.act, y, tx, ty);
-      __syncthreads();
-      db[l] += row_sum(S.act, unit, half);
-    }
-    // dA0 = dZ0 W0 [128 samples x 32 channels]: 4 samples x 4 channels a thread
-    {
-      const int cg = lane_x(lane), sg = warp * 4 + lane_y(lane);
-      float4 g[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
-        const float *w = st.take() + cg * 4;
-        const float *a = S.act + c * 64 * kTile;
-#pragma unroll 16
-        for (int kk = 0; kk < 64; ++kk) {
-          const float4 av = *reinterpret_cast<const float4 *>(
-              a + kk * kTile + ((sg ^ act_swz(kk)) << 2));
-          const float4 wv = *reinterpret_cast<const float4 *>(w + kk * kE);
-          const float s4[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            g[i].x = fmaf(s4[i], wv.x, g[i].x); g[i].y = fmaf(s4[i], wv.y, g[i].y);
-            g[i].z = fmaf(s4[i], wv.z, g[i].z); g[i].w = fmaf(s4[i], wv.w, g[i].w);
-          }
-        }
-      }
-      // grad_values[feats[v, k]] += w_k g, summed over the thread's
-      // consecutive samples of one voxel before the atomics
-      int64_t prev = -1;
-      float4 sum[8];
-      auto flush = [&]() {
-        if (prev < 0) return;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int64_t key = p.feats[prev * 8 + k];
-          if (key >= 0 && key < p.n_keys) atomicAdd(p.g_values + key * (kE / 4) + cg, sum[k]);
-        }
-      };
-#pragma unroll 1
-      for (int i = 0; i < 4; ++i) {
-        const int64_t s = s0 + sg * 4 + i;
-        int64_t v = s < ns ? (int64_t)p.vox[s] : -1;
-        if (v >= p.n_vox) v = -1;
-        if (v < 0) continue;
-        if (v != prev) {
-          flush();
-          prev = v;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        const float4 x = p.xyzd[s];
-        const float q[3] = {(x.x - p.centers[v * 3 + 0]) / p.voxel_size + 0.5f,
-                            (x.y - p.centers[v * 3 + 1]) / p.voxel_size + 0.5f,
-                            (x.z - p.centers[v * 3 + 2]) / p.voxel_size + 0.5f};
-        const float4 gi = i == 0 ? g[0] : i == 1 ? g[1] : i == 2 ? g[2] : g[3];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float w = corner_weight(q, k);
-          sum[k].x = fmaf(w, gi.x, sum[k].x); sum[k].y = fmaf(w, gi.y, sum[k].y);
-          sum[k].z = fmaf(w, gi.z, sum[k].z); sum[k].w = fmaf(w, gi.w, sum[k].w);
-        }
-      }
-      flush();
-    }
+    if (s0 + unit < ns)
+      reinterpret_cast<float2 *>(p.out + s0 + unit)[half] =
+          make_float2(__fadd_rn(o0, S.b4[half * 2]), __fadd_rn(o1, S.b4[half * 2 + 1]));
   }
   cp_wait<0>();
-  if (!BWD) return;
-  float *sm = p.small + (int64_t)(blockIdx.x * 2 + half) * kSmall;
-#pragma unroll
-  for (int o = 0; o < 4; ++o) {
-    float *a = sm + o * kHid + unit, *b = sm + (4 + o) * kHid + unit;
-    *a = p.add ? *a + dw4[o] : dw4[o];
-    *b = p.add ? *b + db[o] : db[o];
-  }
-  __syncthreads();
-  if (t < kTile) S.dout[t] = db4;
-  __syncthreads();
-  if (t < 4) {
-    float s = 0.0f;
-    for (int i = 0; i < kTile; ++i) s += reinterpret_cast<const float *>(S.dout + i)[t];
-    float *d = p.db4 + blockIdx.x * 4 + t;
-    *d = p.add ? *d + s : s;
-  }
-}
-
-// dW_l = dZ_l^T A_l over a range of the chunk's samples: blocks 0..3 kSplit - 1
-// are layers 1..3 (128 x 128), the rest layer 0 (128 x 32). 16 samples per
-// cp.async stage, both operands [sample][unit] as they lie in memory. Adds to
-// (or overwrites) the block's slot.
-__global__ void __launch_bounds__(kT, 2) weight_grad_kernel(int64_t ns, int64_t rows,
-                                                            const float *__restrict__ acts,
-                                                            const float *__restrict__ grads,
-                                                            float *__restrict__ part, int add) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  float *sx = reinterpret_cast<float *>(smem_raw);           // dZ rows
-  float *sy = sx + kGradStages * kRows * kHid;               // A rows
-  const int t = threadIdx.x;
-  const int b = blockIdx.x;
-  const int l = b < 3 * kSplit ? 1 + b / kSplit : 0;
-  const int j = b < 3 * kSplit ? b % kSplit : b - 3 * kSplit;
-  const int splits = l ? kSplit : kSplit0;
-  const int64_t per = ((ns + splits - 1) / splits + kRows - 1) / kRows * kRows;
-  const int64_t r0 = j * per < ns ? j * per : ns, r1 = r0 + per < ns ? r0 + per : ns;
-  const int64_t steps = (r1 - r0 + kRows - 1) / kRows;
-  const float *X = grads + (int64_t)l * rows * kHid;
-  const float *Y = l ? acts + rows * kE + (int64_t)(l - 1) * rows * kHid : acts;
-  const int wy = l ? kHid : kE;                              // width of A rows
-  auto issue = [&](int64_t step) {
-    if (step < steps) {
-      const int slot = (int)(step % kGradStages);
-      const int64_t base = r0 + step * kRows;
-      for (int q = t; q < kRows * kHid / 4; q += kT) {
-        const int64_t r = base + (q >> 5);
-        cp16(sx + slot * kRows * kHid + q * 4, X + (r < r1 ? r : r0) * kHid + (q & 31) * 4,
-             r < r1 ? 16 : 0);
-      }
-      const int w4 = wy / 4;
-      for (int q = t; q < kRows * w4; q += kT) {
-        const int64_t r = base + q / w4;
-        cp16(sy + slot * kRows * kHid + q * 4, Y + (r < r1 ? r : r0) * wy + (q % w4) * 4,
-             r < r1 ? 16 : 0);
-      }
-    }
-    cp_commit();
-  };
-  for (int q = 0; q < kGradStages - 1; ++q) issue(q);
-  const int lane = t & 31, warp = t >> 5;
-  if (l) {
-    const int tx = (warp >> 2) * 8 + lane_x(lane), ty = (warp & 3) * 4 + lane_y(lane);
-    uint64_t acc[8][4];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[a][c] = 0;
-#pragma unroll 1
-    for (int64_t step = 0; step < steps; ++step) {
-      cp_wait<kGradStages - 2>();
-      __syncthreads();
-      issue(step + kGradStages - 1);
-      const float *x = sx + (step % kGradStages) * kRows * kHid + ty * 4;
-      const float *y = sy + (step % kGradStages) * kRows * kHid + tx * 4;
-#pragma unroll
-      for (int s = 0; s < kRows; ++s) {
-        const float4 x0 = *reinterpret_cast<const float4 *>(x + s * kHid);
-        const float4 x1 = *reinterpret_cast<const float4 *>(x + s * kHid + 64);
-        const ulonglong2 y0 = *reinterpret_cast<const ulonglong2 *>(y + s * kHid);
-        const ulonglong2 y1 = *reinterpret_cast<const ulonglong2 *>(y + s * kHid + 64);
-        outer(acc, x0, x1, y0, y1);
-      }
-    }
-    float *P = part + (int64_t)b * kHid * kHid;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      float *row = P + ((a < 4 ? 0 : 64) + ty * 4 + (a & 3)) * kHid + tx * 4;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float4 v;
-        unpk(acc[a][2 * h], v.x, v.y);
-        unpk(acc[a][2 * h + 1], v.z, v.w);
-        float4 *d = reinterpret_cast<float4 *>(row + h * 64);
-        if (add) {
-          const float4 o = *d;
-          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-        }
-        *d = v;
-      }
-    }
-  } else {
-    const int kg = lane_x(lane), ng = warp * 4 + lane_y(lane);   // 4 channels, 4 units
-    float4 g[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-    for (int64_t step = 0; step < steps; ++step) {
-      cp_wait<kGradStages - 2>();
-      __syncthreads();
-      issue(step + kGradStages - 1);
-      const float *x = sx + (step % kGradStages) * kRows * kHid + ng * 4;
-      const float *y = sy + (step % kGradStages) * kRows * kHid + kg * 4;
-#pragma unroll
-      for (int s = 0; s < kRows; ++s) {
-        const float4 xv = *reinterpret_cast<const float4 *>(x + s * kHid);
-        const float4 yv = *reinterpret_cast<const float4 *>(y + s * kE);
-        const float x4[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          g[i].x = fmaf(x4[i], yv.x, g[i].x); g[i].y = fmaf(x4[i], yv.y, g[i].y);
-          g[i].z = fmaf(x4[i], yv.z, g[i].z); g[i].w = fmaf(x4[i], yv.w, g[i].w);
-        }
-      }
-    }
-    float *P = part + (int64_t)3 * kSplit * kHid * kHid + (int64_t)j * kHid * kE;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float4 *d = reinterpret_cast<float4 *>(P + (ng * 4 + i) * kE + kg * 4);
-      if (add) {
-        const float4 o = *d;
-        g[i].x += o.x; g[i].y += o.y; g[i].z += o.z; g[i].w += o.w;
-      }
-      *d = g[i];
-    }
-  }
-  cp_wait<0>();
-}
-
-struct GradOut {
-  float *w[5], *b[5];
-};
-
-// The field's gradients from the slots, each element's slots added in order.
-__global__ void __launch_bounds__(kT) grad_reduce_kernel(const float *__restrict__ part,
-                                                         const float *__restrict__ small,
-                                                         const float *__restrict__ db4,
-                                                         GradOut out) {
-  int i = blockIdx.x * kT + threadIdx.x;
-  const float *src;
-  float *dst;
-  int n, stride;
-  if (i < 3 * kHid * kHid) {
-    const int l = i / (kHid * kHid), e = i % (kHid * kHid);
-    src = part + (int64_t)l * kSplit * kHid * kHid + e;
-    n = kSplit; stride = kHid * kHid;
-    dst = out.w[l + 1] + e;
-  } else if ((i -= 3 * kHid * kHid) < kHid * kE) {
-    src = part + (int64_t)3 * kSplit * kHid * kHid + i;
-    n = kSplit0; stride = kHid * kE;
-    dst = out.w[0] + i;
-  } else if ((i -= kHid * kE) < kSmall) {
-    src = small + i;
-    n = 2 * kBlocks; stride = kSmall;
-    dst = i < 4 * kHid ? out.w[4] + i : out.b[i / kHid - 4] + i % kHid;
-  } else if ((i -= kSmall) < 4) {
-    src = db4 + i;
-    n = kBlocks; stride = 4;
-    dst = out.b[4] + i;
-  } else {
-    return;
-  }
-  float s = 0.0f;
-#pragma unroll 16
-  for (int k = 0; k < n; ++k) s += src[(int64_t)k * stride];
-  *dst = s;
 }
 
 struct FieldWeights {
@@ -729,12 +368,9 @@ __global__ void __launch_bounds__(kT) pack_weights_kernel(FieldWeights f, float 
   if (i >= kPacked) return;
   float v;
   constexpr int kL0 = kE * kHid, kL = kHid * kHid;
-  if (i < kFwdStages * kStage) {                        // W_l transposed: [k][n]
+  if (i < kW4Off) {                                     // W_l transposed: [k][n]
     const int l = i < kL0 ? 0 : 1 + (i - kL0) / kL, e = i < kL0 ? i : (i - kL0) % kL;
     v = f.w[l][(e % kHid) * (l ? kHid : kE) + e / kHid];
-  } else if (i < kW4Off) {                              // W3, W2, W1, W0
-    const int e = i - kFwdStages * kStage;
-    v = e < 3 * kL ? f.w[3 - e / kL][e % kL] : f.w[0][e - 3 * kL];
   } else if (i < kBiasOff) {
     v = f.w[4][i - kW4Off];
   } else if (i < kB4Off) {
@@ -783,14 +419,6 @@ __global__ void __launch_bounds__(kT) rows_pack_kernel(
   }
 }
 
-bool bad_scene(int64_t ns, const int32_t *vox, const float *xyzd, int64_t n_vox, int64_t n_keys,
-               const float *centers, const int32_t *feats, const float *values,
-               const float *packed) {
-  return ns < 0 || n_vox < 0 || n_keys < 0 ||
-         (ns > 0 && (!vox || !xyzd || !centers || !feats || !values || !packed)) ||
-         ((((uintptr_t)xyzd) | ((uintptr_t)values) | ((uintptr_t)packed)) & 15);
-}
-
 // The points of `in` whose voxel is not kept yet, to `out` (any order).
 __global__ void __launch_bounds__(kT) undecided_kernel(
     const int64_t *__restrict__ in, const unsigned long long *__restrict__ n_in, int64_t cap, int P,
@@ -823,16 +451,6 @@ int launch_train(const TrainParams &p, int64_t blocks, cudaStream_t s) {
     return NSVF_ERR_CUDA;
   field_train_kernel<MODE><<<(int)blocks, kT, sizeof(Smem), s>>>(p);
   return nsvf_launch_status();
-}
-
-// floats of the backward's workspace besides the chunk arrays
-constexpr int64_t kSlotFloats = (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE +
-                                (int64_t)2 * kBlocks * kSmall + (int64_t)kBlocks * 4;
-constexpr int64_t kRowFloats = kE + 7 * kHid;              // A0, A1..A3, dZ0..dZ3
-
-int64_t chunk_rows(int64_t ns, int64_t chunk) {
-  const int64_t c = chunk < ns ? chunk : ns;
-  return (c + kTile - 1) / kTile * kTile;
 }
 
 }  // namespace
@@ -881,6 +499,15 @@ int nsvf_field_train_forward(int64_t n_samples, const int32_t *voxel, const floa
                              int64_t n_voxels, int64_t n_keys, float voxel_size,
                              const float *centers, const int32_t *feats, const float *values,
                              const float *packed, float *out, int32_t *err, void *stream) {
+  return nsvf_field_train_forward_signs(n_samples, voxel, xyz_dist, n_voxels, n_keys, voxel_size,
+                                        centers, feats, values, packed, out, nullptr, err, stream);
+}
+
+int nsvf_field_train_forward_signs(int64_t n_samples, const int32_t *voxel, const float *xyz_dist,
+                                   int64_t n_voxels, int64_t n_keys, float voxel_size,
+                                   const float *centers, const int32_t *feats,
+                                   const float *values, const float *packed, float *out,
+                                   uint8_t *signs, int32_t *err, void *stream) {
   if (bad_scene(n_samples, voxel, xyz_dist, n_voxels, n_keys, centers, feats, values, packed))
     return NSVF_ERR_INVALID;
   if (n_samples == 0) return NSVF_OK;
@@ -897,78 +524,11 @@ int nsvf_field_train_forward(int64_t n_samples, const int32_t *voxel, const floa
   p.values = (const float4 *)values;
   p.packed = packed;
   p.out = (float4 *)out;
+  p.signs = signs;
   p.err = err;
-  const int64_t tiles = (n_samples + kTile - 1) / kTile;
-  return launch_train<kForward>(p, tiles < kBlocks ? tiles : kBlocks, (cudaStream_t)stream);
-}
-
-int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_samples) {
-  if (n_samples < 0 || chunk_samples < 1) return -1;
-  return kSlotFloats + chunk_rows(n_samples, chunk_samples) * kRowFloats;
-}
-
-int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
-                              const float *xyz_dist, int64_t n_voxels, int64_t n_keys,
-                              float voxel_size, const float *centers, const int32_t *feats,
-                              const float *values, const float *packed, const float *grad_out,
-                              float *workspace, int64_t workspace_floats, float *grad_values,
-                              float *const grad_weights[5], float *const grad_biases[5],
-                              void *stream) {
-  if (bad_scene(n_samples, voxel, xyz_dist, n_voxels, n_keys, centers, feats, values, packed) ||
-      chunk_samples < 1 || chunk_samples % kTile || !grad_weights || !grad_biases || !workspace ||
-      (((uintptr_t)workspace) & 15))
-    return NSVF_ERR_INVALID;
-  if (n_samples > 0 && (!grad_out || !grad_values ||
-                        ((((uintptr_t)grad_out) | ((uintptr_t)grad_values)) & 15)))
-    return NSVF_ERR_INVALID;
-  if (workspace_floats < nsvf_field_train_backward_floats(n_samples, chunk_samples))
-    return NSVF_ERR_CAPACITY;
-  GradOut g;
-  for (int l = 0; l < 5; ++l) {
-    if (!grad_weights[l] || !grad_biases[l]) return NSVF_ERR_INVALID;
-    g.w[l] = grad_weights[l];
-    g.b[l] = grad_biases[l];
-  }
-  cudaStream_t s = (cudaStream_t)stream;
-  constexpr int smem = 2 * kGradStages * kRows * kHid * (int)sizeof(float);
-  if (cudaFuncSetAttribute(weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           smem) != cudaSuccess)
-    return NSVF_ERR_CUDA;
-  const int64_t rows = chunk_rows(n_samples, chunk_samples);
-  float *acts = workspace, *grads = acts + rows * (kE + 3 * kHid);
-  float *part = grads + rows * 4 * kHid;
-  float *small = part + (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE;
-  float *db4 = small + (int64_t)2 * kBlocks * kSmall;
-  TrainParams p = {};
-  p.n_vox = n_voxels;
-  p.n_keys = n_keys;
-  p.voxel_size = voxel_size;
-  p.centers = centers;
-  p.feats = feats;
-  p.values = (const float4 *)values;
-  p.packed = packed;
-  p.acts = acts;
-  p.grads = grads;
-  p.rows = rows;
-  p.small = small;
-  p.db4 = db4;
-  p.g_values = (float4 *)grad_values;
-  // (one pass without samples zeroes the slots of an empty batch)
-  for (int64_t a = 0; a == 0 || a < n_samples; a += chunk_samples) {
-    p.ns = n_samples - a < chunk_samples ? n_samples - a : chunk_samples;
-    p.vox = voxel + a;
-    p.xyzd = (const float4 *)xyz_dist + a;
-    p.d_out = (const float4 *)grad_out + a;
-    p.add = a > 0;
-    int st = launch_train<kBackward>(p, kBlocks, s);
-    if (st != NSVF_OK) return st;
-    weight_grad_kernel<<<kBlocks, kT, smem, s>>>(p.ns, rows, acts, grads, part, p.add);
-    st = nsvf_launch_status();
-    if (st != NSVF_OK) return st;
-  }
-  constexpr int n_grads = 3 * kHid * kHid + kHid * kE + kSmall + 4;
-  grad_reduce_kernel<<<nsvf_grid(n_grads, kT), kT, 0, s>>>(part, small, db4, g);
-  return nsvf_launch_status();
+  const int64_t tiles = (n_samples + kTile - 1) / kTile, blocks = tiles < kBlocks ? tiles : kBlocks;
+  return signs ? launch_train<kForwardSigns>(p, blocks, (cudaStream_t)stream)
+               : launch_train<kForward>(p, blocks, (cudaStream_t)stream);
 }
 
 int nsvf_prune_fp32_dev(int64_t n_voxels, int bits, float threshold, float band, int64_t n_keys,

@@ -1,0 +1,1056 @@
+// Backward of the 4 x 128 FP32 field and of the interpolation below it, on
+// the tensor cores in split FP32.
+//
+// Reference: SparseVoxelEncoder.forward (fairnr/modules/encoder.py:558-592)
+// and the field under autograd.
+//
+// The split. A GEMM operand's row (its K elements) is scaled by a power of
+// two to |x| < 1 and cut into three bf16 slices on fixed grids of 2^-8, 2^-17
+// and about 2^-26 (error-free slicing on a common exponent, the scheme of
+// Ozaki, Ogita, Oishi and Rump, 2012). Products of slices on the first grid
+// are multiples of 2^-16 below one, so K = 128 of them add up in an FP32
+// accumulator without any rounding, whatever the order and the rounding of
+// the tensor core. One accumulator takes the products of order 0, a second one
+// those of orders 2 and 1 (three and two, in this sequence; what it loses is a
+// 2^-9th of the first one's last places); the orders left out are below 2^-26
+// of the row's and the column's largest element. The sum of the two rounds
+// once, where a chain of 128 FP32 multiply-adds rounds 128 times.
+//
+// A row with an element that is not finite (or of 2^126 and more) gets the
+// scale NaN: its results are NaN and each of them is then computed by the
+// FP32 chain.
+//
+// Measured on 1.40 M samples (an FP32-pipe version of the two kernels took 6.7
+// + 2.7 ms, at 41 and 50 TFLOP/s of the pipe's 66): 3.3 + 2.1 ms. Errors of
+// the weight gradients against float64: 2.1e-7 to 2.6e-7 of their norm, where
+// FP32 GEMMs over chunks leave 8e-7 to 1.6e-6.
+//
+// field_bwd_kernel: a tile of 128 samples per block and one block per SM:
+// interpolation and layers again (the ReLU signs are the forward's own,
+// which are exact), then dZ_l = dA_{l+1} (z_l > 0), dA_l = dZ_l W_l, then the
+// scatter into the embeddings. TMEM lane = sample, so a row's largest element
+// is found by the four threads that hold it, and its slices go to tensor
+// memory as the next layer's A operand, which leaves shared memory for the
+// weights of two layers. The layer inputs A_l and the gradients dZ_l go to
+// memory as [unit][sample] of a tile (every store a whole line). Stores,
+// scatter and the next tile's gather run beside the MMAs. Bound: a tile's 340
+// MMAs of 64 cycles are 22k of its 83k cycles; the rest is the chain MMA ->
+// epilogue -> MMA of the one tile that fits, the stores (5.9 GB at 1.8 TB/s)
+// and the scatter's atomics.
+// weight_grad_kernel: dW_l = dZ_l^T A_l, db_l = sum dZ_l: K runs over the 128
+// samples of a tile, rows are units; FP32 accumulation over tiles in
+// registers, one slot per block, the slots added in a fixed order. The FP32
+// rows of the next tile arrive by cp.async while a tile is sliced. Bound: MMA
+// issue and slicing by the same warps, 14k cycles a tile and layer of which
+// the MMAs are 3.1k and the 128 KB from memory 5.6k.
+#include "tc_common.cuh"
+#include "train_common.cuh"
+
+using namespace nsvf_tc;
+using namespace nsvf_train;
+
+namespace {
+
+constexpr int kPlane = kHid * kHid * 2;    // bytes of a slice of a 128 x 128 operand
+constexpr int kSmallOp = kHid * kE * 2;    // of a 128 x 32 or 32 x 128 one
+// The weight operands in the order of their use: W0..W3 (rows = units), then
+// W3^T, W2^T, W1^T, W0^T (rows = inputs), three slices each.
+__host__ __device__ constexpr int op_plane(int op) { return op % 7 ? kPlane : kSmallOp; }
+__host__ __device__ constexpr int op_off(int op) {
+  return op ? 3 * kSmallOp + (op - 1) * 3 * kPlane : 0;
+}
+constexpr int kSliceBytes = op_off(7) + 3 * kSmallOp;
+constexpr int kScales = 7 * kHid + kE;     // a power of two per row of every operand
+constexpr int kSliceFloats = kSliceBytes / 4 + kScales;
+
+// rows of 128 samples of a tile in memory: A0 (32), A1..A4, dZ0..dZ3, and dA0
+// as [sample][32]
+constexpr int kRows = 2 * kE + 8 * kHid;
+constexpr int kDA0 = kE + 8 * kHid;
+__host__ __device__ constexpr int a_row(int l) { return l ? kE + (l - 1) * kHid : 0; }
+__host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHid; }
+
+// weight_grad_kernel's blocks, in proportion to a tile's time: layers 1..3 (15k
+// cycles each), layer 0 (10.5k) and the head (10k: an MMA of 16 columns takes
+// 45 of the 64 cycles that one of 128 takes). By rows (37 / 23 / 18) the head's
+// blocks were the last by a third: 2.6 -> 2.2 ms.
+constexpr int kSplit = 35, kSplit0 = 24, kSplit4 = 23;
+static_assert(3 * kSplit + kSplit0 + kSplit4 == kSMs, "one block per SM");
+
+constexpr int kBT = 512;                   // threads of the two kernels
+constexpr int kQ = kHid / 4;               // units of a thread's quarter of a row
+constexpr uint32_t kAccCols = 128;         // columns between the two accumulators
+constexpr uint32_t kACol = 256;            // field_bwd_kernel: A's slices, 64 columns each
+
+__device__ __forceinline__ uint64_t pk(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {   // a - b
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(b), "l"(pk(-1.0f, -1.0f)), "l"(a));
+  return d;
+}
+// the upper halves of two floats (exact for values of at most 8 bits)
+__device__ __forceinline__ uint32_t tops(uint64_t v) {
+  return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632);
+}
+
+// The three bf16 slices of x0, x1 scaled by inv (|x inv| < 1). Adding and
+// subtracting 1.5 2^15 rounds to a multiple of 2^-8, 1.5 2^6 to one of 2^-17;
+// both quotients are at most 256 and so 8 bits; the rest rounds to bf16.
+__device__ __forceinline__ void slice2(float x0, float x1, float inv, uint32_t &h, uint32_t &m,
+                                       uint32_t &l) {
+  const uint64_t t = mul2(pk(x0, x1), pk(inv, inv));
+  const uint64_t hi = add2(add2(t, pk(49152.0f, 49152.0f)), pk(-49152.0f, -49152.0f));
+  const uint64_t r = sub2(t, hi);
+  const uint64_t mi = add2(add2(r, pk(96.0f, 96.0f)), pk(-96.0f, -96.0f));
+  const uint64_t lo = sub2(r, mi);
+  h = tops(hi);
+  m = tops(mi);
+  l = pack_bf16x2(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)));
+}
+
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+
+// The power of two above a row's largest element, whose biased exponent is e
+// (NaN for a row that the slices cannot hold), and its reciprocal.
+__device__ __forceinline__ uint32_t exponent(float m) { return (__float_as_uint(m) >> 23) & 255u; }
+__device__ __forceinline__ float row_scale(uint32_t e, float &inv) {
+  inv = e < 253u ? __uint_as_float((253u - e) << 23) : 0.0f;
+  return __uint_as_float(e < 253u ? (e + 1u) << 23 : 0x7fffffffu);
+}
+
+// Adds the products of three slices each of A (128 rows) and B, K = 16 KS, to
+// the accumulators (first: to zero); issued by one thread. Addresses are of
+// slice 0, strides in bytes. All addresses are constants beyond the operands'
+// descriptors: with a loop of computed ones a MMA took 105 cycles to issue and
+// 64 to run.
+template <int KS, int A_PLANE, int B_PLANE, int N>
+__device__ __forceinline__ void issue_split(uint32_t tmem, uint32_t a, uint32_t b, bool first) {
+  constexpr uint32_t idesc = idesc_bf16_f32(kTile, N);
+  const uint64_t ad = sdesc(a, 128u, KS * 256u), bd = sdesc(b, 128u, KS * 256u);
+#pragma unroll
+  for (int o = 2; o >= 0; --o)
+#pragma unroll
+    for (int i = 0; i <= o; ++i)
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+        mma_bf16(tmem + (o ? kAccCols : 0u), ad + (uint32_t)(i * A_PLANE / 16 + 16 * k),
+                 bd + (uint32_t)((o - i) * B_PLANE / 16 + 16 * k), idesc,
+                 i == 0 && o != 1 && k == 0 && first ? 0u : 1u);
+}
+
+// The same with A's slices in tensor memory at column `a`, KS * 8 columns
+// apart (two elements per column).
+template <int KS, int B_PLANE, int N>
+__device__ __forceinline__ void issue_split_ts(uint32_t tmem, uint32_t a, uint32_t b,
+                                               bool first) {
+  constexpr uint32_t idesc = idesc_bf16_f32(kTile, N);
+  const uint64_t bd = sdesc(b, 128u, KS * 256u);
+#pragma unroll
+  for (int o = 2; o >= 0; --o)
+#pragma unroll
+    for (int i = 0; i <= o; ++i)
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+        mma_bf16_ts(tmem + (o ? kAccCols : 0u), a + (uint32_t)(i * KS * 8 + 8 * k),
+                    bd + (uint32_t)((o - i) * B_PLANE / 16 + 16 * k), idesc,
+                    i == 0 && o != 1 && k == 0 && first ? 0u : 1u);
+}
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes,
+                                          uint64_t *bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)),
+               "r"(bytes)
+               : "memory");
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::
+          "r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// sum over k of x[k xs] w[k ws] in FP32, one fused multiply-add after the
+// other: the elements that the slices cannot hold. (Inlined: around a call the
+// registers of the fast path moved to the stack, 0.9 of 6.0 ms.)
+__device__ __forceinline__ float chain(const float *x, int64_t xs, const float *w, int64_t ws,
+                                       int K) {
+  float s = 0.0f;
+#pragma unroll 1
+  for (int k = 0; k < K; ++k) s = fmaf(x[k * xs], w[k * ws], s);
+  return s;
+}
+
+// Slices of the weight operands, a block per row.
+__global__ void __launch_bounds__(kHid) slice_weights_kernel(const float *__restrict__ packed,
+                                                             uint8_t *__restrict__ slices,
+                                                             float *__restrict__ scales) {
+  __shared__ float part[kHid / 32];
+  const int op = blockIdx.x / kHid, row = blockIdx.x % kHid, k = threadIdx.x;
+  const int l = op < 4 ? op : 7 - op, K = op ? kHid : kE;
+  float x = 0.0f;
+  if (k < K) x = packed[w_off(l) + (op < 4 ? k * kHid + row : row * kHid + k)];
+  float m = fabsf(x);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((k & 31) == 0) part[k >> 5] = m;
+  __syncthreads();
+  m = max_nan(max_nan(part[0], part[1]), max_nan(part[2], part[3]));
+  float inv;
+  const float s = row_scale(exponent(m), inv);
+  if (k == 0) scales[blockIdx.x] = s;
+  if (k >= K) return;
+  uint32_t h, mi, lo;
+  slice2(inv == 0.0f ? 0.0f : x, 0.0f, inv, h, mi, lo);
+  uint8_t *d = slices + op_off(op) + kmajor_off(row, k & ~7, K) + (k & 7) * 2;
+  *reinterpret_cast<uint16_t *>(d) = (uint16_t)h;
+  *reinterpret_cast<uint16_t *>(d + op_plane(op)) = (uint16_t)mi;
+  *reinterpret_cast<uint16_t *>(d + 2 * op_plane(op)) = (uint16_t)lo;
+}
+
+struct BwdParams {
+  int64_t ns;                 // samples of this launch
+  int64_t ns_all;             // of the batch (row length of signs)
+  const int32_t *vox;         // [ns]
+  const float4 *xyzd;         // [ns]
+  int64_t n_vox, n_keys;
+  float voxel_size;
+  const float *centers;       // [n_vox, 3]
+  const int32_t *feats;       // [n_vox, 8]
+  const float4 *values;       // [n_keys, 32]
+  const float *packed;        // kPacked floats
+  const uint8_t *slices;      // kSliceBytes
+  const float *scales;        // kScales
+  const uint4 *signs;         // [4][ns_all], from this launch's first sample
+  const float4 *d_out;        // [ns]
+  float *rows;                // [tiles][kRows][128]
+  float4 *g_values;           // [n_keys, 32]
+  int32_t *err;
+};
+
+struct BwdSmem {
+  uint8_t b[2][3 * kPlane];   // the slices of a layer's weights and of the next one's
+  uint8_t a0[3 * kSmallOp];   // of the tile's embeddings
+  float4 dout[kTile];
+  float scales[kScales];
+  float bias[4 * kHid];
+  float rmax[4][kTile];
+  float rs[kTile];
+  uint64_t mma_done, loaded[2];
+  uint32_t tmem;
+  int abort;
+};
+
+// Slices a thread's elements of its row to tensor memory (column `a` of its
+// lane on, two elements per column).
+__device__ __forceinline__ void slice_row(uint32_t a, const float (&y)[kQ], float inv) {
+#pragma unroll
+  for (int c = 0; c < kQ / 16; ++c) {
+    uint32_t h[8], m[8], l[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      slice2(y[c * 16 + 2 * i], y[c * 16 + 2 * i + 1], inv, h[i], m[i], l[i]);
+    __syncwarp();
+    tmem_st8(a + c * 8, h);
+    tmem_st8(a + kHid / 2 + c * 8, m);
+    tmem_st8(a + kHid + c * 8, l);
+  }
+  tmem_wait_st();
+}
+
+// v = the sums of 16 (8) columns of this thread's TMEM lane
+__device__ __forceinline__ void load_sums(uint32_t tmem, float (&v)[16]) {
+  float a1[16];
+  __syncwarp();
+  tmem_ld16(tmem, v);
+  tmem_ld16(tmem + kAccCols, a1);
+  tmem_wait_ld();
+  // (after the wait: the loads write their registers asynchronously)
+#pragma unroll
+  for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(v[i]), "+f"(a1[i]));
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] += a1[i];
+}
+
+__device__ __forceinline__ void load_sums8(uint32_t tmem, float (&v)[8]) {
+  uint32_t r[2][8];
+  __syncwarp();
+#pragma unroll
+  for (int o = 0; o < 2; ++o)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[o][0]), "=r"(r[o][1]), "=r"(r[o][2]), "=r"(r[o][3]), "=r"(r[o][4]),
+                   "=r"(r[o][5]), "=r"(r[o][6]), "=r"(r[o][7])
+                 : "r"(tmem + o * kAccCols)
+                 : "memory");
+  tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) asm volatile("" : "+r"(r[0][i]), "+r"(r[1][i]));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[0][i]) + __uint_as_float(r[1][i]);
+}
+
+__global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  BwdSmem &S = *reinterpret_cast<BwdSmem *>(smem_raw);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int row = (warp & 3) * 32 + lane, quarter = warp >> 2, c0 = quarter * kQ;
+  for (int i = t; i < 4 * kHid; i += kBT)
+    S.bias[i] = p.packed[kBiasOff + i];
+  for (int i = t; i < kScales; i += kBT) S.scales[i] = p.scales[i];
+  if (t == 0) {
+    mbar_init(&S.mma_done, 1);
+    mbar_init(&S.loaded[0], 1);
+    mbar_init(&S.loaded[1], 1);
+    S.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  constexpr uint32_t kCols = 512;
+  if (warp == 0) tmem_alloc(&S.tmem, kCols);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = S.tmem;
+  const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  volatile int *abort = &S.abort;
+  const int64_t tiles = (p.ns + kTile - 1) / kTile;
+  uint32_t ph_load = 0, ph_mma = 0;          // ph_load: of the two buffers
+  bool ok = true;
+  auto load_op = [&](int op) {               // thread 0
+    bulk_load(S.b[op & 1], p.slices + op_off(op), 3u * op_plane(op), &S.loaded[op & 1]);
+  };
+  // One layer's MMAs on the slices written before the last barrier. What
+  // needs no result follows between start and finish; after finish the
+  // operand after the next is on its way.
+  auto start = [&](int op) {
+    if (t == 0 && mbar_wait(&S.loaded[op & 1], ph_load >> (op & 1) & 1u, abort)) {
+      fence_after_sync();
+      const uint32_t b = smem_u32(S.b[op & 1]);
+      if (op == 0)
+        issue_split<kE / 16, kSmallOp, kSmallOp, kHid>(tmem, smem_u32(S.a0), b, true);
+      else if (op < 7)
+        issue_split_ts<kHid / 16, kPlane, kHid>(tmem, tmem + kACol, b, true);
+      else
+        issue_split_ts<kHid / 16, kSmallOp, kE>(tmem, tmem + kACol, b, true);
+      mma_commit(&S.mma_done);
+    }
+    ph_load ^= 1u << (op & 1);
+  };
+  auto finish = [&](int op, bool more) {
+    ok = mbar_wait(&S.mma_done, ph_mma, abort) && ok;
+    ph_mma ^= 1u;
+    fence_after_sync();
+    if (t == 0 && ok && (op < 6 || more)) load_op((op + 2) & 7);
+  };
+  // Interpolation: 8 threads per sample, 4 channels each (interp.cu's
+  // operations), samples t / 8 + 64 it of the tile.
+  float4 e[kTile * 8 / kBT];
+  auto gather = [&](int64_t tile) {
+    constexpr int N = kTile * 8 / kBT;
+    const int ch = t & 7;
+    int64_t v[N];
+#pragma unroll
+    for (int it = 0; it < N; ++it) {
+      const int64_t s = tile * kTile + it * (kBT / 8) + (t >> 3);
+      v[it] = s < p.ns ? (int64_t)p.vox[s] : -1;
+      if (v[it] >= p.n_vox) v[it] = -1;
+    }
+#pragma unroll
+    for (int it = 0; it < N; ++it) {
+      e[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (v[it] < 0) continue;
+      const int64_t s = tile * kTile + it * (kBT / 8) + (t >> 3);
+      const float4 x = p.xyzd[s];
+      const float cx = p.centers[v[it] * 3], cy = p.centers[v[it] * 3 + 1],
+                  cz = p.centers[v[it] * 3 + 2];
+      int key[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) key[k] = p.feats[v[it] * 8 + k];
+      // (every load before the first use: one wait for the 8 rows)
+      float4 c[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        c[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (key[k] >= 0 && key[k] < p.n_keys)
+          c[k] = __ldg(p.values + (int64_t)key[k] * (kE / 4) + ch);
+      }
+      const float q[3] = {(x.x - cx) / p.voxel_size + 0.5f, (x.y - cy) / p.voxel_size + 0.5f,
+                          (x.z - cz) / p.voxel_size + 0.5f};
+      float4 a = e[it];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (key[k] < 0 || key[k] >= p.n_keys) continue;
+        const float w = corner_weight(q, k);
+        a.x = fmaf(w, c[k].x, a.x); a.y = fmaf(w, c[k].y, a.y);
+        a.z = fmaf(w, c[k].z, a.z); a.w = fmaf(w, c[k].w, a.w);
+      }
+      e[it] = a;
+    }
+  };
+  // grad_values[feats[v, k]] += w_k g, summed over a thread's consecutive
+  // samples of one voxel before the atomics: 4 samples, 4 channels and 4
+  // corners a thread
+  auto scatter = [&](int64_t tile) {
+    const int cg = lane & 7, sg = (warp & 7) * 4 + (lane >> 3), k0 = warp >> 3 << 2;
+    int64_t prev = -1;
+    float4 sum[4];
+    auto flush = [&]() {
+      if (prev < 0) return;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int64_t key = p.feats[prev * 8 + k0 + k];
+        if (key >= 0 && key < p.n_keys) atomicAdd(p.g_values + key * (kE / 4) + cg, sum[k]);
+      }
+    };
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+      const int64_t s = tile * kTile + sg * 4 + i;
+      int64_t v = s < p.ns ? (int64_t)p.vox[s] : -1;
+      if (v >= p.n_vox) v = -1;
+      if (v < 0) continue;
+      if (v != prev) {
+        flush();
+        prev = v;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      const float4 x = p.xyzd[s];
+      const float q[3] = {(x.x - p.centers[v * 3 + 0]) / p.voxel_size + 0.5f,
+                          (x.y - p.centers[v * 3 + 1]) / p.voxel_size + 0.5f,
+                          (x.z - p.centers[v * 3 + 2]) / p.voxel_size + 0.5f};
+      const float4 gi = *reinterpret_cast<const float4 *>(
+          p.rows + (tile * kRows + kDA0) * kTile + (sg * 4 + i) * kE + cg * 4);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float w = corner_weight(q, k0 + k);
+        sum[k].x = fmaf(w, gi.x, sum[k].x); sum[k].y = fmaf(w, gi.y, sum[k].y);
+        sum[k].z = fmaf(w, gi.z, sum[k].z); sum[k].w = fmaf(w, gi.w, sum[k].w);
+      }
+    }
+    flush();
+  };
+  float sa = 0.0f;                           // scale of this thread's row in A
+  float y[kQ];                               // its elements: units c0 + j
+  int64_t last = -1;                         // the tile whose dA0 waits in memory
+  if ((int64_t)blockIdx.x < tiles) {
+    if (t == 0) {
+      load_op(0);
+      load_op(1);
+    }
+    gather(blockIdx.x);
+  }
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t s0 = tile * kTile;
+    float *R = p.rows + tile * kRows * kTile;
+    const bool live = s0 + row < p.ns;
+#pragma unroll
+    for (int it = 0; it < kTile * 8 / kBT; ++it) {
+      const int sl = it * (kBT / 8) + (t >> 3), ch = t & 7;
+      const float4 a = e[it];
+      float m = max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(a.z), fabsf(a.w))), inv;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const float sc = row_scale(exponent(m), inv);
+      if (ch == 0) S.rs[sl] = sc;
+      uint32_t h0, m0, l0, h1, m1, l1;
+      slice2(a.x, a.y, inv, h0, m0, l0);
+      slice2(a.z, a.w, inv, h1, m1, l1);
+      uint8_t *d = S.a0 + kmajor_off(sl, (ch >> 1) * 8, kE) + (ch & 1) * 8;
+      *reinterpret_cast<uint2 *>(d) = make_uint2(h0, h1);
+      *reinterpret_cast<uint2 *>(d + kSmallOp) = make_uint2(m0, m1);
+      *reinterpret_cast<uint2 *>(d + 2 * kSmallOp) = make_uint2(l0, l1);
+      const float ev[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) R[(ch * 4 + j) * kTile + sl] = ev[j];
+    }
+    if (t < kTile)
+      S.dout[t] = s0 + t < p.ns ? p.d_out[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
+    fence_async_smem();
+    fence_before_sync();
+    __syncthreads();
+    sa = S.rs[row];
+    // a layer's signs of this thread's units: unit j at bit 8 (j / 4 % 4) +
+    // j % 4 of word j / 16
+    auto signs = [&](int l, uint32_t (&m)[2]) {
+      uint2 w = make_uint2(0, 0);
+      if (live)
+        w = reinterpret_cast<const uint2 *>(p.signs + (int64_t)l * p.ns_all + s0 + row)[quarter & 1];
+      m[0] = w.x >> ((quarter >> 1) * 4);
+      m[1] = w.y >> ((quarter >> 1) * 4);
+    };
+    auto bit = [](const uint32_t (&m)[2], int j) {
+      return (m[j >> 4] >> (((j >> 2) & 3) * 8 + (j & 3))) & 1u;
+    };
+    auto store = [&](int first_row) {
+      float *out = R + (first_row + c0) * kTile + row;
+#pragma unroll
+      for (int j = 0; j < kQ; ++j) out[j * kTile] = y[j];
+    };
+    // Ends a layer: joins the row's quarters and, where `slice`, puts its
+    // slices in A. top: the largest |y|, NaN where fix(j) has to give y[j]
+    // again (it reads rows of memory written before the barrier). False:
+    // unwind.
+    auto rows_done = [&](float top, bool slice, auto fix) {
+      S.rmax[quarter][row] = top;
+      if (!__syncthreads_and(ok && top == top)) {
+        if (!__syncthreads_and(ok)) return false;
+        if (top != top) {
+          top = 0.0f;
+#pragma unroll
+          for (int j = 0; j < kQ; ++j) {
+            if (y[j] != y[j]) y[j] = fix(j);
+            top = max_nan(top, fabsf(y[j]));
+          }
+          S.rmax[quarter][row] = top;
+        }
+        __syncthreads();
+      }
+      if (!slice) return true;
+      float inv;
+      sa = row_scale(exponent(max_nan(max_nan(S.rmax[0][row], S.rmax[1][row]),
+                                      max_nan(S.rmax[2][row], S.rmax[3][row]))),
+                     inv);
+      slice_row(tmem_row + kACol + c0 / 2, y, inv);
+      fence_before_sync();
+      __syncthreads();
+      return true;
+    };
+#pragma unroll 1
+    for (int l = 0; l < 4; ++l) {
+      uint32_t m[2];
+      signs(l, m);
+      start(l);
+      if (l) store(a_row(l));
+      if (l == 1 && last >= 0) scatter(last);
+      finish(l, true);
+      const float *sc = S.scales + l * kHid + c0, *bias = S.bias + l * kHid + c0;
+      float top = 0.0f;
+#pragma unroll
+      for (int c = 0; c < kQ / 16; ++c) {
+        float v[16];
+        load_sums(tmem_row + c0 + c * 16, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int j = c * 16 + i;
+          const float z = fmaf(v[i] * sc[j], sa, bias[j]);
+          y[j] = bit(m, j) || z != z ? z : 0.0f;
+          top = max_nan(top, fabsf(y[j]));
+        }
+      }
+      if (!rows_done(top, l < 3, [&](int j) {
+            const float z = chain(R + a_row(l) * kTile + row, kTile, p.packed + w_off(l) + c0 + j,
+                                  kHid, l ? kHid : kE) +
+                            bias[j];
+            return bit(m, j) || z != z ? z : 0.0f;
+          }))
+        goto out;
+    }
+    store(a_row(4));
+    // dA4 = d_out W4
+    {
+      const float4 d = S.dout[row];
+      const float4 *w4 = reinterpret_cast<const float4 *>(p.packed + kW4Off + c0);
+#pragma unroll
+      for (int j = 0; j < kQ; j += 4) {
+        const float4 a = __ldg(w4 + j / 4), b = __ldg(w4 + kHid / 4 + j / 4),
+                     c = __ldg(w4 + kHid / 2 + j / 4), e4 = __ldg(w4 + 3 * kHid / 4 + j / 4);
+        y[j] = fmaf(d.w, e4.x, fmaf(d.z, c.x, fmaf(d.y, b.x, d.x * a.x)));
+        y[j + 1] = fmaf(d.w, e4.y, fmaf(d.z, c.y, fmaf(d.y, b.y, d.x * a.y)));
+        y[j + 2] = fmaf(d.w, e4.z, fmaf(d.z, c.z, fmaf(d.y, b.z, d.x * a.z)));
+        y[j + 3] = fmaf(d.w, e4.w, fmaf(d.z, c.w, fmaf(d.y, b.w, d.x * a.w)));
+      }
+    }
+#pragma unroll 1
+    for (int l = 3; l >= 0; --l) {
+      uint32_t m[2];
+      signs(l, m);
+      float top = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kQ; ++j) {
+        y[j] *= bit(m, j) ? 1.0f : 0.0f;
+        top = max_nan(top, fabsf(y[j]));
+      }
+      if (!rows_done(top, true, [&](int j) {
+            if (l == 3) return y[j];
+            return chain(R + dz_row(l + 1) * kTile + row, kTile,
+                         p.packed + w_off(l + 1) + (c0 + j) * kHid, 1, kHid) *
+                   (bit(m, j) ? 1.0f : 0.0f);
+          }))
+        goto out;
+      const int op = 7 - l;
+      start(op);
+      store(dz_row(l));
+      if (l == 1 && tile + gridDim.x < tiles) gather(tile + gridDim.x);
+      finish(op, tile + gridDim.x < tiles);
+      if (l == 0) break;
+      const float *sc = S.scales + op * kHid + c0;
+#pragma unroll
+      for (int c = 0; c < kQ / 16; ++c) {
+        float v[16];
+        load_sums(tmem_row + c0 + c * 16, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[c * 16 + i] = v[i] * sc[c * 16 + i] * sa;
+      }
+    }
+    // dA0: 8 channels a thread
+    {
+      float v[8], nan = 0.0f;               // 0 or NaN
+      load_sums8(tmem_row + quarter * 8, v);
+      float *g = R + kDA0 * kTile + row * kE + quarter * 8;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = v[i] * S.scales[7 * kHid + quarter * 8 + i] * sa;
+        nan = max_nan(nan, v[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i += 4)
+        *reinterpret_cast<float4 *>(g + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      fence_before_sync();
+      if (!__syncthreads_and(ok && nan == nan)) {
+        if (!__syncthreads_and(ok)) goto out;
+#pragma unroll 1
+        for (int i = 0; i < 8 && nan != nan; ++i)
+          if (g[i] != g[i])
+            g[i] = chain(R + dz_row(0) * kTile + row, kTile,
+                         p.packed + w_off(0) + (quarter * 8 + i) * kHid, 1, kHid);
+        __syncthreads();
+      }
+    }
+    last = tile;
+  }
+  if (last >= 0) scatter(last);
+out:
+  if (t == 0 && S.abort) {
+    // a wait ran out: give the copy and the MMAs in flight one more limit
+    int never = 0;
+    if (p.err) atomicOr(p.err, 8);
+    for (int i = 0; i < 2; ++i) {
+      mbar_wait(&S.loaded[i], ph_load >> i & 1u, &never);
+      never = 0;
+    }
+    mbar_wait(&S.mma_done, ph_mma, &never);
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  if (warp == 0) tmem_dealloc(tmem, kCols);
+}
+
+// The two operands of a tile in FP32, and the slices of Y for half a tile's
+// samples (K = 64) in two stages; X's slices are in tensor memory.
+constexpr int kHalfPlane = kHid * 64 * 2;
+struct GradSmem {
+  float in[2][kHid * kTile];  // X, Y: rows of 32 16-byte chunks, chunk c at c ^ (row & 7)
+  uint8_t y[2][3 * kHalfPlane];
+  uint8_t top[2][4][kHid];    // X, Y: the largest exponent in each quarter of a row
+  float ys[2][kHid];          // Y's scales, by parity of the tile
+  uint64_t done;
+  uint32_t tmem;
+  int abort;
+};
+
+__device__ __forceinline__ void cp_async(void *dst, const void *src, int size, bool fill) {
+  if (size == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
+  else                                       // 4 bytes, zero where !fill
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(fill ? 4 : 0)
+                 : "memory");
+}
+
+// dW = X^T Y of one layer over some of the chunk's tiles, X = dZ (A4 for the
+// head), Y = A (d_out). A thread slices 32 samples (a quarter of each half of
+// the tile) of row t % 128 of both.
+__global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
+                                                             const float *__restrict__ rows,
+                                                             const float *__restrict__ d_out,
+                                                             float *__restrict__ part,
+                                                             float *__restrict__ bias_part, int add,
+                                                             int32_t *err) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  GradSmem &S = *reinterpret_cast<GradSmem *>(smem_raw);
+  const int t = threadIdx.x, warp = t >> 5, b = blockIdx.x;
+  const int l = b < 3 * kSplit ? 1 + b / kSplit : b < 3 * kSplit + kSplit0 ? 0 : 4;
+  const int j = l == 0 ? b - 3 * kSplit : l == 4 ? b - 3 * kSplit - kSplit0 : b % kSplit;
+  const int splits = l == 0 ? kSplit0 : l == 4 ? kSplit4 : kSplit;
+  const int ny = l == 0 ? kE : l == 4 ? 16 : kHid;           // columns of the result
+  const int yrows = l == 4 ? 4 : ny;                         // rows of Y with data
+  const int64_t xrow = l == 4 ? a_row(4) : dz_row(l), yrow = l == 4 ? 0 : a_row(l);
+  // TMEM lane = row of X and of the result
+  const int row = t & (kHid - 1), quarter = t >> 7;
+  const int ncol = ny == kHid ? 32 : ny == kE || quarter < 2 ? 8 : 0;
+  const int c0 = ny == kHid ? quarter * 32 : quarter * 8;
+  if (t == 0) {
+    mbar_init(&S.done, 1);
+    S.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (l == 4)                                // rows 4..15 stay zero
+    for (int i = t; i < (int)sizeof(S.y) / 16; i += kBT)
+      reinterpret_cast<uint4 *>(S.y)[i] = make_uint4(0, 0, 0, 0);
+  constexpr uint32_t kCols = 512;
+  if (warp == 0) tmem_alloc(&S.tmem, kCols);
+  fence_async_smem();
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = S.tmem;
+  const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  constexpr uint32_t kXCol = 2 * kAccCols, kXHalf = 3 * 32;  // slices of a half: 32 columns each
+  volatile int *abort = &S.abort;
+  const int64_t tiles = (ns + kTile - 1) / kTile;
+  float acc[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+  float sum = 0.0f, comp = 0.0f;             // of the thread's samples of its row (db), Kahan
+  float v[2][32];                            // X, Y: samples h * 64 + quarter * 16 + 0..15
+  float inv[2], xs = 0.0f, xs_prev = 0.0f;
+  bool ok = true;
+  // copies of a tile's rows to S.in
+  auto fetch = [&](int64_t tile) {
+    const float *R = rows + tile * kRows * kTile;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      if (g && l == 4) {
+        // sample t / 4, output t % 4
+        const int64_t s = tile * kTile + (t >> 2);
+        const int u = t & 3, c = (t >> 4) ^ u;
+        cp_async(S.in[1] + u * kTile + c * 4 + ((t >> 2) & 3), d_out + (s < ns ? s : 0) * 4 + u, 4,
+                 s < ns);
+      } else {
+        const float *src = R + (g ? yrow : xrow) * kTile;
+        const int n = (g ? ny : kHid) * 32;
+#pragma unroll
+        for (int k = 0; k < kHid * 32 / kBT; ++k) {
+          const int i = t + k * kBT, r = i >> 5, c = i & 31;
+          if (i < n) cp_async(S.in[g] + r * kTile + ((c ^ (r & 7)) << 2), src + i * 4, 16, true);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // the fetched tile to registers, its scales; the next one on its way
+  auto take = [&](int64_t next, int buf) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      if (g && row >= yrows) continue;
+      const float *in = S.in[g] + row * kTile;
+      float m = 0.0f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int at = (c >> 2) * 16 + quarter * 4 + (c & 3);
+        const float4 a = *reinterpret_cast<const float4 *>(in + ((at ^ (row & 7)) << 2));
+        v[g][c * 4] = a.x; v[g][c * 4 + 1] = a.y; v[g][c * 4 + 2] = a.z; v[g][c * 4 + 3] = a.w;
+        m = max_nan(m, max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(a.z), fabsf(a.w))));
+      }
+      S.top[g][quarter][row] = (uint8_t)exponent(m);
+    }
+    ok = __syncthreads_and(ok);
+    if (next < tiles) fetch(next);
+    xs_prev = xs;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      if (g && row >= yrows) continue;
+      const float sc = row_scale(max(max(S.top[g][0][row], S.top[g][1][row]),
+                                     max(S.top[g][2][row], S.top[g][3][row])),
+                                 inv[g]);
+      if (!g) xs = sc;
+      else if (quarter == 0) S.ys[buf][row] = sc;
+    }
+    if (l != 4 || row < 4) {
+      float s[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) s[i] = l == 4 ? v[1][i] : v[0][i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) s[i] += s[i + o];
+      const float a = s[0] - comp, w = sum + a;
+      comp = fabsf(w) <= 3.4e38f ? (w - sum) - a : 0.0f;
+      sum = w;
+    }
+  };
+  // adds the finished result of `tile` (X's scale x) to acc
+  auto drain = [&](int64_t tile, int buf, float x) {
+    fence_after_sync();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c * 8 >= ncol) break;
+      float d[8];
+      load_sums8(tmem_row + c0 + c * 8, d);
+      float nan = 0.0f;                      // 0 or NaN
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        d[i] = d[i] * S.ys[buf][c0 + c * 8 + i] * x;
+        nan = max_nan(nan, d[i]);
+      }
+      if (nan != nan) {
+        const float *X = rows + (tile * kRows + xrow + row) * kTile;
+        const float *Y = l == 4 ? d_out + tile * kTile * 4 : rows + (tile * kRows + yrow) * kTile;
+        const int K = ns - tile * kTile < kTile ? (int)(ns - tile * kTile) : kTile;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int n = c0 + c * 8 + i;
+          if (d[i] != d[i] && n < yrows)
+            d[i] = l == 4 ? chain(X, 1, Y + n, 4, K) : chain(X, 1, Y + n * kTile, 1, K);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[c * 8 + i] += d[i];
+    }
+  };
+  int64_t n = 0;                             // tiles begun
+  if (j < tiles) fetch(j);
+  for (int64_t tile = j; tile < tiles; tile += splits, ++n) {
+    const int buf = (int)(n & 1);
+    take(tile + splits, buf);
+    if (!ok) break;
+    if (n > 0) {
+      ok = mbar_wait(&S.done, (uint32_t)(n - 1) & 1u, abort);
+      drain(tile - splits, buf ^ 1, xs_prev);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t a[3][8];
+#pragma unroll
+      for (int g = 1; g >= 0; --g) {
+        if (g && row >= yrows) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          slice2(v[g][h * 16 + 2 * i], v[g][h * 16 + 2 * i + 1], inv[g], a[0][i], a[1][i], a[2][i]);
+        if (g) {
+#pragma unroll
+          for (int o = 0; o < 3; ++o) {
+            uint8_t *d = S.y[h] + o * kHalfPlane + kmajor_off(row, quarter * 16, 64);
+            *reinterpret_cast<uint4 *>(d) = make_uint4(a[o][0], a[o][1], a[o][2], a[o][3]);
+            *reinterpret_cast<uint4 *>(d + 128) = make_uint4(a[o][4], a[o][5], a[o][6], a[o][7]);
+          }
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int o = 0; o < 3; ++o) tmem_st8(tmem_row + kXCol + h * kXHalf + o * 32 + quarter * 8, a[o]);
+      tmem_wait_st();
+      fence_async_smem();
+      fence_before_sync();
+      ok = __syncthreads_and(ok);
+      if (t == 0 && ok) {
+        fence_after_sync();
+        const uint32_t x = tmem + kXCol + h * kXHalf, y = smem_u32(S.y[h]);
+        if (ny == kHid)
+          issue_split_ts<4, kHalfPlane, kHid>(tmem, x, y, h == 0);
+        else if (ny == kE)
+          issue_split_ts<4, kHalfPlane, kE>(tmem, x, y, h == 0);
+        else
+          issue_split_ts<4, kHalfPlane, 16>(tmem, x, y, h == 0);
+        if (h == 1) mma_commit(&S.done);
+      }
+    }
+    if (!ok) break;
+  }
+  if (n > 0 && ok) {
+    ok = mbar_wait(&S.done, (uint32_t)(n - 1) & 1u, abort);
+    if (__syncthreads_and(ok)) drain(j + (n - 1) * splits, (int)(n - 1) & 1, xs);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (S.abort && t == 0) {
+    // a wait ran out: give the MMAs in flight one more limit
+    int never = 0;
+    if (err) atomicOr(err, 8);
+    mbar_wait(&S.done, n > 0 ? (uint32_t)(n - 1) & 1u : 0u, &never);
+  }
+  // slots: layers 1..3 [128][128], layer 0 [128][32], head [128][4]
+  float *P = part + (l == 0   ? (int64_t)3 * kSplit * kHid * kHid + (int64_t)j * kHid * kE
+                     : l == 4 ? (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE +
+                                    (int64_t)j * kHid * 4
+                              : (int64_t)b * kHid * kHid) +
+             (int64_t)row * yrows + c0;
+#pragma unroll
+  for (int i = 0; i < 32; i += 4) {
+    if (i >= ncol || c0 + i >= yrows) break;
+    float4 *d = reinterpret_cast<float4 *>(P + i);
+    float4 o = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+    if (add) {
+      const float4 w = *d;
+      o.x += w.x; o.y += w.y; o.z += w.z; o.w += w.w;
+    }
+    *d = o;
+  }
+  __syncthreads();
+  float *const sums = S.in[0];
+  sums[quarter * kHid + row] = sum;
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  if (t < kHid) {
+    const float s =
+        (sums[t] + sums[kHid + t]) + (sums[2 * kHid + t] + sums[3 * kHid + t]);
+    float *d = bias_part + (int64_t)b * kHid + t;
+    *d = add ? *d + s : s;
+  }
+  if (warp == 0) tmem_dealloc(tmem, kCols);
+}
+
+static_assert(sizeof(BwdSmem) <= 232448 && sizeof(GradSmem) <= 232448, "shared memory");
+
+constexpr int64_t kPartFloats =
+    (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE + (int64_t)kSplit4 * kHid * 4;
+
+struct GradOut {
+  float *w[5], *b[5];
+};
+
+// The field's gradients from the slots, each element's slots added in order.
+__global__ void __launch_bounds__(kT) grad_reduce_kernel(const float *__restrict__ part,
+                                                         const float *__restrict__ bias_part,
+                                                         GradOut out) {
+  int i = blockIdx.x * kT + threadIdx.x;
+  const float *src;
+  float *dst;
+  int n, stride;
+  if (i < 3 * kHid * kHid) {
+    const int l = i / (kHid * kHid), e = i % (kHid * kHid);
+    src = part + (int64_t)l * kSplit * kHid * kHid + e;
+    n = kSplit; stride = kHid * kHid;
+    dst = out.w[l + 1] + e;
+  } else if ((i -= 3 * kHid * kHid) < kHid * kE) {
+    src = part + (int64_t)3 * kSplit * kHid * kHid + i;
+    n = kSplit0; stride = kHid * kE;
+    dst = out.w[0] + i;
+  } else if ((i -= kHid * kE) < kHid * 4) {
+    src = part + (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE + i;
+    n = kSplit4; stride = kHid * 4;
+    dst = out.w[4] + (i & 3) * kHid + (i >> 2);
+  } else if ((i -= kHid * 4) < 4 * kHid) {
+    const int l = i / kHid;
+    src = bias_part + (int64_t)(l ? (l - 1) * kSplit : 3 * kSplit) * kHid + i % kHid;
+    n = l ? kSplit : kSplit0; stride = kHid;
+    dst = out.b[l] + i % kHid;
+  } else if ((i -= 4 * kHid) < 4) {
+    src = bias_part + (int64_t)(3 * kSplit + kSplit0) * kHid + i;
+    n = kSplit4; stride = kHid;
+    dst = out.b[4] + i;
+  } else {
+    return;
+  }
+  float s = 0.0f, c = 0.0f;                  // compensated (Kahan)
+#pragma unroll 8
+  for (int k = 0; k < n; ++k) {
+    const float a = src[(int64_t)k * stride] - c, b = s + a;
+    c = fabsf(b) <= 3.4e38f ? (b - s) - a : 0.0f;
+    s = b;
+  }
+  *dst = s;
+}
+
+// floats of the workspace besides a chunk's rows
+constexpr int64_t kFixedFloats = kPartFloats + (int64_t)kSMs * kHid + (kSliceFloats + 31) / 32 * 32;
+
+int64_t chunk_rows(int64_t ns, int64_t chunk) {
+  const int64_t c = chunk < ns ? chunk : ns;
+  return (c + kTile - 1) / kTile * kTile;
+}
+
+}  // namespace
+
+extern "C" {
+
+int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_samples) {
+  if (n_samples < 0 || chunk_samples < 1) return -1;
+  return kFixedFloats + chunk_rows(n_samples, chunk_samples) * kRows;
+}
+
+int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
+                              const float *xyz_dist, int64_t n_voxels, int64_t n_keys,
+                              float voxel_size, const float *centers, const int32_t *feats,
+                              const float *values, const float *packed, const uint8_t *signs,
+                              const float *grad_out, float *workspace, int64_t workspace_floats,
+                              float *grad_values, float *const grad_weights[5],
+                              float *const grad_biases[5], int32_t *err, void *stream) {
+  if (bad_scene(n_samples, voxel, xyz_dist, n_voxels, n_keys, centers, feats, values, packed) ||
+      chunk_samples < 1 || chunk_samples % kTile || !grad_weights || !grad_biases || !workspace ||
+      !packed || (((uintptr_t)workspace) & 15))
+    return NSVF_ERR_INVALID;
+  if (n_samples > 0 &&
+      (!grad_out || !grad_values || !signs ||
+       ((((uintptr_t)grad_out) | ((uintptr_t)grad_values) | ((uintptr_t)signs)) & 15)))
+    return NSVF_ERR_INVALID;
+  if (workspace_floats < nsvf_field_train_backward_floats(n_samples, chunk_samples))
+    return NSVF_ERR_CAPACITY;
+  GradOut g;
+  for (int l = 0; l < 5; ++l) {
+    if (!grad_weights[l] || !grad_biases[l]) return NSVF_ERR_INVALID;
+    g.w[l] = grad_weights[l];
+    g.b[l] = grad_biases[l];
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  if (cudaFuncSetAttribute(field_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(BwdSmem)) != cudaSuccess ||
+      cudaFuncSetAttribute(weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GradSmem)) != cudaSuccess)
+    return NSVF_ERR_CUDA;
+  float *rows = workspace;
+  uint8_t *slices =
+      (uint8_t *)(rows + chunk_rows(n_samples, chunk_samples) * kRows);
+  float *scales = (float *)(slices + kSliceBytes);
+  float *part = (float *)slices + (kSliceFloats + 31) / 32 * 32;
+  float *bias_part = part + kPartFloats;
+  int st;
+  if (n_samples > 0) {
+    slice_weights_kernel<<<kScales, kHid, 0, s>>>(packed, slices, scales);
+    if ((st = nsvf_launch_status()) != NSVF_OK) return st;
+  }
+  BwdParams p = {};
+  p.ns_all = n_samples;
+  p.n_vox = n_voxels;
+  p.n_keys = n_keys;
+  p.voxel_size = voxel_size;
+  p.centers = centers;
+  p.feats = feats;
+  p.values = (const float4 *)values;
+  p.packed = packed;
+  p.slices = slices;
+  p.scales = scales;
+  p.rows = rows;
+  p.g_values = (float4 *)grad_values;
+  p.err = err;
+  // (one pass without samples zeroes the slots of an empty batch)
+  for (int64_t a = 0; a == 0 || a < n_samples; a += chunk_samples) {
+    p.ns = n_samples - a < chunk_samples ? n_samples - a : chunk_samples;
+    p.vox = voxel + a;
+    p.xyzd = (const float4 *)xyz_dist + a;
+    p.signs = (const uint4 *)signs + a;
+    p.d_out = (const float4 *)grad_out + a;
+    if (p.ns > 0) {
+      const int64_t tiles = (p.ns + kTile - 1) / kTile;
+      field_bwd_kernel<<<(int)(tiles < kSMs ? tiles : kSMs), kBT, sizeof(BwdSmem), s>>>(p);
+      if ((st = nsvf_launch_status()) != NSVF_OK) return st;
+    }
+    weight_grad_kernel<<<kSMs, kBT, sizeof(GradSmem), s>>>(p.ns, rows, (const float *)p.d_out, part,
+                                                          bias_part, a > 0, err);
+    if ((st = nsvf_launch_status()) != NSVF_OK) return st;
+  }
+  constexpr int n_grads = 3 * kHid * kHid + kHid * kE + 8 * kHid + 4;
+  grad_reduce_kernel<<<nsvf_grid(n_grads, kT), kT, 0, s>>>(part, bias_part, g);
+  return nsvf_launch_status();
+}
+
+}  // extern "C"

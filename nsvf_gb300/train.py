@@ -5,16 +5,18 @@ The reference trains through autograd and keeps every ray chunk's graph
 alive until the loss's backward (fairnr/modules/renderer.py:135-232): the
 [samples, 8, 32] corner gathers and every MLP activation of the whole batch.
 Here `RayBatch` is one torch.autograd.Function per batch of rays that keeps
-its compacted samples (voxel ids, positions, depths, lengths: 28 bytes each)
-and their field values. Its backward runs
+its compacted samples (voxel ids, positions, depths, lengths: 28 bytes each),
+their field values and the signs of their pre-activations (64 bytes). Its
+backward runs
 
   compositing backward     nsvf_composite_rows_backward (transmittance prefix
                            recomputed in the kernel), with the free energy's:
                            d sigma = d fe * dist * 7 where sigma > 0
   field backward           nsvf_field_train_backward: per chunk of samples,
                            interpolation and activations again, dZ = dA (Z >
-                           0), dA = dZ W through all layers of a tile in
-                           shared memory, then dW = dZ^T A, db = sum dZ
+                           0), dA = dZ W through all layers of a tile, then
+                           dW = dZ^T A, db = sum dZ, on the tensor cores in
+                           split FP32
   interpolation backward   float4 atomics into the corner embeddings, from the
                            same tiles
 
@@ -148,9 +150,9 @@ class RayChunk(Function):
         return (g_values, *grads) + (None,) * 8
 
 
-# Samples of one wave of nsvf_field_train_backward: 304 blocks (two per SM) of
-# one 128-sample tile. A chunk is whole waves, so that no SM idles between the
-# chunks of a batch.
+# Samples of two waves of nsvf_field_train_backward: 152 blocks (one per SM) of
+# one 128-sample tile each. A chunk is a multiple, so that no SM idles between
+# the chunks of a batch.
 WAVE = 304 * 128
 
 
@@ -180,20 +182,23 @@ class RayBatch(Function):
         f = lambda *shape: torch.empty(*shape, dtype=torch.float32, device=dev)
         vox = torch.empty(max(ns, 1), dtype=torch.int32, device=dev)
         xyzd, depth, field = f(max(ns, 1), 4), f(max(ns, 1)), f(max(ns, 1), 4)
+        signs = torch.empty(4, max(ns, 1), 16, dtype=torch.uint8, device=dev) \
+            if any(ctx.needs_input_grad) else None
         if ns:
             check(LIB.nsvf_train_rows_pack(R, M, _p(sidx), _p(xyz), _p(dists), _p(depths),
                                            _p(offset), _p(vox), _p(xyzd), _p(depth), stream),
                   "train_rows_pack")
             packed = RayBatch._packed(params, stream)
-            check(LIB.nsvf_field_train_forward(
+            check(LIB.nsvf_field_train_forward_signs(
                 ns, _p(vox), _p(xyzd), centers.size(0), values.size(0), float(voxel_size),
-                _p(centers), _p(feats), _p(values), _p(packed), _p(field),
+                _p(centers), _p(feats), _p(values), _p(packed), _p(field), _p(signs),
                 _p(ext.error_word(dev)), stream), "field_train_forward")
         colors, out_depth, missed = f(R, 3), f(R), f(R)
         check(LIB.nsvf_composite_rows(R, _p(offset), _p(field), _p(xyzd), _p(depth), SIGMA_SCALE,
                                       _p(colors), _p(out_depth), _p(missed), int(bool(kahan)),
                                       stream), "composite_rows")
-        ctx.save_for_backward(values, *params, vox, xyzd, depth, offset, field, centers, feats)
+        ctx.save_for_backward(values, *params, vox, xyzd, depth, offset, field, signs, centers,
+                              feats)
         ctx.voxel_size, ctx.kahan, ctx.ns = float(voxel_size), bool(kahan), ns
         waves = max(1, round(ns * int(chunk_rays) / max(R, 1) / WAVE))
         ctx.chunk = waves * WAVE
@@ -211,7 +216,7 @@ class RayBatch(Function):
     def backward(ctx, g_colors, g_depth, g_missed):
         saved = ctx.saved_tensors
         values, params = saved[0], saved[1:11]
-        vox, xyzd, depth, offset, field, centers, feats = saved[11:]
+        vox, xyzd, depth, offset, field, signs, centers, feats = saved[11:]
         dev = values.device
         stream = ext.ctypes_stream(dev)
         R, ns = offset.numel() - 1, ctx.ns
@@ -230,8 +235,9 @@ class RayBatch(Function):
             packed = RayBatch._packed(params, stream)
             check(LIB.nsvf_field_train_backward(
                 ns, ctx.chunk, _p(vox), _p(xyzd), centers.size(0), values.size(0), ctx.voxel_size,
-                _p(centers), _p(feats), _p(values), _p(packed), _p(g_field), _p(work), n,
-                _p(g_values), _ptrs(grads[0::2]), _ptrs(grads[1::2]), stream),
+                _p(centers), _p(feats), _p(values), _p(packed), _p(signs), _p(g_field), _p(work),
+                n, _p(g_values), _ptrs(grads[0::2]), _ptrs(grads[1::2]), _p(ext.error_word(dev)),
+                stream),
                 "field_train_backward")
         return (g_values, *grads) + (None,) * 9
 

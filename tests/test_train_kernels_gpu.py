@@ -126,6 +126,107 @@ def test_forward_bits_of_a_gemm_chain(cuda, ns):
     assert torch.equal(out, x)
 
 
+def _field_grads(cuda, ns, dout, seed, chunk):
+    """The field's forward with signs and its backward on random samples, and
+    the FP32 layers of the same samples: (grads, grad_values), (acts, pre,
+    params, scene)."""
+    from nsvf_gb300 import ext, train
+    from nsvf_gb300._lib import LIB, check
+    from nsvf_gb300.functional import trilinear_embed
+    n_vox = 61
+    vs, centers, feats, values, params = _scene(cuda, n_vox, seed)
+    g = torch.Generator().manual_seed(seed)
+    vid = torch.randint(0, n_vox, (ns,), generator=g, dtype=torch.int32).to(cuda)
+    xyz = (centers[vid.long()] + (torch.rand(ns, 3, generator=g).to(cuda) - 0.5) * vs).contiguous()
+    xyzd = torch.cat([xyz, torch.ones(ns, 1, device=cuda)], 1).contiguous()
+    stream, err = ext.ctypes_stream(cuda), ext.error_word(cuda)
+    packed = train.RayBatch._packed(params, stream)
+    out = torch.empty(ns, 4, device=cuda)
+    signs = torch.zeros(4, ns, 16, dtype=torch.uint8, device=cuda)
+    scene = (n_vox, values.size(0), vs, centers.data_ptr(), feats.data_ptr(), values.data_ptr(),
+             packed.data_ptr())
+    check(LIB.nsvf_field_train_forward_signs(ns, vid.data_ptr(), xyzd.data_ptr(), *scene,
+                                             out.data_ptr(), signs.data_ptr(), err.data_ptr(),
+                                             stream), "forward")
+    n = int(LIB.nsvf_field_train_backward_floats(ns, chunk))
+    work = torch.empty(n, device=cuda)
+    gv, grads = torch.zeros_like(values), [torch.empty_like(p) for p in params]
+    check(LIB.nsvf_field_train_backward(
+        ns, chunk, vid.data_ptr(), xyzd.data_ptr(), *scene, signs.data_ptr(), dout.data_ptr(),
+        work.data_ptr(), n, gv.data_ptr(), train._ptrs(grads[0::2]), train._ptrs(grads[1::2]),
+        err.data_ptr(), stream), "backward")
+    ext.check_errors(cuda)
+    acts, pre = [trilinear_embed(vid, xyz, centers, feats, values, vs)], []
+    for l in range(4):
+        pre.append(torch.addmm(params[2 * l + 1], acts[-1], params[2 * l].t()))
+        acts.append(torch.relu(pre[-1]))
+    return (grads, gv), (acts, pre, params, (vid, xyz, centers, feats, values, vs))
+
+
+def _chain_grads(acts, pre, params, dout):
+    grads, dz = [None] * 10, dout
+    for l in range(4, -1, -1):
+        grads[2 * l], grads[2 * l + 1] = dz.t() @ acts[l], dz.sum(0)
+        da = dz @ params[2 * l]
+        if l:
+            dz = da * (pre[l - 1] > 0)
+    return grads, da
+
+
+# one sample, a tile's edges, fewer tiles than splits, several chunks; the
+# samples' gradients of one size, and over many orders of magnitude
+@pytest.mark.parametrize("ns,spread", [(1, 0.0), (127, 4.0), (128, 0.0), (129, 1.0), (5000, 12.0),
+                                       (60000, 0.0), (60000, 3.0)])
+def test_split_backward_against_float64(cuda, ns, spread):
+    """The tensor-core backward against float64 with the FP32 forward's ReLU
+    signs. Each of at most nine contractions in a row is good to about 2^-23
+    of its result's norm, the FP32 sums over tiles and slots to a few more:
+    2^-18 in all; the embeddings' float4 atomics add up to 1,000 samples."""
+    g = torch.Generator().manual_seed(ns)
+    dout = (torch.randn(ns, 4, generator=g) *
+            torch.exp(spread * torch.randn(ns, 1, generator=g))).to(cuda)
+    (grads, gv), (acts, pre, params, scene) = _field_grads(cuda, ns, dout, ns, 304 * 128)
+    vid, xyz, centers, feats, values, vs = scene
+    p64 = [p.double() for p in params]
+    q = (xyz.double() - centers[vid.long()].double()) / float(np.float32(vs)) + 0.5
+    w = [1, 1, 1, 1, 1, 1, 1, 1]
+    for k in range(8):
+        for d, bit in enumerate((4, 2, 1)):
+            w[k] = w[k] * (q[:, d] if k & bit else 1 - q[:, d])
+    keys = feats[vid.long()].long()
+    a64 = [sum(w[k][:, None] * values.double()[keys[:, k]] for k in range(8))]
+    for l in range(4):
+        a64.append((a64[-1] @ p64[2 * l].t() + p64[2 * l + 1]) * (pre[l] > 0))
+    ref, da = _chain_grads(a64, pre, p64, dout.double())
+    ref_v = torch.zeros_like(values, dtype=torch.float64)
+    for k in range(8):
+        ref_v.index_add_(0, keys[:, k], w[k][:, None] * da)
+    for a, b in zip([*grads, gv], [*ref, ref_v]):
+        assert float((a.double() - b).norm()) <= 2.0 ** -18 * float(b.norm())
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 9e37, 1e-40])
+def test_split_backward_rows_the_slices_cannot_hold(cuda, value):
+    """A gradient that is not finite, near the largest float, or denormal: the
+    same infinities and NaNs as FP32 GEMMs, and the same finite values."""
+    ns = 300
+    g = torch.Generator().manual_seed(3)
+    dout = torch.randn(ns, 4, generator=g)
+    dout[::97, 1] = value
+    dout = dout.to(cuda)
+    (grads, gv), (acts, pre, params, _) = _field_grads(cuda, ns, dout, 9, 304 * 128)
+    ref, _ = _chain_grads(acts, pre, params, dout)
+    for a, b in zip(grads, ref):
+        assert torch.equal(a.isnan(), b.isnan())
+        assert torch.equal(a.isinf(), b.isinf())
+        m = b.isfinite()
+        assert torch.equal(a[b.isinf()], b[b.isinf()])
+        if m.any():
+            assert float((a[m] - b[m]).double().norm()) <= 1e-5 * float(b[m].double().norm())
+    if value != value or abs(value) == float("inf"):
+        assert not gv.isfinite().all()
+
+
 def test_other_widths_keep_the_general_path(cuda):
     """A field that is not 4 x 128 trains through RayChunk."""
     from nsvf_gb300 import train
