@@ -14,20 +14,13 @@
 // row lie in the same voxel, so its corner rows stay in registers until the
 // voxel changes, and so do the backward's eight corner sums, whose float4
 // atomics were the bound. Measured at 1.26 M samples: see there.
-#include "common.cuh"
+#include "interp_run.cuh"
+
+using namespace nsvf_interp;
 
 namespace {
 
 constexpr int kBlock = 256;
-
-// w_k for corner k from p (q_kd in {0,1}: p*q + (1-p)*(1-q) reduces to p or
-// 1-p exactly), multiplied in dimension order like torch's prod.
-__device__ __forceinline__ float corner_w(const float p[3], int k) {
-  float a = (k & 4) ? p[0] : 1.0f - p[0];
-  float b = (k & 2) ? p[1] : 1.0f - p[1];
-  float c = (k & 1) ? p[2] : 1.0f - p[2];
-  return a * b * c;
-}
 
 // Voxel ids outside [0, n_vox) and corner ids outside [0, n_keys) are not
 // read: the sample's embedding is 0 there and bit 2 of *err is set.
@@ -136,55 +129,6 @@ __global__ void __launch_bounds__(kBlock) trilinear_bwd_kernel(
 // and 228 (203, 170), and groups that walk 32 samples with the next batch's
 // loads in flight 85 and 222. Floor 30 and 55 us: the embeddings written; read,
 // and the table updated. Blocks of 256: 84 and 148 us, of 512: 88 and 164.
-constexpr int kLanes = 8, kRun = 4, kRunBlock = 128;
-
-template <typename FeatT>
-struct Group {
-  int64_t v[kRun];          // voxel of each sample, -1 where there is none
-  int key[kRun];            // this lane's corner of it, -1 where it is out of range
-  float mine[3];            // trilinear coordinates of sample (lane & 3)
-
-  template <typename IdxT>
-  __device__ __forceinline__ void load(int64_t s0, int64_t ns, float voxel_size, int64_t n_vox,
-                                       int64_t n_keys, const IdxT *__restrict__ sidx,
-                                       const float *__restrict__ xyz,
-                                       const float *__restrict__ centers,
-                                       const FeatT *__restrict__ feats, int lane, int32_t *err) {
-    const int64_t s = s0 + (lane & (kRun - 1));
-    int64_t my = -1;
-    mine[0] = mine[1] = mine[2] = 0.0f;
-    if (s < ns) {
-      my = (int64_t)sidx[s];
-      if (my < 0 || my >= n_vox) {
-        if (err) atomicOr(err, 4);
-        my = -1;
-      } else {
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          mine[d] = (xyz[s * 3 + d] - centers[my * 3 + d]) / voxel_size + 0.5f;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kRun; ++i) {
-      v[i] = __shfl_sync(0xffffffffu, my, i, kLanes);
-      if (i > 0 && v[i] == v[i - 1]) {
-        key[i] = key[i - 1];
-        continue;
-      }
-      key[i] = -1;
-      if (v[i] < 0) continue;
-      const int64_t k = (int64_t)feats[v[i] * 8 + lane];
-      if (k >= 0 && k < n_keys) key[i] = (int)k;
-      else if (err) atomicOr(err, 4);
-    }
-  }
-  __device__ __forceinline__ bool change(int i) const { return i == 0 || v[i] != v[i - 1]; }
-  __device__ __forceinline__ void coords(int i, float (&p)[3]) const {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) p[d] = __shfl_sync(0xffffffffu, mine[d], i, kLanes);
-  }
-};
-
 template <typename IdxT, typename FeatT>
 __global__ void __launch_bounds__(kRunBlock) trilinear_fwd_run_kernel(
     int64_t ns, float voxel_size, int64_t n_vox, int64_t n_keys, const IdxT *__restrict__ sidx,
@@ -195,7 +139,7 @@ __global__ void __launch_bounds__(kRunBlock) trilinear_fwd_run_kernel(
   const int64_t s0 = t / kLanes * kRun;
   const int ch = threadIdx.x % kLanes;
   Group<FeatT> g;
-  g.load(s0, ns, voxel_size, n_vox, n_keys, sidx, xyz, centers, feats, ch, err);
+  g.template load<3>(s0, ns, voxel_size, n_vox, n_keys, sidx, xyz, centers, feats, ch, err);
   float4 x[8];
   unsigned mask = 0;
 #pragma unroll
@@ -248,7 +192,7 @@ __global__ void __launch_bounds__(kRunBlock, GV && GX ? 6 : 8) trilinear_bwd_run
   for (int i = 0; i < kRun; ++i)
     ge[i] = s0 + i < ns ? grad_emb[(s0 + i) * kLanes + ch] : make_float4(0.f, 0.f, 0.f, 0.f);
   Group<FeatT> g;
-  g.load(s0, ns, voxel_size, n_vox, n_keys, sidx, xyz, centers, feats, ch, nullptr);
+  g.template load<3>(s0, ns, voxel_size, n_vox, n_keys, sidx, xyz, centers, feats, ch, nullptr);
   float d[kRun][3];
 #pragma unroll
   for (int i = 0; i < kRun; ++i) d[i][0] = d[i][1] = d[i][2] = 0.0f;

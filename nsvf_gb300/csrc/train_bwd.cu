@@ -20,29 +20,35 @@
 // scale NaN: its results are NaN and each of them is then computed by the
 // FP32 chain.
 //
-// Measured on 1.40 M samples (an FP32-pipe version of the two kernels took 6.7
-// + 2.7 ms, at 41 and 50 TFLOP/s of the pipe's 66): 3.3 + 2.1 ms. Errors of
-// the weight gradients against float64: 2.1e-7 to 2.6e-7 of their norm, where
-// FP32 GEMMs over chunks leave 8e-7 to 1.6e-6.
+// Measured on 1.40 M samples: 4.8 ms (the interpolation 0.3, field_bwd_kernel
+// 2.5, weight_grad_kernel 1.9; versions on the FP32 pipe took 6.7 + 2.7 ms, at
+// 41 and 50 of the pipe's 66 TFLOP/s). Errors of the weight gradients against
+// float64: 2e-7 of their norm, where FP32 GEMMs over chunks leave 8e-7 to
+// 1.6e-6 (2.5e-7 and up to 2.8e-5 in training batches with far samples).
 //
-// field_bwd_kernel: a tile of 128 samples per block and one block per SM:
-// interpolation and layers again (the ReLU signs are the forward's own,
-// which are exact), then dZ_l = dA_{l+1} (z_l > 0), dA_l = dZ_l W_l, then the
-// scatter into the embeddings. TMEM lane = sample, so a row's largest element
-// is found by the four threads that hold it, and its slices go to tensor
-// memory as the next layer's A operand, which leaves shared memory for the
-// weights of two layers. The layer inputs A_l and the gradients dZ_l go to
-// memory as [unit][sample] of a tile (every store a whole line). Stores,
-// scatter and the next tile's gather run beside the MMAs. Bound: a tile's 340
-// MMAs of 64 cycles are 22k of its 83k cycles; the rest is the chain MMA ->
-// epilogue -> MMA of the one tile that fits, the stores (5.9 GB at 1.8 TB/s)
-// and the scatter's atomics.
+// field_bwd_kernel: a tile of 128 samples per block and one block per SM: the
+// layers again (the ReLU signs are the forward's own, which are exact), then
+// dZ_l = dA_{l+1} (z_l > 0), dA_l = dZ_l W_l. TMEM lane = sample, so a row's
+// largest element is found by the four threads that hold it, and its slices go
+// to tensor memory as the next layer's A operand, which leaves shared memory
+// for the weights of two layers. The layer inputs A_l and the gradients dZ_l
+// go to memory as [unit][sample] of a tile (every store a whole line), beside
+// the MMAs. Bound: the chain MMA (340 of 64 cycles) -> epilogue (1.7-2.2k) ->
+// slices (1.7-2.1k) of the one tile that fits an SM, eight times a tile, 64k
+// cycles; the stores fill the MMAs' time (64 KB a layer at 27 bytes a cycle).
+// A lane of the computing warps as the issuer: 3.3 ms, behind its warp's share
+// of the stores.
 // weight_grad_kernel: dW_l = dZ_l^T A_l, db_l = sum dZ_l: K runs over the 128
-// samples of a tile, rows are units; FP32 accumulation over tiles in
+// samples of a tile, rows are units. A sample far outside its voxel has
+// activations some thousand times the others', and often next to no gradient;
+// on a common exponent the others would lose ten bits to it. So A_l is stored
+// divided by its sample's power of two (all samples alike), and dZ_l is
+// multiplied by it before it is sliced; the products are the same. FP32 accumulation over tiles in
 // registers, one slot per block, the slots added in a fixed order. The FP32
-// rows of the next tile arrive by cp.async while a tile is sliced. Bound: MMA
-// issue and slicing by the same warps, 14k cycles a tile and layer of which
-// the MMAs are 3.1k and the 128 KB from memory 5.6k.
+// rows of the next tile arrive by cp.async while a tile is sliced. Bound: the
+// instructions and the barriers of slicing and draining, 13k cycles a tile and
+// layer, of which the MMAs run beside 3.1k and the 128 KB from memory 5.6k.
+#include "interp_run.cuh"
 #include "tc_common.cuh"
 #include "train_common.cuh"
 
@@ -63,10 +69,11 @@ constexpr int kSliceBytes = op_off(7) + 3 * kSmallOp;
 constexpr int kScales = 7 * kHid + kE;     // a power of two per row of every operand
 constexpr int kSliceFloats = kSliceBytes / 4 + kScales;
 
-// rows of 128 samples of a tile in memory: A0 (32), A1..A4, dZ0..dZ3, and dA0
-// as [sample][32]
-constexpr int kRows = 2 * kE + 8 * kHid;
-constexpr int kDA0 = kE + 8 * kHid;
+// rows of 128 samples of a tile in memory: A0 (32), A1..A4, dZ0..dZ3, dA0 as
+// [sample][32], and the scales of A0..A4. A_l is stored divided by its sample's
+// scale, the power of two above the sample's largest element (NaN and the
+// element itself where row_scale has none).
+constexpr int kDA0 = kE + 8 * kHid, kScale = kDA0 + kE, kRows = kScale + 5;
 __host__ __device__ constexpr int a_row(int l) { return l ? kE + (l - 1) * kHid : 0; }
 __host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHid; }
 
@@ -77,7 +84,10 @@ __host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHi
 constexpr int kSplit = 35, kSplit0 = 24, kSplit4 = 23;
 static_assert(3 * kSplit + kSplit0 + kSplit4 == kSMs, "one block per SM");
 
-constexpr int kBT = 512;                   // threads of the two kernels
+// threads of the two tensor-core kernels that compute; a fifth warpgroup's
+// first lane issues the MMAs. Of the 640 x 96 registers at the launch (61,440)
+// the computing warpgroups take 512 x 112 and the fifth keeps 128 x 32.
+constexpr int kBT = 512, kMmaWarp = kBT / 32, kThreads = kBT + 128;
 constexpr int kQ = kHid / 4;               // units of a thread's quarter of a row
 constexpr uint32_t kAccCols = 128;         // columns between the two accumulators
 constexpr uint32_t kACol = 256;            // field_bwd_kernel: A's slices, 64 columns each
@@ -137,32 +147,16 @@ __device__ __forceinline__ float row_scale(uint32_t e, float &inv) {
 }
 
 // Adds the products of three slices each of A (128 rows) and B, K = 16 KS, to
-// the accumulators (first: to zero); issued by one thread. Addresses are of
-// slice 0, strides in bytes. All addresses are constants beyond the operands'
-// descriptors: with a loop of computed ones a MMA took 105 cycles to issue and
-// 64 to run.
-template <int KS, int A_PLANE, int B_PLANE, int N>
-__device__ __forceinline__ void issue_split(uint32_t tmem, uint32_t a, uint32_t b, bool first) {
-  constexpr uint32_t idesc = idesc_bf16_f32(kTile, N);
-  const uint64_t ad = sdesc(a, 128u, KS * 256u), bd = sdesc(b, 128u, KS * 256u);
-#pragma unroll
-  for (int o = 2; o >= 0; --o)
-#pragma unroll
-    for (int i = 0; i <= o; ++i)
-#pragma unroll
-      for (int k = 0; k < KS; ++k)
-        mma_bf16(tmem + (o ? kAccCols : 0u), ad + (uint32_t)(i * A_PLANE / 16 + 16 * k),
-                 bd + (uint32_t)((o - i) * B_PLANE / 16 + 16 * k), idesc,
-                 i == 0 && o != 1 && k == 0 && first ? 0u : 1u);
-}
-
-// The same with A's slices in tensor memory at column `a`, KS * 8 columns
-// apart (two elements per column).
+// the accumulators (first: to zero); issued by one thread. A's slices are in
+// tensor memory at column `a`, KS * 8 columns apart (two elements per column),
+// B's in shared memory at `b`. All addresses are constants beyond these: with
+// a loop of computed descriptors a MMA took 105 cycles to issue and 64 to run.
 template <int KS, int B_PLANE, int N>
 __device__ __forceinline__ void issue_split_ts(uint32_t tmem, uint32_t a, uint32_t b,
                                                bool first) {
   constexpr uint32_t idesc = idesc_bf16_f32(kTile, N);
-  const uint64_t bd = sdesc(b, 128u, KS * 256u);
+  uint64_t bd = sdesc(b, 128u, KS * 256u);
+  asm volatile("" : "+l"(bd), "+r"(a));
 #pragma unroll
   for (int o = 2; o >= 0; --o)
 #pragma unroll
@@ -172,6 +166,26 @@ __device__ __forceinline__ void issue_split_ts(uint32_t tmem, uint32_t a, uint32
         mma_bf16_ts(tmem + (o ? kAccCols : 0u), a + (uint32_t)(i * KS * 8 + 8 * k),
                     bd + (uint32_t)((o - i) * B_PLANE / 16 + 16 * k), idesc,
                     i == 0 && o != 1 && k == 0 && first ? 0u : 1u);
+}
+
+// A barrier of the computing threads: whether `ok` holds for all of them.
+__device__ __forceinline__ bool sync_and(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)ok), "n"(kBT)
+      : "memory");
+  return r != 0;
+}
+// This warp's slices are written (every thread past its fences).
+__device__ __forceinline__ void slices_ready(uint64_t *bar) {
+  fence_before_sync();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes,
@@ -196,6 +210,8 @@ __device__ __forceinline__ float chain(const float *x, int64_t xs, const float *
   for (int k = 0; k < K; ++k) s = fmaf(x[k * xs], w[k * ws], s);
   return s;
 }
+// A stored value's scale: 1 where the value is stored as it is.
+__device__ __forceinline__ float scale_of(float s) { return s == s ? s : 1.0f; }
 
 // Slices of the weight operands, a block per row.
 __global__ void __launch_bounds__(kHid) slice_weights_kernel(const float *__restrict__ packed,
@@ -224,9 +240,8 @@ __global__ void __launch_bounds__(kHid) slice_weights_kernel(const float *__rest
   *reinterpret_cast<uint16_t *>(d + 2 * op_plane(op)) = (uint16_t)lo;
 }
 
-struct BwdParams {
+struct InterpParams {
   int64_t ns;                 // samples of this launch
-  int64_t ns_all;             // of the batch (row length of signs)
   const int32_t *vox;         // [ns]
   const float4 *xyzd;         // [ns]
   int64_t n_vox, n_keys;
@@ -234,25 +249,140 @@ struct BwdParams {
   const float *centers;       // [n_vox, 3]
   const int32_t *feats;       // [n_vox, 8]
   const float4 *values;       // [n_keys, 32]
+  float *rows;                // [tiles][kRows][128]
+  float4 *g_values;           // [n_keys, 32]
+};
+
+// Interpolation of a chunk as interp.cu's run kernel does it (groups of 8
+// lanes, 4 consecutive samples each), to [channel][sample] of a tile: a block
+// has 64 samples and turns them in shared memory. Tiles are filled up with
+// zeros. Kernels of their own, this one and the next: field_bwd_kernel's one
+// block per SM has no second one to wait for memory behind (8k + 13k of a
+// tile's 86k cycles were these two, and three warps for them alone could not
+// keep up: 123k).
+constexpr int kRunSamples = nsvf_interp::kRunBlock / nsvf_interp::kLanes * nsvf_interp::kRun;
+__global__ void __launch_bounds__(nsvf_interp::kRunBlock) interp_rows_kernel(const InterpParams p) {
+  using namespace nsvf_interp;
+  __shared__ float out[kE][kRunSamples + 1], scale[kRunSamples];
+  const int t = threadIdx.x, ch = t % kLanes, sl = t / kLanes * kRun;
+  Group<int32_t> g;
+  g.load<4>(blockIdx.x * (int64_t)kRunSamples + sl, p.ns, p.voxel_size, p.n_vox, p.n_keys, p.vox,
+            reinterpret_cast<const float *>(p.xyzd), p.centers, p.feats, ch, nullptr);
+  float4 x[8];
+  unsigned mask = 0;
+#pragma unroll
+  for (int i = 0; i < kRun; ++i) {
+    float q[3];
+    g.coords(i, q);
+    int key[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) key[k] = __shfl_sync(0xffffffffu, g.key[i], k, kLanes);
+    if (g.change(i)) {
+      mask = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (key[k] >= 0) {
+          x[k] = __ldg(p.values + (int64_t)key[k] * kLanes + ch);
+          mask |= 1u << k;
+        }
+      }
+    }
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (mask != 0xffu && !((mask >> k) & 1u)) continue;
+      const float w = corner_w(q, k);
+      e.x = fmaf(w, x[k].x, e.x); e.y = fmaf(w, x[k].y, e.y);
+      e.z = fmaf(w, x[k].z, e.z); e.w = fmaf(w, x[k].w, e.w);
+    }
+    float m = max_nan(max_nan(fabsf(e.x), fabsf(e.y)), max_nan(fabsf(e.z), fabsf(e.w))), inv;
+#pragma unroll
+    for (int o = 1; o < kLanes; o <<= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float sc = row_scale(exponent(m), inv);
+    if (sc != sc) inv = 1.0f;
+    out[ch * 4][sl + i] = e.x * inv; out[ch * 4 + 1][sl + i] = e.y * inv;
+    out[ch * 4 + 2][sl + i] = e.z * inv; out[ch * 4 + 3][sl + i] = e.w * inv;
+    if (ch == 0) scale[sl + i] = sc;
+  }
+  __syncthreads();
+  const int64_t s = blockIdx.x * (int64_t)kRunSamples;
+  float *R = p.rows + s / kTile * kRows * kTile + s % kTile;
+  if (t < kRunSamples) R[kScale * kTile + t] = scale[t];
+#pragma unroll
+  for (int i = t; i < kE * kRunSamples; i += kRunBlock)
+    R[i / kRunSamples * kTile + i % kRunSamples] = out[i / kRunSamples][i % kRunSamples];
+}
+
+// grad_values[feats[v, k]] += w_k dA0, as interp.cu's run kernel: corner sums
+// over the consecutive samples of one voxel, then float4 atomics.
+__global__ void __launch_bounds__(nsvf_interp::kRunBlock, 8) interp_grad_kernel(
+    const InterpParams p) {
+  using namespace nsvf_interp;
+  const int64_t s0 = (blockIdx.x * (int64_t)kRunBlock + threadIdx.x) / kLanes * kRun;
+  const int ch = threadIdx.x % kLanes;
+  const float4 *G = reinterpret_cast<const float4 *>(
+      p.rows + (s0 / kTile * kRows + kDA0) * kTile + s0 % kTile * kE);
+  float4 ge[kRun];
+#pragma unroll
+  for (int i = 0; i < kRun; ++i)
+    ge[i] = s0 + i < p.ns ? G[i * kLanes + ch] : make_float4(0.f, 0.f, 0.f, 0.f);
+  Group<int32_t> g;
+  g.load<4>(s0, p.ns, p.voxel_size, p.n_vox, p.n_keys, p.vox,
+            reinterpret_cast<const float *>(p.xyzd), p.centers, p.feats, ch, nullptr);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float4 sum[4];
+    int last[4] = {-1, -1, -1, -1};          // rows of the sums
+    auto flush = [&]() {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (last[k] >= 0) atomicAdd(p.g_values + (int64_t)last[k] * kLanes + ch, sum[k]);
+    };
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+      float q[3];
+      g.coords(i, q);
+      int key[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) key[k] = __shfl_sync(0xffffffffu, g.key[i], h * 4 + k, kLanes);
+      if (g.change(i)) {
+        if (i > 0) flush();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          last[k] = key[k];
+          sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float w = corner_w(q, h * 4 + k);
+        sum[k].x = fmaf(w, ge[i].x, sum[k].x); sum[k].y = fmaf(w, ge[i].y, sum[k].y);
+        sum[k].z = fmaf(w, ge[i].z, sum[k].z); sum[k].w = fmaf(w, ge[i].w, sum[k].w);
+      }
+    }
+    flush();
+  }
+}
+
+struct BwdParams {
+  int64_t ns;                 // samples of this launch
+  int64_t ns_all;             // of the batch (row length of signs)
   const float *packed;        // kPacked floats
   const uint8_t *slices;      // kSliceBytes
   const float *scales;        // kScales
   const uint4 *signs;         // [4][ns_all], from this launch's first sample
   const float4 *d_out;        // [ns]
   float *rows;                // [tiles][kRows][128]
-  float4 *g_values;           // [n_keys, 32]
   int32_t *err;
 };
 
 struct BwdSmem {
   uint8_t b[2][3 * kPlane];   // the slices of a layer's weights and of the next one's
-  uint8_t a0[3 * kSmallOp];   // of the tile's embeddings
-  float4 dout[kTile];
   float scales[kScales];
   float bias[4 * kHid];
-  float rmax[4][kTile];
-  float rs[kTile];
-  uint64_t mma_done, loaded[2];
+  uint8_t top[4][kTile];      // the largest exponent in each quarter of a row
+  uint64_t mma_done, ready, loaded[2];
   uint32_t tmem;
   int abort;
 };
@@ -305,16 +435,17 @@ __device__ __forceinline__ void load_sums8(uint32_t tmem, float (&v)[8]) {
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[0][i]) + __uint_as_float(r[1][i]);
 }
 
-__global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
+__global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   BwdSmem &S = *reinterpret_cast<BwdSmem *>(smem_raw);
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int row = (warp & 3) * 32 + lane, quarter = warp >> 2, c0 = quarter * kQ;
-  for (int i = t; i < 4 * kHid; i += kBT)
+  for (int i = t; i < 4 * kHid; i += kThreads)
     S.bias[i] = p.packed[kBiasOff + i];
-  for (int i = t; i < kScales; i += kBT) S.scales[i] = p.scales[i];
+  for (int i = t; i < kScales; i += kThreads) S.scales[i] = p.scales[i];
   if (t == 0) {
     mbar_init(&S.mma_done, 1);
+    mbar_init(&S.ready, kBT / 32);
     mbar_init(&S.loaded[0], 1);
     mbar_init(&S.loaded[1], 1);
     S.abort = 0;
@@ -329,161 +460,88 @@ __global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
   const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   volatile int *abort = &S.abort;
   const int64_t tiles = (p.ns + kTile - 1) / kTile;
-  uint32_t ph_load = 0, ph_mma = 0;          // ph_load: of the two buffers
+  uint32_t ph_mma = 0;
   bool ok = true;
-  auto load_op = [&](int op) {               // thread 0
-    bulk_load(S.b[op & 1], p.slices + op_off(op), 3u * op_plane(op), &S.loaded[op & 1]);
-  };
-  // One layer's MMAs on the slices written before the last barrier. What
-  // needs no result follows between start and finish; after finish the
-  // operand after the next is on its way.
-  auto start = [&](int op) {
-    if (t == 0 && mbar_wait(&S.loaded[op & 1], ph_load >> (op & 1) & 1u, abort)) {
-      fence_after_sync();
-      const uint32_t b = smem_u32(S.b[op & 1]);
-      if (op == 0)
-        issue_split<kE / 16, kSmallOp, kSmallOp, kHid>(tmem, smem_u32(S.a0), b, true);
-      else if (op < 7)
-        issue_split_ts<kHid / 16, kPlane, kHid>(tmem, tmem + kACol, b, true);
-      else
-        issue_split_ts<kHid / 16, kSmallOp, kE>(tmem, tmem + kACol, b, true);
-      mma_commit(&S.mma_done);
+  if (warp >= kMmaWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n");
+    // every layer: the MMAs when its slices and its weights are there, then
+    // the weights of the layer after the next
+    if (t == kBT && (int64_t)blockIdx.x < tiles) {
+      auto load_op = [&](int op) {
+        bulk_load(S.b[op & 1], p.slices + op_off(op), 3u * op_plane(op), &S.loaded[op & 1]);
+      };
+      uint32_t ph_load = 0;                  // of the two buffers
+      load_op(0);
+      load_op(1);
+      for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x)
+#pragma unroll 1
+        for (int op = 0; op < 8 && ok; ++op) {
+          ok = mbar_wait(&S.ready, ph_mma, abort) &&
+               mbar_wait(&S.loaded[op & 1], ph_load >> (op & 1) & 1u, abort);
+          if (!ok) break;
+          ph_load ^= 1u << (op & 1);
+          fence_after_sync();
+          const uint32_t b = smem_u32(S.b[op & 1]);
+          if (op == 0)
+            issue_split_ts<kE / 16, kSmallOp, kHid>(tmem, tmem + kACol, b, true);
+          else if (op < 7)
+            issue_split_ts<kHid / 16, kPlane, kHid>(tmem, tmem + kACol, b, true);
+          else
+            issue_split_ts<kHid / 16, kSmallOp, kE>(tmem, tmem + kACol, b, true);
+          mma_commit(&S.mma_done);
+          ok = mbar_wait(&S.mma_done, ph_mma, abort);
+          ph_mma ^= 1u;
+          if (ok && (op < 6 || tile + gridDim.x < tiles)) load_op((op + 2) & 7);
+        }
+      if (!ok) {
+        // a wait ran out: give what is in flight one more limit
+        if (p.err) atomicOr(p.err, 8);
+        for (int i = 0; i < 2; ++i) {
+          int never = 0;
+          mbar_wait(&S.loaded[i], ph_load >> i & 1u, &never);
+        }
+        int never = 0;
+        mbar_wait(&S.mma_done, ph_mma, &never);
+      }
     }
-    ph_load ^= 1u << (op & 1);
-  };
-  auto finish = [&](int op, bool more) {
+    __syncwarp();
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n");
+  // Waits for a layer's MMAs.
+  auto finish = [&] {
     ok = mbar_wait(&S.mma_done, ph_mma, abort) && ok;
     ph_mma ^= 1u;
     fence_after_sync();
-    if (t == 0 && ok && (op < 6 || more)) load_op((op + 2) & 7);
-  };
-  // Interpolation: 8 threads per sample, 4 channels each (interp.cu's
-  // operations), samples t / 8 + 64 it of the tile.
-  float4 e[kTile * 8 / kBT];
-  auto gather = [&](int64_t tile) {
-    constexpr int N = kTile * 8 / kBT;
-    const int ch = t & 7;
-    int64_t v[N];
-#pragma unroll
-    for (int it = 0; it < N; ++it) {
-      const int64_t s = tile * kTile + it * (kBT / 8) + (t >> 3);
-      v[it] = s < p.ns ? (int64_t)p.vox[s] : -1;
-      if (v[it] >= p.n_vox) v[it] = -1;
-    }
-#pragma unroll
-    for (int it = 0; it < N; ++it) {
-      e[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (v[it] < 0) continue;
-      const int64_t s = tile * kTile + it * (kBT / 8) + (t >> 3);
-      const float4 x = p.xyzd[s];
-      const float cx = p.centers[v[it] * 3], cy = p.centers[v[it] * 3 + 1],
-                  cz = p.centers[v[it] * 3 + 2];
-      int key[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) key[k] = p.feats[v[it] * 8 + k];
-      // (every load before the first use: one wait for the 8 rows)
-      float4 c[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        c[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (key[k] >= 0 && key[k] < p.n_keys)
-          c[k] = __ldg(p.values + (int64_t)key[k] * (kE / 4) + ch);
-      }
-      const float q[3] = {(x.x - cx) / p.voxel_size + 0.5f, (x.y - cy) / p.voxel_size + 0.5f,
-                          (x.z - cz) / p.voxel_size + 0.5f};
-      float4 a = e[it];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (key[k] < 0 || key[k] >= p.n_keys) continue;
-        const float w = corner_weight(q, k);
-        a.x = fmaf(w, c[k].x, a.x); a.y = fmaf(w, c[k].y, a.y);
-        a.z = fmaf(w, c[k].z, a.z); a.w = fmaf(w, c[k].w, a.w);
-      }
-      e[it] = a;
-    }
-  };
-  // grad_values[feats[v, k]] += w_k g, summed over a thread's consecutive
-  // samples of one voxel before the atomics: 4 samples, 4 channels and 4
-  // corners a thread
-  auto scatter = [&](int64_t tile) {
-    const int cg = lane & 7, sg = (warp & 7) * 4 + (lane >> 3), k0 = warp >> 3 << 2;
-    int64_t prev = -1;
-    float4 sum[4];
-    auto flush = [&]() {
-      if (prev < 0) return;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int64_t key = p.feats[prev * 8 + k0 + k];
-        if (key >= 0 && key < p.n_keys) atomicAdd(p.g_values + key * (kE / 4) + cg, sum[k]);
-      }
-    };
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-      const int64_t s = tile * kTile + sg * 4 + i;
-      int64_t v = s < p.ns ? (int64_t)p.vox[s] : -1;
-      if (v >= p.n_vox) v = -1;
-      if (v < 0) continue;
-      if (v != prev) {
-        flush();
-        prev = v;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) sum[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      const float4 x = p.xyzd[s];
-      const float q[3] = {(x.x - p.centers[v * 3 + 0]) / p.voxel_size + 0.5f,
-                          (x.y - p.centers[v * 3 + 1]) / p.voxel_size + 0.5f,
-                          (x.z - p.centers[v * 3 + 2]) / p.voxel_size + 0.5f};
-      const float4 gi = *reinterpret_cast<const float4 *>(
-          p.rows + (tile * kRows + kDA0) * kTile + (sg * 4 + i) * kE + cg * 4);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float w = corner_weight(q, k0 + k);
-        sum[k].x = fmaf(w, gi.x, sum[k].x); sum[k].y = fmaf(w, gi.y, sum[k].y);
-        sum[k].z = fmaf(w, gi.z, sum[k].z); sum[k].w = fmaf(w, gi.w, sum[k].w);
-      }
-    }
-    flush();
   };
   float sa = 0.0f;                           // scale of this thread's row in A
   float y[kQ];                               // its elements: units c0 + j
-  int64_t last = -1;                         // the tile whose dA0 waits in memory
-  if ((int64_t)blockIdx.x < tiles) {
-    if (t == 0) {
-      load_op(0);
-      load_op(1);
-    }
-    gather(blockIdx.x);
-  }
+  // the embeddings of this thread's sample, 8 channels, and their scale
+  float e[8], es;
+  auto load_e = [&](int64_t tile) {
+    const float *R = p.rows + tile * kRows * kTile + row;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) e[j] = R[(quarter * 8 + j) * kTile];
+    es = R[kScale * kTile];
+  };
+  if ((int64_t)blockIdx.x < tiles) load_e(blockIdx.x);
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t s0 = tile * kTile;
     float *R = p.rows + tile * kRows * kTile;
     const bool live = s0 + row < p.ns;
+    {
+      sa = es;
+      uint32_t a[3][4];
 #pragma unroll
-    for (int it = 0; it < kTile * 8 / kBT; ++it) {
-      const int sl = it * (kBT / 8) + (t >> 3), ch = t & 7;
-      const float4 a = e[it];
-      float m = max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(a.z), fabsf(a.w))), inv;
+      for (int i = 0; i < 4; ++i) slice2(e[2 * i], e[2 * i + 1], 1.0f, a[0][i], a[1][i], a[2][i]);
+      __syncwarp();
 #pragma unroll
-      for (int o = 1; o < 8; o <<= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
-      const float sc = row_scale(exponent(m), inv);
-      if (ch == 0) S.rs[sl] = sc;
-      uint32_t h0, m0, l0, h1, m1, l1;
-      slice2(a.x, a.y, inv, h0, m0, l0);
-      slice2(a.z, a.w, inv, h1, m1, l1);
-      uint8_t *d = S.a0 + kmajor_off(sl, (ch >> 1) * 8, kE) + (ch & 1) * 8;
-      *reinterpret_cast<uint2 *>(d) = make_uint2(h0, h1);
-      *reinterpret_cast<uint2 *>(d + kSmallOp) = make_uint2(m0, m1);
-      *reinterpret_cast<uint2 *>(d + 2 * kSmallOp) = make_uint2(l0, l1);
-      const float ev[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) R[(ch * 4 + j) * kTile + sl] = ev[j];
+      for (int o = 0; o < 3; ++o)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(
+                         tmem_row + kACol + o * (kE / 2) + quarter * 4),
+                     "r"(a[o][0]), "r"(a[o][1]), "r"(a[o][2]), "r"(a[o][3]));
+      tmem_wait_st();
+      slices_ready(&S.ready);
     }
-    if (t < kTile)
-      S.dout[t] = s0 + t < p.ns ? p.d_out[s0 + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-    fence_async_smem();
-    fence_before_sync();
-    __syncthreads();
-    sa = S.rs[row];
     // a layer's signs of this thread's units: unit j at bit 8 (j / 4 % 4) +
     // j % 4 of word j / 16
     auto signs = [&](int l, uint32_t (&m)[2]) {
@@ -496,19 +554,25 @@ __global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
     auto bit = [](const uint32_t (&m)[2], int j) {
       return (m[j >> 4] >> (((j >> 2) & 3) * 8 + (j & 3))) & 1u;
     };
-    auto store = [&](int first_row) {
+    auto store = [&](int first_row, float by) {
       float *out = R + (first_row + c0) * kTile + row;
 #pragma unroll
-      for (int j = 0; j < kQ; ++j) out[j * kTile] = y[j];
+      for (int j = 0; j < kQ; ++j) out[j * kTile] = y[j] * by;
     };
+    // A_l divided by its scale, and the scale
+    auto store_a = [&](int l, float inv) {
+      store(a_row(l), sa == sa ? inv : 1.0f);
+      if (quarter == 0) R[(kScale + l) * kTile + row] = sa;
+    };
+    float inv = 0.0f;                        // 1 / sa
     // Ends a layer: joins the row's quarters and, where `slice`, puts its
     // slices in A. top: the largest |y|, NaN where fix(j) has to give y[j]
     // again (it reads rows of memory written before the barrier). False:
     // unwind.
     auto rows_done = [&](float top, bool slice, auto fix) {
-      S.rmax[quarter][row] = top;
-      if (!__syncthreads_and(ok && top == top)) {
-        if (!__syncthreads_and(ok)) return false;
+      S.top[quarter][row] = (uint8_t)exponent(top);
+      if (!sync_and(ok && top == top)) {
+        if (!sync_and(ok)) return false;
         if (top != top) {
           top = 0.0f;
 #pragma unroll
@@ -516,28 +580,23 @@ __global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
             if (y[j] != y[j]) y[j] = fix(j);
             top = max_nan(top, fabsf(y[j]));
           }
-          S.rmax[quarter][row] = top;
+          S.top[quarter][row] = (uint8_t)exponent(top);
         }
-        __syncthreads();
+        sync_and(true);
       }
-      if (!slice) return true;
-      float inv;
-      sa = row_scale(exponent(max_nan(max_nan(S.rmax[0][row], S.rmax[1][row]),
-                                      max_nan(S.rmax[2][row], S.rmax[3][row]))),
+      sa = row_scale(max(max(S.top[0][row], S.top[1][row]), max(S.top[2][row], S.top[3][row])),
                      inv);
+      if (!slice) return true;
       slice_row(tmem_row + kACol + c0 / 2, y, inv);
-      fence_before_sync();
-      __syncthreads();
+      slices_ready(&S.ready);
       return true;
     };
 #pragma unroll 1
     for (int l = 0; l < 4; ++l) {
       uint32_t m[2];
       signs(l, m);
-      start(l);
-      if (l) store(a_row(l));
-      if (l == 1 && last >= 0) scatter(last);
-      finish(l, true);
+      if (l) store_a(l, inv);
+      finish();
       const float *sc = S.scales + l * kHid + c0, *bias = S.bias + l * kHid + c0;
       float top = 0.0f;
 #pragma unroll
@@ -553,17 +612,17 @@ __global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
         }
       }
       if (!rows_done(top, l < 3, [&](int j) {
-            const float z = chain(R + a_row(l) * kTile + row, kTile, p.packed + w_off(l) + c0 + j,
-                                  kHid, l ? kHid : kE) +
-                            bias[j];
+            const float z = fmaf(chain(R + a_row(l) * kTile + row, kTile,
+                                       p.packed + w_off(l) + c0 + j, kHid, l ? kHid : kE),
+                                 scale_of(R[(kScale + l) * kTile + row]), bias[j]);
             return bit(m, j) || z != z ? z : 0.0f;
           }))
         goto out;
     }
-    store(a_row(4));
+    store_a(4, inv);
     // dA4 = d_out W4
     {
-      const float4 d = S.dout[row];
+      const float4 d = live ? p.d_out[s0 + row] : make_float4(0.f, 0.f, 0.f, 0.f);
       const float4 *w4 = reinterpret_cast<const float4 *>(p.packed + kW4Off + c0);
 #pragma unroll
       for (int j = 0; j < kQ; j += 4) {
@@ -593,10 +652,9 @@ __global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
           }))
         goto out;
       const int op = 7 - l;
-      start(op);
-      store(dz_row(l));
-      if (l == 1 && tile + gridDim.x < tiles) gather(tile + gridDim.x);
-      finish(op, tile + gridDim.x < tiles);
+      store(dz_row(l), 1.0f);
+      if (l == 1 && tile + gridDim.x < tiles) load_e(tile + gridDim.x);
+      finish();
       if (l == 0) break;
       const float *sc = S.scales + op * kHid + c0;
 #pragma unroll
@@ -620,30 +678,18 @@ __global__ void __launch_bounds__(kBT, 1) field_bwd_kernel(const BwdParams p) {
 #pragma unroll
       for (int i = 0; i < 8; i += 4)
         *reinterpret_cast<float4 *>(g + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-      fence_before_sync();
-      if (!__syncthreads_and(ok && nan == nan)) {
-        if (!__syncthreads_and(ok)) goto out;
+      if (!sync_and(ok && nan == nan)) {
+        if (!sync_and(ok)) goto out;
 #pragma unroll 1
         for (int i = 0; i < 8 && nan != nan; ++i)
           if (g[i] != g[i])
             g[i] = chain(R + dz_row(0) * kTile + row, kTile,
                          p.packed + w_off(0) + (quarter * 8 + i) * kHid, 1, kHid);
-        __syncthreads();
+        sync_and(true);
       }
     }
-    last = tile;
   }
-  if (last >= 0) scatter(last);
-out:
-  if (t == 0 && S.abort) {
-    // a wait ran out: give the copy and the MMAs in flight one more limit
-    int never = 0;
-    if (p.err) atomicOr(p.err, 8);
-    for (int i = 0; i < 2; ++i) {
-      mbar_wait(&S.loaded[i], ph_load >> i & 1u, &never);
-      never = 0;
-    }
-    mbar_wait(&S.mma_done, ph_mma, &never);
+out:;
   }
   fence_before_sync();
   __syncthreads();
@@ -656,10 +702,11 @@ out:
 constexpr int kHalfPlane = kHid * 64 * 2;
 struct GradSmem {
   float in[2][kHid * kTile];  // X, Y: rows of 32 16-byte chunks, chunk c at c ^ (row & 7)
+  float scale[kTile];         // of A's samples
   uint8_t y[2][3 * kHalfPlane];
   uint8_t top[2][4][kHid];    // X, Y: the largest exponent in each quarter of a row
   float ys[2][kHid];          // Y's scales, by parity of the tile
-  uint64_t done;
+  uint64_t done, ready[2];    // ready: of a half's slices
   uint32_t tmem;
   int abort;
 };
@@ -677,7 +724,7 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, int size, b
 // dW = X^T Y of one layer over some of the chunk's tiles, X = dZ (A4 for the
 // head), Y = A (d_out). A thread slices 32 samples (a quarter of each half of
 // the tile) of row t % 128 of both.
-__global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
+__global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
                                                              const float *__restrict__ rows,
                                                              const float *__restrict__ d_out,
                                                              float *__restrict__ part,
@@ -698,11 +745,13 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
   const int c0 = ny == kHid ? quarter * 32 : quarter * 8;
   if (t == 0) {
     mbar_init(&S.done, 1);
+    mbar_init(&S.ready[0], kBT / 32);
+    mbar_init(&S.ready[1], kBT / 32);
     S.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (l == 4)                                // rows 4..15 stay zero
-    for (int i = t; i < (int)sizeof(S.y) / 16; i += kBT)
+    for (int i = t; i < (int)sizeof(S.y) / 16; i += kThreads)
       reinterpret_cast<uint4 *>(S.y)[i] = make_uint4(0, 0, 0, 0);
   constexpr uint32_t kCols = 512;
   if (warp == 0) tmem_alloc(&S.tmem, kCols);
@@ -712,16 +761,45 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
   fence_after_sync();
   const uint32_t tmem = S.tmem;
   const uint32_t tmem_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  constexpr uint32_t kXCol = 2 * kAccCols, kXHalf = 3 * 32;  // slices of a half: 32 columns each
   volatile int *abort = &S.abort;
   const int64_t tiles = (ns + kTile - 1) / kTile;
+  constexpr uint32_t kXCol = 2 * kAccCols, kXHalf = 3 * 32;  // slices of a half: 32 columns each
+  bool ok = true;
+  if (warp >= kMmaWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n");
+    if (t == kBT) {
+      int64_t n = 0;
+      for (int64_t tile = j; tile < tiles && ok; tile += splits, ++n)
+#pragma unroll 1
+        for (int h = 0; h < 2 && ok; ++h) {
+          ok = mbar_wait(&S.ready[h], (uint32_t)n & 1u, abort);
+          if (!ok) break;
+          fence_after_sync();
+          const uint32_t x = tmem + kXCol + h * kXHalf, y = smem_u32(S.y[h]);
+          if (ny == kHid)
+            issue_split_ts<4, kHalfPlane, kHid>(tmem, x, y, h == 0);
+          else if (ny == kE)
+            issue_split_ts<4, kHalfPlane, kE>(tmem, x, y, h == 0);
+          else
+            issue_split_ts<4, kHalfPlane, 16>(tmem, x, y, h == 0);
+          if (h == 1) mma_commit(&S.done);
+        }
+      if (!ok) {
+        // a wait ran out: give the MMAs in flight one more limit
+        int never = 0;
+        if (err) atomicOr(err, 8);
+        mbar_wait(&S.done, n > 0 ? (uint32_t)(n - 1) & 1u : 0u, &never);
+      }
+    }
+    __syncwarp();
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n");
   float acc[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
   float sum = 0.0f, comp = 0.0f;             // of the thread's samples of its row (db), Kahan
   float v[2][32];                            // X, Y: samples h * 64 + quarter * 16 + 0..15
   float inv[2], xs = 0.0f, xs_prev = 0.0f;
-  bool ok = true;
   // copies of a tile's rows to S.in
   auto fetch = [&](int64_t tile) {
     const float *R = rows + tile * kRows * kTile;
@@ -743,27 +821,40 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
         }
       }
     }
+    if (t < kTile / 4)
+      cp_async(S.scale + t * 4, R + (kScale + l) * kTile + t * 4, 16, true);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   // the fetched tile to registers, its scales; the next one on its way
   auto take = [&](int64_t next, int buf) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
+    sync_and(true);
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
       if (g && row >= yrows) continue;
       const float *in = S.in[g] + row * kTile;
-      float m = 0.0f;
+      float m = 0.0f, s = 0.0f;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const int at = (c >> 2) * 16 + quarter * 4 + (c & 3);
-        const float4 a = *reinterpret_cast<const float4 *>(in + ((at ^ (row & 7)) << 2));
+        float4 a = *reinterpret_cast<const float4 *>(in + ((at ^ (row & 7)) << 2));
+        if (g == (l == 4)) {
+          // dZ (d_out): its sum for db, and times the scale of A's sample
+          s += (a.x + a.y) + (a.z + a.w);
+          const float4 by = *reinterpret_cast<const float4 *>(S.scale + at * 4);
+          a.x *= by.x; a.y *= by.y; a.z *= by.z; a.w *= by.w;
+        }
         v[g][c * 4] = a.x; v[g][c * 4 + 1] = a.y; v[g][c * 4 + 2] = a.z; v[g][c * 4 + 3] = a.w;
         m = max_nan(m, max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(a.z), fabsf(a.w))));
       }
+      if (g == (l == 4)) {
+        const float a = s - comp, w = sum + a;
+        comp = fabsf(w) <= 3.4e38f ? (w - sum) - a : 0.0f;
+        sum = w;
+      }
       S.top[g][quarter][row] = (uint8_t)exponent(m);
     }
-    ok = __syncthreads_and(ok);
+    ok = sync_and(ok);
     if (next < tiles) fetch(next);
     xs_prev = xs;
 #pragma unroll
@@ -774,18 +865,6 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
                                  inv[g]);
       if (!g) xs = sc;
       else if (quarter == 0) S.ys[buf][row] = sc;
-    }
-    if (l != 4 || row < 4) {
-      float s[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) s[i] = l == 4 ? v[1][i] : v[0][i];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int i = 0; i < o; ++i) s[i] += s[i + o];
-      const float a = s[0] - comp, w = sum + a;
-      comp = fabsf(w) <= 3.4e38f ? (w - sum) - a : 0.0f;
-      sum = w;
     }
   };
   // adds the finished result of `tile` (X's scale x) to acc
@@ -809,8 +888,16 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int n = c0 + c * 8 + i;
-          if (d[i] != d[i] && n < yrows)
-            d[i] = l == 4 ? chain(X, 1, Y + n, 4, K) : chain(X, 1, Y + n * kTile, 1, K);
+          if (d[i] != d[i] && n < yrows) {
+            const float *y = l == 4 ? Y + n : Y + n * kTile, *by = rows + (tile * kRows + kScale + l) * kTile;
+            const int ys = l == 4 ? 4 : 1;
+            float s = 0.0f;
+#pragma unroll 1
+            for (int k = 0; k < K; ++k)
+              s = l == 4 ? fmaf(X[k] * scale_of(by[k]), y[k * ys], s)
+                         : fmaf(X[k], y[k * ys] * scale_of(by[k]), s);
+            d[i] = s;
+          }
         }
       }
 #pragma unroll
@@ -850,33 +937,14 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
       for (int o = 0; o < 3; ++o) tmem_st8(tmem_row + kXCol + h * kXHalf + o * 32 + quarter * 8, a[o]);
       tmem_wait_st();
       fence_async_smem();
-      fence_before_sync();
-      ok = __syncthreads_and(ok);
-      if (t == 0 && ok) {
-        fence_after_sync();
-        const uint32_t x = tmem + kXCol + h * kXHalf, y = smem_u32(S.y[h]);
-        if (ny == kHid)
-          issue_split_ts<4, kHalfPlane, kHid>(tmem, x, y, h == 0);
-        else if (ny == kE)
-          issue_split_ts<4, kHalfPlane, kE>(tmem, x, y, h == 0);
-        else
-          issue_split_ts<4, kHalfPlane, 16>(tmem, x, y, h == 0);
-        if (h == 1) mma_commit(&S.done);
-      }
+      slices_ready(&S.ready[h]);
     }
-    if (!ok) break;
   }
   if (n > 0 && ok) {
     ok = mbar_wait(&S.done, (uint32_t)(n - 1) & 1u, abort);
-    if (__syncthreads_and(ok)) drain(j + (n - 1) * splits, (int)(n - 1) & 1, xs);
+    if (sync_and(ok)) drain(j + (n - 1) * splits, (int)(n - 1) & 1, xs);
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  if (S.abort && t == 0) {
-    // a wait ran out: give the MMAs in flight one more limit
-    int never = 0;
-    if (err) atomicOr(err, 8);
-    mbar_wait(&S.done, n > 0 ? (uint32_t)(n - 1) & 1u : 0u, &never);
-  }
   // slots: layers 1..3 [128][128], layer 0 [128][32], head [128][4]
   float *P = part + (l == 0   ? (int64_t)3 * kSplit * kHid * kHid + (int64_t)j * kHid * kE
                      : l == 4 ? (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE +
@@ -894,18 +962,19 @@ __global__ void __launch_bounds__(kBT, 1) weight_grad_kernel(int64_t ns,
     }
     *d = o;
   }
-  __syncthreads();
+  sync_and(true);
   float *const sums = S.in[0];
   sums[quarter * kHid + row] = sum;
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
+  sync_and(true);
   if (t < kHid) {
-    const float s =
-        (sums[t] + sums[kHid + t]) + (sums[2 * kHid + t] + sums[3 * kHid + t]);
+    const float s = (sums[t] + sums[kHid + t]) + (sums[2 * kHid + t] + sums[3 * kHid + t]);
     float *d = bias_part + (int64_t)b * kHid + t;
     *d = add ? *d + s : s;
   }
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
   if (warp == 0) tmem_dealloc(tmem, kCols);
 }
 
@@ -1020,31 +1089,39 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
   }
   BwdParams p = {};
   p.ns_all = n_samples;
-  p.n_vox = n_voxels;
-  p.n_keys = n_keys;
-  p.voxel_size = voxel_size;
-  p.centers = centers;
-  p.feats = feats;
-  p.values = (const float4 *)values;
   p.packed = packed;
   p.slices = slices;
   p.scales = scales;
   p.rows = rows;
-  p.g_values = (float4 *)grad_values;
   p.err = err;
+  InterpParams q = {};
+  q.n_vox = n_voxels;
+  q.n_keys = n_keys;
+  q.voxel_size = voxel_size;
+  q.centers = centers;
+  q.feats = feats;
+  q.values = (const float4 *)values;
+  q.rows = rows;
+  q.g_values = (float4 *)grad_values;
   // (one pass without samples zeroes the slots of an empty batch)
   for (int64_t a = 0; a == 0 || a < n_samples; a += chunk_samples) {
     p.ns = n_samples - a < chunk_samples ? n_samples - a : chunk_samples;
-    p.vox = voxel + a;
-    p.xyzd = (const float4 *)xyz_dist + a;
+    q.ns = p.ns;
+    q.vox = voxel + a;
+    q.xyzd = (const float4 *)xyz_dist + a;
     p.signs = (const uint4 *)signs + a;
     p.d_out = (const float4 *)grad_out + a;
     if (p.ns > 0) {
       const int64_t tiles = (p.ns + kTile - 1) / kTile;
-      field_bwd_kernel<<<(int)(tiles < kSMs ? tiles : kSMs), kBT, sizeof(BwdSmem), s>>>(p);
+      interp_rows_kernel<<<nsvf_grid(tiles * kTile, kRunSamples), nsvf_interp::kRunBlock, 0, s>>>(
+          q);
+      if ((st = nsvf_launch_status()) != NSVF_OK) return st;
+      field_bwd_kernel<<<(int)(tiles < kSMs ? tiles : kSMs), kThreads, sizeof(BwdSmem), s>>>(p);
+      if ((st = nsvf_launch_status()) != NSVF_OK) return st;
+      interp_grad_kernel<<<nsvf_grid(p.ns, kRunSamples), nsvf_interp::kRunBlock, 0, s>>>(q);
       if ((st = nsvf_launch_status()) != NSVF_OK) return st;
     }
-    weight_grad_kernel<<<kSMs, kBT, sizeof(GradSmem), s>>>(p.ns, rows, (const float *)p.d_out, part,
+    weight_grad_kernel<<<kSMs, kThreads, sizeof(GradSmem), s>>>(p.ns, rows, (const float *)p.d_out, part,
                                                           bias_part, a > 0, err);
     if ((st = nsvf_launch_status()) != NSVF_OK) return st;
   }

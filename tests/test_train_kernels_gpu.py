@@ -126,7 +126,7 @@ def test_forward_bits_of_a_gemm_chain(cuda, ns):
     assert torch.equal(out, x)
 
 
-def _field_grads(cuda, ns, dout, seed, chunk):
+def _field_grads(cuda, ns, dout, seed, chunk, far=None):
     """The field's forward with signs and its backward on random samples, and
     the FP32 layers of the same samples: (grads, grad_values), (acts, pre,
     params, scene)."""
@@ -138,6 +138,8 @@ def _field_grads(cuda, ns, dout, seed, chunk):
     g = torch.Generator().manual_seed(seed)
     vid = torch.randint(0, n_vox, (ns,), generator=g, dtype=torch.int32).to(cuda)
     xyz = (centers[vid.long()] + (torch.rand(ns, 3, generator=g).to(cuda) - 0.5) * vs).contiguous()
+    if far is not None:
+        xyz[far] += 40 * vs
     xyzd = torch.cat([xyz, torch.ones(ns, 1, device=cuda)], 1).contiguous()
     stream, err = ext.ctypes_stream(cuda), ext.error_word(cuda)
     packed = train.RayBatch._packed(params, stream)
@@ -174,10 +176,14 @@ def _chain_grads(acts, pre, params, dout):
 
 
 # one sample, a tile's edges, fewer tiles than splits, several chunks; the
-# samples' gradients of one size, and over many orders of magnitude
-@pytest.mark.parametrize("ns,spread", [(1, 0.0), (127, 4.0), (128, 0.0), (129, 1.0), (5000, 12.0),
-                                       (60000, 0.0), (60000, 3.0)])
-def test_split_backward_against_float64(cuda, ns, spread):
+# samples' gradients of one size, and over many orders of magnitude; samples far
+# outside their voxel, whose activations are some thousand times the others',
+# without a gradient of their own
+@pytest.mark.parametrize("ns,spread,far", [(1, 0.0, None), (127, 4.0, None), (128, 0.0, None),
+                                           (129, 1.0, None), (5000, 12.0, None),
+                                           (60000, 0.0, None), (60000, 3.0, None),
+                                           (128, 0.0, 17), (5000, 0.0, 100)])
+def test_split_backward_against_float64(cuda, ns, spread, far):
     """The tensor-core backward against float64 with the FP32 forward's ReLU
     signs. Each of at most nine contractions in a row is good to about 2^-23
     of its result's norm, the FP32 sums over tiles and slots to a few more:
@@ -185,7 +191,10 @@ def test_split_backward_against_float64(cuda, ns, spread):
     g = torch.Generator().manual_seed(ns)
     dout = (torch.randn(ns, 4, generator=g) *
             torch.exp(spread * torch.randn(ns, 1, generator=g))).to(cuda)
-    (grads, gv), (acts, pre, params, scene) = _field_grads(cuda, ns, dout, ns, 304 * 128)
+    far = slice(far, None, far) if far else None
+    if far:
+        dout[far] = 0
+    (grads, gv), (acts, pre, params, scene) = _field_grads(cuda, ns, dout, ns, 304 * 128, far)
     vid, xyz, centers, feats, values, vs = scene
     p64 = [p.double() for p in params]
     q = (xyz.double() - centers[vid.long()].double()) / float(np.float32(vs)) + 0.5
