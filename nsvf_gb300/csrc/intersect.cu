@@ -394,16 +394,15 @@ constexpr int kRaysPerBlock = kRayBlock / kLanesPerRay;  // 32
 // A warp walks 8 rays; the 4 lanes of a ray's group each own two child
 // slots (lane j: children j and j + 4). Expanding a node = each lane loads
 // its two children's ids and boxes and runs their slab tests; ballots give
-// the node's 8-bit masks of hit children and hit leaves. The descent stack
-// is spread over the group: lane j keeps, for levels j, j + 4, j + 8 and
-// j + 12 (one byte each), the mask of hit children not visited yet (and
-// which of them are leaves); the child ids of each level sit in shared
-// memory. The next node to expand -- the highest unvisited child of the
-// deepest non-empty level -- comes from the group's mask of non-empty levels
-// (each lane's stack bytes as bits, OR-ed over the group by two xor
-// shuffles) and one shuffle from the level's owner lane, the same on all 4
-// lanes. The per-ray bookkeeping (ballots, stack, pick) is shared by twice
-// as many rays per warp instruction as with one child per lane.
+// the node's 8-bit mask of hit children and whether one of them is no leaf. The
+// descent stack is 16 such masks (children not visited yet, one byte per
+// level) in two registers, the same on the group's 4 lanes; the child ids of
+// each level, the sign bit marking leaves, sit in shared memory. The next node
+// to expand -- the highest unvisited child of the deepest non-empty level -- is
+// the stack's highest bit. Bound: instruction issue (70 % of the slots), 1.3 M
+// warp steps of 8 rays for a frame's 640,000 rays. With the stack's bytes
+// spread over the 4 lanes, four shuffles a pick and a second mask for the
+// leaves the kernel took 555 us, so 513.
 // When every hit child of a node is a leaf -- always the case for trees made
 // by build_octree, whose leaves all sit under depth-0 nodes -- the DFS visits
 // them consecutively, so the group emits them at once, the lane of child c
@@ -597,7 +596,6 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
   const uint32_t full = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane / kLanesPerRay, j = lane % kLanesPerRay;  // ray slot, child slots j + P c
-  const int g0 = lane - j;                           // the group's first lane
   const uint32_t gshift = (uint32_t)(kLanesPerRay * grp);
   const int slot = warp * kRaysPerWarp + grp;        // ray slot in the block
   // Ray-list mode (ray_list != NULL): slot q of the launch takes ray
@@ -654,18 +652,20 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
       level = 0;
     }
   }
-  // lane j's share of the stack: byte k holds level j + P k (P lanes per ray)
-  constexpr int P = kLanesPerRay, NC = 8 / P, NLV = kSvoLevels / P;
+  constexpr int P = kLanesPerRay, NC = 8 / P;
   constexpr uint32_t PM = (1u << P) - 1u;
-  using Stack = typename std::conditional<(NLV * 8 > 32), uint64_t, uint32_t>::type;
-  Stack stk = 0, stl = 0;               // unvisited hit children; those that are leaves
+  // the stack, the same on the group's lanes: the unvisited hit children, child
+  // c of level l at bit 8 l + c, so the highest bit is the next one to visit
+  static_assert(kSvoLevels == 16, "sixteen one-byte levels");
+  uint64_t stk0 = 0, stk1 = 0;           // levels 0..7, 8..15
   int node = n - 1;                      // the node to expand next (valid when `expand`)
   bool expand = level == 0;
-  int64_t steps = 0;
+  const uint32_t limit = n < (1 << 28) ? 8u * (uint32_t)n : 0x7fffffffu;
+  uint32_t steps = 0;
   // Every group runs the loop until all groups of the warp are done. All
   // warp-wide operations run on all 32 lanes every iteration; only
-  // lane-local work is predicated on `expand` / `pick`. Every value the
-  // group steers by (level, cnt, node, top, t, u) is the same on its lanes.
+  // lane-local work is predicated on `expand`. Every value the group steers by
+  // (level, cnt, node, the stack) is the same on its lanes.
   while (__any_sync(full, expand)) {
     // 1. expand `node`: lane j tests children j + P c
     bool hit[NC];
@@ -725,16 +725,17 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
         }
       }
     }
-    uint32_t hm = 0, lm = 0;
+    uint32_t hm = 0;
+    bool inner = false;                   // a hit child of this lane is no leaf
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       hm |= ((__ballot_sync(full, hit[c]) >> gshift) & PM) << (P * c);
-      lm |= ((__ballot_sync(full, hit[c] && cbw[c] < 0.0f) >> gshift) & PM) << (P * c);
+      inner = inner || (hit[c] && !(cbw[c] < 0.0f));
     }
-    if (expand && ++steps > 8 * (int64_t)n) { bad = true; expand = false; }
-    int top = level - 1;                  // deepest stack level that may hold children
+    inner = ((__ballot_sync(full, inner) >> gshift) & PM) != 0;
+    if (expand && ++steps > limit) { bad = true; expand = false; }
     if (expand) {
-      if (hm != 0 && hm == lm) {
+      if (hm != 0 && !inner) {
         // all hit children are leaves: emit them now, highest index first
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
@@ -747,88 +748,53 @@ __global__ void __launch_bounds__(kRayBlock) svo_kernel(
       } else if (hm != 0) {
         const int base = level * kRaysPerBlock + slot;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) s_child[base * 8 + j + P * c] = cid[c];
+        for (int c = 0; c < NC; ++c)
+          s_child[base * 8 + j + P * c] = cid[c] | (cbw[c] < 0.0f ? INT32_MIN : 0);
         if (j == 0) s_node[base] = node;
-        if (j == level % P) {
-          const int sh = (level / P) * 8;
-          stk = (stk & ~((Stack)0xffu << sh)) | ((Stack)hm << sh);
-          stl = (stl & ~((Stack)0xffu << sh)) | ((Stack)lm << sh);
-        }
-        top = level;
+        const uint64_t push = (uint64_t)hm << ((level & 7) * 8);
+        if (level < 8) stk0 |= push;
+        else stk1 |= push;
       }
     }
     __syncwarp();                         // s_child / s_node writes -> the group's reads
     // 2. the next node to expand: the highest unvisited child of the deepest
-    // non-empty level <= top. A leaf found there is emitted and the pick
-    // repeats.
-    bool pick = expand && cnt < n_max;
+    // non-empty level. A leaf found there is emitted and the pick repeats.
     int next = -1;
-    while (__any_sync(full, pick)) {
-      // bit l of L: level l (<= top) still has unvisited children. Level
-      // P k + j is byte k of lane j: each lane sets bits j + P k for its
-      // non-empty bytes, and two xor shuffles OR them over the group.
-      static_assert(P == 4 && NLV == 4, "four one-byte levels per lane");
-      uint32_t own = 0;
-      if (pick && top >= 0) {
-        const uint32_t s32 = (uint32_t)stk;
-        // the high bit of every non-zero byte
-        const uint32_t nzb = (((s32 & 0x7f7f7f7fu) + 0x7f7f7f7fu) | s32) & 0x80808080u;
-        // bytes 0..3 (bits 7, 15, 23, 31) to bits 0, 4, 8, 12
-        const uint32_t sp = ((nzb >> 7) & 0x1u) | ((nzb >> 11) & 0x10u) | ((nzb >> 15) & 0x100u) |
-                            ((nzb >> 19) & 0x1000u);
-        own = (sp << j) & ((2u << top) - 1u);  // levels 0..top (top <= 15)
-      }
-      uint32_t L = own;
-      L |= __shfl_xor_sync(full, L, 1);
-      L |= __shfl_xor_sync(full, L, 2);
-      const int t = (pick && L != 0) ? 31 - __clz(L) : -1;
-      uint32_t mine = 0, isleaf = 0;
-      int u = 0;
-      if (t >= 0 && j == t % P) {
-        const int sh = (t / P) * 8;
-        mine = (uint32_t)(stk >> sh) & 0xffu;
-        u = 31 - __clz(mine);
-        isleaf = (uint32_t)(stl >> (sh + u)) & 1u;
-        stk &= ~((Stack)1u << (sh + u));
-      }
-      const int src = g0 + (t >= 0 ? t % P : 0);
-      u = __shfl_sync(full, u, src);
-      isleaf = __shfl_sync(full, isleaf, src);
-      if (pick) {
-        if (t < 0) {
-          pick = false;                   // the stack is empty: the ray is done
+    while (expand && cnt < n_max && (stk0 | stk1) != 0) {
+      const bool up = stk1 != 0;
+      const uint64_t w = up ? stk1 : stk0;
+      const int bit = 63 - __clzll((long long)w);
+      const uint64_t rest = w & ~(1ull << bit);
+      if (up) stk1 = rest;
+      else stk0 = rest;
+      const int t = (bit >> 3) + (up ? 8 : 0), u = bit & 7;
+      const int base = t * kRaysPerBlock + slot;
+      const int ch = s_child[base * 8 + u];
+      if (ch >= 0) {
+        if (t + 1 >= kSvoLevels) {
+          bad = true;
         } else {
-          const int base = t * kRaysPerBlock + slot;
-          const int ch = s_child[base * 8 + u];
-          top = t;
-          if (isleaf) {
-            if (j == 0) {
-              float a, b2;
-              if (TIGHT) {
-                const float *cb = reinterpret_cast<const float *>(
-                                      CB + (int64_t)s_node[base] * 12 + 3 * (u & 3)) + (u >> 2);
-                const float f[6] = {cb[0], cb[4], cb[8], cb[2], cb[6], cb[10]};
-                slab_faces(ox, oy, oz, ix, iy, iz, f, a, b2);
-              } else {
-                const float *cb =
-                    reinterpret_cast<const float *>(CB + (int64_t)s_node[base] * 8 + 2 * (u & 3)) +
-                    (u >> 2);
-                slab(cb[0], cb[2], cb[4], -cb[6], a, b2);
-              }
-              I[cnt] = ch; LO[cnt] = a; HI[cnt] = b2;
-            }
-            ++cnt;
-            if (cnt >= n_max) pick = false;
-          } else if (t + 1 >= kSvoLevels) {
-            bad = true;
-            pick = false;
-          } else {
-            next = ch;
-            level = t + 1;
-            pick = false;
-          }
+          next = ch;
+          level = t + 1;
         }
+        break;
       }
+      if (j == 0) {
+        float a, b2;
+        if (TIGHT) {
+          const float *cb = reinterpret_cast<const float *>(CB + (int64_t)s_node[base] * 12 +
+                                                            3 * (u & 3)) + (u >> 2);
+          const float f[6] = {cb[0], cb[4], cb[8], cb[2], cb[6], cb[10]};
+          slab_faces(ox, oy, oz, ix, iy, iz, f, a, b2);
+        } else {
+          const float *cb =
+              reinterpret_cast<const float *>(CB + (int64_t)s_node[base] * 8 + 2 * (u & 3)) +
+              (u >> 2);
+          slab(cb[0], cb[2], cb[4], -cb[6], a, b2);
+        }
+        I[cnt] = ch & INT32_MAX; LO[cnt] = a; HI[cnt] = b2;
+      }
+      ++cnt;
     }
     if (expand) {
       if (next >= 0) node = next;
