@@ -20,11 +20,14 @@
 // scale NaN: its results are NaN and each of them is then computed by the
 // FP32 chain.
 //
-// Measured on 1.40 M samples: 4.8 ms (the interpolation 0.3, field_bwd_kernel
-// 2.5, weight_grad_kernel 1.9; versions on the FP32 pipe took 6.7 + 2.7 ms, at
-// 41 and 50 of the pipe's 66 TFLOP/s). Errors of the weight gradients against
-// float64: 2e-7 of their norm, where FP32 GEMMs over chunks leave 8e-7 to
-// 1.6e-6 (2.5e-7 and up to 2.8e-5 in training batches with far samples).
+// Errors of these sums against float64: 2e-7 of the gradient's norm, where
+// FP32 GEMMs over chunks leave 8e-7 to 1.6e-6, and up to 3.4e-5 in batches with
+// far samples; there layers 2 and 3, where that is more than 1e-5, are summed
+// as the GEMMs sum them (weight_chain_kernel).
+//
+// Measured on 1.40 M samples: 5.7 ms (the interpolation 0.3, field_bwd_kernel 2.5,
+// weight_chain_kernel 1.8, weight_grad_kernel 1.1; all on the FP32 pipe took
+// 6.7 + 2.7 ms, at 41 and 50 of the pipe's 66 TFLOP/s).
 //
 // field_bwd_kernel: a tile of 128 samples per block and one block per SM: the
 // layers again (the ReLU signs are the forward's own, which are exact), then
@@ -38,7 +41,8 @@
 // cycles; the stores fill the MMAs' time (64 KB a layer at 27 bytes a cycle).
 // A lane of the computing warps as the issuer: 3.3 ms, behind its warp's share
 // of the stores.
-// weight_grad_kernel: dW_l = dZ_l^T A_l, db_l = sum dZ_l: K runs over the 128
+// weight_grad_kernel (layers 0, 1 and the head): dW_l = dZ_l^T A_l, db_l = sum
+// dZ_l: K runs over the 128
 // samples of a tile, rows are units. A sample far outside its voxel has
 // activations some thousand times the others', and often next to no gradient;
 // on a common exponent the others would lose ten bits to it. So A_l is stored
@@ -77,12 +81,16 @@ constexpr int kDA0 = kE + 8 * kHid, kScale = kDA0 + kE, kRows = kScale + 5;
 __host__ __device__ constexpr int a_row(int l) { return l ? kE + (l - 1) * kHid : 0; }
 __host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHid; }
 
-// weight_grad_kernel's blocks, in proportion to a tile's time: layers 1..3 (15k
-// cycles each), layer 0 (10.5k) and the head (10k: an MMA of 16 columns takes
-// 45 of the 64 cycles that one of 128 takes). By rows (37 / 23 / 18) the head's
-// blocks were the last by a third: 2.6 -> 2.2 ms.
-constexpr int kSplit = 35, kSplit0 = 24, kSplit4 = 23;
-static_assert(3 * kSplit + kSplit0 + kSplit4 == kSMs, "one block per SM");
+// weight_grad_kernel's blocks, in proportion to a tile's time: layer 1 (15k
+// cycles), layer 0 (10.5k) and the head (10k: an MMA of 16 columns takes 45 of
+// the 64 cycles that one of 128 takes).
+constexpr int kSplit1 = 64, kSplit0 = 45, kSplit4 = 43;
+static_assert(kSplit1 + kSplit0 + kSplit4 == kSMs, "one block per SM");
+// weight_chain_kernel's blocks of layers 2 and 3 (each), with two chains per
+// element, and the samples of a batch that share a set of chains: about 9,000
+// a chain
+constexpr int kChains = kSMs / 2;
+constexpr int64_t kChainSamples = 1400000;
 
 // threads of the two tensor-core kernels that compute; a fifth warpgroup's
 // first lane issues the MMAs. Of the 640 x 96 registers at the launch (61,440)
@@ -559,10 +567,11 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
 #pragma unroll
       for (int j = 0; j < kQ; ++j) out[j * kTile] = y[j] * by;
     };
-    // A_l divided by its scale, and the scale
+    // A_l divided by its scale, and the scale (as it is for the FP32 chains)
     auto store_a = [&](int l, float inv) {
-      store(a_row(l), sa == sa ? inv : 1.0f);
-      if (quarter == 0) R[(kScale + l) * kTile + row] = sa;
+      const bool chained = l == 2 || l == 3;
+      store(a_row(l), sa == sa && !chained ? inv : 1.0f);
+      if (quarter == 0) R[(kScale + l) * kTile + row] = chained ? 1.0f : sa;
     };
     float inv = 0.0f;                        // 1 / sa
     // Ends a layer: joins the row's quarters and, where `slice`, puts its
@@ -697,6 +706,14 @@ out:;
   if (warp == 0) tmem_dealloc(tmem, kCols);
 }
 
+// slots of partial sums (floats): weight_grad_kernel's of layer 1, layer 0 and
+// the head, weight_chain_kernel's of layers 2 and 3, and its chains
+constexpr int64_t kPart0 = (int64_t)kSplit1 * kHid * kHid;
+constexpr int64_t kPart4 = kPart0 + (int64_t)kSplit0 * kHid * kE;
+constexpr int64_t kPart2 = kPart4 + (int64_t)kSplit4 * kHid * 4;
+constexpr int64_t kPartChains = kPart2 + (int64_t)2 * kChains * kHid * kHid;
+constexpr int64_t kPartFloats = kPartChains + (int64_t)2 * kChains * kHid * kHid * 2;
+
 // The two operands of a tile in FP32, and the slices of Y for half a tile's
 // samples (K = 64) in two stages; X's slices are in tensor memory.
 constexpr int kHalfPlane = kHid * 64 * 2;
@@ -733,9 +750,9 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   GradSmem &S = *reinterpret_cast<GradSmem *>(smem_raw);
   const int t = threadIdx.x, warp = t >> 5, b = blockIdx.x;
-  const int l = b < 3 * kSplit ? 1 + b / kSplit : b < 3 * kSplit + kSplit0 ? 0 : 4;
-  const int j = l == 0 ? b - 3 * kSplit : l == 4 ? b - 3 * kSplit - kSplit0 : b % kSplit;
-  const int splits = l == 0 ? kSplit0 : l == 4 ? kSplit4 : kSplit;
+  const int l = b < kSplit1 ? 1 : b < kSplit1 + kSplit0 ? 0 : 4;
+  const int j = l == 0 ? b - kSplit1 : l == 4 ? b - kSplit1 - kSplit0 : b;
+  const int splits = l == 0 ? kSplit0 : l == 4 ? kSplit4 : kSplit1;
   const int ny = l == 0 ? kE : l == 4 ? 16 : kHid;           // columns of the result
   const int yrows = l == 4 ? 4 : ny;                         // rows of Y with data
   const int64_t xrow = l == 4 ? a_row(4) : dz_row(l), yrow = l == 4 ? 0 : a_row(l);
@@ -945,11 +962,8 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
     if (sync_and(ok)) drain(j + (n - 1) * splits, (int)(n - 1) & 1, xs);
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  // slots: layers 1..3 [128][128], layer 0 [128][32], head [128][4]
-  float *P = part + (l == 0   ? (int64_t)3 * kSplit * kHid * kHid + (int64_t)j * kHid * kE
-                     : l == 4 ? (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE +
-                                    (int64_t)j * kHid * 4
-                              : (int64_t)b * kHid * kHid) +
+  // slots: layer 1 [128][128], layer 0 [128][32], head [128][4]
+  float *P = part + (l == 0 ? kPart0 : l == 4 ? kPart4 : 0) + (int64_t)j * kHid * yrows +
              (int64_t)row * yrows + c0;
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {
@@ -980,8 +994,136 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
 
 static_assert(sizeof(BwdSmem) <= 232448 && sizeof(GradSmem) <= 232448, "shared memory");
 
-constexpr int64_t kPartFloats =
-    (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE + (int64_t)kSplit4 * kHid * 4;
+// dW_l = dZ_l^T A_l of layers 2 and 3 in chains of FP32 multiply-adds, and db_l.
+// A block takes consecutive tiles of a chunk and goes on with the chains where
+// it left them in the chunk before. Thread (tx, ty) has units tx + 16 j of dZ
+// and ty + 16 i of A, and per element one chain of the even and one of the odd
+// samples: two samples per fma.rn.f32x2, operands as they lie in memory.
+//
+// Why chains: after a far sample's product an FP32 chain loses those of 2^-24
+// of it and less. In a batch with far samples FP32 GEMMs over chunks of 200k
+// samples (24 chains each) lose up to 3.4e-5 of dW3's and 1.5e-5 of dW2's norm
+// to that, which exact sums do not; these chains are of that length, so that a
+// batch's gradients stay within 1.2e-5 of the GEMM path's (RayChunk), where
+// they were up to 3.4e-5 away with exact sums (12 batches of 8,192 rays).
+// Bound: the FP32 pipe; 256 us for 194,560 samples (50 of its 66 TFLOP/s): 8 x
+// 8 elements a thread and all eight chunks unrolled; 8 x 4 and twice the
+// threads 283, one chunk an iteration 272, rows of elements all forwards 281.
+struct ChainSmem {
+  float x[3][kHid * 32], y[3][kHid * 32];  // 32 samples; 16-byte chunk c of a row at c ^ (row & 7)
+};
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
+}
+__global__ void __launch_bounds__(kT, 1) weight_chain_kernel(int64_t ns,
+                                                              const float *__restrict__ rows,
+                                                              uint64_t *__restrict__ chains,
+                                                              float *__restrict__ part,
+                                                              float *__restrict__ bias_part,
+                                                              int begin, int end, int add,
+                                                              int bias_add) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  ChainSmem &S = *reinterpret_cast<ChainSmem *>(smem_raw);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, b = blockIdx.x;
+  // (lanes that differ in bit 0 share tx: see train.cu's lane_x)
+  const int tx = (warp >> 2) * 8 + ((lane >> 1) & 7);
+  const int ty = (warp & 3) * 4 + ((lane & 1) | ((lane >> 4) << 1));
+  const int l = 2 + b / kChains, j = b % kChains;
+  const int64_t tiles = (ns + kTile - 1) / kTile, per = (tiles + kChains - 1) / kChains;
+  const int64_t first = j * per, last = first + per < tiles ? first + per : tiles;
+  const int stages = last > first ? (int)(last - first) * 4 : 0;
+  const int xrow = dz_row(l), yrow = a_row(l);
+  // stage i: a quarter of a tile, zeros behind the last sample
+  auto issue = [&](int i) {
+    if (i < stages) {
+      const int64_t tile = first + i / 4;
+      const float *R = rows + tile * kRows * kTile + (i & 3) * 32 + (t & 7) * 4;
+      const int64_t left = (ns - tile * kTile - (i & 3) * 32 - (t & 7) * 4) * 4;
+      const int bytes = left >= 16 ? 16 : left > 0 ? (int)left : 0;
+#pragma unroll
+      for (int k = 0; k < kHid * 8 / kT; ++k) {
+        const int r = (t >> 3) + k * (kT / 8), at = r * 32 + (((t & 7) ^ (r & 7)) << 2);
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                           smem_u32((g ? S.y[i % 3] : S.x[i % 3]) + at)),
+                       "l"(R + (int64_t)((g ? yrow : xrow) + r) * kTile), "r"(bytes)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  issue(0);
+  issue(1);
+  uint64_t acc[8][8];
+  uint64_t *C = chains + (int64_t)b * kHid * kHid + t;
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[n][k] = begin ? 0 : C[(n * 8 + k) * kT];
+  float sum = 0.0f, comp = 0.0f;             // db: half of row t / 2 of every stage, Kahan
+#pragma unroll 1
+  for (int i = 0; i < stages; ++i) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    issue(i + 2);
+    const float *X = S.x[i % 3] + tx * 32, *Y = S.y[i % 3] + ty * 32;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int cx = (c ^ (tx & 7)) << 2, cy = (c ^ (ty & 7)) << 2;
+      ulonglong2 x[8];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) x[n] = *reinterpret_cast<const ulonglong2 *>(X + n * 512 + cx);
+      ulonglong2 y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) y[k] = *reinterpret_cast<const ulonglong2 *>(Y + k * 512 + cy);
+      // every other row of elements backwards: neighbouring FMAs share an operand
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int n = k & 1 ? 7 - i : i;
+          fma2(acc[n][k], x[n].x, y[k].x);
+        }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int n = k & 1 ? 7 - i : i;
+          fma2(acc[n][k], x[n].y, y[k].y);
+        }
+    }
+    const float *D = S.x[i % 3] + (t >> 1) * 32;
+    float s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 a =
+          *reinterpret_cast<const float4 *>(D + ((((t & 1) * 4 + q) ^ ((t >> 1) & 7)) << 2));
+      s += (a.x + a.y) + (a.z + a.w);
+    }
+    const float a = s - comp, w = sum + a;
+    comp = fabsf(w) <= 3.4e38f ? (w - sum) - a : 0.0f;
+    sum = w;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  float *P = part + (int64_t)b * kHid * kHid + tx * kHid + ty;
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (!end) {
+        C[(n * 8 + k) * kT] = acc[n][k];
+      } else {
+        float &d = P[n * 16 * kHid + k * 16];
+        const float w = __uint_as_float((uint32_t)acc[n][k]) +
+                        __uint_as_float((uint32_t)(acc[n][k] >> 32));
+        d = add ? d + w : w;
+      }
+    }
+  const float s = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
+  float *d = bias_part + (int64_t)b * kHid + (t >> 1);
+  if (!(t & 1)) *d = bias_add ? *d + s : s;
+}
 
 struct GradOut {
   float *w[5], *b[5];
@@ -996,25 +1138,26 @@ __global__ void __launch_bounds__(kT) grad_reduce_kernel(const float *__restrict
   float *dst;
   int n, stride;
   if (i < 3 * kHid * kHid) {
-    const int l = i / (kHid * kHid), e = i % (kHid * kHid);
-    src = part + (int64_t)l * kSplit * kHid * kHid + e;
-    n = kSplit; stride = kHid * kHid;
-    dst = out.w[l + 1] + e;
+    const int l = i / (kHid * kHid) + 1, e = i % (kHid * kHid);
+    src = part + (l > 1 ? kPart2 + (int64_t)(l - 2) * kChains * kHid * kHid : 0) + e;
+    n = l > 1 ? kChains : kSplit1; stride = kHid * kHid;
+    dst = out.w[l] + e;
   } else if ((i -= 3 * kHid * kHid) < kHid * kE) {
-    src = part + (int64_t)3 * kSplit * kHid * kHid + i;
+    src = part + kPart0 + i;
     n = kSplit0; stride = kHid * kE;
     dst = out.w[0] + i;
   } else if ((i -= kHid * kE) < kHid * 4) {
-    src = part + (int64_t)3 * kSplit * kHid * kHid + (int64_t)kSplit0 * kHid * kE + i;
+    src = part + kPart4 + i;
     n = kSplit4; stride = kHid * 4;
     dst = out.w[4] + (i & 3) * kHid + (i >> 2);
   } else if ((i -= kHid * 4) < 4 * kHid) {
     const int l = i / kHid;
-    src = bias_part + (int64_t)(l ? (l - 1) * kSplit : 3 * kSplit) * kHid + i % kHid;
-    n = l ? kSplit : kSplit0; stride = kHid;
+    src = bias_part + (int64_t)(l == 0 ? kSplit1 : l == 1 ? 0 : kSMs + (l - 2) * kChains) * kHid +
+          i % kHid;
+    n = l == 0 ? kSplit0 : l == 1 ? kSplit1 : kChains; stride = kHid;
     dst = out.b[l] + i % kHid;
   } else if ((i -= 4 * kHid) < 4) {
-    src = bias_part + (int64_t)(3 * kSplit + kSplit0) * kHid + i;
+    src = bias_part + (int64_t)(kSplit1 + kSplit0) * kHid + i;
     n = kSplit4; stride = kHid;
     dst = out.b[4] + i;
   } else {
@@ -1031,7 +1174,7 @@ __global__ void __launch_bounds__(kT) grad_reduce_kernel(const float *__restrict
 }
 
 // floats of the workspace besides a chunk's rows
-constexpr int64_t kFixedFloats = kPartFloats + (int64_t)kSMs * kHid + (kSliceFloats + 31) / 32 * 32;
+constexpr int64_t kFixedFloats = kPartFloats + (int64_t)(kSMs + 2 * kChains) * kHid + (kSliceFloats + 31) / 32 * 32;
 
 int64_t chunk_rows(int64_t ns, int64_t chunk) {
   const int64_t c = chunk < ns ? chunk : ns;
@@ -1074,7 +1217,9 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
   if (cudaFuncSetAttribute(field_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)sizeof(BwdSmem)) != cudaSuccess ||
       cudaFuncSetAttribute(weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(GradSmem)) != cudaSuccess)
+                           (int)sizeof(GradSmem)) != cudaSuccess ||
+      cudaFuncSetAttribute(weight_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(ChainSmem)) != cudaSuccess)
     return NSVF_ERR_CUDA;
   float *rows = workspace;
   uint8_t *slices =
@@ -1103,8 +1248,14 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
   q.values = (const float4 *)values;
   q.rows = rows;
   q.g_values = (float4 *)grad_values;
+  // the chains begin anew every `group` chunks
+  const int64_t chunks = (n_samples + chunk_samples - 1) / chunk_samples;
+  const int64_t groups = n_samples > kChainSamples
+                             ? (n_samples + kChainSamples / 2) / kChainSamples : 1;
+  const int64_t group = chunks > groups ? (chunks + groups - 1) / groups : 1;
+  int64_t k = 0;                             // chunk
   // (one pass without samples zeroes the slots of an empty batch)
-  for (int64_t a = 0; a == 0 || a < n_samples; a += chunk_samples) {
+  for (int64_t a = 0; a == 0 || a < n_samples; a += chunk_samples, ++k) {
     p.ns = n_samples - a < chunk_samples ? n_samples - a : chunk_samples;
     q.ns = p.ns;
     q.vox = voxel + a;
@@ -1123,6 +1274,11 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
     }
     weight_grad_kernel<<<kSMs, kThreads, sizeof(GradSmem), s>>>(p.ns, rows, (const float *)p.d_out, part,
                                                           bias_part, a > 0, err);
+    if ((st = nsvf_launch_status()) != NSVF_OK) return st;
+    weight_chain_kernel<<<2 * kChains, kT, sizeof(ChainSmem), s>>>(
+        p.ns, rows, (uint64_t *)(part + kPartChains), part + kPart2,
+        bias_part + (int64_t)kSMs * kHid, k % group == 0, k % group == group - 1 || k + 1 >= chunks,
+        k >= group, a > 0);
     if ((st = nsvf_launch_status()) != NSVF_OK) return st;
   }
   constexpr int n_grads = 3 * kHid * kHid + kHid * kE + 8 * kHid + 4;

@@ -16,7 +16,7 @@ backward runs
                            interpolation and activations again, dZ = dA (Z >
                            0), dA = dZ W through all layers of a tile, then
                            dW = dZ^T A, db = sum dZ, on the tensor cores in
-                           split FP32
+                           split FP32 (dW2 and dW3 in FP32 chains)
   interpolation backward   float4 atomics into the corner embeddings, from the
                            same tiles
 

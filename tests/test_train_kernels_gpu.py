@@ -214,6 +214,26 @@ def test_split_backward_against_float64(cuda, ns, spread, far):
         assert float((a.double() - b).norm()) <= 2.0 ** -18 * float(b.norm())
 
 
+@pytest.mark.parametrize("ns,chunks", [(300, 1), (100000, 3), (2150000, 13)])
+def test_weight_chains_across_chunks(cuda, ns, chunks):
+    """Weight gradients of one chunk, of several that share their FP32 chains,
+    and of more samples than one set of chains takes. At most 9,300 additions
+    round in a chain, as a random walk by 2^-24 each: 2^-17 of the norm."""
+    g = torch.Generator().manual_seed(ns)
+    dout = torch.randn(ns, 4, generator=g).to(cuda)
+    chunk = -(-ns // chunks) // 128 * 128 + 128
+    (grads, _), (acts, pre, params, _) = _field_grads(cuda, ns, dout, ns, chunk)
+    p64 = [p.double() for p in params]
+    ref = [0] * 10
+    for i in range(0, ns, 250000):
+        s = slice(i, i + 250000)
+        part, _ = _chain_grads([a[s].double() for a in acts], [z[s] for z in pre], p64,
+                               dout[s].double())
+        ref = [r + q for r, q in zip(ref, part)]
+    for a, b in zip(grads, ref):
+        assert float((a.double() - b).norm()) <= 2.0 ** -17 * float(b.norm())
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 9e37, 1e-40])
 def test_split_backward_rows_the_slices_cannot_hold(cuda, value):
     """A gradient that is not finite, near the largest float, or denormal: the
