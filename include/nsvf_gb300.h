@@ -724,7 +724,9 @@ int nsvf_prune_screen_bf16(int64_t n_voxels, int bits, int rule, float step, flo
 /* prune_screen_live_bf16: the screen without scores, on sub^3 of each voxel's
  * points (sub per axis, both faces among them; 2 <= sub <= bits, all points for
  * sub == bits) and, with `live` (int32 [n_voxels], n_live one int64), only for
- * the voxels that keep does not hold yet. Two calls, a few points of every
+ * the voxels that keep does not hold yet (all their points: in parts, each on
+ * the voxels that the part before left; live and n_live then hold the last
+ * part's). Two calls, a few points of every
  * voxel and then all points of the rest, set the same keep flags and list the
  * undecided points of every voxel not kept. */
 int nsvf_prune_screen_live_bf16(int64_t n_voxels, int bits, int sub, int rule, float threshold,
