@@ -285,12 +285,15 @@ def sample_rays(encoder, ray_start, ray_dir, states=None):
                                                    inter['min_depth'], inter['max_depth'],
                                                    encoder.step_size)
     hits = hits.reshape(-1)
-    sub = {k: v.reshape(-1, v.shape[-1])[hits] if v.dim() == 3 else v.reshape(-1)[hits]
+    # the hit rays' rows, found once: indexing by the mask finds them (and
+    # waits for their number) for each of seven tensors again
+    rows = hits.nonzero()[:, 0]
+    sub = {k: (v.reshape(-1, v.shape[-1]) if v.dim() == 3 else v.reshape(-1))[rows]
            for k, v in inter.items()}
     smp = encoder.ray_sample(sub)
     o = ray_start.reshape(-1, 3)
-    o = o[hits] if o.shape[0] == R else o.expand(int(hits.sum()), 3)
-    d = ray_dir.reshape(-1, 3)[hits]
+    o = o[rows] if o.shape[0] == R else o.expand(rows.numel(), 3)
+    d = ray_dir.reshape(-1, 3)[rows]
     xyz = o[:, None, :] + d[:, None, :] * smp['sampled_point_depth'][..., None]
     return hits, smp['sampled_point_voxel_idx'], smp['sampled_point_depth'], \
         smp['sampled_point_distance'], xyz.contiguous()
@@ -298,7 +301,7 @@ def sample_rays(encoder, ray_start, ray_dir, states=None):
 
 def render_batch(encoder, field, ray_start, ray_dir, chunk_rays=1024, states=None, kahan=False,
                  samples=None):
-    """Colours [R, 3] of a batch of rays through RayChunk (differentiable
+    """Colours [R, 3] of a batch of rays through RayBatch or RayChunk (differentiable
     with respect to the encoder's `values` and the field's parameters), with
     the background filled in for missed rays and the missed part of hit
     rays (fairnr/models/nsvf.py:89-110)."""
