@@ -305,6 +305,26 @@ def test_prune_fp32_stage_keeps_the_mask(cuda, n_vox, bits, rule):
         assert torch.equal(keep2, want) and none is None
 
 
+@pytest.mark.parametrize("n_vox,bits", [(60, 3), (60, 4), (60, 7), (6, 40), (6, 41)])
+def test_prune_in_parts_keeps_the_mask(cuda, n_vox, bits):
+    """The screen of all points at the edges of its rule (four parts from 4 to
+    40 points per axis), and where the parts do not divide the points: the
+    mask of the screen in one pass over all points."""
+    from nsvf_gb300 import ext
+    from nsvf_gb300.field import StandInField
+    from nsvf_gb300.mlp import TensorCoreMLP
+    vs, centers, feats, values, params = _scene(cuda, n_vox, n_vox)
+    mlp = TensorCoreMLP(StandInField(weights=[(params[2 * l].cpu(), params[2 * l + 1].cpu())
+                                              for l in range(5)]).to(cuda))
+    score = mlp.prune_scores(centers, feats, values, vs, bits=bits, rule=1, step=0.01)
+    for th in (float(score.median()), float(score.max()) * 0.999):
+        keep = [mlp.prune_mask(centers, feats, values, vs, th=max(th, 1e-6), bits=bits, rule=1,
+                               step=0.01, band=band, scores=s)[0]
+                for band in (0.02, 0.5) for s in (True, False)]
+        ext.check_errors(cuda)
+        assert all(torch.equal(k, keep[0]) for k in keep)
+
+
 @pytest.mark.parametrize("ns", [1, 7, 257, 90001])
 @pytest.mark.parametrize("E,dtypes", [(4, (torch.int64, torch.int64)),
                                       (32, (torch.int64, torch.int64)),
