@@ -42,16 +42,16 @@
 // A lane of the computing warps as the issuer: 3.3 ms, behind its warp's share
 // of the stores.
 // weight_grad_kernel (layers 0, 1 and the head): dW_l = dZ_l^T A_l, db_l = sum
-// dZ_l: K runs over the 128
-// samples of a tile, rows are units. A sample far outside its voxel has
-// activations some thousand times the others', and often next to no gradient;
-// on a common exponent the others would lose ten bits to it. So A_l is stored
-// divided by its sample's power of two (all samples alike), and dZ_l is
-// multiplied by it before it is sliced; the products are the same. FP32 accumulation over tiles in
-// registers, one slot per block, the slots added in a fixed order. The FP32
-// rows of the next tile arrive by cp.async while a tile is sliced. Bound: the
-// instructions and the barriers of slicing and draining, 13k cycles a tile and
-// layer, of which the MMAs run beside 3.1k and the 128 KB from memory 5.6k.
+// dZ_l: K runs over the 128 samples of a tile, rows are units. A sample far
+// outside its voxel has activations some thousand times the others', and often
+// next to no gradient; on a common exponent the others would lose ten bits to
+// it. So A_l is stored divided by its sample's power of two (all samples
+// alike), and dZ_l is multiplied by it before it is sliced; the products are
+// the same. FP32 accumulation over tiles in registers, one slot per block, the
+// slots added in a fixed order. The FP32 rows of the next tile arrive by
+// cp.async while a tile is sliced. Bound: the instructions and the barriers of
+// slicing and draining, 11k cycles a tile of layer 1, of which the MMAs run
+// beside 3.1k and the 128 KB from memory 5.6k.
 #include "interp_run.cuh"
 #include "tc_common.cuh"
 #include "train_common.cuh"
