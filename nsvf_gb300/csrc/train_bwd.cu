@@ -389,7 +389,9 @@ struct BwdSmem {
   uint8_t b[2][3 * kPlane];   // the slices of a layer's weights and of the next one's
   float scales[kScales];
   float bias[4 * kHid];
-  uint8_t top[4][kTile];      // the largest exponent in each quarter of a row
+  // the largest exponent in each quarter of a row, of this layer and of the
+  // one before: a quarter may write the next layer's while another still reads
+  uint8_t top[2][4][kTile];
   uint64_t mma_done, ready, loaded[2];
   uint32_t tmem;
   int abort;
@@ -576,10 +578,12 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
     float inv = 0.0f;                        // 1 / sa
     // Ends a layer: joins the row's quarters and, where `slice`, puts its
     // slices in A. top: the largest |y|, NaN where fix(j) has to give y[j]
-    // again (it reads rows of memory written before the barrier). False:
-    // unwind.
-    auto rows_done = [&](float top, bool slice, auto fix) {
-      S.top[quarter][row] = (uint8_t)exponent(top);
+    // again (it reads rows of memory written before the barrier). turn: 0 and 1
+    // in turn, so that the next call's barrier lies between this one's reads of
+    // S.top and the next write to the same half. False: unwind.
+    auto rows_done = [&](float top, int turn, bool slice, auto fix) {
+      auto &tops = S.top[turn];
+      tops[quarter][row] = (uint8_t)exponent(top);
       if (!sync_and(ok && top == top)) {
         if (!sync_and(ok)) return false;
         if (top != top) {
@@ -589,12 +593,11 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
             if (y[j] != y[j]) y[j] = fix(j);
             top = max_nan(top, fabsf(y[j]));
           }
-          S.top[quarter][row] = (uint8_t)exponent(top);
+          tops[quarter][row] = (uint8_t)exponent(top);
         }
         sync_and(true);
       }
-      sa = row_scale(max(max(S.top[0][row], S.top[1][row]), max(S.top[2][row], S.top[3][row])),
-                     inv);
+      sa = row_scale(max(max(tops[0][row], tops[1][row]), max(tops[2][row], tops[3][row])), inv);
       if (!slice) return true;
       slice_row(tmem_row + kACol + c0 / 2, y, inv);
       slices_ready(&S.ready);
@@ -620,7 +623,7 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
           top = max_nan(top, fabsf(y[j]));
         }
       }
-      if (!rows_done(top, l < 3, [&](int j) {
+      if (!rows_done(top, l & 1, l < 3, [&](int j) {
             const float z = fmaf(chain(R + a_row(l) * kTile + row, kTile,
                                        p.packed + w_off(l) + c0 + j, kHid, l ? kHid : kE),
                                  scale_of(R[(kScale + l) * kTile + row]), bias[j]);
@@ -653,7 +656,7 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
         y[j] *= bit(m, j) ? 1.0f : 0.0f;
         top = max_nan(top, fabsf(y[j]));
       }
-      if (!rows_done(top, true, [&](int j) {
+      if (!rows_done(top, ~l & 1, true, [&](int j) {
             if (l == 3) return y[j];
             return chain(R + dz_row(l + 1) * kTile + row, kTile,
                          p.packed + w_off(l + 1) + (c0 + j) * kHid, 1, kHid) *

@@ -374,3 +374,60 @@ def test_interpolation_runs(cuda, ns, E, dtypes):
     assert float((emb.detach().double() - ref.detach()).abs().max()) <= 1e-5
     assert float((gx.double() - rx).norm()) <= 2e-6 * float(rx.norm()) + 1e-12
     assert float((gv.double() - rv).norm()) <= 2e-6 * float(rv.norm()) + 1e-12
+
+
+@pytest.mark.parametrize("ns", [128, 152 * 128 * 3 + 1])
+def test_head_gradient_of_uneven_quarters(cuda, ns):
+    """dW4 where the four threads that hold a sample's last activations find
+    largest elements far apart (units of one quarter scaled by 2^20 and the
+    head's columns by 2^-20, which leaves the field as it is): all of them have
+    to divide by the power of two that is stored beside the row. Against float64
+    with the test above's 2^-18 of a column block's norm, and the same bits from
+    every launch (each block has several tiles at the larger size)."""
+    from nsvf_gb300.functional import trilinear_embed
+    from nsvf_gb300 import ext, train
+    from nsvf_gb300._lib import LIB, check
+    n_vox = 61
+    vs, centers, feats, values, params = _scene(cuda, n_vox, 4)
+    for q, scale in enumerate((1.0, 2.0 ** 20, 2.0 ** -20, 2.0 ** 10)):
+        u = slice(32 * q, 32 * q + 32)
+        params[6][u] *= scale
+        params[7][u] *= scale
+        params[8][:, u] /= scale
+    g = torch.Generator().manual_seed(ns)
+    vid = torch.randint(0, n_vox, (ns,), generator=g, dtype=torch.int32).to(cuda)
+    xyz = (centers[vid.long()] + (torch.rand(ns, 3, generator=g).to(cuda) - 0.5) * vs).contiguous()
+    xyzd = torch.cat([xyz, torch.ones(ns, 1, device=cuda)], 1).contiguous()
+    dout = torch.randn(ns, 4, generator=g).to(cuda)
+    stream, err = ext.ctypes_stream(cuda), ext.error_word(cuda)
+    packed = train.RayBatch._packed(params, stream)
+    out = torch.empty(ns, 4, device=cuda)
+    signs = torch.zeros(4, ns, 16, dtype=torch.uint8, device=cuda)
+    scene = (n_vox, values.size(0), vs, centers.data_ptr(), feats.data_ptr(), values.data_ptr(),
+             packed.data_ptr())
+    check(LIB.nsvf_field_train_forward_signs(ns, vid.data_ptr(), xyzd.data_ptr(), *scene,
+                                             out.data_ptr(), signs.data_ptr(), err.data_ptr(),
+                                             stream), "forward")
+    chunk = -(-ns // 128) * 128
+    n = int(LIB.nsvf_field_train_backward_floats(ns, chunk))
+    work = torch.empty(n, device=cuda)
+    first = None
+    for _ in range(10):
+        gv, grads = torch.zeros_like(values), [torch.empty_like(p) for p in params]
+        check(LIB.nsvf_field_train_backward(
+            ns, chunk, vid.data_ptr(), xyzd.data_ptr(), *scene, signs.data_ptr(), dout.data_ptr(),
+            work.data_ptr(), n, gv.data_ptr(), train._ptrs(grads[0::2]), train._ptrs(grads[1::2]),
+            err.data_ptr(), stream), "backward")
+        first = first or grads
+        assert all(torch.equal(a, b) for a, b in zip(grads, first))
+    ext.check_errors(cuda)
+    x = trilinear_embed(vid, xyz, centers, feats, values, vs)
+    x64 = x.double()
+    for l in range(4):
+        z = torch.addmm(params[2 * l + 1], x, params[2 * l].t())
+        x64 = (x64 @ params[2 * l].double().t() + params[2 * l + 1].double()) * (z > 0)
+        x = torch.relu(z)
+    ref = dout.double().t() @ x64
+    for q in range(4):
+        a, b = first[8][:, 32 * q:32 * q + 32].double(), ref[:, 32 * q:32 * q + 32]
+        assert float((a - b).norm()) <= 2.0 ** -18 * float(b.norm())
