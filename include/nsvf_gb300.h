@@ -671,10 +671,11 @@ int nsvf_field_samples_fp8_dev(int64_t capacity, const int64_t *n_samples_dev,
                                void *stream);
 
 /* wait_timeout_selftest: the failure path of the kernels' bounded waits,
- * without a fault. One CTA waits on an mbarrier phase that never completes;
- * after limit_ns (1 ns .. 1 s) the wait gives up, bit 3 (8) of *err is set
- * (the bit the tensor-core kernels set on a timed-out wait) and the kernel
- * returns, leaving the context usable. No reference counterpart (the
+ * without a fault. One warp of a CTA waits on an mbarrier phase that never
+ * completes, another one on a complete phase; after limit_ns (1 ns .. 1 s) the
+ * wait gives up, the warps join their results, bit 3 (8) of *err is set (the
+ * bit the tensor-core kernels set on a timed-out wait; bit 0 where a warp took
+ * the wait for a good one) and the kernel returns, leaving the context usable. No reference counterpart (the
  * reference's kernels have no waits). */
 int nsvf_wait_timeout_selftest(uint64_t limit_ns, int32_t *err, void *stream);
 

@@ -1015,21 +1015,29 @@ bool set_weights_fp8(MlpParams &p, const void *const weights[5], const float *co
   return true;
 }
 
-// One CTA waits, with the kernels' bounded wait, on an mbarrier phase that
-// never completes (nothing arrives). The wait gives up after limit_ns; the
-// kernel records bit 3 (8) in err, as the MLP kernels do on a timeout, and
-// returns normally.
+// The kernels' bounded wait in one CTA of two warps: the first one waits on an
+// mbarrier phase that never completes (nothing arrives) and gives up after
+// limit_ns, the second one on a phase that is complete. Both join their results
+// (barrier_and), as a block does before its next barrier; the kernel records
+// bit 3 (8) in err, as the tensor-core kernels do on a timeout (and bit 0 where
+// a warp is told that all waits ended well), and returns normally.
 __global__ void wait_timeout_kernel(uint64_t limit_ns, int32_t *err) {
-  __shared__ uint64_t bar;
-  __shared__ int abort_flag;
+  __shared__ uint64_t bar[2];
+  __shared__ int abort_flag[2];
+  const int w = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    abort_flag = 0;
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    abort_flag[0] = abort_flag[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
-  const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar, 0, &abort_flag, limit_ns));
-  if (!ok && threadIdx.x == 0 && err) atomicOr(err, 8);
+  if (threadIdx.x == 32) mbar_arrive(&bar[1]);
+  bool ok = mbar_wait(&bar[w], 0, &abort_flag[w], limit_ns);
+  ok = barrier_and<64>(ok);
+  if (ok) ok = barrier_and<64>(ok);          // one more, where all waits ended well
+  ok = barrier_and<64>(ok);
+  if ((threadIdx.x & 31) == 0 && err) atomicOr(err, ok ? 1 : 8);
 }
 
 }  // namespace
@@ -1307,7 +1315,7 @@ int nsvf_field_samples_fp8(int64_t n_samples, const int32_t *voxel, const float 
 
 int nsvf_wait_timeout_selftest(uint64_t limit_ns, int32_t *err, void *stream) {
   if (!err || limit_ns == 0 || limit_ns > 1000000000ull) return NSVF_ERR_INVALID;
-  wait_timeout_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(limit_ns, err);
+  wait_timeout_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(limit_ns, err);
   return nsvf_launch_status();
 }
 

@@ -284,6 +284,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   return false;
 }
 
+// A barrier (number 1) of kThreads threads: whether `ok` holds for all of them.
+// A wait may run out for some threads of a block and end well for others, so
+// its result has to pass through here before it decides on another barrier.
+template <int kThreads>
+__device__ __forceinline__ bool barrier_and(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)ok), "n"(kThreads)
+      : "memory");
+  return r != 0;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t *>(&h);

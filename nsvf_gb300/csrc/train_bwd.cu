@@ -177,18 +177,7 @@ __device__ __forceinline__ void issue_split_ts(uint32_t tmem, uint32_t a, uint32
 }
 
 // A barrier of the computing threads: whether `ok` holds for all of them.
-__device__ __forceinline__ bool sync_and(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)ok), "n"(kBT)
-      : "memory");
-  return r != 0;
-}
+__device__ __forceinline__ bool sync_and(bool ok) { return barrier_and<kBT>(ok); }
 // This warp's slices are written (every thread past its fences).
 __device__ __forceinline__ void slices_ready(uint64_t *bar) {
   fence_before_sync();
@@ -960,8 +949,8 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
       slices_ready(&S.ready[h]);
     }
   }
-  if (n > 0 && ok) {
-    ok = mbar_wait(&S.done, (uint32_t)(n - 1) & 1u, abort);
+  if (n > 0) {                               // the same n on all threads, ok not
+    ok = ok && mbar_wait(&S.done, (uint32_t)(n - 1) & 1u, abort);
     if (sync_and(ok)) drain(j + (n - 1) * splits, (int)(n - 1) & 1, xs);
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");

@@ -192,3 +192,16 @@ def test_bounded_wait_times_out_and_leaves_the_context_usable(cuda):
     ext.check_errors(cuda)
     np.testing.assert_allclose(out.cpu().numpy(), mlp.reference_bf16(emb).cpu().numpy(),
                                atol=2e-3 * (out.abs().max().item() + 1e-6), rtol=1e-2)
+
+
+@pytest.mark.parametrize("limit_ns", [1, 1_000_000])
+def test_wait_that_runs_out_for_some_threads_ends_for_all(cuda, limit_ns):
+    """A wait that ends well in one warp and runs out in another: both leave
+    the block's barriers the same number of times, and both are told so."""
+    from nsvf_gb300 import ext
+    from nsvf_gb300._lib import LIB
+    for _ in range(20):
+        err = torch.zeros(1, dtype=torch.int32, device=cuda)
+        assert LIB.nsvf_wait_timeout_selftest(limit_ns, err.data_ptr(),
+                                              ext.ctypes_stream(cuda)) == 0
+        assert int(err.item()) == 8
