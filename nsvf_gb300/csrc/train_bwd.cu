@@ -4,26 +4,36 @@
 // Reference: SparseVoxelEncoder.forward (fairnr/modules/encoder.py:558-592)
 // and the field under autograd.
 //
-// The split. A GEMM operand's row (its K elements) is scaled by a power of
-// two to |x| < 1 and cut into three bf16 slices on fixed grids of 2^-8, 2^-17
-// and about 2^-26 (error-free slicing on a common exponent, the scheme of
-// Ozaki, Ogita, Oishi and Rump, 2012). Products of slices on the first grid
-// are multiples of 2^-16 below one, so K = 128 of them add up in an FP32
-// accumulator without any rounding, whatever the order and the rounding of
-// the tensor core. One accumulator takes the products of order 0, a second one
-// those of orders 2 and 1 (three and two, in this sequence; what it loses is a
-// 2^-9th of the first one's last places); the orders left out are below 2^-26
-// of the row's and the column's largest element. The sum of the two rounds
-// once, where a chain of 128 FP32 multiply-adds rounds 128 times.
+// The split. Every element of a GEMM operand is cut into three bf16 slices,
+// each rounded to nearest, after its row (its K elements) was scaled by a power
+// of two to |x| < 1: all 24 bits of the element, whatever else its row holds,
+// down to 2^-109 of the row's largest. Of the nine products of slices the six
+// of orders 0 to 2 (in steps of 2^-8) are taken; the others are 2^-23 of the
+// element's product at most and 2^-26 typically. Two accumulators: one takes
+// the first half of the products of order 0, the second one those of orders 2
+// and 1 and then the other half. The tensor core's adder truncates, so that
+// sums of half the length lose less: all products of order 0 in one accumulator
+// doubled the errors below. The two are added once, where a chain of 128 FP32
+// multiply-adds rounds 128 times.
+//
+// Why slices of the elements' own: on a grid common to the row (2^-8, 2^-17 and
+// about 2^-26 of its largest element) the products of the first slices add up
+// without any rounding, but an element of 1e-6 of the largest keeps few bits.
+// Gradients of units that are active only in samples behind a surface were
+// off by up to 2e-5 of the sum of their terms' absolute values, and everything
+// by 4 % in a field whose units differ by 2^24 in size.
 //
 // A row with an element that is not finite (or of 2^126 and more) gets the
 // scale NaN: its results are NaN and each of them is then computed by the
 // FP32 chain.
 //
-// Errors of these sums against float64: 2e-7 of the gradient's norm, where
-// FP32 GEMMs over chunks leave 8e-7 to 1.6e-6, and up to 3.4e-5 in batches with
-// far samples; there layers 2 and 3, where that is more than 1e-5, are summed
-// as the GEMMs sum them (weight_chain_kernel).
+// Errors against float64 over 128 to 200,000 samples (gradients alike,
+// log-normal of sigma 6, a few 1e6 times the others, units of 2^-12 to 2^12 in
+// size): 1.1e-7 to 3.2e-7 of the norm, FP32 GEMMs 1.9e-7 to 1.5e-6; single
+// elements, relative to the sum of their terms' absolute values, 0.2 to 0.95 of
+// the GEMMs' in the root mean square. In batches with far samples FP32 GEMMs
+// over chunks leave up to 3.4e-5 of the norm; layers 2 and 3, where that is more
+// than 1e-5, are summed as the GEMMs sum them (weight_chain_kernel).
 //
 // Measured on 1.40 M samples: 5.7 ms (the interpolation 0.3, field_bwd_kernel 2.5,
 // weight_chain_kernel 1.8, weight_grad_kernel 1.1; all on the FP32 pipe took
@@ -105,11 +115,6 @@ __device__ __forceinline__ uint64_t pk(float lo, float hi) {
   asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "f"(lo), "f"(hi));
   return d;
 }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
@@ -120,24 +125,24 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {   // a - b
   asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(b), "l"(pk(-1.0f, -1.0f)), "l"(a));
   return d;
 }
-// the upper halves of two floats (exact for values of at most 8 bits)
-__device__ __forceinline__ uint32_t tops(uint64_t v) {
-  return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632);
+// two bf16 as two floats
+__device__ __forceinline__ uint64_t widen(uint32_t v) {
+  return pk(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
 }
 
-// The three bf16 slices of x0, x1 scaled by inv (|x inv| < 1). Adding and
-// subtracting 1.5 2^15 rounds to a multiple of 2^-8, 1.5 2^6 to one of 2^-17;
-// both quotients are at most 256 and so 8 bits; the rest rounds to bf16.
+// The three bf16 slices of x0, x1 scaled by inv (|x inv| < 1), each rounded to
+// nearest: both differences are exact, and the three add up to x inv wherever
+// that is above 2^-109.
 __device__ __forceinline__ void slice2(float x0, float x1, float inv, uint32_t &h, uint32_t &m,
                                        uint32_t &l) {
   const uint64_t t = mul2(pk(x0, x1), pk(inv, inv));
-  const uint64_t hi = add2(add2(t, pk(49152.0f, 49152.0f)), pk(-49152.0f, -49152.0f));
-  const uint64_t r = sub2(t, hi);
-  const uint64_t mi = add2(add2(r, pk(96.0f, 96.0f)), pk(-96.0f, -96.0f));
-  const uint64_t lo = sub2(r, mi);
-  h = tops(hi);
-  m = tops(mi);
-  l = pack_bf16x2(__uint_as_float((uint32_t)lo), __uint_as_float((uint32_t)(lo >> 32)));
+  auto pack = [](uint64_t v) {
+    return pack_bf16x2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+  };
+  h = pack(t);
+  const uint64_t r = sub2(t, widen(h));
+  m = pack(r);
+  l = pack(sub2(r, widen(m)));
 }
 
 __device__ __forceinline__ float max_nan(float a, float b) {
@@ -155,11 +160,12 @@ __device__ __forceinline__ float row_scale(uint32_t e, float &inv) {
 }
 
 // Adds the products of three slices each of A (128 rows) and B, K = 16 KS, to
-// the accumulators (first: to zero); issued by one thread. A's slices are in
+// the accumulators (first: to zero), those of order 0 with k < 16 KS0 to the
+// first one and all others to the second; issued by one thread. A's slices are in
 // tensor memory at column `a`, KS * 8 columns apart (two elements per column),
 // B's in shared memory at `b`. All addresses are constants beyond these: with
 // a loop of computed descriptors a MMA took 105 cycles to issue and 64 to run.
-template <int KS, int B_PLANE, int N>
+template <int KS, int B_PLANE, int N, int KS0>
 __device__ __forceinline__ void issue_split_ts(uint32_t tmem, uint32_t a, uint32_t b,
                                                bool first) {
   constexpr uint32_t idesc = idesc_bf16_f32(kTile, N);
@@ -170,10 +176,12 @@ __device__ __forceinline__ void issue_split_ts(uint32_t tmem, uint32_t a, uint32
 #pragma unroll
     for (int i = 0; i <= o; ++i)
 #pragma unroll
-      for (int k = 0; k < KS; ++k)
-        mma_bf16_ts(tmem + (o ? kAccCols : 0u), a + (uint32_t)(i * KS * 8 + 8 * k),
+      for (int k = 0; k < KS; ++k) {
+        const bool low = o == 0 && k < KS0;
+        mma_bf16_ts(tmem + (low ? 0u : kAccCols), a + (uint32_t)(i * KS * 8 + 8 * k),
                     bd + (uint32_t)((o - i) * B_PLANE / 16 + 16 * k), idesc,
-                    i == 0 && o != 1 && k == 0 && first ? 0u : 1u);
+                    first && i == 0 && k == 0 && (o == 2 || low) ? 0u : 1u);
+      }
 }
 
 // A barrier of the computing threads: whether `ok` holds for all of them.
@@ -482,11 +490,11 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
           fence_after_sync();
           const uint32_t b = smem_u32(S.b[op & 1]);
           if (op == 0)
-            issue_split_ts<kE / 16, kSmallOp, kHid>(tmem, tmem + kACol, b, true);
+            issue_split_ts<kE / 16, kSmallOp, kHid, 1>(tmem, tmem + kACol, b, true);
           else if (op < 7)
-            issue_split_ts<kHid / 16, kPlane, kHid>(tmem, tmem + kACol, b, true);
+            issue_split_ts<kHid / 16, kPlane, kHid, 4>(tmem, tmem + kACol, b, true);
           else
-            issue_split_ts<kHid / 16, kSmallOp, kE>(tmem, tmem + kACol, b, true);
+            issue_split_ts<kHid / 16, kSmallOp, kE, 4>(tmem, tmem + kACol, b, true);
           mma_commit(&S.mma_done);
           ok = mbar_wait(&S.mma_done, ph_mma, abort);
           ph_mma ^= 1u;
@@ -730,6 +738,14 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, int size, b
                  : "memory");
 }
 
+// The MMAs of half a tile, the first ones of the first half in one accumulator
+// and of the second in the other.
+template <int N>
+__device__ __forceinline__ void issue_half(uint32_t tmem, uint32_t x, uint32_t y, int h) {
+  if (h == 0) issue_split_ts<4, kHalfPlane, N, 4>(tmem, x, y, true);
+  else issue_split_ts<4, kHalfPlane, N, 0>(tmem, x, y, false);
+}
+
 // dW = X^T Y of one layer over some of the chunk's tiles, X = dZ (A4 for the
 // head), Y = A (d_out). A thread slices 32 samples (a quarter of each half of
 // the tile) of row t % 128 of both.
@@ -785,12 +801,9 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
           if (!ok) break;
           fence_after_sync();
           const uint32_t x = tmem + kXCol + h * kXHalf, y = smem_u32(S.y[h]);
-          if (ny == kHid)
-            issue_split_ts<4, kHalfPlane, kHid>(tmem, x, y, h == 0);
-          else if (ny == kE)
-            issue_split_ts<4, kHalfPlane, kE>(tmem, x, y, h == 0);
-          else
-            issue_split_ts<4, kHalfPlane, 16>(tmem, x, y, h == 0);
+          if (ny == kHid) issue_half<kHid>(tmem, x, y, h);
+          else if (ny == kE) issue_half<kE>(tmem, x, y, h);
+          else issue_half<16>(tmem, x, y, h);
           if (h == 1) mma_commit(&S.done);
         }
       if (!ok) {

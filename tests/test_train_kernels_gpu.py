@@ -126,7 +126,7 @@ def test_forward_bits_of_a_gemm_chain(cuda, ns):
     assert torch.equal(out, x)
 
 
-def _field_grads(cuda, ns, dout, seed, chunk, far=None):
+def _field_grads(cuda, ns, dout, seed, chunk, far=None, rescale=None):
     """The field's forward with signs and its backward on random samples, and
     the FP32 layers of the same samples: (grads, grad_values), (acts, pre,
     params, scene)."""
@@ -135,6 +135,8 @@ def _field_grads(cuda, ns, dout, seed, chunk, far=None):
     from nsvf_gb300.functional import trilinear_embed
     n_vox = 61
     vs, centers, feats, values, params = _scene(cuda, n_vox, seed)
+    if rescale is not None:
+        rescale(params)
     g = torch.Generator().manual_seed(seed)
     vid = torch.randint(0, n_vox, (ns,), generator=g, dtype=torch.int32).to(cuda)
     xyz = (centers[vid.long()] + (torch.rand(ns, 3, generator=g).to(cuda) - 0.5) * vs).contiguous()
@@ -431,3 +433,52 @@ def test_head_gradient_of_uneven_quarters(cuda, ns):
     for q in range(4):
         a, b = first[8][:, 32 * q:32 * q + 32].double(), ref[:, 32 * q:32 * q + 32]
         assert float((a - b).norm()) <= 2.0 ** -18 * float(b.norm())
+
+
+@pytest.mark.parametrize("units", [0, 12])
+@pytest.mark.parametrize("ns,large", [(1, []), (127, [5]), (128, [5, 70]), (129, [128]), (300, [7])])
+def test_small_elements_of_the_gradients(cuda, ns, large, units):
+    """Single elements: of units that are active only in samples whose
+    gradients are 1e-6 of the largest, and of layers whose units differ by 2^24
+    in size (scaled by powers of two, which leaves the field as it is). Against
+    float64 with the forward's ReLU signs, each element relative to the sum of
+    its terms' absolute values: at most six contractions of 128 or ns terms in
+    FP32, each a random walk of 2^-24 a term whose largest of 1e5 elements is
+    4.5 deviations: 2^-17.5, with a factor of 3 left 2^-16."""
+    g = torch.Generator().manual_seed(ns + units)
+    dout = torch.randn(ns, 4, generator=g)
+    dout[large] *= 1e6
+    dout = dout.to(cuda)
+
+    def rescale(params):
+        for l in range(4):
+            s = 2.0 ** (units * torch.randint(-1, 2, (128,), generator=g).float()).to(cuda)
+            params[2 * l] *= s[:, None]
+            params[2 * l + 1] *= s
+            params[2 * l + 2] /= s
+
+    (grads, gv), (acts, pre, params, scene) = _field_grads(cuda, ns, dout, ns, 304 * 128,
+                                                           rescale=rescale)
+    vid, xyz, centers, feats, values, vs = scene
+    p64 = [p.double() for p in params]
+    q = (xyz.double() - centers[vid.long()].double()) / float(np.float32(vs)) + 0.5
+    w = [1, 1, 1, 1, 1, 1, 1, 1]
+    for k in range(8):
+        for d, bit in enumerate((4, 2, 1)):
+            w[k] = w[k] * (q[:, d] if k & bit else 1 - q[:, d])
+    keys = feats[vid.long()].long()
+    v64 = values.double()
+    a = [sum(w[k][:, None] * v64[keys[:, k]] for k in range(8))]
+    size = [sum(w[k].abs()[:, None] * v64[keys[:, k]].abs() for k in range(8))]
+    for l in range(4):
+        on = (pre[l] > 0).double()
+        a.append((a[-1] @ p64[2 * l].t() + p64[2 * l + 1]) * on)
+        size.append((size[-1] @ p64[2 * l].abs().t() + p64[2 * l + 1].abs()) * on)
+    ref, da = _chain_grads(a, pre, p64, dout.double())
+    sizes, dsize = _chain_grads(size, pre, [p.abs() for p in p64], dout.double().abs())
+    ref_v, size_v = (torch.zeros_like(v64) for _ in range(2))
+    for k in range(8):
+        ref_v.index_add_(0, keys[:, k], w[k][:, None] * da)
+        size_v.index_add_(0, keys[:, k], w[k].abs()[:, None] * dsize)
+    for x, b, s in zip([*grads, gv], [*ref, ref_v], [*sizes, size_v]):
+        assert bool(((x.double() - b).abs() <= 2.0 ** -16 * s).all())
