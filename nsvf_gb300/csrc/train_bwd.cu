@@ -52,16 +52,12 @@
 // A lane of the computing warps as the issuer: 3.3 ms, behind its warp's share
 // of the stores.
 // weight_grad_kernel (layers 0, 1 and the head): dW_l = dZ_l^T A_l, db_l = sum
-// dZ_l: K runs over the 128 samples of a tile, rows are units. A sample far
-// outside its voxel has activations some thousand times the others', and often
-// next to no gradient; on a common exponent the others would lose ten bits to
-// it. So A_l is stored divided by its sample's power of two (all samples
-// alike), and dZ_l is multiplied by it before it is sliced; the products are
-// the same. FP32 accumulation over tiles in registers, one slot per block, the
-// slots added in a fixed order. The FP32 rows of the next tile arrive by
-// cp.async while a tile is sliced. Bound: the instructions and the barriers of
-// slicing and draining, 11k cycles a tile of layer 1, of which the MMAs run
-// beside 3.1k and the 128 KB from memory 5.6k.
+// dZ_l: K runs over the 128 samples of a tile, rows are units. FP32 accumulation
+// over tiles in registers, one slot per block, the slots added in a fixed order.
+// The FP32 rows of the next tile arrive by cp.async while a tile is sliced.
+// Bound: the instructions and the barriers of slicing and draining, 11k cycles a
+// tile of layer 1, of which the MMAs run beside 3.1k and the 128 KB from memory
+// 5.6k.
 #include "interp_run.cuh"
 #include "tc_common.cuh"
 #include "train_common.cuh"
@@ -84,10 +80,8 @@ constexpr int kScales = 7 * kHid + kE;     // a power of two per row of every op
 constexpr int kSliceFloats = kSliceBytes / 4 + kScales;
 
 // rows of 128 samples of a tile in memory: A0 (32), A1..A4, dZ0..dZ3, dA0 as
-// [sample][32], and the scales of A0..A4. A_l is stored divided by its sample's
-// scale, the power of two above the sample's largest element (NaN and the
-// element itself where row_scale has none).
-constexpr int kDA0 = kE + 8 * kHid, kScale = kDA0 + kE, kRows = kScale + 5;
+// [sample][32], and the scales of A0's samples (row_scale)
+constexpr int kDA0 = kE + 8 * kHid, kScale = kDA0 + kE, kRows = kScale + 1;
 __host__ __device__ constexpr int a_row(int l) { return l ? kE + (l - 1) * kHid : 0; }
 __host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHid; }
 
@@ -154,9 +148,16 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // The power of two above a row's largest element, whose biased exponent is e
 // (NaN for a row that the slices cannot hold), and its reciprocal.
 __device__ __forceinline__ uint32_t exponent(float m) { return (__float_as_uint(m) >> 23) & 255u; }
-__device__ __forceinline__ float row_scale(uint32_t e, float &inv) {
-  inv = e < 253u ? __uint_as_float((253u - e) << 23) : 0.0f;
+__device__ __forceinline__ float row_scale(uint32_t e) {
   return __uint_as_float(e < 253u ? (e + 1u) << 23 : 0x7fffffffu);
+}
+__device__ __forceinline__ float reciprocal(float scale) {
+  return scale == scale ? __uint_as_float((254u << 23) - __float_as_uint(scale)) : 0.0f;
+}
+__device__ __forceinline__ float row_scale(uint32_t e, float &inv) {
+  const float s = row_scale(e);
+  inv = reciprocal(s);
+  return s;
 }
 
 // Adds the products of three slices each of A (128 rows) and B, K = 16 KS, to
@@ -215,8 +216,6 @@ __device__ __forceinline__ float chain(const float *x, int64_t xs, const float *
   for (int k = 0; k < K; ++k) s = fmaf(x[k * xs], w[k * ws], s);
   return s;
 }
-// A stored value's scale: 1 where the value is stored as it is.
-__device__ __forceinline__ float scale_of(float s) { return s == s ? s : 1.0f; }
 
 // Slices of the weight operands, a block per row.
 __global__ void __launch_bounds__(kHid) slice_weights_kernel(const float *__restrict__ packed,
@@ -301,14 +300,12 @@ __global__ void __launch_bounds__(nsvf_interp::kRunBlock) interp_rows_kernel(con
       e.x = fmaf(w, x[k].x, e.x); e.y = fmaf(w, x[k].y, e.y);
       e.z = fmaf(w, x[k].z, e.z); e.w = fmaf(w, x[k].w, e.w);
     }
-    float m = max_nan(max_nan(fabsf(e.x), fabsf(e.y)), max_nan(fabsf(e.z), fabsf(e.w))), inv;
+    float m = max_nan(max_nan(fabsf(e.x), fabsf(e.y)), max_nan(fabsf(e.z), fabsf(e.w)));
 #pragma unroll
     for (int o = 1; o < kLanes; o <<= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const float sc = row_scale(exponent(m), inv);
-    if (sc != sc) inv = 1.0f;
-    out[ch * 4][sl + i] = e.x * inv; out[ch * 4 + 1][sl + i] = e.y * inv;
-    out[ch * 4 + 2][sl + i] = e.z * inv; out[ch * 4 + 3][sl + i] = e.w * inv;
-    if (ch == 0) scale[sl + i] = sc;
+    out[ch * 4][sl + i] = e.x; out[ch * 4 + 1][sl + i] = e.y;
+    out[ch * 4 + 2][sl + i] = e.z; out[ch * 4 + 3][sl + i] = e.w;
+    if (ch == 0) scale[sl + i] = row_scale(exponent(m));
   }
   __syncthreads();
   const int64_t s = blockIdx.x * (int64_t)kRunSamples;
@@ -537,9 +534,10 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
     const bool live = s0 + row < p.ns;
     {
       sa = es;
+      const float inv = reciprocal(sa);
       uint32_t a[3][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) slice2(e[2 * i], e[2 * i + 1], 1.0f, a[0][i], a[1][i], a[2][i]);
+      for (int i = 0; i < 4; ++i) slice2(e[2 * i], e[2 * i + 1], inv, a[0][i], a[1][i], a[2][i]);
       __syncwarp();
 #pragma unroll
       for (int o = 0; o < 3; ++o)
@@ -561,18 +559,11 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
     auto bit = [](const uint32_t (&m)[2], int j) {
       return (m[j >> 4] >> (((j >> 2) & 3) * 8 + (j & 3))) & 1u;
     };
-    auto store = [&](int first_row, float by) {
+    auto store = [&](int first_row) {
       float *out = R + (first_row + c0) * kTile + row;
 #pragma unroll
-      for (int j = 0; j < kQ; ++j) out[j * kTile] = y[j] * by;
+      for (int j = 0; j < kQ; ++j) out[j * kTile] = y[j];
     };
-    // A_l divided by its scale, and the scale (as it is for the FP32 chains)
-    auto store_a = [&](int l, float inv) {
-      const bool chained = l == 2 || l == 3;
-      store(a_row(l), sa == sa && !chained ? inv : 1.0f);
-      if (quarter == 0) R[(kScale + l) * kTile + row] = chained ? 1.0f : sa;
-    };
-    float inv = 0.0f;                        // 1 / sa
     // Ends a layer: joins the row's quarters and, where `slice`, puts its
     // slices in A. top: the largest |y|, NaN where fix(j) has to give y[j]
     // again (it reads rows of memory written before the barrier). turn: 0 and 1
@@ -594,6 +585,7 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
         }
         sync_and(true);
       }
+      float inv;
       sa = row_scale(max(max(tops[0][row], tops[1][row]), max(tops[2][row], tops[3][row])), inv);
       if (!slice) return true;
       slice_row(tmem_row + kACol + c0 / 2, y, inv);
@@ -604,7 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
     for (int l = 0; l < 4; ++l) {
       uint32_t m[2];
       signs(l, m);
-      if (l) store_a(l, inv);
+      if (l) store(a_row(l));
       finish();
       const float *sc = S.scales + l * kHid + c0, *bias = S.bias + l * kHid + c0;
       float top = 0.0f;
@@ -621,14 +613,13 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
         }
       }
       if (!rows_done(top, l & 1, l < 3, [&](int j) {
-            const float z = fmaf(chain(R + a_row(l) * kTile + row, kTile,
-                                       p.packed + w_off(l) + c0 + j, kHid, l ? kHid : kE),
-                                 scale_of(R[(kScale + l) * kTile + row]), bias[j]);
+            const float z = chain(R + a_row(l) * kTile + row, kTile, p.packed + w_off(l) + c0 + j,
+                                  kHid, l ? kHid : kE) + bias[j];
             return bit(m, j) || z != z ? z : 0.0f;
           }))
         goto out;
     }
-    store_a(4, inv);
+    store(a_row(4));
     // dA4 = d_out W4
     {
       const float4 d = live ? p.d_out[s0 + row] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -661,7 +652,7 @@ __global__ void __launch_bounds__(kThreads, 1) field_bwd_kernel(const BwdParams 
           }))
         goto out;
       const int op = 7 - l;
-      store(dz_row(l), 1.0f);
+      store(dz_row(l));
       if (l == 1 && tile + gridDim.x < tiles) load_e(tile + gridDim.x);
       finish();
       if (l == 0) break;
@@ -719,7 +710,6 @@ constexpr int64_t kPartFloats = kPartChains + (int64_t)2 * kChains * kHid * kHid
 constexpr int kHalfPlane = kHid * 64 * 2;
 struct GradSmem {
   float in[2][kHid * kTile];  // X, Y: rows of 32 16-byte chunks, chunk c at c ^ (row & 7)
-  float scale[kTile];         // of A's samples
   uint8_t y[2][3 * kHalfPlane];
   uint8_t top[2][4][kHid];    // X, Y: the largest exponent in each quarter of a row
   float ys[2][kHid];          // Y's scales, by parity of the tile
@@ -843,8 +833,6 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
         }
       }
     }
-    if (t < kTile / 4)
-      cp_async(S.scale + t * 4, R + (kScale + l) * kTile + t * 4, 16, true);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   // the fetched tile to registers, its scales; the next one on its way
@@ -859,13 +847,8 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const int at = (c >> 2) * 16 + quarter * 4 + (c & 3);
-        float4 a = *reinterpret_cast<const float4 *>(in + ((at ^ (row & 7)) << 2));
-        if (g == (l == 4)) {
-          // dZ (d_out): its sum for db, and times the scale of A's sample
-          s += (a.x + a.y) + (a.z + a.w);
-          const float4 by = *reinterpret_cast<const float4 *>(S.scale + at * 4);
-          a.x *= by.x; a.y *= by.y; a.z *= by.z; a.w *= by.w;
-        }
+        const float4 a = *reinterpret_cast<const float4 *>(in + ((at ^ (row & 7)) << 2));
+        if (g == (l == 4)) s += (a.x + a.y) + (a.z + a.w);   // dZ (d_out): its sum for db
         v[g][c * 4] = a.x; v[g][c * 4 + 1] = a.y; v[g][c * 4 + 2] = a.z; v[g][c * 4 + 3] = a.w;
         m = max_nan(m, max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(a.z), fabsf(a.w))));
       }
@@ -911,14 +894,7 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(int64_t ns,
         for (int i = 0; i < 8; ++i) {
           const int n = c0 + c * 8 + i;
           if (d[i] != d[i] && n < yrows) {
-            const float *y = l == 4 ? Y + n : Y + n * kTile, *by = rows + (tile * kRows + kScale + l) * kTile;
-            const int ys = l == 4 ? 4 : 1;
-            float s = 0.0f;
-#pragma unroll 1
-            for (int k = 0; k < K; ++k)
-              s = l == 4 ? fmaf(X[k] * scale_of(by[k]), y[k * ys], s)
-                         : fmaf(X[k], y[k * ys] * scale_of(by[k]), s);
-            d[i] = s;
+            d[i] = l == 4 ? chain(X, 1, Y + n, 4, K) : chain(X, 1, Y + n * kTile, 1, K);
           }
         }
       }
