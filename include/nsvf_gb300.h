@@ -792,7 +792,10 @@ int nsvf_compact_scan(int64_t n, const uint8_t *hits, int64_t *pix, int64_t *n_h
  *    order) and grad_values (added to, float4 atomics), the activations
  *    recomputed (with the forward's signs) for chunk_samples (a multiple of
  *    128) samples at a time in a workspace of field_train_backward_floats()
- *    floats. A tensor-core wait that runs out sets err bit 3. */
+ *    floats. A tensor-core wait that runs out sets err bit 3;
+ *  - field_train_chain_chunks: the chunks over which the FP32 sums of layers 2
+ *    and 3 go on (64 additions per 128 samples of a block, 76 blocks) before
+ *    they begin anew: at most 9,216 additions, or one chunk. */
 int nsvf_train_rows_count(int64_t rays, int max_steps, const int32_t *sampled_idx, int32_t *count,
                           void *stream);
 int nsvf_train_rows_pack(int64_t rays, int max_steps, const int32_t *sampled_idx, const float *xyz,
@@ -820,6 +823,7 @@ int nsvf_composite_rows_backward(int64_t rays, const int64_t *offset, const floa
                                  const float *grad_missed, float *grad_field, int kahan,
                                  void *stream);
 int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_samples);
+int64_t nsvf_field_train_chain_chunks(int64_t n_samples, int64_t chunk_samples);
 int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
                               const float *xyz_dist, int64_t n_voxels, int64_t n_keys,
                               float voxel_size, const float *centers, const int32_t *feats,

@@ -117,6 +117,7 @@ def _load():
         "nsvf_composite_rows": ([i64, P, P, P, P, f32, P, P, P, i32, P], i32),
         "nsvf_composite_rows_backward": ([i64, P, P, P, P, f32, P, P, P, P, i32, P], i32),
         "nsvf_field_train_backward_floats": ([i64, i64], i64),
+        "nsvf_field_train_chain_chunks": ([i64, i64], i64),
         "nsvf_field_train_backward": ([i64, i64, P, P, i64, i64, f32, P, P, P, P, P, P, P, i64, P,
                                        P, P, P, P], i32),
     }
@@ -165,4 +166,5 @@ def exported_symbols():
         "nsvf_field_train_pack", "nsvf_field_train_forward", "nsvf_composite_rows",
         "nsvf_composite_rows_backward", "nsvf_field_train_backward_floats",
         "nsvf_field_train_backward", "nsvf_field_train_forward_signs",
+        "nsvf_field_train_chain_chunks",
     ]

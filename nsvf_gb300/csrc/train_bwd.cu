@@ -91,10 +91,10 @@ __host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHi
 constexpr int kSplit1 = 64, kSplit0 = 45, kSplit4 = 43;
 static_assert(kSplit1 + kSplit0 + kSplit4 == kSMs, "one block per SM");
 // weight_chain_kernel's blocks of layers 2 and 3 (each), with two chains per
-// element, and the samples of a batch that share a set of chains: about 9,000
-// a chain
+// element, and the longest chain (in additions) that goes on from one chunk into
+// the next: that of an FP32 GEMM over a chunk of 1,024 rays is about 8,700
 constexpr int kChains = kSMs / 2;
-constexpr int64_t kChainSamples = 1400000;
+constexpr int64_t kChainLimit = 9216;
 
 // threads of the two tensor-core kernels that compute; a fifth warpgroup's
 // first lane issues the MMAs. Of the 640 x 96 registers at the launch (61,440)
@@ -984,8 +984,8 @@ static_assert(sizeof(BwdSmem) <= 232448 && sizeof(GradSmem) <= 232448, "shared m
 // Why chains: after a far sample's product an FP32 chain loses those of 2^-24
 // of it and less. In a batch with far samples FP32 GEMMs over chunks of 200k
 // samples (24 chains each) lose up to 3.4e-5 of dW3's and 1.5e-5 of dW2's norm
-// to that, which exact sums do not; these chains are of that length, so that a
-// batch's gradients stay within 1.2e-5 of the GEMM path's (RayChunk), where
+// to that, which exact sums do not; these chains are not longer, and so that a
+// batch's gradients stay near the GEMM path's (RayChunk): within 2e-5, where
 // they were up to 3.4e-5 away with exact sums (12 batches of 8,192 rays).
 // Bound: the FP32 pipe; 256 us for 194,560 samples (50 of its 66 TFLOP/s): 8 x
 // 8 elements a thread and all eight chunks unrolled; 8 x 4 and twice the
@@ -1171,6 +1171,18 @@ int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_sample
   return kFixedFloats + chunk_rows(n_samples, chunk_samples) * kRows;
 }
 
+// A chunk adds as many additions to a chain as half of a block's tiles have
+// samples. As many chunks go on with it as its limit allows, in even parts.
+int64_t nsvf_field_train_chain_chunks(int64_t n_samples, int64_t chunk_samples) {
+  if (n_samples < 0 || chunk_samples < 1) return -1;
+  const int64_t chunks = (n_samples + chunk_samples - 1) / chunk_samples;
+  const int64_t tiles = (chunk_samples + kTile - 1) / kTile;
+  const int64_t most = kChainLimit / ((tiles + kChains - 1) / kChains * (kTile / 2));
+  if (most < 2 || chunks < 2) return 1;
+  const int64_t groups = (chunks + most - 1) / most;
+  return (chunks + groups - 1) / groups;
+}
+
 int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
                               const float *xyz_dist, int64_t n_voxels, int64_t n_keys,
                               float voxel_size, const float *centers, const int32_t *feats,
@@ -1229,11 +1241,8 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
   q.values = (const float4 *)values;
   q.rows = rows;
   q.g_values = (float4 *)grad_values;
-  // the chains begin anew every `group` chunks
   const int64_t chunks = (n_samples + chunk_samples - 1) / chunk_samples;
-  const int64_t groups = n_samples > kChainSamples
-                             ? (n_samples + kChainSamples / 2) / kChainSamples : 1;
-  const int64_t group = chunks > groups ? (chunks + groups - 1) / groups : 1;
+  const int64_t group = nsvf_field_train_chain_chunks(n_samples, chunk_samples);
   int64_t k = 0;                             // chunk
   // (one pass without samples zeroes the slots of an empty batch)
   for (int64_t a = 0; a == 0 || a < n_samples; a += chunk_samples, ++k) {

@@ -482,3 +482,24 @@ def test_small_elements_of_the_gradients(cuda, ns, large, units):
         size_v.index_add_(0, keys[:, k], w[k].abs()[:, None] * dsize)
     for x, b, s in zip([*grads, gv], [*ref, ref_v], [*sizes, size_v]):
         assert bool(((x.double() - b).abs() <= 2.0 ** -16 * s).all())
+
+
+@pytest.mark.parametrize("ns,chunk", [(100000, 640), (1700000, 5 * 304 * 128)])
+def test_weight_chains_of_several_sets(cuda, ns, chunk):
+    """Gradients where the FP32 chains begin anew on the way (chunks of few
+    tiles; more samples than one set takes): at most 9,216 additions round in a
+    chain, as a random walk by 2^-24 each: 2^-17 of the norm."""
+    from nsvf_gb300._lib import LIB
+    assert LIB.nsvf_field_train_chain_chunks(ns, chunk) < -(-ns // chunk)
+    g = torch.Generator().manual_seed(ns)
+    dout = torch.randn(ns, 4, generator=g).to(cuda)
+    (grads, _), (acts, pre, params, _) = _field_grads(cuda, ns, dout, ns, chunk)
+    p64 = [p.double() for p in params]
+    ref = [0] * 10
+    for i in range(0, ns, 250000):
+        s = slice(i, i + 250000)
+        part, _ = _chain_grads([a[s].double() for a in acts], [z[s] for z in pre], p64,
+                               dout[s].double())
+        ref = [r + q for r, q in zip(ref, part)]
+    for a, b in zip(grads, ref):
+        assert float((a.double() - b).norm()) <= 2.0 ** -17 * float(b.norm())
