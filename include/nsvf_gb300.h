@@ -792,7 +792,8 @@ int nsvf_compact_scan(int64_t n, const uint8_t *hits, int64_t *pix, int64_t *n_h
  *    order) and grad_values (added to, float4 atomics), the activations
  *    recomputed (with the forward's signs) for chunk_samples (a multiple of
  *    128) samples at a time in a workspace of field_train_backward_floats()
- *    floats. A tensor-core wait that runs out sets err bit 3;
+ *    floats. A tensor-core wait that runs out sets err bit 3; where that bit is
+ *    set at the end (or was already), all gradients and grad_values are NaN;
  *  - field_train_chain_chunks: the chunks over which the FP32 sums of layers 2
  *    and 3 go on (64 additions per 128 samples of a block, 76 blocks) before
  *    they begin anew: at most 9,216 additions, or one chunk. */

@@ -1111,10 +1111,18 @@ struct GradOut {
 };
 
 // The field's gradients from the slots, each element's slots added in order.
+// NaN, and NaN in grad_values, where a wait ran out (bit 3 of *err): an update
+// with what was summed so far would not be noticed.
 __global__ void __launch_bounds__(kT) grad_reduce_kernel(const float *__restrict__ part,
                                                          const float *__restrict__ bias_part,
-                                                         GradOut out) {
+                                                         GradOut out, float *__restrict__ g_values,
+                                                         int64_t n_values,
+                                                         const int32_t *__restrict__ err) {
   int i = blockIdx.x * kT + threadIdx.x;
+  const bool failed = err && (*err & 8) != 0;
+  const float nan = __int_as_float(0x7fffffff);
+  if (failed)
+    for (int64_t k = i; k < n_values; k += (int64_t)gridDim.x * kT) g_values[k] = nan;
   const float *src;
   float *dst;
   int n, stride;
@@ -1151,7 +1159,7 @@ __global__ void __launch_bounds__(kT) grad_reduce_kernel(const float *__restrict
     c = fabsf(b) <= 3.4e38f ? (b - s) - a : 0.0f;
     s = b;
   }
-  *dst = s;
+  *dst = failed ? nan : s;
 }
 
 // floats of the workspace besides a chunk's rows
@@ -1272,7 +1280,8 @@ int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const in
     if ((st = nsvf_launch_status()) != NSVF_OK) return st;
   }
   constexpr int n_grads = 3 * kHid * kHid + kHid * kE + 8 * kHid + 4;
-  grad_reduce_kernel<<<nsvf_grid(n_grads, kT), kT, 0, s>>>(part, bias_part, g);
+  grad_reduce_kernel<<<nsvf_grid(n_grads, kT), kT, 0, s>>>(
+      part, bias_part, g, grad_values, n_samples > 0 ? n_keys * kE : 0, err);
   return nsvf_launch_status();
 }
 

@@ -503,3 +503,29 @@ def test_weight_chains_of_several_sets(cuda, ns, chunk):
         ref = [r + q for r, q in zip(ref, part)]
     for a, b in zip(grads, ref):
         assert float((a.double() - b).norm()) <= 2.0 ** -17 * float(b.norm())
+
+
+@pytest.mark.parametrize("rays,steps", [(1, 1), (200, 40)])
+def test_gradients_behind_a_wait_that_ran_out_are_nan(cuda, rays, steps):
+    """A wait of the backward that runs out records bit 3 (8) in the error word
+    and leaves partial sums. Set by hand here: every gradient is NaN, so that no
+    optimizer takes them for gradients, and the word still says why; without
+    it the same call gives finite ones."""
+    from nsvf_gb300 import ext, train
+    vs, centers, feats, values, params = _scene(cuda, 20, 1)
+    idx, xyz, dists, depths = _rows(cuda, rays, steps, 20, vs, centers, 3)
+    idx[0, 0] = 4
+    values.requires_grad_(True)
+    for p in params:
+        p.requires_grad_(True)
+    word = ext.error_word(cuda)
+    for bits in (8, 0):
+        word.zero_()
+        out = train.RayBatch.apply(values, *params, idx, xyz, dists, depths, centers, feats, vs,
+                                   False, 1024)
+        word.fill_(bits)
+        grads = torch.autograd.grad(out[0].sum(), [values, *params])
+        assert int(word.item()) == bits
+        word.zero_()
+        for g in grads:
+            assert bool(g.isnan().all()) if bits else bool(g.isfinite().all())
