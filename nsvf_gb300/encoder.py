@@ -349,10 +349,13 @@ class SparseVoxelEncoder(nn.Module):
     @torch.no_grad()
     def pruning_exact(self, mlp, th=0.5, bits=16, use_step=False, apply=True):
         """pruning() on the GPU with the mask decided exactly: the tensor-core
-        BF16 pass screens every point and the points it cannot decide are
-        evaluated in double-float (TensorCoreMLP.prune_mask). The mask is the
-        reference rule's without rounding error. Returns the keep mask over
-        the currently kept voxels (applied to `keep` unless apply=False)."""
+        BF16 pass screens the points, those it cannot decide are evaluated in
+        FP32, and what that cannot decide in double-float
+        (TensorCoreMLP.prune_mask). The mask is the reference rule's without
+        rounding error. Returns the keep mask over the currently kept voxels
+        (applied to `keep` unless apply=False); last_prune_undecided_points is
+        the number of points that the BF16 pass left undecided in voxels it
+        had not kept before it came to them."""
         states = self.precompute(id=None)
         centers = states['voxel_center_xyz'].float().contiguous()
         feats = states['voxel_vertex_idx'].int().contiguous()

@@ -165,7 +165,8 @@ class TensorCoreMLP:
         and the number of points that the BF16 pass left undecided. With
         scores=False (the second result is then None) the BF16 pass first
         takes a few points of every voxel and then all points of the voxels
-        that those do not keep."""
+        that those do not keep; the number is then of the points it left
+        undecided there, each counted once."""
         if not 0.0 < th < 1.0:
             raise ValueError("pruning threshold must lie in (0, 1), got %r" % (th,))
         if rule == 1 and not step > 0.0:
@@ -205,11 +206,12 @@ class TensorCoreMLP:
                     for g, lv, nl in ((sub, None, None), (bits, live, n_live)):
                         if lv is None and bits < 4:
                             continue
+                        # (the second pass lists the first one's points again)
+                        out = (lv.data_ptr(), nl.data_ptr(), lst.data_ptr(), n_list.data_ptr(),
+                               cap) if lv is not None else (None, None, None, None, 0)
                         check(LIB.nsvf_prune_screen_live_bf16(
                             V, int(bits), int(g), int(rule), float(T), float(band), *common,
-                            keep.data_ptr(), lv.data_ptr() if lv is not None else None,
-                            nl.data_ptr() if nl is not None else None, lst.data_ptr(),
-                            n_list.data_ptr(), cap, None, stream), "prune_screen_live_bf16")
+                            keep.data_ptr(), *out, None, stream), "prune_screen_live_bf16")
             n = int(n_list.item())
             if n <= cap:
                 break

@@ -529,3 +529,26 @@ def test_gradients_behind_a_wait_that_ran_out_are_nan(cuda, rays, steps):
         word.zero_()
         for g in grads:
             assert bool(g.isnan().all()) if bits else bool(g.isfinite().all())
+
+
+@pytest.mark.parametrize("n_vox,bits", [(5, 3), (5, 4), (3, 12), (2, 41)])
+def test_undecided_points_are_listed_once(cuda, n_vox, bits):
+    """With a band that leaves every point undecided: each point once, whether
+    the screen goes over all points at once, or over a few of every voxel first
+    and the rest in parts; and no other mask than the narrow band's."""
+    from nsvf_gb300 import ext
+    from nsvf_gb300.field import StandInField
+    from nsvf_gb300.mlp import TensorCoreMLP
+    vs, centers, feats, values, params = _scene(cuda, n_vox, n_vox)
+    params[7] += 1.0                   # active units at every point: M > 0
+    mlp = TensorCoreMLP(StandInField(weights=[(params[2 * l].cpu(), params[2 * l + 1].cpu())
+                                              for l in range(5)]).to(cuda))
+    score = mlp.prune_scores(centers, feats, values, vs, bits=bits, rule=1, step=0.01)
+    th = max(float(score.median()), 1e-6)
+    want = mlp.prune_mask(centers, feats, values, vs, th=th, bits=bits, rule=1, step=0.01)[0]
+    for scores in (True, False):
+        keep, _, n = mlp.prune_mask(centers, feats, values, vs, th=th, bits=bits, rule=1,
+                                    step=0.01, band=1e6, scores=scores)
+        ext.check_errors(cuda)
+        assert n == n_vox * bits ** 3
+        assert torch.equal(keep, want)
