@@ -40,11 +40,25 @@ constexpr int kRayBlock = 128;
 // 706 us, so 30 us and 2 us for the boxes.
 constexpr int kAabbGroup = 32;
 constexpr int kAabbWarps = 8;
-// One group, or up to eight for few rays, do without boxes: their launch costs
-// more than the tests (147 voxels: 4,096 rays 8 us without and 9 us with
-// boxes; 640,000 rays 307 and 201 us, where a thread per ray took 227 us).
+// Up to eight groups do without boxes while there are few rays: their launch
+// costs more than the tests (147 voxels: 4,096 rays 8 us without and 9 us with
+// boxes; 64 voxels: 65,536 rays 23 and 28).
 __host__ __forceinline__ bool aabb_no_boxes(int n, int64_t rays) {
-  return n <= kAabbGroup || (n <= 8 * kAabbGroup && rays <= 16384);
+  return n <= kAabbGroup || (n <= 2 * kAabbGroup && rays < 131072) ||
+         (n <= 8 * kAabbGroup && rays <= 16384);
+}
+// With rays to fill the device several times over, a warp takes 32 of them
+// (aabb_many_kernel). 640,000 rays of a view, 20 slots, in us (a warp per ray;
+// this; a thread per ray without boxes): 33 voxels 171, 60, 175; 147 voxels 202,
+// 86, 227, through random voxels 298, 205, 261, and a list in random order 349,
+// 206, 255; 1,000 voxels 189, 118, 883, random order 304, 255, 884; 1,000
+// without boxes 1,240, 803, 883. With boxes and more than 256 voxels a warp per
+// ray is the faster one up to some 300,000 rays (1,000 voxels, 131,072 rays of a
+// view 42 and 76), except for lists in random order (271 and 228 through random
+// voxels).
+__host__ __forceinline__ bool aabb_many(int n, int64_t rays, bool boxes) {
+  if (n <= 8 * kAabbGroup) return rays >= (boxes ? 131072 : 65536);
+  return rays >= (boxes ? 524288 : 131072);
 }
 
 __device__ __forceinline__ float warp_fmin(float x) {
@@ -82,6 +96,55 @@ __global__ void __launch_bounds__(kAabbWarps * 32) aabb_boxes_kernel(
   }
 }
 
+// One ray's slab tests.
+struct AabbRay {
+  float ox, oy, oz, ix, iy, iz;
+  bool fast;
+
+  __device__ __forceinline__ void load(const float *__restrict__ ray_start,
+                                       const float *__restrict__ ray_dir, int64_t r) {
+    ox = ray_start[r * 3 + 0]; oy = ray_start[r * 3 + 1]; oz = ray_start[r * 3 + 2];
+    ix = nsvf_rcp(ray_dir[r * 3 + 0]); iy = nsvf_rcp(ray_dir[r * 3 + 1]);
+    iz = nsvf_rcp(ray_dir[r * 3 + 2]);
+    fast = isfinite(ix) && isfinite(iy) && isfinite(iz);
+  }
+  __device__ __forceinline__ bool voxel(float cx, float cy, float cz, float hv, float &lo,
+                                        float &hi) const {
+    const float sx = ix >= 0.0f ? 1.0f : -1.0f, sy = iy >= 0.0f ? 1.0f : -1.0f,
+                sz = iz >= 0.0f ? 1.0f : -1.0f;
+    return fast ? nsvf_slab_fast(ox, oy, oz, ix, iy, iz, sx, sy, sz, cx, cy, cz, hv, lo, hi)
+                : nsvf_slab(ox, oy, oz, ix, iy, iz, cx, cy, cz, hv, lo, hi);
+  }
+  // the ray of lane q (the whole warp)
+  __device__ __forceinline__ AabbRay of_lane(int q) const {
+    const uint32_t full = 0xffffffffu;
+    AabbRay o;
+    o.ox = __shfl_sync(full, ox, q); o.oy = __shfl_sync(full, oy, q);
+    o.oz = __shfl_sync(full, oz, q); o.ix = __shfl_sync(full, ix, q);
+    o.iy = __shfl_sync(full, iy, q); o.iz = __shfl_sync(full, iz, q);
+    o.fast = (__ballot_sync(full, fast) >> q) & 1u;
+    return o;
+  }
+  // nsvf_slab_fast's operations on a box's near and far faces; true for every
+  // box where that is not `fast`
+  __device__ __forceinline__ bool box(const float4 &p, const float4 &q) const {
+    const float nx = ix >= 0.0f ? p.x : -p.w, fx = ix >= 0.0f ? -p.w : p.x;
+    const float ny = iy >= 0.0f ? p.y : -q.x, fy = iy >= 0.0f ? -q.x : p.y;
+    const float nz = iz >= 0.0f ? p.z : -q.y, fz = iz >= 0.0f ? -q.y : p.z;
+    float lo = 0.0f, hi = 100000.0f, u;
+    lo = fmaxf(lo, __fadd_rn(__fmul_rn(__fsub_rn(nx, ox), ix), 0.0f));
+    u = __fmul_rn(__fsub_rn(fx, ox), ix);
+    hi = (u < hi) ? u : hi;
+    lo = fmaxf(lo, __fadd_rn(__fmul_rn(__fsub_rn(ny, oy), iy), 0.0f));
+    u = __fmul_rn(__fsub_rn(fy, oy), iy);
+    hi = (u < hi) ? u : hi;
+    lo = fmaxf(lo, __fadd_rn(__fmul_rn(__fsub_rn(nz, oz), iz), 0.0f));
+    u = __fmul_rn(__fsub_rn(fz, oz), iz);
+    hi = (u < hi) ? u : hi;
+    return !fast || !(lo > hi);
+  }
+};
+
 __global__ void __launch_bounds__(kAabbWarps * 32) aabb_kernel(
     int64_t rays, int m, int b_pts, int n, float hv, int n_max,
     const float *__restrict__ ray_start, const float *__restrict__ ray_dir,
@@ -95,42 +158,19 @@ __global__ void __launch_bounds__(kAabbWarps * 32) aabb_kernel(
   const int groups = (n + kAabbGroup - 1) / kAabbGroup;
   const int64_t set = b_pts == 1 ? 0 : r / m;
   const float *P = points + set * n * 3;
-  const float ox = ray_start[r * 3 + 0], oy = ray_start[r * 3 + 1], oz = ray_start[r * 3 + 2];
-  const float ix = nsvf_rcp(ray_dir[r * 3 + 0]), iy = nsvf_rcp(ray_dir[r * 3 + 1]),
-              iz = nsvf_rcp(ray_dir[r * 3 + 2]);
-  const bool fast = isfinite(ix) && isfinite(iy) && isfinite(iz);
-  const float sx = ix >= 0.0f ? 1.0f : -1.0f, sy = iy >= 0.0f ? 1.0f : -1.0f,
-              sz = iz >= 0.0f ? 1.0f : -1.0f;
+  AabbRay ray;
+  ray.load(ray_start, ray_dir, r);
   auto voxel = [&](int k, float &lo, float &hi) {
-    if (k >= n) return false;
-    const float cx = P[(int64_t)k * 3], cy = P[(int64_t)k * 3 + 1], cz = P[(int64_t)k * 3 + 2];
-    return fast ? nsvf_slab_fast(ox, oy, oz, ix, iy, iz, sx, sy, sz, cx, cy, cz, hv, lo, hi)
-                : nsvf_slab(ox, oy, oz, ix, iy, iz, cx, cy, cz, hv, lo, hi);
-  };
-  // nsvf_slab_fast's operations on a box's near and far faces
-  auto box = [&](int64_t g) {
-    const float4 p = boxes[g * 2], q = boxes[g * 2 + 1];
-    const float nx = sx > 0.0f ? p.x : -p.w, fx = sx > 0.0f ? -p.w : p.x;
-    const float ny = sy > 0.0f ? p.y : -q.x, fy = sy > 0.0f ? -q.x : p.y;
-    const float nz = sz > 0.0f ? p.z : -q.y, fz = sz > 0.0f ? -q.y : p.z;
-    float lo = 0.0f, hi = 100000.0f, u;
-    lo = fmaxf(lo, __fadd_rn(__fmul_rn(__fsub_rn(nx, ox), ix), 0.0f));
-    u = __fmul_rn(__fsub_rn(fx, ox), ix);
-    hi = (u < hi) ? u : hi;
-    lo = fmaxf(lo, __fadd_rn(__fmul_rn(__fsub_rn(ny, oy), iy), 0.0f));
-    u = __fmul_rn(__fsub_rn(fy, oy), iy);
-    hi = (u < hi) ? u : hi;
-    lo = fmaxf(lo, __fadd_rn(__fmul_rn(__fsub_rn(nz, oz), iz), 0.0f));
-    u = __fmul_rn(__fsub_rn(fz, oz), iz);
-    hi = (u < hi) ? u : hi;
-    return !(lo > hi);
+    return k < n && ray.voxel(P[(int64_t)k * 3], P[(int64_t)k * 3 + 1], P[(int64_t)k * 3 + 2], hv,
+                              lo, hi);
   };
   int32_t *I = idx + r * n_max;
   float *LO = min_depth + r * n_max, *HI = max_depth + r * n_max;
   int cnt = 0;
   for (int g0 = 0; g0 < groups && cnt < n_max; g0 += 32) {
+    const int64_t g = set * groups + g0 + lane;
     const bool in = g0 + lane < groups;
-    uint32_t gm = __ballot_sync(full, in && (!boxes || !fast || box(set * groups + g0 + lane)));
+    uint32_t gm = __ballot_sync(full, in && (!boxes || ray.box(boxes[g * 2], boxes[g * 2 + 1])));
     while (gm && cnt < n_max) {
       // two groups at a time: their loads are independent
       const int ga = g0 + __ffs(gm) - 1;
@@ -148,6 +188,89 @@ __global__ void __launch_bounds__(kAabbWarps * 32) aabb_kernel(
     }
   }
   for (int l = cnt + lane; l < n_max; l += 32) { I[l] = -1; LO[l] = 0.0f; HI[l] = 0.0f; }
+}
+
+// The same for many rays, 32 per warp: each lane tests its ray against a group's
+// box. Where few rays hit it, they are taken one by one, a lane per voxel as
+// above; otherwise all at once, a lane per ray, which needs no ballots and loads
+// a voxel once for 32 rays. The rest of the rows is filled by the warp, row by
+// row.
+constexpr int kAabbManyWarps = 4;
+constexpr int kAabbFew = 20;                 // (a ray alone takes about 43 instructions, all 32 1,056)
+__global__ void __launch_bounds__(kAabbManyWarps * 32) aabb_many_kernel(
+    int64_t rays, int m, int b_pts, int n, float hv, int n_max,
+    const float *__restrict__ ray_start, const float *__restrict__ ray_dir,
+    const float *__restrict__ points, const float4 *__restrict__ boxes, int32_t *__restrict__ idx,
+    float *__restrict__ min_depth, float *__restrict__ max_depth) {
+  __shared__ float4 tile[kAabbManyWarps][kAabbGroup];
+  const uint32_t full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t below = (1u << lane) - 1u;
+  float4 *V = tile[threadIdx.x >> 5];
+  // a warp's rays are of one point set
+  const int64_t per_row = b_pts == 1 ? rays : m, warps = (per_row + 31) / 32;
+  const int64_t w = blockIdx.x * (int64_t)kAabbManyWarps + (threadIdx.x >> 5);
+  const int64_t set = w / warps, in_row = w % warps * 32;
+  if (set * per_row >= rays) return;
+  const int64_t r0 = set * per_row + in_row;
+  const int n_rays = per_row - in_row < 32 ? (int)(per_row - in_row) : 32;
+  const int groups = (n + kAabbGroup - 1) / kAabbGroup;
+  const float *P = points + set * n * 3;
+  const int64_t r = r0 + (lane < n_rays ? lane : 0);
+  AabbRay ray;
+  ray.load(ray_start, ray_dir, r);
+  int cnt = lane < n_rays ? 0 : n_max;
+  for (int g = 0; g < groups; ++g) {
+    bool go = cnt < n_max;
+    if (__all_sync(full, !go)) break;
+    if (boxes) {
+      const float4 p = __ldg(boxes + (set * groups + g) * 2);
+      const float4 q = __ldg(boxes + (set * groups + g) * 2 + 1);
+      go = go && ray.box(p, q);
+    }
+    uint32_t who = __ballot_sync(full, go);
+    if (who == 0) continue;
+    const int k0 = g * kAabbGroup, len = n - k0 < kAabbGroup ? n - k0 : kAabbGroup;
+    float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < len) {
+      const float *c = P + (int64_t)(k0 + lane) * 3;
+      mine = make_float4(c[0], c[1], c[2], 0.0f);
+    }
+    if (boxes && __popc(who) <= kAabbFew) {
+      for (; who; who &= who - 1) {
+        const int q = __ffs(who) - 1;
+        const AabbRay one = ray.of_lane(q);
+        const int at0 = __shfl_sync(full, cnt, q);
+        float lo, hi;
+        const bool hit = one.voxel(mine.x, mine.y, mine.z, hv, lo, hi) && lane < len;
+        const uint32_t hm = __ballot_sync(full, hit);
+        const int pos = at0 + __popc(hm & below);
+        if (hit && pos < n_max) {
+          const int64_t at = (r0 + q) * n_max + pos;
+          idx[at] = k0 + lane; min_depth[at] = lo; max_depth[at] = hi;
+        }
+        if (lane == q) cnt = min(n_max, cnt + __popc(hm));
+      }
+      continue;
+    }
+    __syncwarp();                            // the last group's voxels are done with
+    V[lane] = mine;
+    __syncwarp();
+    for (int k = 0; k < len; ++k) {
+      const float4 c = V[k];
+      float lo, hi;
+      if (ray.voxel(c.x, c.y, c.z, hv, lo, hi) && cnt < n_max) {
+        const int64_t at = r * n_max + cnt;
+        idx[at] = k0 + k; min_depth[at] = lo; max_depth[at] = hi;
+        ++cnt;
+      }
+    }
+  }
+  for (int q = 0; q < n_rays; ++q)
+    for (int l = __shfl_sync(full, cnt, q) + lane; l < n_max; l += 32) {
+      const int64_t at = (r0 + q) * n_max + l;
+      idx[at] = -1; min_depth[at] = 0.0f; max_depth[at] = 0.0f;
+    }
 }
 
 // ----------------------------------------------------------------- SVO ----
@@ -1024,9 +1147,16 @@ static int aabb_launch(int b, int b_pts, int n, int m, float voxelsize, int n_ma
         b_pts, n, voxelsize * 0.5f, points, boxes);
     nsvf_count_launch();
   }
-  aabb_kernel<<<(int)grid, kAabbWarps * 32, 0, s>>>(rays, m, b_pts, n, voxelsize * 0.5f, n_max,
-                                                    ray_start, ray_dir, points, boxes, idx,
-                                                    min_depth, max_depth);
+  if (aabb_many(n, rays, boxes != nullptr)) {
+    const int64_t per_row = b_pts == 1 ? rays : m, warps = rays / per_row * ((per_row + 31) / 32);
+    aabb_many_kernel<<<nsvf_grid(warps, kAabbManyWarps), kAabbManyWarps * 32, 0, s>>>(
+        rays, m, b_pts, n, voxelsize * 0.5f, n_max, ray_start, ray_dir, points, boxes, idx,
+        min_depth, max_depth);
+  } else {
+    aabb_kernel<<<(int)grid, kAabbWarps * 32, 0, s>>>(rays, m, b_pts, n, voxelsize * 0.5f, n_max,
+                                                      ray_start, ray_dir, points, boxes, idx,
+                                                      min_depth, max_depth);
+  }
   return nsvf_launch_status();
 }
 

@@ -569,3 +569,41 @@ def test_aabb_boxes_equal_oracle(cuda, n, order):
         out = ext.aabb_intersect(_t(o, cuda), _t(d, cuda), _t(pts[None], cuda), vs, n_max)
         for a, b in zip(out, ref):
             assert np.array_equal(_np(a), b)
+
+
+@pytest.mark.parametrize("n,b,m", [(1, 1, 65536), (33, 1, 65539), (64, 2, 65537), (65, 1, 131072),
+                                   (256, 2, 65567), (257, 1, 131075), (257, 1, 524289)])
+def test_aabb_many_rays_equal_oracle(cuda, n, b, m):
+    """From 65,536 rays on a warp takes 32 rays: the oracle's hits at the edges
+    of the rule, for rays that do not fill the last warp of a set, sets of
+    their own, lists in grid and in random order, with NaN and infinite
+    centres, rays along the axes, and rows that fill up."""
+    from nsvf_gb300 import ext
+    from nsvf_gb300._lib import LIB, check
+    rng = np.random.RandomState(n + m)
+    vs = 0.05
+    g = np.stack(np.meshgrid(*[np.arange(-8, 9)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    sets = np.stack([g[np.linalg.norm(g, axis=1) < 8][:n], g[rng.permutation(len(g))[:n]]])
+    pts = (sets[:b] if m % 2 else sets[1:][:b]).astype(np.float32) * np.float32(vs)
+    pts[:, 7::37, 0] = np.nan
+    pts[:, 5::41, 1] = np.inf
+    o = rng.uniform(-0.6, 0.6, (b, m, 3)).astype(np.float32)
+    d = rng.normal(size=(b, m, 3)).astype(np.float32)
+    d[:, 1::3] = rng.normal(size=(b, 1, 3)) + 0.1 * d[:, 1::3]      # (much the same way)
+    d /= np.linalg.norm(d, axis=-1, keepdims=True)
+    d[:, ::7, rng.randint(3)] = 0.0
+    d[:, 1::11] = np.float32([0, 0, -1])
+    o[:, 2::9] = np.round(o[:, 2::9] / (vs / 2)) * np.float32(vs / 2)
+    od, dd, pd = (_t(x, cuda) for x in (o, d, pts))
+    for n_max in (1, 20):
+        ref = cpu.aabb_intersect(o, d, pts, vs, n_max)
+        for a, r in zip(ext.aabb_intersect(od, dd, pd, vs, n_max), ref):
+            assert np.array_equal(_np(a), r)
+        # the C entry without boxes
+        out = [torch.full((b, m, n_max), 7, dtype=t, device=cuda)
+               for t in (torch.int32, torch.float32, torch.float32)]
+        check(LIB.nsvf_aabb_intersect(b, b, n, m, vs, n_max, od.data_ptr(), dd.data_ptr(),
+                                      pd.data_ptr(), *(t.data_ptr() for t in out),
+                                      ext.ctypes_stream(cuda)), "aabb_intersect")
+        for a, r in zip(out, ref):
+            assert np.array_equal(_np(a), r)
