@@ -28,3 +28,20 @@ def test_chain_chunks_rejects_what_the_backward_does():
     from nsvf_gb300._lib import LIB
     assert LIB.nsvf_field_train_chain_chunks(-1, 128) == -1
     assert LIB.nsvf_field_train_chain_chunks(5, 0) == -1
+
+
+@pytest.mark.parametrize("ns,rays,chunk_rays,want", [
+    (0, 0, 1024, 128), (1, 1, 1, 128), (1000, 10, 1, 128), (1300, 10, 1, 256),
+    (WAVE // 2 * 8, 8, 1, WAVE), (WAVE // 2 * 8 - 8, 8, 1, WAVE // 2),
+    (340000, 2048, 64, 84 * 128), (1400000, 8192, 1024, 4 * WAVE), (1400000, 8192, 8192, 36 * WAVE)])
+def test_backward_chunk_follows_chunk_rays(ns, rays, chunk_rays, want):
+    """A caller who lowers chunk_rays gets a chunk, and a workspace, as much
+    smaller; from half a wave of the GPU on the chunk is whole waves."""
+    from nsvf_gb300 import train
+    from nsvf_gb300._lib import LIB
+    chunk = train.chunk_samples(ns, rays, chunk_rays)
+    assert chunk == want
+    n = ns * chunk_rays / max(rays, 1)
+    assert chunk <= max(2 * n, n + 128)
+    fixed = LIB.nsvf_field_train_backward_floats(0, 128)
+    assert LIB.nsvf_field_train_backward_floats(ns, chunk) - fixed <= 1100 * min(chunk, ns + 128)
