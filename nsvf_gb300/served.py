@@ -153,7 +153,6 @@ def _frame_buffers(scene, R, stream):
          "probs": e(R, H), "steps": e(R), "count": e(R, dtype=i32),
          "offset": off[:R + 1], "counts": off[R:R + 5], "zero": off[R:], "scan_words": off[R + 5:],
          "scan_ws": torch.empty(int(LIB.nsvf_sample_scan_bytes(R)), dtype=torch.uint8, device=dev),
-         "ws": ext._svo_workspace(1, scene.octree_centers.shape[0], dev),
          "bg": torch.tensor(list(scene.bg), dtype=torch.float32, device=dev),
          "err": off[R + 4:R + 5].view(i32)[:1],
          "counts_host": torch.zeros(5, dtype=i64).pin_memory(), "cap": 0,
@@ -389,6 +388,8 @@ def render_frame(scene, ray_start, ray_dir, kahan=True, out=None, mlp="tc", exac
             scene.svo_grid.intersect_into(R, H, _p(ro), _p(rd), _p(b["idx"]), _p(b["lo"]),
                                           _p(b["hi"]), _p(b["hits"]), stream, padded=False)
     else:
+        if "ws" not in b:                    # the leaf grid needs none
+            b["ws"] = ext._svo_workspace(1, n_nodes, dev)
         with ext._timed("svo_intersect_sorted", dev):
             check(LIB.nsvf_svo_intersect_sorted(1, 1, n_nodes, R, scene.voxel_size, H, _p(ro),
                                                 _p(rd), _p(scene.octree_centers),

@@ -449,3 +449,21 @@ def test_frame_outputs_in_other_forms(cuda):
     for o in (a, b):
         for k in ("colors", "depths", "missed"):
             assert torch.equal(o[k], ref[k])
+
+
+def test_traversal_workspace_only_where_it_is_used(cuda):
+    """Frames through the leaf grid hold no workspace of the depth-first
+    traversal (228 bytes a node); frames that ask for that traversal do, and
+    are the same."""
+    from nsvf_gb300 import scenes
+    from nsvf_gb300.served import SceneState, render_frame
+    enc, field, _, _ = _scene(cuda, 0.25, 1.0, 60.0, 0.5, 20)
+    sc = SceneState(enc, field)
+    rs, rd = (torch.from_numpy(a).to(cuda) for a in scenes.small_view(0))
+    assert sc.svo_grid.ok
+    a = render_frame(sc, rs, rd)
+    assert all("ws" not in b for b in sc._frames.values())
+    b = render_frame(sc, rs, rd, traversal="dfs")
+    assert all("ws" in b for b in sc._frames.values())
+    for k in ("colors", "depths", "missed"):
+        assert torch.equal(a[k], b[k])
