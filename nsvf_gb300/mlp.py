@@ -39,6 +39,9 @@ class TensorCoreMLP:
         # samples far outside their voxel (nsvf_field_exact_dev)
         self.wt32 = [w.t().contiguous() for w in self.w32]
         self._wtp = (ctypes.c_void_p * 5)(*[t.data_ptr() for t in self.wt32])
+        # the same copies as [out, in], for pruning's FP32 stage
+        self.wc32 = [t.t().contiguous() for t in self.wt32]
+        self._wcp = (ctypes.c_void_p * 5)(*[t.data_ptr() for t in self.wc32])
         self.fp8 = None
 
     E4M3_MAX = 448.0
@@ -148,8 +151,11 @@ class TensorCoreMLP:
     # 0.005 M (c2 pruning field, 768k points), so 0.02 leaves a factor 4.
     PRUNE_BAND = 0.02
 
-    # The FP32 pass's band is PRUNE_BAND / 64 (nsvf_prune_fp32_dev).
+    # The FP32 pass's band is PRUNE_BAND / 64 (nsvf_prune_fp32_dev). Up to
+    # FP32_FROM points go to double-float at once: these take less than the
+    # launches and buffers before them.
     FP32_BAND = 64.0
+    FP32_FROM = 512
 
     def prune_mask(self, centers, feats, values, voxel_size, th=0.5, bits=8, rule=1, step=0.0,
                    band=PRUNE_BAND, scores=True):
@@ -219,13 +225,11 @@ class TensorCoreMLP:
         # double-float costs about 60 times FP32 a point (131 against 2.2 us per
         # thousand), so FP32 decides what it can first: the c2 pass's 23.0 ms
         # of double-float become 0.39 ms of FP32 and 0.07 ms
-        if n and band > 0.0 and 1e-30 < T < 1e30:
-            # the weights of the double-float pass, as they are laid out there
-            w = [t.t().contiguous() for t in self.wt32]
+        if n > self.FP32_FROM and band > 0.0 and 1e-30 < T < 1e30:
+            # (the weights of the double-float pass)
             packed = torch.empty(int(LIB.nsvf_field_train_packed_floats()), dtype=torch.float32,
                                  device=dev)
-            check(LIB.nsvf_field_train_pack((ctypes.c_void_p * 5)(*[t.data_ptr() for t in w]),
-                                            self._bp, packed.data_ptr(), stream),
+            check(LIB.nsvf_field_train_pack(self._wcp, self._bp, packed.data_ptr(), stream),
                   "field_train_pack")
             live = torch.empty(cap, dtype=torch.int64, device=dev)
             n_live = torch.zeros(1, dtype=torch.int64, device=dev)

@@ -552,3 +552,29 @@ def test_undecided_points_are_listed_once(cuda, n_vox, bits):
         ext.check_errors(cuda)
         assert n == n_vox * bits ** 3
         assert torch.equal(keep, want)
+
+
+@pytest.mark.parametrize("n_vox,bits", [(65535, 4), (65536, 4), (12300, 7), (66, 40), (62, 41)])
+def test_prune_of_many_points_in_parts_keeps_the_mask(cuda, n_vox, bits):
+    """From 4 M points on the screen of all points goes in four parts (4 to 40
+    points per axis): the mask of the screen in one pass, with undecided points
+    on both sides of the number from which FP32 comes before double-float."""
+    from nsvf_gb300 import ext
+    from nsvf_gb300.field import StandInField
+    from nsvf_gb300.mlp import TensorCoreMLP
+    vs, centers, feats, values, params = _scene(cuda, n_vox, n_vox)
+    mlp = TensorCoreMLP(StandInField(weights=[(params[2 * l].cpu(), params[2 * l + 1].cpu())
+                                              for l in range(5)]).to(cuda))
+    score = mlp.prune_scores(centers, feats, values, vs, bits=bits, rule=1, step=0.01)
+    seen = []
+    for th in (float(score.median()), float(score.max()) * 0.999):
+        keep = []
+        for band in (0.02, 1e-4):
+            for s in (True, False):
+                k, _, n = mlp.prune_mask(centers, feats, values, vs, th=max(th, 1e-6), bits=bits,
+                                         rule=1, step=0.01, band=band, scores=s)
+                keep.append(k)
+                seen.append(n > mlp.FP32_FROM)
+            assert torch.equal(keep[-1], keep[-2])
+        ext.check_errors(cuda)
+    assert any(seen) and not all(seen)
