@@ -242,8 +242,8 @@ def prune_bench(dev, sc, bits=8, th=0.5):
         torch.cuda.synchronize(dev)
         fp32_ms.append(s1.elapsed_time(e1))
     keep_fp32 = alpha >= th
-    # the exact pass: BF16 screen with the error scale M, double-float
-    # evaluation of the undecided points (TensorCoreMLP.prune_mask)
+    # the exact pass: BF16 screen with the error scale M, FP32 evaluation of the
+    # undecided points, double-float of what that leaves (TensorCoreMLP.prune_mask)
     mlp.prune_mask(centers[:256], feats[:256], values, vs, th=th, bits=bits, rule=1, step=step)
     torch.cuda.synchronize(dev)
     ex_ms = []
@@ -258,8 +258,9 @@ def prune_bench(dev, sc, bits=8, th=0.5):
     return {"workload": "c2 pruning pass: %d voxels x %d^3 points, keep max(1-exp(-relu(s)*step)) >= %g; "
                         "density row of the field scaled by %g" % (V, bits, th, PRUNE_SIGMA_SCALE),
             "exact_ms": round(min(ex_ms), 3),
-            "exact_path": "BF16 tensor-core screen (error scale M = sum |W4[0]| h) + double-float "
-                          "evaluation of the undecided points; mask of the rule without rounding error",
+            "exact_path": "BF16 tensor-core screen (error scale M = sum |W4[0]| h) + FP32 and then "
+                          "double-float evaluation of the undecided points; mask of the rule without "
+                          "rounding error",
             "undecided_points": n_undecided, "points": V * bits ** 3,
             "kept_exact": int(keep_exact.sum()),
             "mask_mismatches_exact_vs_fp32": int((keep_exact != keep_fp32).sum()),

@@ -761,7 +761,7 @@ int nsvf_prune_exact_dev(int64_t n_voxels, int bits, int rule, double threshold,
  * zeros into zero_words 8-byte words.
  * compact_scan: nsvf_compact_hits without a prefix sum to prepare: pix and
  * *n_hit from the flags in one pass; ws: nsvf_compact_scan_words(n) 8-byte
- * words, zeroed by the caller (bit 8 of *err: a bounded wait gave up). */
+ * words, zeroed by the caller (bit 3 (8) of *err: a bounded wait gave up). */
 int nsvf_frame_begin(int64_t n, const float bg[3], float bg_depth, float *color, float *depth,
                      float *missed, const float *origin, float *ray_start, void *zero,
                      int64_t zero_words, void *stream);

@@ -35,8 +35,8 @@
 // over chunks leave up to 3.4e-5 of the norm; layers 2 and 3, where that is more
 // than 1e-5, are summed as the GEMMs sum them (weight_chain_kernel).
 //
-// Measured on 1.40 M samples: 5.7 ms (the interpolation 0.3, field_bwd_kernel 2.5,
-// weight_chain_kernel 1.8, weight_grad_kernel 1.1; all on the FP32 pipe took
+// Measured on 1.40 M samples: 5.5 ms (the interpolation 0.3, field_bwd_kernel 2.4,
+// weight_chain_kernel 1.8, weight_grad_kernel 1.0; all on the FP32 pipe took
 // 6.7 + 2.7 ms, at 41 and 50 of the pipe's 66 TFLOP/s).
 //
 // field_bwd_kernel: a tile of 128 samples per block and one block per SM: the
@@ -46,11 +46,11 @@
 // to tensor memory as the next layer's A operand, which leaves shared memory
 // for the weights of two layers. The layer inputs A_l and the gradients dZ_l
 // go to memory as [unit][sample] of a tile (every store a whole line), beside
-// the MMAs. Bound: the chain MMA (340 of 64 cycles) -> epilogue (1.7-2.2k) ->
-// slices (1.7-2.1k) of the one tile that fits an SM, eight times a tile, 64k
+// the MMAs. Bound: the chain MMA (340 of 64 cycles) -> epilogue -> slices (about
+// 2k cycles each) of the one tile that fits an SM, eight times a tile, 61k
 // cycles; the stores fill the MMAs' time (64 KB a layer at 27 bytes a cycle).
-// A lane of the computing warps as the issuer: 3.3 ms, behind its warp's share
-// of the stores.
+// A lane of the computing warps as the issuer: 0.8 ms more, behind its warp's
+// share of the stores.
 // weight_grad_kernel (layers 0, 1 and the head): dW_l = dZ_l^T A_l, db_l = sum
 // dZ_l: K runs over the 128 samples of a tile, rows are units. FP32 accumulation
 // over tiles in registers, one slot per block, the slots added in a fixed order.
@@ -85,9 +85,9 @@ constexpr int kDA0 = kE + 8 * kHid, kScale = kDA0 + kE, kRows = kScale + 1;
 __host__ __device__ constexpr int a_row(int l) { return l ? kE + (l - 1) * kHid : 0; }
 __host__ __device__ constexpr int dz_row(int l) { return kE + 4 * kHid + l * kHid; }
 
-// weight_grad_kernel's blocks, in proportion to a tile's time: layer 1 (15k
-// cycles), layer 0 (10.5k) and the head (10k: an MMA of 16 columns takes 45 of
-// the 64 cycles that one of 128 takes).
+// weight_grad_kernel's blocks, in proportion to a tile's time: layer 1 (11k
+// cycles), layer 0 (0.70 of that) and the head (0.67: an MMA of 16 columns takes
+// 45 of the 64 cycles that one of 128 takes).
 constexpr int kSplit1 = 64, kSplit0 = 45, kSplit4 = 43;
 static_assert(kSplit1 + kSplit0 + kSplit4 == kSMs, "one block per SM");
 // weight_chain_kernel's blocks of layers 2 and 3 (each), with two chains per

@@ -151,9 +151,11 @@ class TensorCoreMLP:
     # 0.005 M (c2 pruning field, 768k points), so 0.02 leaves a factor 4.
     PRUNE_BAND = 0.02
 
-    # The FP32 pass's band is PRUNE_BAND / 64 (nsvf_prune_fp32_dev). Up to
-    # FP32_FROM points go to double-float at once: these take less than the
-    # launches and buffers before them.
+    # The FP32 pass's band is PRUNE_BAND / 64 (nsvf_prune_fp32_dev), 3.1e-4 M:
+    # FP32's error of sigma is at most 3.4e-7 M and BF16's 6.5e-3 M (twelve shell
+    # and ball fields of 24,000 to 4 M points), so where the screen's band holds,
+    # this one does. Up to FP32_FROM points go to double-float at once: these
+    # take less than the launches and buffers before them.
     FP32_BAND = 64.0
     FP32_FROM = 512
 

@@ -5,8 +5,8 @@ The reference trains through autograd and keeps every ray chunk's graph
 alive until the loss's backward (fairnr/modules/renderer.py:135-232): the
 [samples, 8, 32] corner gathers and every MLP activation of the whole batch.
 Here `RayBatch` is one torch.autograd.Function per batch of rays that keeps
-its compacted samples (voxel ids, positions, depths, lengths: 28 bytes each),
-their field values and the signs of their pre-activations (64 bytes). Its
+its compacted samples (voxel ids, positions, depths, lengths: 24 bytes each),
+their field values (16) and the signs of their pre-activations (64). Its
 backward runs
 
   compositing backward     nsvf_composite_rows_backward (transmittance prefix
