@@ -727,10 +727,10 @@ int nsvf_prune_screen_bf16(int64_t n_voxels, int bits, int rule, float step, flo
  * sub == bits) and, with `live` (int32 [n_voxels], n_live one int64), only for
  * the voxels that keep does not hold yet (all their points: in parts, each on
  * the voxels that the part before left; live and n_live then hold the last
- * part's). Without `live` n_list may be NULL: nothing is listed. Two calls, a
- * few points of every voxel with no list and then all points of the rest, set
- * the same keep flags and list the undecided points of every voxel not kept,
- * each once (and some of voxels kept by a part that came with them or later). */
+ * part's). Two calls, a few points of every voxel with list_cap 0 (nothing is
+ * listed, *n_list counts) and then all points of the rest, set the same keep
+ * flags and list the undecided points of every voxel not kept, each once (and
+ * some of voxels kept by a part that came with them or later). */
 int nsvf_prune_screen_live_bf16(int64_t n_voxels, int bits, int sub, int rule, float threshold,
                                 float band, int64_t n_keys, float voxel_size,
                                 const float *centers, const int32_t *feats, const float *values,

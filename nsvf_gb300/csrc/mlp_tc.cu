@@ -573,7 +573,7 @@ __device__ __forceinline__ void head_store(const MlpParams &p, const float *bias
       const float M = v[4];
       const float lo = sigma - p.prune_c * M, hi = sigma + p.prune_c * M;
       const bool certain = live && (p.rule == 1 ? lo >= p.prune_T : lo > p.prune_T);
-      const bool maybe = live && !certain && hi >= p.prune_T && p.n_plist;
+      const bool maybe = live && !certain && hi >= p.prune_T;
       if (MODE == kScreen && (certain || maybe)) {
         int point;
         screen_row(p, r, vv, point);
@@ -588,7 +588,7 @@ __device__ __forceinline__ void head_store(const MlpParams &p, const float *bias
         base = __shfl_sync(0xffffffffu, base, leader);
         if (maybe) {
           const unsigned long long k = base + __popc(m & ((1u << lane) - 1u));
-          if ((int64_t)k < p.plist_cap) p.plist[k] = r;
+          if (k < (unsigned long long)p.plist_cap) p.plist[k] = r;   // (any count)
           else if (p.err) atomicOr(p.err, 16);
         }
       }
@@ -1194,7 +1194,7 @@ int nsvf_prune_screen_live_bf16(int64_t n_voxels, int bits, int sub, int rule, f
     return NSVF_ERR_INVALID;
   if (n_voxels == 0) return NSVF_OK;
   MlpParams p = {};
-  if (!centers || !feats || !values || !keep || (live && !n_list) || (list_cap > 0 && !list) ||
+  if (!centers || !feats || !values || !keep || !n_list || (list_cap > 0 && !list) ||
       !set_weights(p, weights, biases))
     return NSVF_ERR_INVALID;
   if ((((uintptr_t)values) | ((uintptr_t)feats)) & 15) return NSVF_ERR_INVALID;

@@ -196,7 +196,7 @@ class TensorCoreMLP:
         # 4 points per axis 87 %)
         sub = 4 if bits >= 12 else 2
         live = torch.empty(V, dtype=torch.int32, device=dev) if not scores else None
-        n_live = torch.empty(1, dtype=torch.int64, device=dev) if not scores else None
+        n_live = torch.zeros(1, dtype=torch.int64, device=dev) if not scores else None
         common = (values.size(0), float(voxel_size), centers.data_ptr(), feats.data_ptr(),
                   values.data_ptr(), self._wp, self._bp)
         for _ in range(3):
@@ -214,9 +214,11 @@ class TensorCoreMLP:
                     for g, lv, nl in ((sub, None, None), (bits, live, n_live)):
                         if lv is None and bits < 4:
                             continue
-                        # (the second pass lists the first one's points again)
+                        # the first pass lists nothing (the second one goes
+                        # over its points again) and counts into n_live, which
+                        # the second one sets anew
                         out = (lv.data_ptr(), nl.data_ptr(), lst.data_ptr(), n_list.data_ptr(),
-                               cap) if lv is not None else (None, None, None, None, 0)
+                               cap) if lv is not None else (None, None, None, n_live.data_ptr(), 0)
                         check(LIB.nsvf_prune_screen_live_bf16(
                             V, int(bits), int(g), int(rule), float(T), float(band), *common,
                             keep.data_ptr(), *out, None, stream), "prune_screen_live_bf16")
