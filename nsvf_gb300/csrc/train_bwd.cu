@@ -984,9 +984,11 @@ static_assert(sizeof(BwdSmem) <= 232448 && sizeof(GradSmem) <= 232448, "shared m
 // Why chains: after a far sample's product an FP32 chain loses those of 2^-24
 // of it and less. In a batch with far samples FP32 GEMMs over chunks of 200k
 // samples (24 chains each) lose up to 3.4e-5 of dW3's and 1.5e-5 of dW2's norm
-// to that, which exact sums do not; these chains are not longer, and so that a
-// batch's gradients stay near the GEMM path's (RayChunk): within 2e-5, where
-// they were up to 3.4e-5 away with exact sums (12 batches of 8,192 rays).
+// to that, which exact sums do not. With these chains a batch's dW3 is 3.3e-6 of
+// its norm (median of 100 batches of 8,192 rays; 2.4e-5 at most) from the GEMM
+// path's (RayChunk) and as far from float64 as that (1.4e-5, 40 batches); in
+// one chain over all 1.7 M samples, 11,200 additions, 4.7e-6 and 1.6e-5; half
+// the length 6e-6 and 1.3e-5. With exact sums 3.4e-5 apart at most in 12 batches.
 // Bound: the FP32 pipe; 256 us for 194,560 samples (50 of its 66 TFLOP/s): 8 x
 // 8 elements a thread and all eight chunks unrolled; 8 x 4 and twice the
 // threads 283, one chunk an iteration 272, rows of elements all forwards 281.
@@ -1180,15 +1182,13 @@ int64_t nsvf_field_train_backward_floats(int64_t n_samples, int64_t chunk_sample
 }
 
 // A chunk adds as many additions to a chain as half of a block's tiles have
-// samples. As many chunks go on with it as its limit allows, in even parts.
+// samples. As many chunks go on with it as its limit allows.
 int64_t nsvf_field_train_chain_chunks(int64_t n_samples, int64_t chunk_samples) {
   if (n_samples < 0 || chunk_samples < 1) return -1;
   const int64_t chunks = (n_samples + chunk_samples - 1) / chunk_samples;
   const int64_t tiles = (chunk_samples + kTile - 1) / kTile;
   const int64_t most = kChainLimit / ((tiles + kChains - 1) / kChains * (kTile / 2));
-  if (most < 2 || chunks < 2) return 1;
-  const int64_t groups = (chunks + most - 1) / most;
-  return (chunks + groups - 1) / groups;
+  return most < 2 || chunks < 2 ? 1 : most < chunks ? most : chunks;
 }
 
 int nsvf_field_train_backward(int64_t n_samples, int64_t chunk_samples, const int32_t *voxel,
